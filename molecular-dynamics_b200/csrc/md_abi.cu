@@ -271,6 +271,10 @@ struct md_forcefield {
     bool side_pending = false;               // ev_done marks energy sums the system's stream has not joined
     DevBuf<double> out;  // [0] pe, [1] virial, [2] inside
     DevBuf<unsigned long long> inside_count;
+    // all-pairs forces: own pairs inside the cutoff per particle, their offsets, and the pairs' (E, W) in order
+    DevBuf<int> own_pairs;
+    DevBuf<long long> own_off, own_tiles;
+    DevBuf<double2> pair_rec;
     DevBuf<long long> fx_acc;  // fixed-point accumulators of the float kernels: pe, virial
     double* host_out = nullptr;
 };
@@ -636,6 +640,8 @@ md_status kick_async(md_system* s, double dt);
 // Lists with fewer pairs than this keep each pair's (E, W) for the FP64 energy sums, larger ones its r^2
 // (store_pair_rec)
 constexpr long long kTermsMaxPairs = 4'000'000;
+// (E, W) records the all-pairs sums hold at once (256 MB)
+constexpr long long kAllPairsRecords = 1ll << 24;
 
 // A kernel launch carrying a scheduling priority: the launch keeps it when a CUDA graph records it (a graph's
 // nodes do not take the priority of the stream they were captured from)
@@ -1552,13 +1558,48 @@ md_status md_forces_all_pairs(md_forcefield* ff, md_system* s, double* pe, doubl
     const int n = static_cast<int>(s->n);
     MD_TRY(join_energy(ff, s));
     MD_CUDA(ff->out.reserve(4));
+    MD_CUDA(cudaMemsetAsync(ff->out.p, 0, 3 * sizeof(double), s->stream));
     if (n > 0) {
-        k_force_all_pairs<<<blocks_for(n, 128), 128, 0, s->stream>>>(s->pos.p, n, s->box, ff->lj, s->force.p);
+        MD_CUDA(ff->own_pairs.reserve(n));
+        MD_CUDA(ff->own_off.reserve(static_cast<size_t>(n) + 1));
+        MD_CUDA(ff->own_tiles.reserve(scan_tiles_needed(n)));
+        k_all_pairs<false><<<blocks_for(n, 4), 128, 0, s->stream>>>(s->pos.p, n, s->box, ff->lj, 0, n, s->force.p,
+                                                                    ff->own_pairs.p, nullptr, 0, nullptr);
         MD_CHECK_LAUNCH();
-        k_energy_all_pairs<<<1, 32, 0, s->stream>>>(s->pos.p, n, s->box, ff->lj, ff->out.p);
-        MD_CHECK_LAUNCH();
-    } else {
-        MD_CUDA(cudaMemsetAsync(ff->out.p, 0, 3 * sizeof(double), s->stream));
+        exclusive_scan<int, long long>(ff->own_pairs.p, n, ff->own_off.p, ff->own_tiles.p, s->stream);
+        MD_CHECK_SCAN();
+        long long pairs = 0;
+        MD_CUDA(cudaMemcpyAsync(&pairs, ff->own_off.p + n, sizeof(long long), cudaMemcpyDeviceToHost, s->stream));
+        MD_TRY(sync(s));
+        // the pairs inside the cutoff, as many particles at a time as their records fit (one pass but for very
+        // large systems), each pass going on from the sums of the one before
+        std::vector<long long> off;
+        if (pairs > kAllPairsRecords) {
+            off.resize(static_cast<size_t>(n) + 1);
+            MD_CUDA(cudaMemcpyAsync(off.data(), ff->own_off.p, sizeof(long long) * off.size(), cudaMemcpyDeviceToHost,
+                                    s->stream));
+            MD_TRY(sync(s));
+        }
+        for (int a = 0; a < n;) {
+            int b = n;
+            const long long first = off.empty() ? 0 : off[a];
+            if (!off.empty())
+                b = std::max(a + 1, static_cast<int>(std::upper_bound(off.begin() + a, off.end(),
+                                                                      first + kAllPairsRecords) - off.begin()) - 1);
+            const long long last = off.empty() ? pairs : off[b];
+            if (last > first) {
+                const size_t records = static_cast<size_t>(last - first);
+                if (ff->pair_rec.count < records)  // with headroom: the pair count drifts from step to step
+                    MD_CUDA(ff->pair_rec.reserve(records + records / 8));
+                k_all_pairs<true><<<blocks_for(b - a, 4), 128, 0, s->stream>>>(
+                    s->pos.p, n, s->box, ff->lj, a, b, nullptr, nullptr, ff->own_off.p, first, ff->pair_rec.p);
+                MD_CHECK_LAUNCH();
+                k_sum_pairs<<<1, 2 * kOrderedThreads, 0, s->stream>>>(ff->pair_rec.p, last - first, ff->out.p,
+                                                                      static_cast<double>(last));
+                MD_CHECK_LAUNCH();
+            }
+            a = b;
+        }
     }
     double out[3];
     MD_CUDA(cudaMemcpyAsync(out, ff->out.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));

@@ -4,8 +4,11 @@
 #pragma once
 
 #include "md_common.cuh"
+#include "md_ordered.cuh"
 
 namespace md {
+
+constexpr int kChainValues = 8;  // values per thread of a one-block ordered sum (45 KB of shared memory)
 
 // ---- forces -----------------------------------------------------------------------------------------
 
@@ -474,80 +477,79 @@ __global__ void k_rdf_sample(const double4* __restrict__ pos, int n, Box box, co
 // ---- O(N^2) forces ----------------------------------------------------------------------------------------
 
 // computeForces(System&) (src/Forcefield.cpp:39-78). Particle p receives, in the reference's loop order,
-// -F(i, p) for i = 0 .. p-1 and then +F(p, j) for j = p+1 .. n-1; pairs at or beyond the cutoff are skipped.
-__global__ void k_force_all_pairs(const double4* __restrict__ pos, int n, Box box, LJ lj, double* __restrict__ force) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
+// -F(i, p) for i = 0 .. p-1 and then +F(p, j) for j = p+1 .. n-1; pairs at or beyond the cutoff are skipped. The
+// potential and virial are one sequential sum over the pairs (i, j > i) inside the cutoff in loop order, from 0.0.
+//
+// One warp per particle: the lanes test 32 partners at a time and the few inside the cutoff are then added one after
+// another in partner order, from shuffled terms, by every lane alike. Both signs take the one form +F dx(p, i), which
+// is the same double (min_image is odd, IEEE subtraction antisymmetric). Bound by the FP64 pipe: about 40 double
+// operations a pair tested (three minimum images; their rounding is skipped within a quarter box).
+// own[p] = pairs (p, j > p) inside the cutoff. With `rec` (kRecords), the (E, W) of those pairs are written instead,
+// in order, at rec[off[p] - off0] for the particles [p0, p1); ordered_sum adds them with the serial sum's bits.
+template <bool kRecords>
+__global__ void __launch_bounds__(128) k_all_pairs(const double4* __restrict__ pos, int n, Box box, LJ lj, int p0,
+                                                   int p1, double* __restrict__ force, int* __restrict__ own,
+                                                   const long long* __restrict__ off, long long off0,
+                                                   double2* __restrict__ rec) {
+    const int p = p0 + static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (p >= p1) return;
     const double4 pp = pos[p];
-    double f[3] = {0.0, 0.0, 0.0};
-    for (int i = 0; i < n; ++i) {
-        if (i == p) continue;
-        const double4 a = i < p ? pos[i] : pp;
-        const double4 b = i < p ? pp : pos[i];
-        const double dx = min_image(dsub(a.x, b.x), box);
-        const double dy = min_image(dsub(a.y, b.y), box);
-        const double dz = min_image(dsub(a.z, b.z), box);
-        const double r2 = norm2(dx, dy, dz);
-        if (r2 >= lj.rc2) continue;
-        double fr, e;
-        pair_terms(r2, lj, fr, e);
-        if (i < p) {
-            f[0] = dsub(f[0], dmul(fr, dx));
-            f[1] = dsub(f[1], dmul(fr, dy));
-            f[2] = dsub(f[2], dmul(fr, dz));
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    int hits = 0;
+    double2* out = kRecords ? rec + (off[p] - off0) : nullptr;
+    for (int i0 = kRecords ? (p + 1) & ~31 : 0; i0 < n; i0 += 32) {
+        const int i = i0 + lane;
+        bool in = i < n && (kRecords ? i > p : i != p);
+        double dx = 0.0, dy = 0.0, dz = 0.0, r2 = 0.0;
+        if (in) {
+            const double4 q = pos[i];
+            dx = min_image(dsub(pp.x, q.x), box);
+            dy = min_image(dsub(pp.y, q.y), box);
+            dz = min_image(dsub(pp.z, q.z), box);
+            r2 = norm2(dx, dy, dz);
+            in = kRecords ? r2 < lj.rc2 : !(r2 >= lj.rc2);  // (a NaN separation enters the forces, not the sums)
+        }
+        unsigned mask = __ballot_sync(0xffffffffu, in);
+        if (!mask) continue;
+        double fr = 0.0, e = 0.0;
+        if (in) pair_terms(r2, lj, fr, e);
+        if (kRecords) {
+            if (in) out[hits + __popc(mask & ((1u << lane) - 1u))] = make_double2(e, dmul(fr, r2));
+            hits += __popc(mask);
         } else {
-            f[0] = dadd(f[0], dmul(fr, dx));
-            f[1] = dadd(f[1], dmul(fr, dy));
-            f[2] = dadd(f[2], dmul(fr, dz));
+            hits += __popc(__ballot_sync(0xffffffffu, in && i > p && r2 < lj.rc2));
+            dx = dmul(fr, dx);
+            dy = dmul(fr, dy);
+            dz = dmul(fr, dz);
+            while (mask) {
+                const int t = __ffs(mask) - 1;
+                mask &= mask - 1;
+                fx = dadd(fx, __shfl_sync(0xffffffffu, dx, t));
+                fy = dadd(fy, __shfl_sync(0xffffffffu, dy, t));
+                fz = dadd(fz, __shfl_sync(0xffffffffu, dz, t));
+            }
         }
     }
-    force[p] = f[0];
-    force[static_cast<size_t>(n) + p] = f[1];
-    force[2 * static_cast<size_t>(n) + p] = f[2];
+    if (!kRecords && lane == 0) {
+        force[p] = fx;
+        force[static_cast<size_t>(n) + p] = fy;
+        force[2 * static_cast<size_t>(n) + p] = fz;
+        own[p] = hits;
+    }
 }
 
-// The all-pairs potential, virial and inside count: one sequential sum over pairs (i, j > i) in the
-// reference's loop order, started from 0.0. One warp: lanes evaluate 32 pairs at a time, lane 0 adds them.
-__global__ void k_energy_all_pairs(const double4* __restrict__ pos, int n, Box box, LJ lj, double* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    double pe = 0.0, w = 0.0, ins = 0.0;
-    for (int i = 0; i < n; ++i) {
-        const double4 pi = pos[i];
-        for (int j0 = i + 1; j0 < n; j0 += 32) {
-            const int j = j0 + lane;
-            double e = 0.0, vir = 0.0;
-            bool in = false;
-            if (j < n) {
-                const double4 pj = pos[j];
-                const double dx = min_image(dsub(pi.x, pj.x), box);
-                const double dy = min_image(dsub(pi.y, pj.y), box);
-                const double dz = min_image(dsub(pi.z, pj.z), box);
-                const double r2 = norm2(dx, dy, dz);
-                if (r2 < lj.rc2) {
-                    double fr;
-                    pair_terms(r2, lj, fr, e);
-                    vir = dmul(fr, r2);
-                    in = true;
-                }
-            }
-            const unsigned mask = __ballot_sync(0xffffffffu, in);
-            const int m = n - j0 < 32 ? n - j0 : 32;
-            for (int t = 0; t < m; ++t) {
-                const double et = __shfl_sync(0xffffffffu, e, t);
-                const double wt = __shfl_sync(0xffffffffu, vir, t);
-                if (lane == 0 && ((mask >> t) & 1u)) {
-                    pe = dadd(pe, et);
-                    w = dadd(w, wt);
-                    ins = dadd(ins, 1.0);
-                }
-            }
-        }
-    }
-    if (lane == 0) {
-        out[0] = pe;
-        out[1] = w;
-        out[2] = ins;
-    }
+// The all-pairs records added to the running (potential, virial) in out[0..1]; out[2] = inside pairs so far. One block.
+__global__ void __launch_bounds__(2 * kOrderedThreads) k_sum_pairs(const double2* __restrict__ rec, long long m,
+                                                                   double* __restrict__ out, double inside) {
+    __shared__ OrderedSmem<2, kChainValues> sm;
+    if (threadIdx.x < 2) sm.run[threadIdx.x] = out[threadIdx.x];
+    ordered_sum(sm, m, [&](long long k, double* v) {
+        const double2 r = rec[k];
+        v[0] = r.x;
+        v[1] = r.y;
+    });
+    if (threadIdx.x < 2) out[threadIdx.x] = sm.run[threadIdx.x];
+    if (threadIdx.x == 0) out[2] = inside;
 }
 
 }  // namespace md
