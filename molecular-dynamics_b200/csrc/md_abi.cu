@@ -772,9 +772,16 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
                         s->pos.p, n, nl->grid.start.p, nl->cell_sorted.p, tg, ff->lj, nl->rows.p, nl->cap,
                         nl->counts.p, s->force.p, ff->inside_count.p, ka, nl->half_off.p, ew, rec_cap);
                 } else if (variant == 2) {
-                    k_force_fp64_quads<kTerms><<<blocks_for(n, 128), 128, 0, s->stream>>>(
-                        s->pos.p, n, s->box, ff->lj, nl->rows.p, nl->cap, nl->counts.p, s->force.p, ff->inside_count.p,
-                        kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt, nl->half_off.p, ew, rec_cap);
+                    auto go = [&](auto kernel, int lanes) {
+                        kernel<<<blocks_for(static_cast<long long>(n) * lanes, 128), 128, 0, s->stream>>>(
+                            s->pos.p, n, s->box, ff->lj, nl->rows.p, nl->cap, nl->counts.p, s->force.p,
+                            ff->inside_count.p, kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt, nl->half_off.p, ew,
+                            rec_cap);
+                    };
+                    if (n <= kFp64Lanes16) go(k_force_fp64_lanes<kTerms, 16>, 16);
+                    else if (n <= kFp64Lanes8) go(k_force_fp64_lanes<kTerms, 8>, 8);
+                    else if (n <= kFp64Lanes4) go(k_force_fp64_lanes<kTerms, 4>, 4);
+                    else go(k_force_fp64_quads<kTerms>, 1);
                 } else {
                     k_force_fp64<kTerms><<<blocks_for(n, 128), 128, 0, s->stream>>>(
                         s->pos.p, n, s->box, ff->lj, nl->rows.p, nl->cap, nl->counts.p, s->force.p, ff->inside_count.p,

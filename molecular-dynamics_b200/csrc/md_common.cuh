@@ -32,6 +32,17 @@ __device__ __forceinline__ uint4 row_quad_stream(const uint32_t* __restrict__ ro
 }
 inline size_t row_buffer_entries(long long n, int cap) { return static_cast<size_t>((n + 31) / 32) * 32 * cap; }
 
+// One position with a single 32-byte load (the device arrays of double4 are 32-byte aligned: whole allocations)
+__device__ __forceinline__ double4 load_pos(const double4* __restrict__ p) {
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+// Four doubles with a single 32-byte store (p 32-byte aligned)
+__device__ __forceinline__ void store_4(double* p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }

@@ -98,6 +98,9 @@ __global__ void k_force_fp64(const double4* __restrict__ pos, int n, Box box, LJ
 // odd (round() and the |d| <= L/4 shortcut are symmetric) and IEEE subtraction antisymmetric, so each sum sees
 // the reference's nonzero terms in the reference's order; a masked 0.0 leaves a sum unchanged because a sum
 // that starts at +0.0 never becomes -0.0.
+// Positions come in by one 32-byte load each (two of 16 bytes: 266 us at N = 864,000 without records, now 254), and
+// the r^2 records go out by whole aligned quads of 32 bytes, shifted into place in registers (stored one by one: 493 us
+// with records, now 352). What bounds it: gather and store latency at 40 % of the FP64 pipe's time.
 template <bool kTerms>
 __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restrict__ pos, int n, Box box, LJ lj,
                                                           const uint32_t* __restrict__ rows, int cap,
@@ -107,9 +110,9 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
                                                           double half_dt, const long long* __restrict__ half_off,
                                                           double* __restrict__ pair_r2, long long rec_cap) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long ins = 0;
+    unsigned ins = 0;
     if (i < n) {
-        const double4 pi = pos[i];
+        const double4 pi = load_pos(pos + i);
         const int2 c = counts[i];
         const int m = c.x + c.y;
         const int quads = (m + 3) >> 2;
@@ -118,13 +121,18 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
         const uint4* rq = reinterpret_cast<const uint4*>(rows) + static_cast<size_t>(i >> 5) * (cap >> 2) * 32 + (i & 31);
         uint4 nq = make_uint4(0, 0, 0, 0);
         if (quads > 0) nq = __ldcs(rq);
+        // r^2 records: record k of the array belongs to the aligned quad k >> 2, which is written whole once its four
+        // are known; the quads at either end of the particle's range are shared with its neighbours
+        const int shift = static_cast<int>(pb & 3);
+        double h0 = 0.0, h1 = 0.0, h2 = 0.0;  // the last records of the open aligned quad
         for (int q = 0; q < quads; ++q) {
             const uint4 eq = nq;
             if (q + 1 < quads) nq = __ldcs(rq + 32 * (q + 1));
             const uint32_t ent[4] = {eq.x, eq.y, eq.z, eq.w};
             double4 pj[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) pj[u] = pos[4 * q + u < m ? static_cast<int>(ent[u] & kIndexMask) : 0];
+            for (int u = 0; u < 4; ++u) pj[u] = load_pos(pos + (4 * q + u < m ? static_cast<int>(ent[u] & kIndexMask) : 0));
+            double r[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int sl = 4 * q + u;
@@ -138,10 +146,39 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
                 fx = dadd(fx, in ? dmul(f, dx) : 0.0);
                 fy = dadd(fy, in ? dmul(f, dy) : 0.0);
                 fz = dadd(fz, in ? dmul(f, dz) : 0.0);
+                r[u] = r2;
                 if (sl < c.x) {
                     ins += in ? 1u : 0u;
-                    if (pair_r2) store_pair_rec<kTerms>(pair_r2, pb + sl, r2, f, e, in, rec_cap);
+                    if (kTerms && pair_r2) store_pair_rec<kTerms>(pair_r2, pb + sl, r2, f, e, in, rec_cap);
                 }
+            }
+            if (!kTerms && pair_r2 && 4 * q < c.x) {
+                // the aligned quad that ends inside this step's four: `shift` held back, 4 - shift new
+                const double a0 = shift == 0 ? r[0] : shift == 1 ? h2 : shift == 2 ? h1 : h0;
+                const double a1 = shift == 0 ? r[1] : shift == 1 ? r[0] : shift == 2 ? h2 : h1;
+                const double a2 = shift == 0 ? r[2] : shift == 1 ? r[1] : shift == 2 ? r[0] : h2;
+                const double a3 = shift == 0 ? r[3] : shift == 1 ? r[2] : shift == 2 ? r[1] : r[0];
+                const long long k = pb - shift + 4 * q;
+                const int s0 = 4 * q - shift;  // row entry of a0
+                if (s0 >= 0 && s0 + 4 <= c.x && k + 4 <= rec_cap) {
+                    store_4(pair_r2 + k, a0, a1, a2, a3);
+                } else {
+                    if (s0 >= 0 && s0 < c.x && k < rec_cap) pair_r2[k] = a0;
+                    if (s0 >= -1 && s0 + 1 < c.x && k + 1 < rec_cap) pair_r2[k + 1] = a1;
+                    if (s0 >= -2 && s0 + 2 < c.x && k + 2 < rec_cap) pair_r2[k + 2] = a2;
+                    if (s0 + 3 < c.x && k + 3 < rec_cap) pair_r2[k + 3] = a3;
+                }
+                if (4 * q + 4 >= c.x) {  // the last step with own pairs: the records still held back
+                    const int s1 = s0 + 4;
+                    const double b0 = shift == 1 ? r[3] : shift == 2 ? r[2] : r[1];
+                    const double b1 = shift == 2 ? r[3] : r[2];
+                    if (shift >= 1 && s1 < c.x && k + 4 < rec_cap) pair_r2[k + 4] = b0;
+                    if (shift >= 2 && s1 + 1 < c.x && k + 5 < rec_cap) pair_r2[k + 5] = b1;
+                    if (shift >= 3 && s1 + 2 < c.x && k + 6 < rec_cap) pair_r2[k + 6] = r[3];
+                }
+                h0 = r[1];
+                h1 = r[2];
+                h2 = r[3];
             }
         }
         const double F[3] = {fx, fy, fz};
@@ -152,8 +189,83 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
             if (kick_vel) kick_vel[o] = dadd(kick_vel[o], ddiv(dmul(half_dt, F[k]), mass[i]));
         }
     }
-    ins = warp_sum_u64(ins);
-    if ((threadIdx.x & 31) == 0 && ins) atomicAdd(inside, ins);
+    const unsigned total = __reduce_add_sync(0xffffffffu, ins);
+    if ((threadIdx.x & 31) == 0 && total) atomicAdd(inside, static_cast<unsigned long long>(total));
+}
+
+// The sums of k_force_fp64_quads with kLanes threads per particle: the lanes evaluate kLanes row entries at once and
+// leave the terms in shared memory, where three of them add the x, y and z terms one after another in row order, so the
+// sums are the same. Entries are read two steps and positions one step ahead. The energy records of consecutive row
+// entries go out side by side.
+// For small systems: a thread per particle leaves most of the GPU without a warp (2,048 particles are 64 of them) and
+// walks its row in one long chain of gathers. Measured with records stored (B200, us; threads per particle 1 / 4 / 8 /
+// 16): N = 500: 37 / 18 / 13 / 11; 2,048: 37 / 18 / 14 / 12; 10,976: 37 / 19 / 16 / 22; 32,000: 40 / 26 / 30 / 35;
+// 108,000: 54 / 61 / 70 / 84. The lines between them follow: past about 70,000 particles the GPU is full either way and
+// the shared-memory pass only costs.
+constexpr int kFp64Lanes16 = 8192, kFp64Lanes8 = 24576, kFp64Lanes4 = 72000;
+template <bool kTerms, int kLanes>
+__global__ void __launch_bounds__(128) k_force_fp64_lanes(const double4* __restrict__ pos, int n, Box box, LJ lj,
+                                                          const uint32_t* __restrict__ rows, int cap,
+                                                          const int2* __restrict__ counts, double* __restrict__ force,
+                                                          unsigned long long* __restrict__ inside,
+                                                          double* __restrict__ kick_vel, const double* __restrict__ mass,
+                                                          double half_dt, const long long* __restrict__ half_off,
+                                                          double* __restrict__ pair_r2, long long rec_cap) {
+    constexpr int kGroups = 32 / kLanes, kPad = kLanes + 1, kRow = kGroups * kPad + 1;
+    __shared__ double s_t[4][3 * kRow];
+    const int lane = threadIdx.x & 31, g = lane / kLanes, u = lane % kLanes;
+    const int i = static_cast<int>((blockIdx.x * 128 + threadIdx.x) / kLanes);
+    double* terms = s_t[threadIdx.x >> 5] + g * kPad;  // component k of the group's entry t at terms[k * kRow + t]
+    const bool real = i < n;
+    const int2 c = real ? counts[i] : make_int2(0, 0);
+    const int m = c.x + c.y;
+    const double4 pi = real ? load_pos(pos + i) : make_double4(0.0, 0.0, 0.0, 0.0);
+    const long long pb = pair_r2 && real ? half_off[i] : 0;
+    // the longest row of the warp's particles: every lane takes part in the warp's steps
+    int steps = (m + kLanes - 1) / kLanes;
+#pragma unroll
+    for (int o = kLanes; o < 32; o <<= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, o));
+    auto entry = [&](int s) { return s < m ? static_cast<int>(rows[row_index(i, s, cap)] & kIndexMask) : 0; };
+    unsigned ins = 0;
+    double sum = 0.0;
+    int j1 = entry(u + kLanes);
+    double4 pj = load_pos(pos + entry(u));
+    for (int q = 0; q < steps; ++q) {
+        const int s = q * kLanes + u;
+        const double dx = min_image(dsub(pi.x, pj.x), box);
+        const double dy = min_image(dsub(pi.y, pj.y), box);
+        const double dz = min_image(dsub(pi.z, pj.z), box);
+        pj = load_pos(pos + j1);
+        j1 = entry(s + 2 * kLanes);
+        const double r2 = norm2(dx, dy, dz);
+        const bool in = s < m && r2 < lj.rc2;
+        double f, e;
+        pair_terms(in ? r2 : 1.0, lj, f, e);
+        terms[u] = in ? dmul(f, dx) : 0.0;
+        terms[kRow + u] = in ? dmul(f, dy) : 0.0;
+        terms[2 * kRow + u] = in ? dmul(f, dz) : 0.0;
+        if (s < c.x) {
+            ins += in ? 1u : 0u;
+            if (pair_r2) store_pair_rec<kTerms>(pair_r2, pb + s, r2, f, e, in, rec_cap);
+        }
+        __syncwarp();
+        if (u < 3) {
+            const double* mine = terms + u * kRow;
+            double t[kLanes];
+#pragma unroll
+            for (int k = 0; k < kLanes; ++k) t[k] = mine[k];
+#pragma unroll
+            for (int k = 0; k < kLanes; ++k) sum = dadd(sum, t[k]);
+        }
+        __syncwarp();
+    }
+    if (real && u < 3) {
+        const size_t o = static_cast<size_t>(u) * n + i;
+        force[o] = sum;
+        if (kick_vel) kick_vel[o] = dadd(kick_vel[o], ddiv(dmul(half_dt, sum), mass[i]));
+    }
+    ins = __reduce_add_sync(0xffffffffu, ins);
+    if (lane == 0 && ins) atomicAdd(inside, static_cast<unsigned long long>(ins));
 }
 
 constexpr int kEnergyWarps = 4;  // warps per block of the blocked kinetic-energy sums
