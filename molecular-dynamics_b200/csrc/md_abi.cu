@@ -317,11 +317,9 @@ md_status kinetic_async(md_system* s) {
         return MD_OK;
     }
     MD_CUDA(s->ke_blocks.reserve(nb));
-    const size_t smem = kEnergyWarps * kChunk * sizeof(double);
-    k_kinetic_blocks<<<blocks_for(nb, kEnergyWarps), kEnergyWarps * 32, smem, s->stream>>>(s->vel.p, s->mass.p, n,
-                                                                                          s->ke_blocks.p, nb);
+    k_kinetic_blocks<<<nb, kOrderedThreads, 0, s->stream>>>(s->vel.p, s->mass.p, n, s->ke_blocks.p);
     MD_CHECK_LAUNCH();
-    k_sum_blocks<<<1, 32, 0, s->stream>>>(s->ke_blocks.p, nb, s->scal.p + kScalKE);
+    k_sum_blocks<<<1, kChainThreads, 0, s->stream>>>(s->ke_blocks.p, nb, s->scal.p + kScalKE);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
@@ -587,7 +585,7 @@ md_status profile_collect(md_system* s) {
 // Autotuner of the list force kernel: with tiles available, the first force call of a list (per precision)
 // times the global-gather kernel (variant 0) and the shared-memory tile kernel (variant 1) on the current
 // state, two launches each after a warm-up, and keeps the faster. Both variants give the same bits, so the
-// choice never changes a result. md_nlist_set_force_variant pins a variant instead.
+// choice never changes a result. md_nlist_set_force_variant pins a variant instead. FP64 always takes variant 2.
 template <typename Launch>
 md_status choose_variant(md_system* s, md_nlist* nl, int prec, Launch&& launch) {
     // variants available: 0 always, 1 with tiles; for FP64 2 (branch-free quads); for the float modes 2, 3
@@ -597,6 +595,12 @@ md_status choose_variant(md_system* s, md_nlist* nl, int prec, Launch&& launch) 
     if (nl->variant[prec] >= 0 && ((mask >> nl->variant[prec]) & 1u)) return MD_OK;
     if (mask == 1u) {
         nl->variant[prec] = 0;
+        return MD_OK;
+    }
+    if (prec == MD_PREC_FP64 && nl->pinned[prec] < 0) {
+        // nothing to time: with records, variants 0 / 1 / 2 take 63 / 47 / 12 us at N = 2,048, 72 / 56 / 24 at 32,000,
+        // 243 / 295 / 118 at 256,000 and 574 / 763 / 313 at 864,000
+        nl->variant[prec] = 2;
         return MD_OK;
     }
     if (nl->pinned[prec] >= 0 && ((mask >> nl->pinned[prec]) & 1u)) {
@@ -637,9 +641,8 @@ md_status choose_variant(md_system* s, md_nlist* nl, int prec, Launch&& launch) 
 // them). Returns through *fused_ke whether the fused kick also left the step's kinetic energy in
 // s->scal[kScalKE] (float tile kernels only; fixed-point, not the reference's summation order).
 md_status kick_async(md_system* s, double dt);
-// Lists with fewer pairs than this keep each pair's (E, W) for the FP64 energy sums, larger ones its r^2
-// (store_pair_rec)
-constexpr long long kTermsMaxPairs = 4'000'000;
+// Lists of more 1024-pair blocks than this sum them four to a warp (k_pair_block_sums): more warps than the GPU holds
+constexpr int kSingleBlocks = 148 * 16;
 // (E, W) records the all-pairs sums hold at once (256 MB)
 constexpr long long kAllPairsRecords = 1ll << 24;
 
@@ -691,11 +694,10 @@ md_status energy_quiesce(md_forcefield* ff) {
     return MD_OK;
 }
 
-// Both pairs of energy buffers for at least `pairs` pair records of either form (two doubles each; call with
-// nothing queued on the streams)
+// Both pairs of energy buffers for at least `pairs` pair records (call with nothing queued on the streams)
 md_status reserve_energy_records(md_forcefield* ff, long long pairs) {
     const size_t blocks = static_cast<size_t>((pairs + kChunk - 1) / kChunk) + 1;
-    for (DevBuf<double>& r : ff->pair_r2) MD_CUDA(r.reserve(2 * static_cast<size_t>(pairs)));
+    for (DevBuf<double>& r : ff->pair_r2) MD_CUDA(r.reserve(static_cast<size_t>(pairs)));
     for (DevBuf<double2>& e : ff->eblocks) MD_CUDA(e.reserve(blocks));
     return MD_OK;
 }
@@ -742,7 +744,7 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
             if (!capturing) {
                 if (!ff->side) MD_TRY(energy_streams(ff));
                 const auto small = [&](size_t r2, size_t blocks) {
-                    return r2 < 2 * static_cast<size_t>(pairs) || blocks < static_cast<size_t>(nb);
+                    return r2 < static_cast<size_t>(pairs) || blocks < static_cast<size_t>(nb);
                 };
                 if (small(ff->pair_r2[0].count, ff->eblocks[0].count) ||
                     small(ff->pair_r2[1].count, ff->eblocks[1].count)) {
@@ -755,20 +757,18 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
             }
             if (ff->read_pending[b]) MD_CUDA(cudaStreamWaitEvent(s->stream, ff->ev_read[b], 0));
         }
-        const long long rec_cap = sums ? static_cast<long long>(ff->pair_r2[b].count / 2) : 0;
-        const bool terms = (capturing ? rec_cap : pairs) < kTermsMaxPairs;  // the records' form
+        const long long rec_cap = sums ? static_cast<long long>(ff->pair_r2[b].count) : 0;
         if (n > 0) {
             // variant 0: global gathers; 1: shared-memory tile; 2: global gathers a quad of entries at a time,
             // branch-free (all bit-identical). With want_energy the kernel also stores every own pair's r^2 in
             // pair order for the blocked sums below.
-            auto launch_form = [&](int variant, bool kick, double* ew, auto form) -> md_status {
-                constexpr bool kTerms = decltype(form)::value;
+            auto launch = [&](int variant, bool kick, double* ew) -> md_status {
                 if (variant == 1) {
                     const TileGeom& tg = nl->tiles_geom;
                     const size_t smem = sizeof(double4) * tg.max_staged;
-                    MD_CUDA(allow_smem(k_force_fp64_tile<kTerms>, smem));
+                    MD_CUDA(allow_smem(k_force_fp64_tile, smem));
                     const KickArgs ka{kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt};
-                    k_force_fp64_tile<kTerms><<<tile_blocks(tg), kTileThreads, smem, s->stream>>>(
+                    k_force_fp64_tile<<<tile_blocks(tg), kTileThreads, smem, s->stream>>>(
                         s->pos.p, n, nl->grid.start.p, nl->cell_sorted.p, tg, ff->lj, nl->rows.p, nl->cap,
                         nl->counts.p, s->force.p, ff->inside_count.p, ka, nl->half_off.p, ew, rec_cap);
                 } else if (variant == 2) {
@@ -778,21 +778,17 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
                             ff->inside_count.p, kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt, nl->half_off.p, ew,
                             rec_cap);
                     };
-                    if (n <= kFp64Lanes16) go(k_force_fp64_lanes<kTerms, 16>, 16);
-                    else if (n <= kFp64Lanes8) go(k_force_fp64_lanes<kTerms, 8>, 8);
-                    else if (n <= kFp64Lanes4) go(k_force_fp64_lanes<kTerms, 4>, 4);
-                    else go(k_force_fp64_quads<kTerms>, 1);
+                    if (n <= kFp64Lanes16) go(k_force_fp64_lanes<16>, 16);
+                    else if (n <= kFp64Lanes8) go(k_force_fp64_lanes<8>, 8);
+                    else if (n <= kFp64Lanes4) go(k_force_fp64_lanes<4>, 4);
+                    else go(k_force_fp64_quads, 1);
                 } else {
-                    k_force_fp64<kTerms><<<blocks_for(n, 128), 128, 0, s->stream>>>(
+                    k_force_fp64<<<blocks_for(n, 128), 128, 0, s->stream>>>(
                         s->pos.p, n, s->box, ff->lj, nl->rows.p, nl->cap, nl->counts.p, s->force.p, ff->inside_count.p,
                         kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt, nl->half_off.p, ew, rec_cap);
                 }
                 MD_CHECK_LAUNCH();
                 return MD_OK;
-            };
-            auto launch = [&](int variant, bool kick, double* ew) -> md_status {
-                return terms ? launch_form(variant, kick, ew, std::true_type{})
-                             : launch_form(variant, kick, ew, std::false_type{});
             };
             MD_TRY(choose_variant(s, nl, MD_PREC_FP64, [&](int v) { return launch(v, false, nullptr); }));
             MD_CUDA(cudaMemsetAsync(ff->inside_count.p, 0, sizeof(unsigned long long), s->stream));
@@ -819,20 +815,18 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
                 MD_CUDA(cudaEventRecord(ff->ev_force, s->stream));
                 MD_CUDA(cudaStreamWaitEvent(ff->side, ff->ev_force, 0));
                 if (ff->chain_pending[eb]) MD_CUDA(cudaStreamWaitEvent(ff->side, ff->ev_chain[eb], 0));
-                if (terms)
-                    MD_TRY(launch_priority(k_pair_block_sums_terms, blocks_for(grid_blocks, 32 * kPairSumWarpsTerms),
-                                           32 * kPairSumWarpsTerms, ff->side, ff->side_priority,
-                                           reinterpret_cast<const double2*>(ff->pair_r2[b].p), count, sum_cap,
-                                           ff->eblocks[eb].p, ff->enblocks.p + eb));
-                else
-                    MD_TRY(launch_priority(k_pair_block_sums, blocks_for(grid_blocks, 32 * kPairSumWarps),
-                                           32 * kPairSumWarps, ff->side, ff->side_priority, ff->pair_r2[b].p,
-                                           count, sum_cap, ff->lj, ff->eblocks[eb].p, ff->enblocks.p + eb));
+                auto block_sums = [&](auto kernel, int per_warp) {
+                    return launch_priority(kernel, blocks_for(grid_blocks, per_warp * kSumWarps), 32 * kSumWarps, ff->side,
+                                           ff->side_priority, ff->pair_r2[b].p, count, sum_cap, ff->lj, ff->eblocks[eb].p,
+                                           ff->enblocks.p + eb);
+                };
+                if (grid_blocks <= kSingleBlocks) MD_TRY(block_sums(k_pair_block_sums<1>, 1));
+                else MD_TRY(block_sums(k_pair_block_sums<4>, 4));
                 MD_CUDA(cudaEventRecord(ff->ev_read[b], ff->side));
                 ff->read_pending[b] = true;
                 ff->ew_next = b ^ 1;
                 MD_CUDA(cudaStreamWaitEvent(ff->chain, ff->ev_read[b], 0));
-                MD_TRY(launch_priority(k_sum_pair_blocks, 1, 32, ff->chain, ff->side_priority, ff->eblocks[eb].p,
+                MD_TRY(launch_priority(k_sum_pair_blocks, 1, kChainThreads, ff->chain, ff->side_priority, ff->eblocks[eb].p,
                                        ff->enblocks.p + eb, ff->out.p));
                 MD_CUDA(cudaEventRecord(ff->ev_chain[eb], ff->chain));
                 ff->chain_pending[eb] = true;
@@ -1843,13 +1837,11 @@ extern "C" md_status md_kinetic_energy_noalloc(const double* vel3, const double*
     // Every block partial that the sum reads is written first by k_kinetic_blocks, and the result slot is
     // written whole by k_sum_blocks, so nothing left by an earlier call is read and nothing needs clearing.
     if (nb > 0) {
-        const size_t smem = kEnergyWarps * kChunk * sizeof(double);
-        k_kinetic_blocks<<<blocks_for(nb, kEnergyWarps), kEnergyWarps * 32, smem, st>>>(
-            vel3, mass, static_cast<int>(n), scratch, static_cast<int>(nb));
+        k_kinetic_blocks<<<static_cast<unsigned>(nb), kOrderedThreads, 0, st>>>(vel3, mass, static_cast<int>(n), scratch);
         MD_CHECK_LAUNCH();
     }
     // (sum of the .x partials, sum of the .y partials) into the result slot; .x is the kinetic energy
-    k_sum_blocks<<<1, 32, 0, st>>>(scratch, static_cast<int>(nb), result);
+    k_sum_blocks<<<1, kChainThreads, 0, st>>>(scratch, static_cast<int>(nb), result);
     MD_CHECK_LAUNCH();
     MD_CUDA(cudaMemcpyAsync(out, result, sizeof(double), cudaMemcpyDeviceToDevice, st));
     return MD_OK;

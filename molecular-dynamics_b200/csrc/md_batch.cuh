@@ -658,6 +658,8 @@ __global__ void k_b_record_inside(int R, const unsigned long long* __restrict__ 
     if (r < R) out[r] = static_cast<double>(inside[r]);
 }
 
+constexpr int kEnergyWarps = 4;  // warps per block of the ordered sums per replica
+
 // ---- kinetic energy and thermostats ---------------------------------------------------------------------------
 
 // System::kineticEnergy's blocked sum (k_kinetic_blocks) per replica: one warp per 1024-particle block of a

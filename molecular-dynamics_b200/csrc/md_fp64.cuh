@@ -17,25 +17,11 @@ constexpr int kChainValues = 8;  // values per thread of a one-block ordered sum
 // index. Pairs outside the cutoff contribute an exact zero in the reference and are skipped here. The
 // inside-cutoff count is the number of own pairs with r^2 < r_c^2 (a sum of whole numbers, exact).
 // With kick_vel set it also applies the closing half kick, v += (half_dt F) / m, with k_kick's sequence.
-// With pair_r2 set, own pair s of particle i also stores its record for the ordered energy sums at index
-// half_off[i] + s: with `terms`, its (pairEnergy, pairVirial) as a double2, E and (F/r) r^2 inside the cutoff,
-// (0, 0) outside (src/Forcefield.cpp:288-296), which k_pair_block_sums_terms adds; without, its r^2, from which
-// k_pair_block_sums recomputes the two terms with the same pair_terms call (the same operations on the same r^2,
-// so the same bits). The r^2 record halves the traffic, which pays for large lists; for small ones the recomputation
-// lengthens the sums (each lane evaluates its block's 1024 pairs in turn), so they keep the terms. Records past
-// rec_cap, the buffer's size in records, are dropped: only a list rebuilt inside a CUDA graph can outgrow the
-// buffer, and the graph's run then reports the overflow and repeats its steps on the host path.
-template <bool kTerms>
-__device__ __forceinline__ void store_pair_rec(double* rec, long long k, double r2, double f, double e, bool in,
-                                               long long rec_cap) {
-    if (k >= rec_cap) return;
-    if (kTerms)
-        reinterpret_cast<double2*>(rec)[k] = in ? make_double2(e, dmul(f, r2)) : make_double2(0.0, 0.0);
-    else
-        rec[k] = r2;  // the energy term is then never used, and the compiler leaves it out
-}
-
-template <bool kTerms>
+// With pair_r2 set, own pair s of particle i also stores its r^2, inside the cutoff or not, for the ordered energy sums
+// at index half_off[i] + s; k_pair_block_sums recomputes the pair's E and (F/r) r^2 from it with the same pair_terms
+// call (the same operations on the same r^2, so the same bits). Records past rec_cap, the buffer's size in records, are
+// dropped: only a list rebuilt inside a CUDA graph can outgrow the buffer, and the graph's run then reports the overflow
+// and repeats its steps on the host path.
 __global__ void k_force_fp64(const double4* __restrict__ pos, int n, Box box, LJ lj, const uint32_t* __restrict__ rows,
                              int cap, const int2* __restrict__ counts, double* __restrict__ force,
                              unsigned long long* __restrict__ inside, double* __restrict__ kick_vel,
@@ -54,13 +40,10 @@ __global__ void k_force_fp64(const double4* __restrict__ pos, int n, Box box, LJ
             const double dy = min_image(dsub(pi.y, pj.y), box);
             const double dz = min_image(dsub(pi.z, pj.z), box);
             const double r2 = norm2(dx, dy, dz);
-            if (!(r2 < lj.rc2)) {
-                if (pair_r2) store_pair_rec<kTerms>(pair_r2, pb + s, r2, 0.0, 0.0, false, rec_cap);
-                continue;
-            }
+            if (pair_r2 && pb + s < rec_cap) pair_r2[pb + s] = r2;
+            if (!(r2 < lj.rc2)) continue;
             double f, e;
             pair_terms(r2, lj, f, e);
-            if (pair_r2) store_pair_rec<kTerms>(pair_r2, pb + s, r2, f, e, true, rec_cap);
             fx = dadd(fx, dmul(f, dx));
             fy = dadd(fy, dmul(f, dy));
             fz = dadd(fz, dmul(f, dz));
@@ -101,7 +84,6 @@ __global__ void k_force_fp64(const double4* __restrict__ pos, int n, Box box, LJ
 // Positions come in by one 32-byte load each (two of 16 bytes: 266 us at N = 864,000 without records, now 254), and
 // the r^2 records go out by whole aligned quads of 32 bytes, shifted into place in registers (stored one by one: 493 us
 // with records, now 352). What bounds it: gather and store latency at 40 % of the FP64 pipe's time.
-template <bool kTerms>
 __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restrict__ pos, int n, Box box, LJ lj,
                                                           const uint32_t* __restrict__ rows, int cap,
                                                           const int2* __restrict__ counts, double* __restrict__ force,
@@ -147,12 +129,9 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
                 fy = dadd(fy, in ? dmul(f, dy) : 0.0);
                 fz = dadd(fz, in ? dmul(f, dz) : 0.0);
                 r[u] = r2;
-                if (sl < c.x) {
-                    ins += in ? 1u : 0u;
-                    if (kTerms && pair_r2) store_pair_rec<kTerms>(pair_r2, pb + sl, r2, f, e, in, rec_cap);
-                }
+                ins += in && sl < c.x ? 1u : 0u;
             }
-            if (!kTerms && pair_r2 && 4 * q < c.x) {
+            if (pair_r2 && 4 * q < c.x) {
                 // the aligned quad that ends inside this step's four: `shift` held back, 4 - shift new
                 const double a0 = shift == 0 ? r[0] : shift == 1 ? h2 : shift == 2 ? h1 : h0;
                 const double a1 = shift == 0 ? r[1] : shift == 1 ? r[0] : shift == 2 ? h2 : h1;
@@ -203,7 +182,7 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
 // 108,000: 54 / 61 / 70 / 84. The lines between them follow: past about 70,000 particles the GPU is full either way and
 // the shared-memory pass only costs.
 constexpr int kFp64Lanes16 = 8192, kFp64Lanes8 = 24576, kFp64Lanes4 = 72000;
-template <bool kTerms, int kLanes>
+template <int kLanes>
 __global__ void __launch_bounds__(128) k_force_fp64_lanes(const double4* __restrict__ pos, int n, Box box, LJ lj,
                                                           const uint32_t* __restrict__ rows, int cap,
                                                           const int2* __restrict__ counts, double* __restrict__ force,
@@ -246,7 +225,7 @@ __global__ void __launch_bounds__(128) k_force_fp64_lanes(const double4* __restr
         terms[2 * kRow + u] = in ? dmul(f, dz) : 0.0;
         if (s < c.x) {
             ins += in ? 1u : 0u;
-            if (pair_r2) store_pair_rec<kTerms>(pair_r2, pb + s, r2, f, e, in, rec_cap);
+            if (pair_r2 && pb + s < rec_cap) pair_r2[pb + s] = r2;
         }
         __syncwarp();
         if (u < 3) {
@@ -268,152 +247,128 @@ __global__ void __launch_bounds__(128) k_force_fp64_lanes(const double4* __restr
     if (lane == 0 && ins) atomicAdd(inside, static_cast<unsigned long long>(ins));
 }
 
-constexpr int kEnergyWarps = 4;  // warps per block of the blocked kinetic-energy sums
+// Adds x[0], x[stride], ... x[(m - 1) stride] to s one after another. One thread's chain, bound by the latency of an
+// addition (8 cycles): the next eight values are on their way from shared memory while the current ones are added.
+__device__ __forceinline__ double add_in_order(const double* x, int stride, int m, double s) {
+    double v[8];
+    int k = 0;
+    if (m >= 8) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = x[u * stride];
+        for (; k + 16 <= m; k += 8) {
+            double w[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) w[u] = x[(k + 8 + u) * stride];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s = dadd(s, v[u]);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = w[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s = dadd(s, v[u]);
+        k += 8;
+    }
+    for (; k < m; ++k) s = dadd(s, x[k * stride]);
+    return s;
+}
 
 // The inner loop of deterministicSum (include/Parallel.hpp:43-46) over the (pairEnergy, pairVirial) array, whose
 // terms are recomputed here from the r^2 records the force kernel stored: block b sums pairs
 // [1024 b, 1024 b + 1024) from 0.0 one after another, a pair outside the cutoff adding 0.0 as the reference's
-// zero entries do. One lane per block, so a warp advances 32 blocks' ordered sums together; the warp stages 32
-// consecutive records of each of its blocks in shared memory at a time (coalesced 256-byte loads), and each lane
-// then evaluates and adds its block's 32 (the evaluations are independent of the sums, so they overlap).
-constexpr int kPairSumWarps = 4;
+// zero entries do (src/Forcefield.cpp:288-296).
+// A warp advances kBlocks blocks together: its 32 lanes evaluate 256 / kBlocks records of each into shared memory (the
+// next ones already loaded), then 2 kBlocks lanes, one per block and sum, add them in order. kBlocks = 1 finishes
+// soonest, 4 spends the fewest instructions a block (the additions of 8 chains issue together).
+constexpr int kSumWarps = 4;
+constexpr int kSumStage = 256;  // records a warp holds
 // The pair count is rec_cap, or, in a CUDA graph (where it is known only on the device), read from *pair_count
 // (the step's copy of the list's count, so a rebuild for the next step cannot change it under the sums) and capped
 // at rec_cap, the records' buffer size; the grid then covers rec_cap. The block count goes to *nblocks_out for
 // k_sum_pair_blocks.
-__global__ void __launch_bounds__(32 * kPairSumWarps) k_pair_block_sums(const double* __restrict__ pair_r2,
-                                                                        const long long* __restrict__ pair_count,
-                                                                        long long rec_cap, LJ lj,
-                                                                        double2* __restrict__ block_sums,
-                                                                        int* __restrict__ nblocks_out) {
-    __shared__ double tile[kPairSumWarps][32][33];
+template <int kBlocks>
+__global__ void __launch_bounds__(32 * kSumWarps) k_pair_block_sums(const double* __restrict__ pair_r2,
+                                                                    const long long* __restrict__ pair_count,
+                                                                    long long rec_cap, LJ lj,
+                                                                    double2* __restrict__ block_sums,
+                                                                    int* __restrict__ nblocks_out) {
+    constexpr int kEach = kSumStage / kBlocks;  // records of a block per step
+    __shared__ double2 s_term[kSumWarps][kSumStage + kBlocks];
     const long long count = pair_count ? *pair_count : rec_cap;
     const long long pairs = count < rec_cap ? count : rec_cap;
     const int nblocks = static_cast<int>((pairs + kChunk - 1) / kChunk);
     if (blockIdx.x == 0 && threadIdx.x == 0) *nblocks_out = nblocks;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b0 = (blockIdx.x * kPairSumWarps + warp) * 32;  // this warp's first block
+    const int b0 = (blockIdx.x * kSumWarps + warp) * kBlocks;
     if (b0 >= nblocks) return;
-    double(*t)[33] = tile[warp];
-    const int b = b0 + lane;
-    const long long k0 = static_cast<long long>(b) * kChunk;
-    const int m = b < nblocks ? static_cast<int>(pairs - k0 < kChunk ? pairs - k0 : kChunk) : 0;
-    double se = 0.0, sw = 0.0;
-    for (int c = 0; c < kChunk; c += 32) {
-        __syncwarp();
-        for (int r = 0; r < 32; ++r) {  // row r: records [c, c + 32) of block b0 + r, lane = record
-            const long long k = static_cast<long long>(b0 + r) * kChunk + c + lane;
-            t[r][lane] = b0 + r < nblocks && k < pairs ? __ldcs(pair_r2 + k) : lj.rc2;
-        }
-        __syncwarp();
-        const int e = m - c < 32 ? m - c : 32;
-#pragma unroll 4
-        for (int u = 0; u < e; ++u) {
-            const double r2 = t[lane][u];
-            const bool in = r2 < lj.rc2;
-            double f, en;
-            pair_terms(in ? r2 : 1.0, lj, f, en);
-            se = dadd(se, in ? en : 0.0);
-            sw = dadd(sw, in ? dmul(f, r2) : 0.0);
-        }
-    }
-    if (b < nblocks) block_sums[b] = make_double2(se, sw);
-}
-
-// k_pair_block_sums over (pairEnergy, pairVirial) records (the force kernels' `terms` form): the same ordered
-// block sums, each lane adding its block's staged terms, with the same device pair count and block-count report.
-constexpr int kPairSumWarpsTerms = 2;
-__global__ void __launch_bounds__(32 * kPairSumWarpsTerms) k_pair_block_sums_terms(
-    const double2* __restrict__ pair_ew, const long long* __restrict__ pair_count, long long rec_cap,
-    double2* __restrict__ block_sums, int* __restrict__ nblocks_out) {
-    __shared__ double2 tile[kPairSumWarpsTerms][32][33];
-    const long long count = pair_count ? *pair_count : rec_cap;
-    const long long pairs = count < rec_cap ? count : rec_cap;
-    const int nblocks = static_cast<int>((pairs + kChunk - 1) / kChunk);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *nblocks_out = nblocks;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b0 = (blockIdx.x * kPairSumWarpsTerms + warp) * 32;  // this warp's first block
-    if (b0 >= nblocks) return;
-    double2(*t)[33] = tile[warp];
-    const int b = b0 + lane;
-    const long long k0 = static_cast<long long>(b) * kChunk;
-    const int m = b < nblocks ? static_cast<int>(pairs - k0 < kChunk ? pairs - k0 : kChunk) : 0;
-    double se = 0.0, sw = 0.0;
-    for (int c = 0; c < kChunk; c += 32) {
-        __syncwarp();
-        for (int r = 0; r < 32; ++r) {  // row r: records [c, c + 32) of block b0 + r, lane = record
-            const long long k = static_cast<long long>(b0 + r) * kChunk + c + lane;
-            t[r][lane] = b0 + r < nblocks && k < pairs ? pair_ew[k] : make_double2(0.0, 0.0);
-        }
-        __syncwarp();
-        const int e = m - c < 32 ? m - c : 32;
-        for (int u = 0; u < e; ++u) {
-            const double2 x = t[lane][u];
-            se = dadd(se, x.x);
-            sw = dadd(sw, x.y);
-        }
-    }
-    if (b < nblocks) block_sums[b] = make_double2(se, sw);
-}
-
-// The outer loop of deterministicSum (include/Parallel.hpp:52-56): block sums added in order from 0.0.
-// One warp: the lanes stage 256 values at a time in shared memory (the next chunk's loads in flight while
-// lane 0 adds the current one, one value after another, reading eight ahead of the adds).
-__device__ __forceinline__ void sum_blocks(const double2* __restrict__ block_sums, int nblocks,
-                                           double* __restrict__ out) {
-    constexpr int kStage = 256;
-    __shared__ double2 stage[kStage];
-    const int lane = threadIdx.x & 31;
-    double2 next[kStage / 32];
-    auto fetch = [&](int c) {
+    double2* term = s_term[warp];  // record k of block b at term[b (kEach + 1) + k]
+    double r2[kSumStage / 32];
+    auto fetch = [&](int step) {
 #pragma unroll
-        for (int q = 0; q < kStage / 32; ++q) {
-            const int k = c * kStage + q * 32 + lane;
-            next[q] = k < nblocks ? block_sums[k] : make_double2(0.0, 0.0);
+        for (int q = 0; q < kSumStage / 32; ++q) {
+            const int b = q * 32 / kEach, k = q * 32 % kEach + lane;
+            const long long at = static_cast<long long>(b0 + b) * kChunk + step * kEach + k;
+            r2[q] = at < pairs ? __ldcs(pair_r2 + at) : lj.rc2;  // outside: adds 0.0
         }
     };
-    double se = 0.0, sw = 0.0;
-    const int chunks = (nblocks + kStage - 1) / kStage;
-    if (chunks > 0) fetch(0);
-    for (int c = 0; c < chunks; ++c) {
+    fetch(0);
+    double sum = 0.0;
+    for (int step = 0; step < kChunk / kEach; ++step) {
         __syncwarp();
 #pragma unroll
-        for (int q = 0; q < kStage / 32; ++q) stage[q * 32 + lane] = next[q];
-        __syncwarp();
-        if (c + 1 < chunks) fetch(c + 1);
-        if (lane == 0) {
-            const int m = nblocks - c * kStage < kStage ? nblocks - c * kStage : kStage;
-            int t = 0;
-            for (; t + 8 <= m; t += 8) {
-                double2 x[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) x[u] = stage[t + u];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    se = dadd(se, x[u].x);
-                    sw = dadd(sw, x[u].y);
-                }
-            }
-            for (; t < m; ++t) {
-                const double2 x = stage[t];
-                se = dadd(se, x.x);
-                sw = dadd(sw, x.y);
-            }
+        for (int q = 0; q < kSumStage / 32; ++q) {
+            const int b = q * 32 / kEach, k = q * 32 % kEach + lane;
+            const bool in = r2[q] < lj.rc2;
+            double f, e;
+            pair_terms(in ? r2[q] : 1.0, lj, f, e);
+            term[b * (kEach + 1) + k] = in ? make_double2(e, dmul(f, r2[q])) : make_double2(0.0, 0.0);
         }
+        __syncwarp();
+        if (step + 1 < kChunk / kEach) fetch(step + 1);
+        if (lane < 2 * kBlocks)
+            sum = add_in_order(reinterpret_cast<const double*>(term + (lane >> 1) * (kEach + 1)) + (lane & 1), 2, kEach, sum);
     }
-    if (lane == 0) {
-        out[0] = se;
-        out[1] = sw;
-    }
+    const int b = b0 + (lane >> 1);
+    if (lane < 2 * kBlocks && b < nblocks) reinterpret_cast<double*>(block_sums + b)[lane & 1] = sum;
 }
 
-__global__ void k_sum_blocks(const double2* __restrict__ block_sums, int nblocks, double* __restrict__ out) {
+// The outer loop of deterministicSum (include/Parallel.hpp:52-56): block sums added in order from 0.0. One block of
+// kChainThreads. A short list is one chain a sum (8 cycles a value); a long one goes through ordered_sum, which
+// gives the same bits: 31,600 block sums (N = 864,000) took 265 us as a chain.
+constexpr int kChainThreads = 2 * kOrderedThreads;
+constexpr int kChainSerial = 512;  // about where both take 4,500 cycles
+union ChainSmem {
+    OrderedSmem<2, kChainValues> ordered;
+    double2 v[kChainSerial];
+    __device__ ChainSmem() {}
+};
+__device__ __forceinline__ void sum_blocks(const double2* __restrict__ block_sums, int nblocks,
+                                           double* __restrict__ out) {
+    __shared__ ChainSmem sm;
+    if (nblocks <= kChainSerial) {
+        for (int k = threadIdx.x; k < nblocks; k += blockDim.x) sm.v[k] = block_sums[k];
+        __syncthreads();
+        if (threadIdx.x < 2)
+            out[threadIdx.x] = add_in_order(reinterpret_cast<const double*>(sm.v) + threadIdx.x, 2, nblocks, 0.0);
+        return;
+    }
+    if (threadIdx.x < 2) sm.ordered.run[threadIdx.x] = 0.0;
+    ordered_sum(sm.ordered, nblocks, [&](long long k, double* v) {
+        const double2 x = block_sums[k];
+        v[0] = x.x;
+        v[1] = x.y;
+    });
+    if (threadIdx.x < 2) out[threadIdx.x] = sm.ordered.run[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(kChainThreads) k_sum_blocks(const double2* __restrict__ block_sums, int nblocks,
+                                                              double* __restrict__ out) {
     sum_blocks(block_sums, nblocks, out);
 }
 
 // sum_blocks over the 1024-pair blocks of k_pair_block_sums, as many as it reported
-__global__ void k_sum_pair_blocks(const double2* __restrict__ block_sums, const int* __restrict__ nblocks,
-                                  double* __restrict__ out) {
+__global__ void __launch_bounds__(kChainThreads) k_sum_pair_blocks(const double2* __restrict__ block_sums,
+                                                                   const int* __restrict__ nblocks,
+                                                                   double* __restrict__ out) {
     sum_blocks(block_sums, *nblocks, out);
 }
 
@@ -428,27 +383,22 @@ __global__ void k_pairs_fit(const long long* __restrict__ pair_count, long long 
 
 // ---- kinetic energy -----------------------------------------------------------------------------------
 
-// 0.5 * m * (vx^2 + vy^2 + vz^2) over particles [1024 b, 1024 b + 1024) summed in order (src/System.cpp:67-76)
-__global__ void k_kinetic_blocks(const double* __restrict__ vel, const double* __restrict__ mass, int n,
-                                 double2* __restrict__ block_sums, int nblocks) {
-    extern __shared__ double2 sm_ke[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blk = blockIdx.x * kEnergyWarps + warp;
-    if (blk >= nblocks) return;
-    double* v = reinterpret_cast<double*>(sm_ke + warp * (kChunk / 2));
-    const int i0 = blk * kChunk;
+// 0.5 * m * (vx^2 + vy^2 + vz^2) over particles [1024 b, 1024 b + 1024) summed in order (src/System.cpp:67-76), one block
+// of kOrderedThreads each: every load of the block in flight at once, then ordered_sum. The thermostats wait for this sum.
+// (A warp per block, loading 32 at a time with one lane adding: 12.6 us at any N up to 864,000, 7 of them loads.)
+__global__ void __launch_bounds__(kOrderedThreads) k_kinetic_blocks(const double* __restrict__ vel,
+                                                                    const double* __restrict__ mass, int n,
+                                                                    double2* __restrict__ block_sums) {
+    __shared__ OrderedSmem<1, kChunk / kOrderedThreads> sm;
+    const int i0 = blockIdx.x * kChunk;
     const int m = n - i0 < kChunk ? n - i0 : kChunk;
-    for (int t = lane; t < m; t += 32) {
-        const int i = i0 + t;
+    if (threadIdx.x == 0) sm.run[0] = 0.0;
+    ordered_sum(sm, m, [&](long long k, double* v) {
+        const int i = i0 + static_cast<int>(k);
         const double vx = vel[i], vy = vel[static_cast<size_t>(n) + i], vz = vel[2 * static_cast<size_t>(n) + i];
-        v[t] = dmul(dmul(0.5, mass[i]), norm2(vx, vy, vz));
-    }
-    __syncwarp();
-    if (lane == 0) {
-        double s = 0.0;
-        for (int t = 0; t < m; ++t) s = dadd(s, v[t]);
-        block_sums[blk] = make_double2(s, 0.0);
-    }
+        v[0] = dmul(dmul(0.5, mass[i]), norm2(vx, vy, vz));
+    });
+    if (threadIdx.x == 0) block_sums[blockIdx.x] = make_double2(sm.run[0], 0.0);
 }
 
 // ---- integration --------------------------------------------------------------------------------------

@@ -222,7 +222,7 @@ md_status device_rebuild_async(md_system* s, md_forcefield* ff, md_nlist* nl, co
         MD_CHECK_LAUNCH();
         exclusive_scan<int, long long>(nl->tmp_counts.p, n, nl->half_off.p, nl->tiles.p, st);
         MD_CHECK_SCAN();
-        const long long cap = static_cast<long long>(std::min(ff->pair_r2[0].count, ff->pair_r2[1].count) / 2);
+        const long long cap = static_cast<long long>(std::min(ff->pair_r2[0].count, ff->pair_r2[1].count));
         k_pairs_fit<<<1, 1, 0, st>>>(nl->half_off.p + n, cap, s->graph_state.p);
         MD_CHECK_LAUNCH();
     }
@@ -389,8 +389,7 @@ md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_ru
     MD_CUDA(allow_smem(k_force_fp32_tile<true, false>, tile_smem));
     MD_CUDA(allow_smem(k_force_fp32_tile<false, true>, tile_smem));
     MD_CUDA(allow_smem(k_force_fp32_tile<false, false>, tile_smem));
-    MD_CUDA(allow_smem(k_force_fp64_tile<true>, sizeof(double4) * tg.max_staged));
-    MD_CUDA(allow_smem(k_force_fp64_tile<false>, sizeof(double4) * tg.max_staged));
+    MD_CUDA(allow_smem(k_force_fp64_tile, sizeof(double4) * tg.max_staged));
     // FP64: the capture starts with no energy sums queued and the records' first buffers (energy_quiesce)
     MD_TRY(energy_quiesce(ff));
     if (s->profile) {

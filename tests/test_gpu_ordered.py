@@ -33,3 +33,31 @@ def test_all_pairs_sums_bit_exact(md, oracle, n, box, rc):
     assert ff.virial == off.virial and ff.inside_pairs == off.inside
     assert n < 8100 or ff.inside_pairs > 1 << 24
     assert np.array_equal(s.forces(), os_.state().force)
+
+
+def serial(x: np.ndarray) -> float:
+    """0.0 + x[0] + x[1] + ... one after another (numpy's cumulative sum is that loop)"""
+    return float(np.cumsum(np.concatenate([[0.0], x]))[-1])
+
+
+STREAMS = {
+    "positive": lambda r, n: r.uniform(0.1, 2.0, n),
+    "mixed signs": lambda r, n: r.standard_normal(n) * r.standard_normal(n) - 0.1,
+    "walk": lambda r, n: r.standard_normal(n),  # crosses zero and binades again and again
+    "halfway": lambda r, n: np.round(r.uniform(0, 1024, n)) / 2.0 ** 22 + 2.0 ** -30 * (r.integers(0, 2, n)),
+    "scales": lambda r, n: np.ldexp(r.standard_normal(n), r.integers(-40, 40, n)),
+    "mostly zero": lambda r, n: np.where(r.integers(0, 50, n) == 0, r.standard_normal(n), 0.0),
+}
+
+
+@pytest.mark.parametrize("kind", STREAMS)
+@pytest.mark.parametrize("n", [1, 7, 8, 1023, 1025, 512 * 1024, 513 * 1024 + 1, 2200 * 1024 - 5])
+def test_blocked_sum_bit_exact(md, kind, n):
+    """The blocked kinetic-energy sum of any values (unit velocities, signed masses): 1,024 values at a time in order,
+    then the block sums in order, as one chain up to 512 of them and through ordered_sum above"""
+    x = STREAMS[kind](np.random.default_rng(n), n)
+    vel = np.zeros((3, n))
+    vel[0] = 1.0
+    s = md.System.from_arrays(np.zeros((n, 4)), 10.0, vel=vel, mass=2.0 * x)
+    blocks = np.array([serial(x[k:k + 1024]) for k in range(0, n, 1024)])
+    assert s.kinetic_energy() == serial(blocks)
