@@ -4,6 +4,7 @@
 
 #include "md_adjoint.cuh"
 #include "md_batch.cuh"
+#include "md_build.cuh"
 #include "md_cells.cuh"
 #include "md_common.cuh"
 #include "md_fp32.cuh"
@@ -400,6 +401,7 @@ CellOffsets cell_offsets(const md_nlist* nl, const md_system* s);
 #ifndef MD_TILE_HOME_TARGET
 #define MD_TILE_HOME_TARGET 96.0
 #endif
+constexpr int kMaxStage = 4096;  // candidates of a cell held in shared memory (64 KB)
 constexpr double kTileHomeTarget = MD_TILE_HOME_TARGET;  // home particles per tile block aimed at
 
 // Segment length and shared-memory size of the tile kernels for this build. Segments aim at ~96 home
@@ -437,6 +439,48 @@ md_status tile_geometry(md_nlist* nl, md_system* s, bool* use) {
 }
 
 unsigned tile_blocks(const TileGeom& g) { return static_cast<unsigned>(g.ncps) * g.ncps * g.nseg; }
+
+// Parameters of the cell build (md_build.cuh) for a list of radius^2 g.rl2 and cells of per_cell particles on average
+CellBuild cell_build_params(const ListGeom& g, double per_cell) {
+    const double margin = 1e-5 * g.rl2 + 1e-4;
+    CellBuild bp{};
+    bp.geom = g;
+    bp.rl2 = static_cast<float>(g.rl2);
+    bp.margin = static_cast<float>(margin);
+    bp.prune = static_cast<float>(g.rl2 * 1.0001 + 2.0 * margin);  // well past what the test could accept
+    // room for the candidates of nearly every cell of a uniform system (four fifths of 28 cells and six deviations)
+    const double mean = 0.8 * kCellItems * per_cell;
+    bp.stage = (std::min(static_cast<int>(mean + 6.0 * std::sqrt(mean)), kMaxStage) + 31) & ~31;
+    return bp;
+}
+
+// The list build kernel (md_build.cuh) on the system's stream, from the cells, frames and positions of this build; with
+// prepare_only its shared-memory opt-in alone, which a capture may not make. Blocks of 4 warps, 4 particles a warp at a
+// time, spend the fewest instructions (N = 864,000: 514 us; 2 particles: 551; blocks of 2 warps: 720); with few cells, 8
+// warps and 2 particles finish a cell soonest (N = 2,048: 90 us a whole rebuild against 102). Rows too long for the
+// shared memory go through the kernel's thread-per-particle path (stage 0).
+constexpr int kWideBuildCells = 148 * 14;
+constexpr size_t kBuildSmem = 200 * 1024;
+md_status cells_build_async(md_nlist* nl, md_system* s, bool prepare_only = false) {
+    const CellGrid& g = nl->grid;
+    const ListGeom geo{s->box, nl->rl2, g.ncps, 1, nl->cap, static_cast<uint32_t>(s->n) | (kSentinelCode << kCodeShift)};
+    CellBuild bp = cell_build_params(geo, static_cast<double>(s->n) / g.ncells);
+    auto go = [&](auto kernel, int warps, int homes) -> md_status {
+        size_t smem = cell_build_smem(bp.stage, nl->cap, warps, homes);
+        if (smem > kBuildSmem) {
+            bp.stage = 0;
+            smem = 0;
+        }
+        MD_CUDA(allow_smem(kernel, smem));
+        if (prepare_only) return MD_OK;
+        kernel<<<g.ncells, 32 * warps, smem, s->stream>>>(nl->frames.p, s->pos.p, g.start.p,
+                                                          static_cast<float>(s->box.L / g.ncps), bp, nl->rows.p,
+                                                          nl->counts.p, nl->flags.p + 1);
+        MD_CHECK_LAUNCH();
+        return MD_OK;
+    };
+    return g.ncells >= kWideBuildCells ? go(k_nlist_build_cells<4, 4>, 4, 4) : go(k_nlist_build_cells<8, 2>, 8, 2);
+}
 
 // NeighbourList::build (src/NeighbourList.cpp:55-134) on the device. The reference builds the cell list,
 // reorders the system, and builds the cell list again; the second build only recomputes the cells of the
@@ -481,16 +525,7 @@ md_status nlist_build(md_nlist* nl, md_system* s) {
         MD_CUDA(nl->rows.reserve(row_buffer_entries(n, nl->cap)));
         MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, 4 * sizeof(int), s->stream));
         if (n > 0 && nl->use_tiles && nl->build_pin != 0) {
-            const TileGeom& tg = nl->tiles_geom;
-            const double margin = 1e-5 * nl->rl2 + 1e-4;  // float r^2 error is below 1e-5 here
-            BuildParams bp{nl->rl2, static_cast<float>(nl->rl2 - margin), static_cast<float>(nl->rl2 + margin),
-                           nl->cap, static_cast<uint32_t>(n)};
-            const size_t smem = sizeof(float4) * tg.max_staged;
-            MD_CUDA(allow_smem(k_nlist_build_tile, smem));
-            k_nlist_build_tile<<<tile_blocks(tg), kTileThreads, smem, s->stream>>>(
-                nl->frames.p, s->pos.p, nl->grid.start.p, nl->cell_sorted.p, tg, bp, cell_offsets(nl, s), nl->rows.p,
-                nl->counts.p, nl->flags.p + 1);
-            MD_CHECK_LAUNCH();
+            MD_TRY(cells_build_async(nl, s));
             nl->build_kernel = 1;
         } else if (n > 0) {
             ListGeom geo{s->box, nl->rl2, nl->grid.ncps, nl->use_cells ? 1 : 0, nl->cap, sentinel};

@@ -16,6 +16,7 @@
 // so a replica's trajectory is bit-identical to the same system run alone.
 #pragma once
 
+#include "md_build.cuh"
 #include "md_cells.cuh"
 #include "md_common.cuh"
 #include "md_fp32.cuh"
@@ -143,44 +144,54 @@ __global__ void k_b_clear_scale(int R, double2* __restrict__ scale) {
 
 // ---- rebuild ------------------------------------------------------------------------------------------------
 
+// Work items of a replica's list build: its cells, or its tiles in a box under 3 cells per side
+__host__ __device__ __forceinline__ int build_items(const BRep& d) { return d.use_cells ? d.ncells : d.np / kTile; }
+
 // One block. Reads and clears the stale flags, lists the stale replicas and their tiles in replica order
-// (work[0] replicas, work[1] tiles) and counts each replica's rebuild.
+// (work[0] replicas, work[1] tiles, work[2] list-build items, those before stale replica w in stale_items[w]) and counts
+// each replica's rebuild.
 __global__ void __launch_bounds__(kListThreads)
     k_b_stale_lists(const BRep* __restrict__ reps, int R, int* __restrict__ stale, int* __restrict__ stale_reps,
-                    int* __restrict__ stale_tiles, int* __restrict__ work, unsigned long long* __restrict__ rebuilds) {
-    __shared__ int s_warp[2][32];
-    __shared__ int s_base[2];
+                    int* __restrict__ stale_tiles, int* __restrict__ stale_items, int* __restrict__ work,
+                    unsigned long long* __restrict__ rebuilds) {
+    __shared__ int s_warp[3][32];
+    __shared__ int s_base[3];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kWarps = kListThreads / 32;
-    if (threadIdx.x == 0) s_base[0] = s_base[1] = 0;
+    if (threadIdx.x == 0) s_base[0] = s_base[1] = s_base[2] = 0;
     __syncthreads();
     for (int r0 = 0; r0 < R; r0 += kListThreads) {
         const int r = r0 + threadIdx.x;
-        int f = 0, nt = 0, t0 = 0;
+        int f = 0, nt = 0, t0 = 0, ni = 0;
         if (r < R && stale[r]) {
             stale[r] = 0;
             const BRep d = reps[r];
             f = 1;
             nt = d.np / kTile;
             t0 = d.tile_off;
+            ni = build_items(d);
         }
-        const int sf = inclusive_warp_scan(f), st = inclusive_warp_scan(nt);
+        const int sf = inclusive_warp_scan(f), st = inclusive_warp_scan(nt), si = inclusive_warp_scan(ni);
         if (lane == 31) {
             s_warp[0][warp] = sf;
             s_warp[1][warp] = st;
+            s_warp[2][warp] = si;
         }
         __syncthreads();
         if (warp == 0) {
             const int a = inclusive_warp_scan(s_warp[0][lane]);
             const int b = inclusive_warp_scan(s_warp[1][lane]);
+            const int c = inclusive_warp_scan(s_warp[2][lane]);
             s_warp[0][lane] = a;
             s_warp[1][lane] = b;
+            s_warp[2][lane] = c;
         }
         __syncthreads();
         if (f) {
             const int pf = s_base[0] + (warp ? s_warp[0][warp - 1] : 0) + sf - 1;
             const int pt = s_base[1] + (warp ? s_warp[1][warp - 1] : 0) + st - nt;
             stale_reps[pf] = r;
+            stale_items[pf] = s_base[2] + (warp ? s_warp[2][warp - 1] : 0) + si - ni;
             for (int k = 0; k < nt; ++k) stale_tiles[pt + k] = t0 + k;
             rebuilds[r] += 1;
         }
@@ -188,12 +199,14 @@ __global__ void __launch_bounds__(kListThreads)
         if (threadIdx.x == 0) {
             s_base[0] += s_warp[0][kWarps - 1];
             s_base[1] += s_warp[1][kWarps - 1];
+            s_base[2] += s_warp[2][kWarps - 1];
         }
         __syncthreads();
     }
     if (threadIdx.x == 0) {
         work[0] = s_base[0];
         work[1] = s_base[1];
+        work[2] = s_base[2];
     }
 }
 
@@ -344,106 +357,38 @@ __global__ void __launch_bounds__(kTile)
     }
 }
 
-struct BBuild {
-    double rl2;      // (r_c + skin)^2
-    float lo, hi;    // float r^2 below lo: inside, above hi: outside, between: decided in double
-    int cap;         // row capacity
-    uint32_t sentinel;
-};
-
-__device__ __forceinline__ bool within_rl(const double4& a, const double4& b, const Box& box, double rl2) {
-    const double dx = min_image(dsub(a.x, b.x), box);
-    const double dy = min_image(dsub(a.y, b.y), box);
-    const double dz = min_image(dsub(a.z, b.z), box);
-    return norm2(dx, dy, dz) < rl2;
-}
-
-// k_nlist_build for the stale replicas, with slots for indices: the same rows (own pairs in the reference's
-// candidate order, then reverse partners ascending, then sentinels). With cells, candidates are screened with
-// the float frames and only those within rounding of r_l are tested in double, which gives the double test's
-// answer for every pair.
-__global__ void __launch_bounds__(kTile)
-    k_b_nlist_build(const BRep* __restrict__ reps, const int* __restrict__ tile_rep, const int* __restrict__ stale_tiles,
+// The list build of the stale replicas (build_cell, with slots for indices): blocks take their cells in turn, and the
+// tiles of replicas under 3 cells per side, a thread per particle. bp.geom's box and cells per side are set per replica.
+template <int kWarps, int kHomes>
+__global__ void __launch_bounds__(32 * kWarps)
+    k_b_nlist_build(const BRep* __restrict__ reps, const int* __restrict__ stale_reps, const int* __restrict__ stale_items,
                     const int* __restrict__ work, const double4* __restrict__ pos, const float4* __restrict__ frames,
-                    const int* __restrict__ cell_sorted, const int* __restrict__ start, BBuild bp,
-                    uint32_t* __restrict__ rows, int2* __restrict__ counts, int* __restrict__ max_count) {
-    const int nw = work[1];
-    for (int w = blockIdx.x; w < nw; w += gridDim.x) {
-        int r, a;
-        BRep d;
-        if (!stale_slot(reps, tile_rep, stale_tiles, w, r, d, a)) continue;
-        const double4 pi = pos[a];
-        int cnt = 0;
-        auto push = [&](int j, uint32_t code) {
-            if (cnt < bp.cap) rows[row_index(a, cnt, bp.cap)] = static_cast<uint32_t>(j) | (code << kCodeShift);
-            ++cnt;
-        };
-        int own;
-        if (d.use_cells) {
-            const float4 qi = frames[a];
-            const float cellf = static_cast<float>(d.cell);
-            const int* st = start + d.cell_off + r;
-            uint32_t* row = rows + row_index(a, 0, bp.cap);
-            // candidates [j0, j1) of one cell (scan_cell: branch-free float screen, exact shell re-scan);
-            // qo = q_i + the cell's image offset, computed once per candidate cell
-            auto take = [&](int j0, int j1, uint32_t code, const float4& qo) {
-                scan_cell<false>(frames + j0, j0, 0, j1 - j0, qo, code, bp.lo, bp.hi, bp.rl2, bp.cap, pi, pos, d.box, row,
-                                 cnt);
-            };
-            auto shifted = [&](uint32_t code) {
-                const float4 o = code_offset(static_cast<int>(code), cellf);
-                return make_float4(qi.x + o.x, qi.y + o.y, qi.z + o.z, 0.0f);
-            };
-            const int nc = d.ncps;
-            const int c = cell_sorted[a];
-            const int cx = c / (nc * nc), cy = (c / nc) % nc, cz = c % nc;
-            for (int dx = -1; dx <= 1; ++dx) {
-                const int x = (cx + dx + nc) % nc;
-                for (int dy = -1; dy <= 1; ++dy) {
-                    const int y = (cy + dy + nc) % nc;
-                    for (int dz = -1; dz <= 1; ++dz) {
-                        const int cell = (x * nc + y) * nc + (cz + dz + nc) % nc;
-                        const uint32_t code = (dx + 1) * 9 + (dy + 1) * 3 + (dz + 1);
-                        const int e = st[cell + 1];
-                        const int j0 = st[cell] > a + 1 ? st[cell] : a + 1;
-                        if (j0 < e) take(j0, e, code, shifted(code));
-                    }
-                }
-            }
-            own = cnt;
-            int ox[3], oy[3], oz[3];
-            ascending_offsets(cx, nc, ox);
-            ascending_offsets(cy, nc, oy);
-            ascending_offsets(cz, nc, oz);
-            for (int u = 0; u < 3; ++u) {
-                const int x = (cx + ox[u] + nc) % nc;
-                for (int v = 0; v < 3; ++v) {
-                    const int y = (cy + oy[v] + nc) % nc;
-                    for (int q = 0; q < 3; ++q) {
-                        const int cell = (x * nc + y) * nc + (cz + oz[q] + nc) % nc;
-                        const uint32_t code = (ox[u] + 1) * 9 + (oy[v] + 1) * 3 + (oz[q] + 1);
-                        const int e = st[cell + 1] < a ? st[cell + 1] : a;
-                        if (st[cell] < e) take(st[cell], e, code, shifted(code));
-                    }
-                }
-            }
-        } else {
-            // under 3 cells per side every particle of the replica is a candidate (src/NeighbourList.cpp:45-50)
-            const int end = d.off + d.n;
-            for (int j = a + 1; j < end; ++j)
-                if (within_rl(pi, pos[j], d.box, bp.rl2)) push(j, 13u);
-            own = cnt;
-            for (int j = d.off; j < a; ++j)
-                if (within_rl(pi, pos[j], d.box, bp.rl2)) push(j, 13u);
+                    const int* __restrict__ start, CellBuild bp, uint32_t* __restrict__ rows, int2* __restrict__ counts,
+                    int* __restrict__ max_count) {
+    extern __shared__ float4 sm_cell[];
+    __shared__ CellItems t;
+    const int nr = work[0], total = work[2];
+    for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        int lo = 0, hi = nr;  // the replica: last w with stale_items[w] <= item
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (stale_items[mid] <= item) lo = mid; else hi = mid;
         }
-        // a row past the capacity keeps counts within it (so every reader stays in bounds) and reports its
-        // length: the host restores the chunk's starting state and runs it again with a larger capacity
-        const int own_c = own < bp.cap ? own : bp.cap;
-        const int all_c = cnt < bp.cap ? cnt : bp.cap;
-        counts[a] = make_int2(own_c, all_c - own_c);
-        const int padded = (cnt + 7) & ~7;
-        for (int s = cnt; s < padded && s < bp.cap; ++s) rows[row_index(a, s, bp.cap)] = bp.sentinel;
-        atomicMax(max_count, padded);
+        const int r = stale_reps[lo];
+        const BRep d = reps[r];
+        bp.geom.box = d.box;
+        bp.geom.ncps = d.ncps;
+        bp.geom.use_cells = d.use_cells;
+        const int* st = start + d.cell_off + r;
+        if (d.use_cells) {
+            build_cell<kWarps, kHomes>(t, sm_cell, frames, pos, st, item - stale_items[lo], static_cast<float>(d.cell), bp,
+                                       rows, counts, max_count);
+        } else {
+            const int i0 = (item - stale_items[lo]) * kTile;
+            for (int i = i0 + threadIdx.x; i < i0 + kTile && i < d.n; i += 32 * kWarps)
+                build_row(pos, d.off, d.off + d.n, bp.geom, d.off + i, 0, st, rows, counts, max_count);
+        }
+        __syncthreads();  // the shared memory goes to the next item
     }
 }
 

@@ -15,6 +15,8 @@ struct md_batch {
     int R = 0;
     int64_t atoms = 0;
     int slots = 0, tiles = 0, cells = 0, chunks = 0;
+    int build_items = 0;    // list-build work items of all replicas (cells, or tiles of boxes without cells)
+    double per_cell = 0.0;  // particles per cell of the densest replica
     std::vector<BRep> reps_h;
     DevBuf<BRep> reps;
     DevBuf<int> tile_rep, chunk_rep;
@@ -36,7 +38,7 @@ struct md_batch {
     // cells
     DevBuf<int> count, cursor, start;
     // per replica
-    DevBuf<int> stale, stale_reps, stale_tiles, work, pairs, item_off, flags;
+    DevBuf<int> stale, stale_reps, stale_tiles, stale_items, work, pairs, item_off, flags;
     DevBuf<unsigned long long> acc, rebuilds, inside;
     DevBuf<double> ke, chunk_sums, noise, rec, tmp_pe, tmp_w;
     DevBuf<double2> scale, item_sums;
@@ -132,11 +134,30 @@ unsigned per_replica(const md_batch* b, int threads) { return blocks_for(b->R, t
 
 bool float_mode(const md_batch* b) { return b->opt.precision != MD_PREC_FP64; }
 
+// The list build kernel over the stale replicas' cells (prepare_only: its shared-memory opt-in alone, which a capture
+// may not make). Rows too long for the kernel's shared memory go through its thread-per-particle path (stage 0).
+md_status b_build_async(md_batch* b, bool prepare_only) {
+    const ListGeom geo{Box{}, b->rl2, 0, 1, b->cap, static_cast<uint32_t>(b->slots) | (kSentinelCode << kCodeShift)};
+    CellBuild bp = cell_build_params(geo, b->per_cell);
+    size_t smem = cell_build_smem(bp.stage, b->cap, 4, 4);
+    if (smem > kBuildSmem) {
+        bp.stage = 0;
+        smem = 0;
+    }
+    MD_CUDA(allow_smem(k_b_nlist_build<4, 4>, smem));
+    if (prepare_only) return MD_OK;
+    const unsigned grid = static_cast<unsigned>(std::min(b->build_items, 148 * 32));
+    k_b_nlist_build<4, 4><<<grid, 128, smem, b->stream>>>(b->reps.p, b->stale_reps.p, b->stale_items.p, b->work.p, b->pos.p,
+                                                          b->frames.p, b->start.p, bp, b->rows.p, b->counts.p, b->flags.p);
+    MD_CHECK_LAUNCH();
+    return MD_OK;
+}
+
 // The list rebuild of every replica flagged stale (all of them when the flags were set by the host)
 md_status b_rebuild_async(md_batch* b) {
     cudaStream_t st = b->stream;
     k_b_stale_lists<<<1, kListThreads, 0, st>>>(b->reps.p, b->R, b->stale.p, b->stale_reps.p, b->stale_tiles.p,
-                                                 b->work.p, b->rebuilds.p);
+                                                b->stale_items.p, b->work.p, b->rebuilds.p);
     MD_CHECK_LAUNCH();
     const unsigned gt = rebuild_grid(b), gr = replica_grid(b);
     k_b_cell_assign<<<gt, kTile, 0, st>>>(b->reps.p, b->tile_rep.p, b->stale_tiles.p, b->work.p, b->pos.p, b->cell_of.p,
@@ -158,14 +179,7 @@ md_status b_rebuild_async(md_batch* b) {
                                      b->force2.p, b->mass2.p, b->ids2.p, b->cell_sorted.p, b->pos.p, b->vel.p,
                                      b->force.p, b->mass.p, b->ids.p, b->ref_pos.p, b->frames.p);
     MD_CHECK_LAUNCH();
-    const double rl2 = b->rl2;
-    const double margin = 1e-5 * rl2 + 1e-4;  // bound on the float r^2 error of fresh frames (as the tile build)
-    const BBuild bp{rl2, static_cast<float>(rl2 - margin), static_cast<float>(rl2 + margin), b->cap,
-                    static_cast<uint32_t>(b->slots) | (kSentinelCode << kCodeShift)};
-    k_b_nlist_build<<<gt, kTile, 0, st>>>(b->reps.p, b->tile_rep.p, b->stale_tiles.p, b->work.p, b->pos.p, b->frames.p,
-                                          b->cell_sorted.p, b->start.p, bp, b->rows.p, b->counts.p, b->flags.p);
-    MD_CHECK_LAUNCH();
-    return MD_OK;
+    return b_build_async(b, false);
 }
 
 template <bool kFixed, bool kEnergy>
@@ -333,7 +347,9 @@ md_status b_graph(md_batch* b, int len, cudaGraphExec_t* out, uint64_t* kernels)
     uint64_t* saved = g_launches;
     g_launches = &count;
     cudaGraph_t graph = nullptr;
+    MD_TRY(b_build_async(b, true));
     MD_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    g_capturing = true;
     md_status st = MD_OK;
     const int every = b->opt.energy_every;
     for (int k = 0; k < len && st == MD_OK; ++k) {
@@ -343,6 +359,7 @@ md_status b_graph(md_batch* b, int len, cudaGraphExec_t* out, uint64_t* kernels)
         st = b_enqueue_step(b, k, step, rec);
     }
     const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
+    g_capturing = false;
     g_launches = saved;
     if (st != MD_OK) {
         if (graph) cudaGraphDestroy(graph);
@@ -589,6 +606,8 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
         d.use_cells = d.ncps >= 3 ? 1 : 0;  // src/NeighbourList.cpp:69
         d.tile_off = off / kTile;
         d.chunk_off = chunk_off;
+        b->build_items += md::build_items(d);
+        if (d.use_cells) b->per_cell = std::max(b->per_cell, static_cast<double>(d.n) / d.ncells);
         for (int t = 0; t < d.np / kTile; ++t) tile_rep[d.tile_off + t] = r;
         const int nch = (n + kChunk - 1) / kChunk;
         for (int c = 0; c < nch; ++c) chunk_rep.push_back(r);
@@ -629,9 +648,9 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
     chk(b->count.reserve(b->cells));
     chk(b->cursor.reserve(b->cells));
     chk(b->start.reserve(static_cast<size_t>(b->cells) + R));
-    for (auto* buf : {&b->stale, &b->stale_reps, &b->pairs}) chk(buf->reserve(R));
+    for (auto* buf : {&b->stale, &b->stale_reps, &b->stale_items, &b->pairs}) chk(buf->reserve(R));
     chk(b->stale_tiles.reserve(b->tiles));
-    chk(b->work.reserve(2));
+    chk(b->work.reserve(3));
     chk(b->item_off.reserve(R + 1));
     chk(b->flags.reserve(1));
     chk(b->acc.reserve(4 * R));

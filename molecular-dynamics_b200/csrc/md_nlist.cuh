@@ -46,13 +46,12 @@ __device__ __forceinline__ void ascending_offsets(int c, int n, int* d) {
     }
 }
 
-// One thread per particle. counts[i] = (own, reverse); rows beyond `cap` are not written, and max_count
-// records the longest row so the host can grow `cap` and rebuild.
-__global__ void k_nlist_build(const double4* __restrict__ pos, int n, ListGeom g, const int* __restrict__ cell_of,
-                              const int* __restrict__ cell_start, uint32_t* __restrict__ rows,
-                              int2* __restrict__ counts, int* __restrict__ max_count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// The row of particle i by the reference's double test on every candidate, one at a time; cell c is i's, its neighbours'
+// ranges in cell_start (without cells, every particle of [begin, end) is a candidate). Entries past the capacity are counted and not written; the counts stay within it, so every
+// reader stays in bounds, and max_count gets the longest padded row, so the host can grow `cap` and rebuild.
+__device__ __forceinline__ void build_row(const double4* __restrict__ pos, int begin, int end, const ListGeom& g, int i, int c,
+                                          const int* __restrict__ cell_start, uint32_t* __restrict__ rows,
+                                          int2* __restrict__ counts, int* __restrict__ max_count) {
     const double4 pi = pos[i];
     int cnt = 0;
     auto push = [&](int j, uint32_t code) {
@@ -62,7 +61,6 @@ __global__ void k_nlist_build(const double4* __restrict__ pos, int n, ListGeom g
     int own;
     if (g.use_cells) {
         const int nc = g.ncps;
-        const int c = cell_of[i];
         const int cx = c / (nc * nc), cy = (c / nc) % nc, cz = c % nc;
         for (int dx = -1; dx <= 1; ++dx) {
             const int x = (cx + dx + nc) % nc;
@@ -98,16 +96,25 @@ __global__ void k_nlist_build(const double4* __restrict__ pos, int n, ListGeom g
         }
     } else {
         // Box under 3 cells per side: every particle is a candidate (src/NeighbourList.cpp:45-50)
-        for (int j = i + 1; j < n; ++j)
+        for (int j = i + 1; j < end; ++j)
             if (within_list(pi, pos[j], g)) push(j, 13u);
         own = cnt;
-        for (int j = 0; j < i; ++j)
+        for (int j = begin; j < i; ++j)
             if (within_list(pi, pos[j], g)) push(j, 13u);
     }
-    counts[i] = make_int2(own, cnt - own);
+    const int own_c = own < g.cap ? own : g.cap, all_c = cnt < g.cap ? cnt : g.cap;
+    counts[i] = make_int2(own_c, all_c - own_c);
     const int padded = (cnt + 7) & ~7;
     for (int s = cnt; s < padded && s < g.cap; ++s) rows[row_index(i, s, g.cap)] = g.sentinel;
     atomicMax(max_count, padded);
+}
+
+// One thread per particle
+__global__ void k_nlist_build(const double4* __restrict__ pos, int n, ListGeom g, const int* __restrict__ cell_of,
+                              const int* __restrict__ cell_start, uint32_t* __restrict__ rows,
+                              int2* __restrict__ counts, int* __restrict__ max_count) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) build_row(pos, 0, n, g, i, g.use_cells ? cell_of[i] : 0, cell_start, rows, counts, max_count);
 }
 
 __global__ void k_own_counts(const int2* __restrict__ counts, int n, int* __restrict__ own) {

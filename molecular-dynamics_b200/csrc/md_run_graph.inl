@@ -206,15 +206,7 @@ md_status device_rebuild_async(md_system* s, md_forcefield* ff, md_nlist* nl, co
     k_frames<<<blocks_for(n + 1, kThreads), kThreads, 0, st>>>(s->pos.p, n, nl->cell_sorted.p, g.ncps, cell, s->box,
                                                                nl->frames.p);
     MD_CHECK_LAUNCH();
-    const double margin = 1e-5 * nl->rl2 + 1e-4;
-    const BuildParams bp{nl->rl2, static_cast<float>(nl->rl2 - margin), static_cast<float>(nl->rl2 + margin), nl->cap,
-                         static_cast<uint32_t>(n)};
-    const size_t smem = sizeof(float4) * tg.max_staged;
-    MD_CUDA(allow_smem(k_nlist_build_tile, smem));
-    k_nlist_build_tile<<<tile_blocks(tg), kTileThreads, smem, st>>>(nl->frames.p, s->pos.p, g.start.p,
-                                                                    nl->cell_sorted.p, tg, bp, cell_offsets(nl, s),
-                                                                    nl->rows.p, nl->counts.p, nl->flags.p + 1);
-    MD_CHECK_LAUNCH();
+    MD_TRY(cells_build_async(nl, s));
     k_build_done<<<1, 1, 0, st>>>(nl->flags.p + 1, nl->cap, s->graph_state.p, (s->graph_flags & MD_GRAPH_TEST_RERUN) != 0);
     MD_CHECK_LAUNCH();
     if (ff->precision == MD_PREC_FP64) {  // the pair offsets of the energy records, and their count against the buffers
@@ -383,8 +375,8 @@ md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_ru
     RunGraph rg;
     // what a capture may not do: opt the tile kernels in to the recorded tile's shared memory, create the
     // profiling events (two per step)
-    const size_t build_smem = sizeof(float4) * tg.max_staged, tile_smem = sizeof(float4) * (tg.max_staged + 1);
-    MD_CUDA(allow_smem(k_nlist_build_tile, build_smem));
+    const size_t tile_smem = sizeof(float4) * (tg.max_staged + 1);
+    MD_TRY(cells_build_async(nl, s, true));
     MD_CUDA(allow_smem(k_force_fp32_tile<true, true>, tile_smem));
     MD_CUDA(allow_smem(k_force_fp32_tile<true, false>, tile_smem));
     MD_CUDA(allow_smem(k_force_fp32_tile<false, true>, tile_smem));

@@ -1,4 +1,4 @@
-// Shared-memory cell tiles for the list build and the list force kernels (boxes of at least 3 cells per side).
+// Shared-memory cell tiles for the list force kernels (boxes of at least 3 cells per side).
 //
 // Work decomposition: one thread block per "segment" = kk consecutive cells along z of one (x, y) cell
 // column. The block stages into shared memory every particle its home atoms can pair with: the 9 columns
@@ -150,184 +150,6 @@ __device__ __forceinline__ int staged_cell(int code, int h, int span) {
     const int dxy = code / 3;        // (dx + 1) * 3 + (dy + 1)
     const int dz = code % 3 - 1;
     return dxy * span + h + 1 + dz;
-}
-
-// ---- list build -------------------------------------------------------------------------------------------
-
-// NeighbourList::build pass 1 (src/NeighbourList.cpp:75-111) on a tile. Candidates come from staged float
-// frames; a candidate is accepted when float r^2 < r_l^2 - margin, rejected when float r^2 > r_l^2 + margin,
-// and otherwise decided by the reference's exact double test on the global positions (a thin shell of
-// candidates). margin bounds the float error of r^2 (frames are within 1.6 cells' half width of their cell
-// centre, so each coordinate carries under 4e-7 absolute error), which keeps the list bit-identical.
-// Row order: own pairs (j > i) in the reference's candidate order, then the j < i that list i, ascending.
-struct BuildParams {
-    double rl2;
-    float rl2_lo, rl2_hi;  // (r_l^2 - margin, r_l^2 + margin) in float
-    int cap;
-    uint32_t sentinel;     // index of the sentinel particle (n)
-};
-
-// The reference's list test in double (src/NeighbourList.cpp:38-52), kept out of line: only candidates within
-// float rounding of r_l reach it
-__device__ __noinline__ bool exact_within(const double4& pi, const double4& pj, const Box& box, double rl2) {
-    const double ex = min_image(dsub(pi.x, pj.x), box);
-    const double ey = min_image(dsub(pi.y, pj.y), box);
-    const double ez = min_image(dsub(pi.z, pj.z), box);
-    return norm2(ex, ey, ez) < rl2;
-}
-
-// The exact pass of scan_cell: candidates [u0, u1) decided as the float scan does, except those in the thin shell,
-// which the reference's double test decides; appended from the row length cnt on
-__device__ __noinline__ void rescan_cell_exact(const float4* q, int jbase, int u0, int u1, const float4 qo,
-                                               uint32_t code, float lo, float hi, double rl2, int cap,
-                                               const double4 pi, const double4* __restrict__ pos, const Box box,
-                                               uint32_t* row, int& cnt) {
-    for (int u = u0; u < u1; ++u) {
-        const float4 qj = q[u];
-        const float dx = qo.x - qj.x;
-        const float dy = qo.y - qj.y;
-        const float dz = qo.z - qj.z;
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        bool take = r2 < lo;
-        if (!take && r2 <= hi) take = exact_within(pi, pos[jbase + u], box, rl2);
-        if (take) {
-            if (cnt < cap) row[(cnt >> 2) * 128 + (cnt & 3)] = static_cast<uint32_t>(jbase + u) | (code << kCodeShift);
-            ++cnt;
-        }
-    }
-}
-
-// Appends to a row the candidates u in [u0, u1) of one cell that are within r_l of particle i: candidate u has
-// the float frame q[u] and the index jbase + u, qo = q_i + the cell's image offset (the margin covers the
-// rounding of that hoisted sum), row is particle i's interleaved row (entry s at row[(s >> 2) * 128 + (s & 3)])
-// and cnt its length. The loop runs branch-free: a candidate whose float r^2 is below lo = r_l^2 - margin is
-// appended with a predicated store, one above hi = r_l^2 + margin is dropped. If any candidate of the cell falls
-// in the thin shell between, the cell is scanned again from its first slot with the reference's exact double
-// test (src/NeighbourList.cpp:38-52) deciding the shell, rewriting the same slots. Entries past cap are counted
-// and not written. kOutOfLine keeps that re-scan in a separate function (fewer registers in the tiled build's
-// loop; the batch build is faster with it inline).
-template <bool kOutOfLine>
-__device__ __forceinline__ void scan_cell(const float4* q, int jbase, int u0, int u1, const float4& qo, uint32_t code,
-                                          float lo, float hi, double rl2, int cap, const double4& pi,
-                                          const double4* __restrict__ pos, const Box& box, uint32_t* row, int& cnt) {
-    const int cnt0 = cnt;
-    bool shell = false;
-    const uint32_t vbase = static_cast<uint32_t>(jbase) | (code << kCodeShift);  // entry of candidate u: vbase + u
-    // q_j - qo: the negation of qo - q_j in every bit (round-to-nearest is symmetric), x and y in one packed add
-    const float2 nxy = make_float2(-qo.x, -qo.y);
-    const float nz = -qo.z;
-    if (cnt + (u1 - u0) <= cap) {  // every candidate fits: no capacity test per candidate
-        for (int u = u0; u < u1; ++u) {
-            const float4 qj = q[u];
-            const float2 d = __fadd2_rn(make_float2(qj.x, qj.y), nxy);
-            const float dz = __fadd_rn(qj.z, nz);
-            const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, dz * dz));
-            const bool take = r2 < lo;
-            shell |= !take && r2 <= hi;
-            uint32_t* p = row + (cnt + 31 * (cnt & ~3));  // (cnt >> 2) * 128 + (cnt & 3)
-            asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.u32 t, %2, 0;\n\t@t st.global.u32 [%0], %1;\n\t}"
-                         :: "l"(p), "r"(vbase + static_cast<uint32_t>(u)), "r"(static_cast<unsigned>(take)) : "memory");
-            cnt += take ? 1 : 0;
-        }
-    } else {
-        for (int u = u0; u < u1; ++u) {
-            const float4 qj = q[u];
-            const float2 d = __fadd2_rn(make_float2(qj.x, qj.y), nxy);
-            const float dz = __fadd_rn(qj.z, nz);
-            const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, dz * dz));
-            const bool take = r2 < lo;
-            shell |= !take && r2 <= hi;
-            if (take && cnt < cap) row[(cnt >> 2) * 128 + (cnt & 3)] = vbase + static_cast<uint32_t>(u);
-            cnt += take ? 1 : 0;
-        }
-    }
-    if (shell) {
-        cnt = cnt0;
-        if (kOutOfLine) {
-            rescan_cell_exact(q, jbase, u0, u1, qo, code, lo, hi, rl2, cap, pi, pos, box, row, cnt);
-        } else {
-            for (int u = u0; u < u1; ++u) {
-                const float4 qj = q[u];
-                const float dx = qo.x - qj.x;
-                const float dy = qo.y - qj.y;
-                const float dz = qo.z - qj.z;
-                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                bool take = r2 < lo;
-                if (!take && r2 <= hi) take = exact_within(pi, pos[jbase + u], box, rl2);
-                if (take) {
-                    if (cnt < cap) row[(cnt >> 2) * 128 + (cnt & 3)] = static_cast<uint32_t>(jbase + u) | (code << kCodeShift);
-                    ++cnt;
-                }
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kTileThreads) k_nlist_build_tile(
-    const float4* __restrict__ frames, const double4* __restrict__ pos, const int* __restrict__ cell_start,
-    const int* __restrict__ cell_sorted, TileGeom g, BuildParams bp, CellOffsets offs, uint32_t* __restrict__ rows,
-    int2* __restrict__ counts, int* __restrict__ max_count) {
-    extern __shared__ float4 s_q[];
-    __shared__ TileTables t;
-    tile_tables(g, cell_start, t);
-    if (t.total > g.max_staged) {  // the host's bound was wrong: report a full row so it rebuilds bigger
-        if (threadIdx.x == 0) atomicMax(max_count, 1 << 30);
-        return;
-    }
-    stage_tile(frames, s_q, t);
-    cp_async_wait();
-    __syncthreads();
-    const int n = g.ncps;
-    const int span = t.kk + 2;
-    for (int i = t.home_begin + threadIdx.x; i < t.home_end; i += blockDim.x) {
-        const float4 qi = frames[i];
-        const double4 pi = pos[i];
-        const int z = cell_sorted[i] % n;
-        const int h = (z - t.z0 + n) % n;
-        int cnt = 0;
-        // this particle's interleaved row: entry s at row[(s >> 2) * 128 + (s & 3)]
-        uint32_t* row = rows + static_cast<size_t>(i >> 5) * (bp.cap >> 2) * 128 + (i & 31) * 4;
-        auto scan = [&](const float4* q, int gs, int u0, int u1, const float4& qo, uint32_t code) {
-            scan_cell<true>(q, gs, u0, u1, qo, code, bp.rl2_lo, bp.rl2_hi, bp.rl2, bp.cap, pi, pos, g.box, row, cnt);
-        };
-        // own pairs: 27 cells in (dx, dy, dz) order, increasing j inside each (src/CellList.cpp:55-83)
-        for (uint32_t code = 0; code < 27; ++code) {
-            const int sc = staged_cell(static_cast<int>(code), h, span);
-            const float4 o = offs.off[code];
-            const float4 qo = make_float4(qi.x + o.x, qi.y + o.y, qi.z + o.z, 0.0f);
-            const int gs = t.gstart[sc];
-            scan(s_q + t.off[sc], gs, max(0, i + 1 - gs), t.count[sc], qo, code);
-        }
-        const int own = cnt;
-        // the j < i that list i, increasing j: cells in increasing cell id
-        const int cx = t.cx, cy = t.cy;
-        int ox[3], oy[3], oz[3];
-        auto asc = [n](int c, int* d) {
-            if (c == 0) { d[0] = 0; d[1] = 1; d[2] = -1; }
-            else if (c == n - 1) { d[0] = 1; d[1] = -1; d[2] = 0; }
-            else { d[0] = -1; d[1] = 0; d[2] = 1; }
-        };
-        asc(cx, ox);
-        asc(cy, oy);
-        asc(z, oz);
-        for (int a = 0; a < 3; ++a)
-            for (int b = 0; b < 3; ++b)
-                for (int d = 0; d < 3; ++d) {
-                    const uint32_t code = (ox[a] + 1) * 9 + (oy[b] + 1) * 3 + (oz[d] + 1);
-                    const int sc = staged_cell(static_cast<int>(code), h, span);
-                    const float4 o = offs.off[code];
-                    const float4 qo = make_float4(qi.x + o.x, qi.y + o.y, qi.z + o.z, 0.0f);
-                    const int gs = t.gstart[sc];
-                    scan(s_q + t.off[sc], gs, 0, min(t.count[sc], i - gs), qo, code);
-                }
-        // a row past the capacity keeps counts within it (the entries written), so kernels that read the rows
-        // before the host sees max_count stay in bounds; max_count reports the full length
-        const int own_c = min(own, bp.cap), cnt_c = min(cnt, bp.cap);
-        counts[i] = make_int2(own_c, cnt_c - own_c);
-        const int padded = (cnt + 7) & ~7;
-        for (int s = cnt; s < padded && s < bp.cap; ++s) row[(s >> 2) * 128 + (s & 3)] = bp.sentinel | (kSentinelCode << kCodeShift);
-        atomicMax(max_count, padded);
-    }
 }
 
 // ---- float forces -----------------------------------------------------------------------------------------
