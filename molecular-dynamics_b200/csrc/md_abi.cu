@@ -529,9 +529,13 @@ md_status nlist_build(md_nlist* nl, md_system* s) {
             nl->build_kernel = 1;
         } else if (n > 0) {
             ListGeom geo{s->box, nl->rl2, nl->grid.ncps, nl->use_cells ? 1 : 0, nl->cap, sentinel};
-            k_nlist_build<<<blocks_for(n, 128), 128, 0, s->stream>>>(s->pos.p, n, geo, nl->cell_sorted.p,
-                                                                      nl->grid.start.p, nl->rows.p, nl->counts.p,
-                                                                      nl->flags.p + 1);
+            if (nl->use_cells)
+                k_nlist_build<<<blocks_for(n, 128), 128, 0, s->stream>>>(s->pos.p, n, geo, nl->cell_sorted.p,
+                                                                          nl->grid.start.p, nl->rows.p, nl->counts.p,
+                                                                          nl->flags.p + 1);
+            else
+                k_nlist_build_all<<<blocks_for(n, 4), 128, 0, s->stream>>>(s->pos.p, n, geo, nl->rows.p, nl->counts.p,
+                                                                           nl->flags.p + 1);
             MD_CHECK_LAUNCH();
             nl->build_kernel = 0;
         }

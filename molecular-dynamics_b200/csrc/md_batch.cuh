@@ -144,8 +144,9 @@ __global__ void k_b_clear_scale(int R, double2* __restrict__ scale) {
 
 // ---- rebuild ------------------------------------------------------------------------------------------------
 
-// Work items of a replica's list build: its cells, or its tiles in a box under 3 cells per side
-__host__ __device__ __forceinline__ int build_items(const BRep& d) { return d.use_cells ? d.ncells : d.np / kTile; }
+// Work items of a replica's list build: its cells, or groups of kAllGroup slots in a box under 3 cells per side
+constexpr int kAllGroup = 16;
+__host__ __device__ __forceinline__ int build_items(const BRep& d) { return d.use_cells ? d.ncells : d.np / kAllGroup; }
 
 // One block. Reads and clears the stale flags, lists the stale replicas and their tiles in replica order
 // (work[0] replicas, work[1] tiles, work[2] list-build items, those before stale replica w in stale_items[w]) and counts
@@ -357,8 +358,8 @@ __global__ void __launch_bounds__(kTile)
     }
 }
 
-// The list build of the stale replicas (build_cell, with slots for indices): blocks take their cells in turn, and the
-// tiles of replicas under 3 cells per side, a thread per particle. bp.geom's box and cells per side are set per replica.
+// The list build of the stale replicas (build_cell, with slots for indices): blocks take their cells in turn, and groups
+// of particles of replicas under 3 cells per side, a warp per particle. bp.geom's box and cells per side are set per replica.
 template <int kWarps, int kHomes>
 __global__ void __launch_bounds__(32 * kWarps)
     k_b_nlist_build(const BRep* __restrict__ reps, const int* __restrict__ stale_reps, const int* __restrict__ stale_items,
@@ -384,9 +385,9 @@ __global__ void __launch_bounds__(32 * kWarps)
             build_cell<kWarps, kHomes>(t, sm_cell, frames, pos, st, item - stale_items[lo], static_cast<float>(d.cell), bp,
                                        rows, counts, max_count);
         } else {
-            const int i0 = (item - stale_items[lo]) * kTile;
-            for (int i = i0 + threadIdx.x; i < i0 + kTile && i < d.n; i += 32 * kWarps)
-                build_row(pos, d.off, d.off + d.n, bp.geom, d.off + i, 0, st, rows, counts, max_count);
+            const int i0 = (item - stale_items[lo]) * kAllGroup;
+            for (int i = i0 + (threadIdx.x >> 5); i < i0 + kAllGroup && i < d.n; i += kWarps)
+                build_row_all(pos, d.off, d.off + d.n, bp.geom, d.off + i, rows, counts, max_count);
         }
         __syncthreads();  // the shared memory goes to the next item
     }
@@ -394,62 +395,48 @@ __global__ void __launch_bounds__(32 * kWarps)
 
 // ---- forces -------------------------------------------------------------------------------------------------
 
-// computeForcesDeterministic's per-particle sums (k_force_fp64) per replica, with the closing half kick and
-// the replica's inside-cutoff count into acc[4 r + 2]
+// First r^2 record of the replica in slot `off` on: rows name each pair from either end, so cap / 2 records a slot hold
+// them (but for rows cut at the capacity, whose chunk is run again: records past the replica's end are dropped)
+__device__ __forceinline__ long long brecords(int off, int cap) { return static_cast<long long>(off) * (cap >> 1); }
+
+// computeForcesDeterministic's per-particle sums (fp64_row_quads, or Fp64Lanes with kLanes > 1 threads per particle and
+// kLanes blocks per tile) per replica, with the closing half kick, the replica's inside-cutoff count into acc[4 r + 2] and,
+// with pair_r2, the own pairs' r^2 records for the ordered energy sums at the replica's half-list offsets
+template <int kLanes>
 __global__ void __launch_bounds__(kTile)
     k_b_force_fp64(const BRep* __restrict__ reps, const int* __restrict__ tile_rep, const double4* __restrict__ pos,
                    LJ lj, const uint32_t* __restrict__ rows, int cap, const int2* __restrict__ counts,
                    double* __restrict__ force, unsigned long long* __restrict__ acc, double* __restrict__ kick_vel,
-                   const double* __restrict__ mass, double half_dt) {
-    const int r = tile_rep[blockIdx.x];
+                   const double* __restrict__ mass, double half_dt, const int* __restrict__ half_off,
+                   double* __restrict__ pair_r2) {
+    const int t = blockIdx.x / kLanes, part = blockIdx.x % kLanes;
+    const int r = tile_rep[t];
     const BRep d = reps[r];
-    const int i = (blockIdx.x - d.tile_off) * kTile + threadIdx.x;
-    unsigned long long ins = 0;
-    if (i < d.n) {
-        const int a = d.off + i;
-        const double4 pi = pos[a];
-        const int2 c = counts[a];
-        const int m = c.x + c.y;
-        const int quads = (m + 3) >> 2;
-        double fx = 0.0, fy = 0.0, fz = 0.0;
-        // k_force_fp64_quads' loop: a quad of row entries at a time, the next one in flight, every entry evaluated
-        // and masked, the reverse pairs in the own form (the same bits as the reference's two loops)
-        const uint4* rq = reinterpret_cast<const uint4*>(rows) + static_cast<size_t>(a >> 5) * (cap >> 2) * 32 + (a & 31);
-        uint4 nq = make_uint4(0, 0, 0, 0);
-        if (quads > 0) nq = __ldcs(rq);
-        for (int q = 0; q < quads; ++q) {
-            const uint4 eq = nq;
-            if (q + 1 < quads) nq = __ldcs(rq + 32 * (q + 1));
-            const uint32_t ent[4] = {eq.x, eq.y, eq.z, eq.w};
-            double4 pj[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) pj[u] = pos[4 * q + u < m ? static_cast<int>(ent[u] & kIndexMask) : a];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int sl = 4 * q + u;
-                const double dx = min_image(dsub(pi.x, pj[u].x), d.box);
-                const double dy = min_image(dsub(pi.y, pj[u].y), d.box);
-                const double dz = min_image(dsub(pi.z, pj[u].z), d.box);
-                const double r2 = norm2(dx, dy, dz);
-                const bool in = sl < m && r2 < lj.rc2;
-                double f, e;
-                pair_terms(in ? r2 : 1.0, lj, f, e);
-                fx = dadd(fx, in ? dmul(f, dx) : 0.0);
-                fy = dadd(fy, in ? dmul(f, dy) : 0.0);
-                fz = dadd(fz, in ? dmul(f, dz) : 0.0);
-                ins += (in && sl < c.x) ? 1u : 0u;
-            }
+    const int i = (t - d.tile_off) * kTile + part * (kTile / kLanes) + threadIdx.x / kLanes, u = threadIdx.x % kLanes;
+    const bool real = i < d.n;
+    const int a = real ? d.off + i : d.off;
+    const int2 c = real ? counts[a] : make_int2(0, 0);
+    const long long pb = pair_r2 ? brecords(d.off, cap) + half_off[a] : 0, end = brecords(d.off + d.np, cap);
+    unsigned ins = 0;
+    auto finish = [&](int k, double f) {
+        const size_t o = bvec(d, k, a);
+        force[o] = f;
+        if (kick_vel) kick_vel[o] = dadd(kick_vel[o], ddiv(dmul(half_dt, f), mass[a]));
+    };
+    if constexpr (kLanes == 1) {
+        const double3 f = fp64_row_quads(pos, a, d.box, lj, rows, cap, c, pair_r2, pb, end, ins);
+        if (real) {
+            finish(0, f.x);
+            finish(1, f.y);
+            finish(2, f.z);
         }
-        const double F[3] = {fx, fy, fz};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const size_t o = bvec(d, k, a);
-            force[o] = F[k];
-            if (kick_vel) kick_vel[o] = dadd(kick_vel[o], ddiv(dmul(half_dt, F[k]), mass[a]));
-        }
+    } else {
+        __shared__ double s_t[kTile / 32][Fp64Lanes<kLanes>::kTerms];
+        const double f = Fp64Lanes<kLanes>::row(pos, a, d.box, lj, rows, cap, c, s_t[threadIdx.x >> 5], pair_r2, pb, end, ins);
+        if (real && u < 3) finish(u, f);
     }
-    ins = warp_sum_u64(ins);
-    if ((threadIdx.x & 31) == 0 && ins) atomicAdd(&acc[4 * r + 2], ins);
+    ins = __reduce_add_sync(0xffffffffu, ins);
+    if ((threadIdx.x & 31) == 0 && ins) atomicAdd(&acc[4 * r + 2], static_cast<unsigned long long>(ins));
 }
 
 // The float list forces per replica (k_force_fp32_rows and, for replicas under 3 cells per side,
@@ -603,42 +590,32 @@ __global__ void k_b_record_inside(int R, const unsigned long long* __restrict__ 
     if (r < R) out[r] = static_cast<double>(inside[r]);
 }
 
-constexpr int kEnergyWarps = 4;  // warps per block of the ordered sums per replica
-
 // ---- kinetic energy and thermostats ---------------------------------------------------------------------------
 
-// System::kineticEnergy's blocked sum (k_kinetic_blocks) per replica: one warp per 1024-particle block of a
+// System::kineticEnergy's blocked sum (k_kinetic_blocks) per replica: one block per 1024-particle block of a
 // replica; with `scale` the pending thermostat scale is applied to each velocity first (the kinetic energy
 // after scaleVelocities).
-__global__ void k_b_kinetic_blocks(const BRep* __restrict__ reps, const int* __restrict__ chunk_rep, int nchunks,
-                                   const double* __restrict__ vel, const double* __restrict__ mass,
-                                   const double2* __restrict__ scale, double* __restrict__ chunk_sums) {
-    extern __shared__ double sm_kb[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blk = blockIdx.x * kEnergyWarps + warp;
-    if (blk >= nchunks) return;
-    const int r = chunk_rep[blk];
+__global__ void __launch_bounds__(kOrderedThreads)
+    k_b_kinetic_blocks(const BRep* __restrict__ reps, const int* __restrict__ chunk_rep, const double* __restrict__ vel,
+                       const double* __restrict__ mass, const double2* __restrict__ scale, double* __restrict__ chunk_sums) {
+    __shared__ OrderedSmem<1, kChunk / kOrderedThreads> sm;
+    const int r = chunk_rep[blockIdx.x];
     const BRep d = reps[r];
-    double* v = sm_kb + warp * kChunk;
-    const int i0 = (blk - d.chunk_off) * kChunk;
+    const int i0 = (blockIdx.x - d.chunk_off) * kChunk;
     const int m = d.n - i0 < kChunk ? d.n - i0 : kChunk;
     const double2 sc = scale ? scale[r] : make_double2(1.0, 0.0);
-    for (int t = lane; t < m; t += 32) {
-        const int a = d.off + i0 + t;
+    if (threadIdx.x == 0) sm.run[0] = 0.0;
+    ordered_sum(sm, m, [&](long long q, double* v) {
+        const int a = d.off + i0 + static_cast<int>(q);
         double c[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             c[k] = vel[bvec(d, k, a)];
             if (sc.y != 0.0) c[k] = dmul(c[k], sc.x);
         }
-        v[t] = dmul(dmul(0.5, mass[a]), norm2(c[0], c[1], c[2]));
-    }
-    __syncwarp();
-    if (lane == 0) {
-        double s = 0.0;
-        for (int t = 0; t < m; ++t) s = dadd(s, v[t]);
-        chunk_sums[blk] = s;
-    }
+        v[0] = dmul(dmul(0.5, mass[a]), norm2(c[0], c[1], c[2]));
+    });
+    if (threadIdx.x == 0) chunk_sums[blockIdx.x] = sm.run[0];
 }
 
 // deterministicSum's outer loop per replica: its block sums added in order; one warp per replica
@@ -748,68 +725,28 @@ __global__ void __launch_bounds__(kRepScanThreads) k_b_pair_items(int R, const i
 
 // Per replica: energy and virial of each 1024-pair block of the half list in the reference's pair order, summed
 // from 0.0 one after another (deterministicSum's inner loop, include/Parallel.hpp:43-46; pairEnergy/pairVirial
-// of src/Forcefield.cpp:288-296). Each warp takes blocks (items) of all replicas in turn: the lanes evaluate the
-// block's pairs into shared memory, lane 0 adds them in order.
-__global__ void k_b_energy_blocks(const BRep* __restrict__ reps, int R, const int* __restrict__ item_off,
-                                  const int* __restrict__ pairs, const int* __restrict__ half_off,
-                                  const double4* __restrict__ pos, LJ lj, const uint32_t* __restrict__ rows, int cap,
-                                  double2* __restrict__ item_sums) {
-    extern __shared__ double2 sm_bew[];
+// of src/Forcefield.cpp:288-296), from the force kernel's r^2 records (pair_block_sums). Each warp takes blocks (items)
+// of all replicas in turn. (Evaluated from the positions, particle by particle, with one lane adding, the 3,900 blocks of
+// 128 replicas of 500 particles took 120 us.)
+__global__ void __launch_bounds__(32 * kSumWarps)
+    k_b_energy_blocks(const BRep* __restrict__ reps, int R, const int* __restrict__ item_off,
+                      const int* __restrict__ pairs, const double* __restrict__ pair_r2, LJ lj, int cap,
+                      double2* __restrict__ item_sums) {
+    __shared__ double2 s_term[kSumWarps][kSumStage + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double2* ew = sm_bew + warp * kChunk;
     const int total = item_off[R];
-    for (int item = blockIdx.x * kEnergyWarps + warp; item < total; item += gridDim.x * kEnergyWarps) {
+    for (int item = blockIdx.x * kSumWarps + warp; item < total; item += gridDim.x * kSumWarps) {
         int lo = 0, hi = R;  // the replica: last r with item_off[r] <= item
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (item_off[mid] <= item) lo = mid; else hi = mid;
         }
-        const int r = lo;
-        const BRep d = reps[r];
-        const int np = pairs[r];
-        const int k0 = (item - item_off[r]) * kChunk;
-        const int k1 = k0 + kChunk < np ? k0 + kChunk : np;
-        int i = 0;  // first particle whose pairs reach k0
-        if (lane == 0) {
-            int l = 0, h = d.n;
-            while (h - l > 1) {
-                const int mid = (l + h) >> 1;
-                if (half_off[d.off + mid] <= k0) l = mid; else h = mid;
-            }
-            i = l;
-        }
-        i = __shfl_sync(0xffffffffu, i, 0);
-        for (; i < d.n && half_off[d.off + i] < k1; ++i) {
-            const int a = d.off + i;
-            const int b = half_off[a];
-            const int kb = b > k0 ? b : k0;
-            const int e_i = i + 1 < d.n ? half_off[a + 1] : np;
-            const int ke = e_i < k1 ? e_i : k1;
-            const double4 pi = pos[a];
-            for (int k = kb + lane; k < ke; k += 32) {
-                const double4 pj = pos[rows[row_index(a, k - b, cap)] & kIndexMask];
-                const double dx = min_image(dsub(pi.x, pj.x), d.box);
-                const double dy = min_image(dsub(pi.y, pj.y), d.box);
-                const double dz = min_image(dsub(pi.z, pj.z), d.box);
-                const double r2 = norm2(dx, dy, dz);
-                double f, e;
-                pair_terms(r2, lj, f, e);
-                const bool in = r2 < lj.rc2;
-                f = in ? f : 0.0;
-                ew[k - k0] = make_double2(in ? e : 0.0, dmul(f, r2));
-            }
-        }
-        __syncwarp();
-        if (lane == 0) {
-            double se = 0.0, sw = 0.0;
-            for (int t = 0; t < k1 - k0; ++t) {
-                const double2 v = ew[t];
-                se = dadd(se, v.x);
-                sw = dadd(sw, v.y);
-            }
-            item_sums[item] = make_double2(se, sw);
-        }
-        __syncwarp();
+        const BRep d = reps[lo];
+        const int k0 = (item - item_off[lo]) * kChunk;
+        const long long all = pairs[lo], most = brecords(d.np, cap), left = (all < most ? all : most) - k0;
+        const double* rec = pair_r2 + brecords(d.off, cap) + k0;
+        const double sum = pair_block_sums<1>(s_term[warp], lj, [&](int, int k) { return k < left ? __ldcs(rec + k) : lj.rc2; });
+        if (lane < 2) reinterpret_cast<double*>(item_sums + item)[lane] = sum;
     }
 }
 

@@ -41,6 +41,7 @@ struct md_batch {
     DevBuf<int> stale, stale_reps, stale_tiles, stale_items, work, pairs, item_off, flags;
     DevBuf<unsigned long long> acc, rebuilds, inside;
     DevBuf<double> ke, chunk_sums, noise, rec, tmp_pe, tmp_w;
+    DevBuf<double> pair_r2;  // FP64 energies: every replica's own pairs' r^2 (brecords), made with the first that are due
     DevBuf<double2> scale, item_sums;
     // snapshot at the start of a chunk
     DevBuf<double4> s_pos, s_ref;
@@ -206,13 +207,32 @@ md_status b_float_forces(md_batch* b, const md_batch::Variant& v, bool kick) {
     return MD_OK;
 }
 
+// The r^2 records of FP64 energies, for the present row capacity (not inside a capture)
+md_status b_alloc_records(md_batch* b) {
+    MD_CUDA(b->pair_r2.reserve(static_cast<size_t>(b->slots) * (b->cap >> 1)));
+    return MD_OK;
+}
+
 // List forces of every replica with the given kernel variant; with `kick` the closing half kick (and, in float
-// modes, the fused fixed-point kinetic energy); with `energy` the float energy/virial sums
+// modes, the fused fixed-point kinetic energy); with `energy` the float energy/virial sums, or the FP64 sums' r^2 records
+// (after the half-list offsets they go by)
 md_status b_forces(md_batch* b, int variant, bool kick, bool energy) {
     if (!float_mode(b)) {
-        k_b_force_fp64<<<b->tiles, kTile, 0, b->stream>>>(b->reps.p, b->tile_rep.p, b->pos.p, b->lj, b->rows.p, b->cap,
-                                                          b->counts.p, b->force.p, b->acc.p, kick ? b->vel.p : nullptr,
-                                                          b->mass.p, 0.5 * b->opt.dt);
+        if (energy) {
+            k_b_half_offsets<<<replica_grid(b), kRepScanThreads, 0, b->stream>>>(b->reps.p, b->R, b->counts.p, b->half_off.p,
+                                                                              b->pairs.p);
+            MD_CHECK_LAUNCH();
+        }
+        auto go = [&](auto kernel, int lanes) {
+            kernel<<<static_cast<unsigned>(b->tiles) * lanes, kTile, 0, b->stream>>>(
+                b->reps.p, b->tile_rep.p, b->pos.p, b->lj, b->rows.p, b->cap, b->counts.p, b->force.p, b->acc.p,
+                kick ? b->vel.p : nullptr, b->mass.p, 0.5 * b->opt.dt, b->half_off.p, energy ? b->pair_r2.p : nullptr);
+        };
+        // threads per particle by the number of slots, as for a single system (k_force_fp64_lanes)
+        if (b->slots <= kFp64Lanes16) go(k_b_force_fp64<16>, 16);
+        else if (b->slots <= kFp64Lanes8) go(k_b_force_fp64<8>, 8);
+        else if (b->slots <= kFp64Lanes4) go(k_b_force_fp64<4>, 4);
+        else go(k_b_force_fp64<1>, 1);
         MD_CHECK_LAUNCH();
         return MD_OK;
     }
@@ -224,9 +244,8 @@ md_status b_forces(md_batch* b, int variant, bool kick, bool energy) {
 
 // FP64 kinetic energies in the reference's blocked order into `out` (with the pending scale applied if asked)
 md_status b_kinetic_fp64(md_batch* b, bool scaled, double* out) {
-    const size_t smem = kEnergyWarps * kChunk * sizeof(double);
-    k_b_kinetic_blocks<<<blocks_for(b->chunks, kEnergyWarps), kEnergyWarps * 32, smem, b->stream>>>(
-        b->reps.p, b->chunk_rep.p, b->chunks, b->vel.p, b->mass.p, scaled ? b->scale.p : nullptr, b->chunk_sums.p);
+    k_b_kinetic_blocks<<<b->chunks, kOrderedThreads, 0, b->stream>>>(b->reps.p, b->chunk_rep.p, b->vel.p, b->mass.p,
+                                                                     scaled ? b->scale.p : nullptr, b->chunk_sums.p);
     MD_CHECK_LAUNCH();
     k_b_sum_chunks<<<blocks_for(static_cast<long long>(b->R) * 32, kThreads), kThreads, 0, b->stream>>>(
         b->reps.p, b->R, b->chunk_sums.p, out);
@@ -234,17 +253,13 @@ md_status b_kinetic_fp64(md_batch* b, bool scaled, double* out) {
     return MD_OK;
 }
 
-// FP64 energy and virial of every replica in the reference's pair order into pe_out / w_out
+// FP64 energy and virial of every replica in the reference's pair order into pe_out / w_out, from the records of a force
+// launch with `energy`
 md_status b_energy_fp64(md_batch* b, double* pe_out, double* w_out) {
-    k_b_half_offsets<<<replica_grid(b), kRepScanThreads, 0, b->stream>>>(b->reps.p, b->R, b->counts.p, b->half_off.p,
-                                                                      b->pairs.p);
-    MD_CHECK_LAUNCH();
     k_b_pair_items<<<1, kRepScanThreads, 0, b->stream>>>(b->R, b->pairs.p, b->item_off.p);
     MD_CHECK_LAUNCH();
-    const size_t smem = kEnergyWarps * kChunk * sizeof(double2);
-    k_b_energy_blocks<<<148 * 4, kEnergyWarps * 32, smem, b->stream>>>(b->reps.p, b->R, b->item_off.p, b->pairs.p,
-                                                                       b->half_off.p, b->pos.p, b->lj, b->rows.p,
-                                                                       b->cap, b->item_sums.p);
+    k_b_energy_blocks<<<148 * 4, kSumWarps * 32, 0, b->stream>>>(b->reps.p, b->R, b->item_off.p, b->pairs.p, b->pair_r2.p,
+                                                                 b->lj, b->cap, b->item_sums.p);
     MD_CHECK_LAUNCH();
     k_b_sum_items<<<blocks_for(static_cast<long long>(b->R) * 32, kThreads), kThreads, 0, b->stream>>>(
         b->R, b->item_off.p, b->item_sums.p, pe_out, w_out);
@@ -296,7 +311,7 @@ md_status b_enqueue_step(md_batch* b, int k, int64_t step, double* rec) {
     }
     MD_TRY(b_rebuild_async(b));
     const bool sample = rec != nullptr;
-    MD_TRY(b_forces(b, b->variant, true, sample && fl));
+    MD_TRY(b_forces(b, b->variant, true, sample));
     const int R = b->R;
     if (fl) {
         k_b_finish_float<<<per_replica(b, kThreads), kThreads, 0, st>>>(R, b->acc.p, true, b->ke.p,
@@ -348,6 +363,7 @@ md_status b_graph(md_batch* b, int len, cudaGraphExec_t* out, uint64_t* kernels)
     g_launches = &count;
     cudaGraph_t graph = nullptr;
     MD_TRY(b_build_async(b, true));
+    if (!float_mode(b) && b->opt.energy_every > 0) MD_TRY(b_alloc_records(b));
     MD_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     g_capturing = true;
     md_status st = MD_OK;
@@ -698,8 +714,6 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
         const float4 sentinel = make_float4(kSentinelCoord, kSentinelCoord, kSentinelCoord, 0.0f);
         chk(cudaMemcpyAsync(b->frames.p + S, &sentinel, sizeof(float4), cudaMemcpyHostToDevice, b->stream));
         chk(cudaStreamSynchronize(b->stream));
-        chk(cudaFuncSetAttribute(k_b_energy_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kEnergyWarps * kChunk * sizeof(double2))));
     }
     if (st == MD_OK && o.thermostat == 2) {
         b->rng.reserve(replicas);
@@ -883,6 +897,7 @@ md_status md_batch_energy(md_batch* b, double* pe, double* virial, double* ke, d
     if (!b) return fail(MD_ERR_INVALID, "null batch");
     MD_TRY(use_batch(b));
     MD_TRY(b_clear_acc(b));
+    if (!float_mode(b)) MD_TRY(b_alloc_records(b));
     MD_TRY(b_forces(b, b->variant, false, true));
     MD_TRY(b_observables(b, b->tmp_pe.p, b->tmp_w.p, b->ke.p));
     const size_t R = b->R;

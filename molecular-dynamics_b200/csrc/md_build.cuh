@@ -222,7 +222,7 @@ __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const f
         __syncthreads();
         if (t.odd || t.off[kCellItems] > bp.stage) {
             for (int h = threadIdx.x; h < homes; h += 32 * kWarps)
-                build_row(pos, 0, 0, bp.geom, i0 + h, cell, cell_start, rows, counts, max_count);
+                build_row(pos, bp.geom, i0 + h, cell, cell_start, rows, counts, max_count);
             return;
         }
         auto put = [&](int at, unsigned mask, const float4& q, uint32_t entry) {

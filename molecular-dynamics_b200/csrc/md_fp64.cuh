@@ -84,6 +84,78 @@ __global__ void k_force_fp64(const double4* __restrict__ pos, int n, Box box, LJ
 // Positions come in by one 32-byte load each (two of 16 bytes: 266 us at N = 864,000 without records, now 254), and
 // the r^2 records go out by whole aligned quads of 32 bytes, shifted into place in registers (stored one by one: 493 us
 // with records, now 352). What bounds it: gather and store latency at 40 % of the FP64 pipe's time.
+// Particle i's sum and its count of own pairs inside the cutoff (added to ins), with rec its r^2 records from index pb on
+__device__ __forceinline__ double3 fp64_row_quads(const double4* __restrict__ pos, int i, const Box& box, const LJ& lj,
+                                                  const uint32_t* __restrict__ rows, int cap, const int2 c,
+                                                  double* __restrict__ rec, long long pb, long long rec_cap,
+                                                  unsigned& ins) {
+    const double4 pi = load_pos(pos + i);
+    const int m = c.x + c.y;
+    const int quads = (m + 3) >> 2;
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    const uint4* rq = reinterpret_cast<const uint4*>(rows) + static_cast<size_t>(i >> 5) * (cap >> 2) * 32 + (i & 31);
+    uint4 nq = make_uint4(0, 0, 0, 0);
+    if (quads > 0) nq = __ldcs(rq);
+    // record k of the array belongs to the aligned quad k >> 2, which is written whole once its four are known; the quads
+    // at either end of the particle's range are shared with its neighbours
+    const int shift = static_cast<int>(pb & 3);
+    double h0 = 0.0, h1 = 0.0, h2 = 0.0;  // the last records of the open aligned quad
+    for (int q = 0; q < quads; ++q) {
+        const uint4 eq = nq;
+        if (q + 1 < quads) nq = __ldcs(rq + 32 * (q + 1));
+        const uint32_t ent[4] = {eq.x, eq.y, eq.z, eq.w};
+        double4 pj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) pj[u] = load_pos(pos + (4 * q + u < m ? static_cast<int>(ent[u] & kIndexMask) : i));
+        double r[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int sl = 4 * q + u;
+            const double dx = min_image(dsub(pi.x, pj[u].x), box);
+            const double dy = min_image(dsub(pi.y, pj[u].y), box);
+            const double dz = min_image(dsub(pi.z, pj[u].z), box);
+            const double r2 = norm2(dx, dy, dz);
+            const bool in = sl < m && r2 < lj.rc2;
+            double f, e;
+            pair_terms(in ? r2 : 1.0, lj, f, e);
+            fx = dadd(fx, in ? dmul(f, dx) : 0.0);
+            fy = dadd(fy, in ? dmul(f, dy) : 0.0);
+            fz = dadd(fz, in ? dmul(f, dz) : 0.0);
+            r[u] = r2;
+            ins += in && sl < c.x ? 1u : 0u;
+        }
+        if (rec && 4 * q < c.x) {
+            // the aligned quad that ends inside this step's four: `shift` held back, 4 - shift new
+            const double a0 = shift == 0 ? r[0] : shift == 1 ? h2 : shift == 2 ? h1 : h0;
+            const double a1 = shift == 0 ? r[1] : shift == 1 ? r[0] : shift == 2 ? h2 : h1;
+            const double a2 = shift == 0 ? r[2] : shift == 1 ? r[1] : shift == 2 ? r[0] : h2;
+            const double a3 = shift == 0 ? r[3] : shift == 1 ? r[2] : shift == 2 ? r[1] : r[0];
+            const long long k = pb - shift + 4 * q;
+            const int s0 = 4 * q - shift;  // row entry of a0
+            if (s0 >= 0 && s0 + 4 <= c.x && k + 4 <= rec_cap) {
+                store_4(rec + k, a0, a1, a2, a3);
+            } else {
+                if (s0 >= 0 && s0 < c.x && k < rec_cap) rec[k] = a0;
+                if (s0 >= -1 && s0 + 1 < c.x && k + 1 < rec_cap) rec[k + 1] = a1;
+                if (s0 >= -2 && s0 + 2 < c.x && k + 2 < rec_cap) rec[k + 2] = a2;
+                if (s0 + 3 < c.x && k + 3 < rec_cap) rec[k + 3] = a3;
+            }
+            if (4 * q + 4 >= c.x) {  // the last step with own pairs: the records still held back
+                const int s1 = s0 + 4;
+                const double b0 = shift == 1 ? r[3] : shift == 2 ? r[2] : r[1];
+                const double b1 = shift == 2 ? r[3] : r[2];
+                if (shift >= 1 && s1 < c.x && k + 4 < rec_cap) rec[k + 4] = b0;
+                if (shift >= 2 && s1 + 1 < c.x && k + 5 < rec_cap) rec[k + 5] = b1;
+                if (shift >= 3 && s1 + 2 < c.x && k + 6 < rec_cap) rec[k + 6] = r[3];
+            }
+            h0 = r[1];
+            h1 = r[2];
+            h2 = r[3];
+        }
+    }
+    return make_double3(fx, fy, fz);
+}
+
 __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restrict__ pos, int n, Box box, LJ lj,
                                                           const uint32_t* __restrict__ rows, int cap,
                                                           const int2* __restrict__ counts, double* __restrict__ force,
@@ -94,73 +166,9 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned ins = 0;
     if (i < n) {
-        const double4 pi = load_pos(pos + i);
-        const int2 c = counts[i];
-        const int m = c.x + c.y;
-        const int quads = (m + 3) >> 2;
-        const long long pb = pair_r2 ? half_off[i] : 0;
-        double fx = 0.0, fy = 0.0, fz = 0.0;
-        const uint4* rq = reinterpret_cast<const uint4*>(rows) + static_cast<size_t>(i >> 5) * (cap >> 2) * 32 + (i & 31);
-        uint4 nq = make_uint4(0, 0, 0, 0);
-        if (quads > 0) nq = __ldcs(rq);
-        // r^2 records: record k of the array belongs to the aligned quad k >> 2, which is written whole once its four
-        // are known; the quads at either end of the particle's range are shared with its neighbours
-        const int shift = static_cast<int>(pb & 3);
-        double h0 = 0.0, h1 = 0.0, h2 = 0.0;  // the last records of the open aligned quad
-        for (int q = 0; q < quads; ++q) {
-            const uint4 eq = nq;
-            if (q + 1 < quads) nq = __ldcs(rq + 32 * (q + 1));
-            const uint32_t ent[4] = {eq.x, eq.y, eq.z, eq.w};
-            double4 pj[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) pj[u] = load_pos(pos + (4 * q + u < m ? static_cast<int>(ent[u] & kIndexMask) : 0));
-            double r[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int sl = 4 * q + u;
-                const double dx = min_image(dsub(pi.x, pj[u].x), box);
-                const double dy = min_image(dsub(pi.y, pj[u].y), box);
-                const double dz = min_image(dsub(pi.z, pj[u].z), box);
-                const double r2 = norm2(dx, dy, dz);
-                const bool in = sl < m && r2 < lj.rc2;
-                double f, e;
-                pair_terms(in ? r2 : 1.0, lj, f, e);
-                fx = dadd(fx, in ? dmul(f, dx) : 0.0);
-                fy = dadd(fy, in ? dmul(f, dy) : 0.0);
-                fz = dadd(fz, in ? dmul(f, dz) : 0.0);
-                r[u] = r2;
-                ins += in && sl < c.x ? 1u : 0u;
-            }
-            if (pair_r2 && 4 * q < c.x) {
-                // the aligned quad that ends inside this step's four: `shift` held back, 4 - shift new
-                const double a0 = shift == 0 ? r[0] : shift == 1 ? h2 : shift == 2 ? h1 : h0;
-                const double a1 = shift == 0 ? r[1] : shift == 1 ? r[0] : shift == 2 ? h2 : h1;
-                const double a2 = shift == 0 ? r[2] : shift == 1 ? r[1] : shift == 2 ? r[0] : h2;
-                const double a3 = shift == 0 ? r[3] : shift == 1 ? r[2] : shift == 2 ? r[1] : r[0];
-                const long long k = pb - shift + 4 * q;
-                const int s0 = 4 * q - shift;  // row entry of a0
-                if (s0 >= 0 && s0 + 4 <= c.x && k + 4 <= rec_cap) {
-                    store_4(pair_r2 + k, a0, a1, a2, a3);
-                } else {
-                    if (s0 >= 0 && s0 < c.x && k < rec_cap) pair_r2[k] = a0;
-                    if (s0 >= -1 && s0 + 1 < c.x && k + 1 < rec_cap) pair_r2[k + 1] = a1;
-                    if (s0 >= -2 && s0 + 2 < c.x && k + 2 < rec_cap) pair_r2[k + 2] = a2;
-                    if (s0 + 3 < c.x && k + 3 < rec_cap) pair_r2[k + 3] = a3;
-                }
-                if (4 * q + 4 >= c.x) {  // the last step with own pairs: the records still held back
-                    const int s1 = s0 + 4;
-                    const double b0 = shift == 1 ? r[3] : shift == 2 ? r[2] : r[1];
-                    const double b1 = shift == 2 ? r[3] : r[2];
-                    if (shift >= 1 && s1 < c.x && k + 4 < rec_cap) pair_r2[k + 4] = b0;
-                    if (shift >= 2 && s1 + 1 < c.x && k + 5 < rec_cap) pair_r2[k + 5] = b1;
-                    if (shift >= 3 && s1 + 2 < c.x && k + 6 < rec_cap) pair_r2[k + 6] = r[3];
-                }
-                h0 = r[1];
-                h1 = r[2];
-                h2 = r[3];
-            }
-        }
-        const double F[3] = {fx, fy, fz};
+        const double3 f = fp64_row_quads(pos, i, box, lj, rows, cap, counts[i], pair_r2, pair_r2 ? half_off[i] : 0, rec_cap,
+                                         ins);
+        const double F[3] = {f.x, f.y, f.z};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const size_t o = static_cast<size_t>(k) * n + i;
@@ -179,9 +187,65 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
 // For small systems: a thread per particle leaves most of the GPU without a warp (2,048 particles are 64 of them) and
 // walks its row in one long chain of gathers. Measured with records stored (B200, us; threads per particle 1 / 4 / 8 /
 // 16): N = 500: 37 / 18 / 13 / 11; 2,048: 37 / 18 / 14 / 12; 10,976: 37 / 19 / 16 / 22; 32,000: 40 / 26 / 30 / 35;
-// 108,000: 54 / 61 / 70 / 84. The lines between them follow: past about 70,000 particles the GPU is full either way and
-// the shared-memory pass only costs.
-constexpr int kFp64Lanes16 = 8192, kFp64Lanes8 = 24576, kFp64Lanes4 = 72000;
+// 108,000: 54 / 61 / 70 / 84; 65,536 slots of 128 replicas with rows of 124 entries: 55 / 61 (1 / 4). The lines between
+// them follow: past about 50,000 particles the GPU is full either way and the shared-memory pass only costs.
+constexpr int kFp64Lanes16 = 8192, kFp64Lanes8 = 24576, kFp64Lanes4 = 48000;
+template <int kLanes>
+struct Fp64Lanes {
+    static constexpr int kGroups = 32 / kLanes, kPad = kLanes + 1, kRow = kGroups * kPad + 1;
+    static constexpr int kTerms = 3 * kRow;  // doubles of shared memory a warp needs
+    // Lane u of particle i's kLanes (a whole warp calls; c is (0, 0) where there is no particle): component u of the
+    // force in lanes 0 to 2, the lane's count of own pairs inside the cutoff added to ins, and with rec the r^2 records
+    // from index pb on
+    static __device__ __forceinline__ double row(const double4* __restrict__ pos, int i, const Box& box, const LJ& lj,
+                                                 const uint32_t* __restrict__ rows, int cap, const int2 c,
+                                                 double* warp_terms, double* __restrict__ rec, long long pb,
+                                                 long long rec_cap, unsigned& ins) {
+        const int lane = threadIdx.x & 31, u = lane % kLanes;
+        double* terms = warp_terms + (lane / kLanes) * kPad;  // component k of the group's entry t at terms[k * kRow + t]
+        const int m = c.x + c.y;
+        const double4 pi = load_pos(pos + i);
+        // the longest row of the warp's particles: every lane takes part in the warp's steps
+        int steps = (m + kLanes - 1) / kLanes;
+#pragma unroll
+        for (int o = kLanes; o < 32; o <<= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, o));
+        auto entry = [&](int s) { return s < m ? static_cast<int>(rows[row_index(i, s, cap)] & kIndexMask) : i; };
+        double sum = 0.0;
+        int j1 = entry(u + kLanes);
+        double4 pj = load_pos(pos + entry(u));
+        for (int q = 0; q < steps; ++q) {
+            const int s = q * kLanes + u;
+            const double dx = min_image(dsub(pi.x, pj.x), box);
+            const double dy = min_image(dsub(pi.y, pj.y), box);
+            const double dz = min_image(dsub(pi.z, pj.z), box);
+            pj = load_pos(pos + j1);
+            j1 = entry(s + 2 * kLanes);
+            const double r2 = norm2(dx, dy, dz);
+            const bool in = s < m && r2 < lj.rc2;
+            double f, e;
+            pair_terms(in ? r2 : 1.0, lj, f, e);
+            terms[u] = in ? dmul(f, dx) : 0.0;
+            terms[kRow + u] = in ? dmul(f, dy) : 0.0;
+            terms[2 * kRow + u] = in ? dmul(f, dz) : 0.0;
+            if (s < c.x) {
+                ins += in ? 1u : 0u;
+                if (rec && pb + s < rec_cap) rec[pb + s] = r2;
+            }
+            __syncwarp();
+            if (u < 3) {
+                const double* mine = terms + u * kRow;
+                double t[kLanes];
+#pragma unroll
+                for (int k = 0; k < kLanes; ++k) t[k] = mine[k];
+#pragma unroll
+                for (int k = 0; k < kLanes; ++k) sum = dadd(sum, t[k]);
+            }
+            __syncwarp();
+        }
+        return sum;
+    }
+};
+
 template <int kLanes>
 __global__ void __launch_bounds__(128) k_force_fp64_lanes(const double4* __restrict__ pos, int n, Box box, LJ lj,
                                                           const uint32_t* __restrict__ rows, int cap,
@@ -190,61 +254,19 @@ __global__ void __launch_bounds__(128) k_force_fp64_lanes(const double4* __restr
                                                           double* __restrict__ kick_vel, const double* __restrict__ mass,
                                                           double half_dt, const long long* __restrict__ half_off,
                                                           double* __restrict__ pair_r2, long long rec_cap) {
-    constexpr int kGroups = 32 / kLanes, kPad = kLanes + 1, kRow = kGroups * kPad + 1;
-    __shared__ double s_t[4][3 * kRow];
-    const int lane = threadIdx.x & 31, g = lane / kLanes, u = lane % kLanes;
-    const int i = static_cast<int>((blockIdx.x * 128 + threadIdx.x) / kLanes);
-    double* terms = s_t[threadIdx.x >> 5] + g * kPad;  // component k of the group's entry t at terms[k * kRow + t]
+    __shared__ double s_t[4][Fp64Lanes<kLanes>::kTerms];
+    const int i = static_cast<int>((blockIdx.x * 128 + threadIdx.x) / kLanes), u = threadIdx.x % kLanes;
     const bool real = i < n;
-    const int2 c = real ? counts[i] : make_int2(0, 0);
-    const int m = c.x + c.y;
-    const double4 pi = real ? load_pos(pos + i) : make_double4(0.0, 0.0, 0.0, 0.0);
-    const long long pb = pair_r2 && real ? half_off[i] : 0;
-    // the longest row of the warp's particles: every lane takes part in the warp's steps
-    int steps = (m + kLanes - 1) / kLanes;
-#pragma unroll
-    for (int o = kLanes; o < 32; o <<= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, o));
-    auto entry = [&](int s) { return s < m ? static_cast<int>(rows[row_index(i, s, cap)] & kIndexMask) : 0; };
     unsigned ins = 0;
-    double sum = 0.0;
-    int j1 = entry(u + kLanes);
-    double4 pj = load_pos(pos + entry(u));
-    for (int q = 0; q < steps; ++q) {
-        const int s = q * kLanes + u;
-        const double dx = min_image(dsub(pi.x, pj.x), box);
-        const double dy = min_image(dsub(pi.y, pj.y), box);
-        const double dz = min_image(dsub(pi.z, pj.z), box);
-        pj = load_pos(pos + j1);
-        j1 = entry(s + 2 * kLanes);
-        const double r2 = norm2(dx, dy, dz);
-        const bool in = s < m && r2 < lj.rc2;
-        double f, e;
-        pair_terms(in ? r2 : 1.0, lj, f, e);
-        terms[u] = in ? dmul(f, dx) : 0.0;
-        terms[kRow + u] = in ? dmul(f, dy) : 0.0;
-        terms[2 * kRow + u] = in ? dmul(f, dz) : 0.0;
-        if (s < c.x) {
-            ins += in ? 1u : 0u;
-            if (pair_r2 && pb + s < rec_cap) pair_r2[pb + s] = r2;
-        }
-        __syncwarp();
-        if (u < 3) {
-            const double* mine = terms + u * kRow;
-            double t[kLanes];
-#pragma unroll
-            for (int k = 0; k < kLanes; ++k) t[k] = mine[k];
-#pragma unroll
-            for (int k = 0; k < kLanes; ++k) sum = dadd(sum, t[k]);
-        }
-        __syncwarp();
-    }
+    const double f = Fp64Lanes<kLanes>::row(pos, real ? i : 0, box, lj, rows, cap, real ? counts[i] : make_int2(0, 0),
+                                            s_t[threadIdx.x >> 5], pair_r2, pair_r2 && real ? half_off[i] : 0, rec_cap, ins);
     if (real && u < 3) {
         const size_t o = static_cast<size_t>(u) * n + i;
-        force[o] = sum;
-        if (kick_vel) kick_vel[o] = dadd(kick_vel[o], ddiv(dmul(half_dt, sum), mass[i]));
+        force[o] = f;
+        if (kick_vel) kick_vel[o] = dadd(kick_vel[o], ddiv(dmul(half_dt, f), mass[i]));
     }
     ins = __reduce_add_sync(0xffffffffu, ins);
-    if (lane == 0 && ins) atomicAdd(inside, static_cast<unsigned long long>(ins));
+    if ((threadIdx.x & 31) == 0 && ins) atomicAdd(inside, static_cast<unsigned long long>(ins));
 }
 
 // Adds x[0], x[stride], ... x[(m - 1) stride] to s one after another. One thread's chain, bound by the latency of an
@@ -285,30 +307,17 @@ constexpr int kSumStage = 256;  // records a warp holds
 // (the step's copy of the list's count, so a rebuild for the next step cannot change it under the sums) and capped
 // at rec_cap, the records' buffer size; the grid then covers rec_cap. The block count goes to *nblocks_out for
 // k_sum_pair_blocks.
-template <int kBlocks>
-__global__ void __launch_bounds__(32 * kSumWarps) k_pair_block_sums(const double* __restrict__ pair_r2,
-                                                                    const long long* __restrict__ pair_count,
-                                                                    long long rec_cap, LJ lj,
-                                                                    double2* __restrict__ block_sums,
-                                                                    int* __restrict__ nblocks_out) {
+// The warp's part: r2_at(b, k) is record k of its block b (r_c^2 past the end, which adds 0.0); returns, in the lanes
+// below 2 kBlocks, the sum of lane & 1 (energy, virial) of block lane >> 1. term: kSumStage + kBlocks records of shared
+// memory.
+template <int kBlocks, typename Load>
+__device__ __forceinline__ double pair_block_sums(double2* term, const LJ& lj, Load r2_at) {
     constexpr int kEach = kSumStage / kBlocks;  // records of a block per step
-    __shared__ double2 s_term[kSumWarps][kSumStage + kBlocks];
-    const long long count = pair_count ? *pair_count : rec_cap;
-    const long long pairs = count < rec_cap ? count : rec_cap;
-    const int nblocks = static_cast<int>((pairs + kChunk - 1) / kChunk);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *nblocks_out = nblocks;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b0 = (blockIdx.x * kSumWarps + warp) * kBlocks;
-    if (b0 >= nblocks) return;
-    double2* term = s_term[warp];  // record k of block b at term[b (kEach + 1) + k]
-    double r2[kSumStage / 32];
+    const int lane = threadIdx.x & 31;
+    double r2[kSumStage / 32];  // record k of block b goes to term[b (kEach + 1) + k]
     auto fetch = [&](int step) {
 #pragma unroll
-        for (int q = 0; q < kSumStage / 32; ++q) {
-            const int b = q * 32 / kEach, k = q * 32 % kEach + lane;
-            const long long at = static_cast<long long>(b0 + b) * kChunk + step * kEach + k;
-            r2[q] = at < pairs ? __ldcs(pair_r2 + at) : lj.rc2;  // outside: adds 0.0
-        }
+        for (int q = 0; q < kSumStage / 32; ++q) r2[q] = r2_at(q * 32 / kEach, step * kEach + q * 32 % kEach + lane);
     };
     fetch(0);
     double sum = 0.0;
@@ -327,6 +336,27 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_pair_block_sums(const double
         if (lane < 2 * kBlocks)
             sum = add_in_order(reinterpret_cast<const double*>(term + (lane >> 1) * (kEach + 1)) + (lane & 1), 2, kEach, sum);
     }
+    return sum;
+}
+
+template <int kBlocks>
+__global__ void __launch_bounds__(32 * kSumWarps) k_pair_block_sums(const double* __restrict__ pair_r2,
+                                                                    const long long* __restrict__ pair_count,
+                                                                    long long rec_cap, LJ lj,
+                                                                    double2* __restrict__ block_sums,
+                                                                    int* __restrict__ nblocks_out) {
+    __shared__ double2 s_term[kSumWarps][kSumStage + kBlocks];
+    const long long count = pair_count ? *pair_count : rec_cap;
+    const long long pairs = count < rec_cap ? count : rec_cap;
+    const int nblocks = static_cast<int>((pairs + kChunk - 1) / kChunk);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nblocks_out = nblocks;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b0 = (blockIdx.x * kSumWarps + warp) * kBlocks;
+    if (b0 >= nblocks) return;
+    const double sum = pair_block_sums<kBlocks>(s_term[warp], lj, [&](int b, int k) {
+        const long long at = static_cast<long long>(b0 + b) * kChunk + k;
+        return at < pairs ? __ldcs(pair_r2 + at) : lj.rc2;
+    });
     const int b = b0 + (lane >> 1);
     if (lane < 2 * kBlocks && b < nblocks) reinterpret_cast<double*>(block_sums + b)[lane & 1] = sum;
 }

@@ -47,9 +47,9 @@ __device__ __forceinline__ void ascending_offsets(int c, int n, int* d) {
 }
 
 // The row of particle i by the reference's double test on every candidate, one at a time; cell c is i's, its neighbours'
-// ranges in cell_start (without cells, every particle of [begin, end) is a candidate). Entries past the capacity are counted and not written; the counts stay within it, so every
+// ranges in cell_start. Entries past the capacity are counted and not written; the counts stay within it, so every
 // reader stays in bounds, and max_count gets the longest padded row, so the host can grow `cap` and rebuild.
-__device__ __forceinline__ void build_row(const double4* __restrict__ pos, int begin, int end, const ListGeom& g, int i, int c,
+__device__ __forceinline__ void build_row(const double4* __restrict__ pos, const ListGeom& g, int i, int c,
                                           const int* __restrict__ cell_start, uint32_t* __restrict__ rows,
                                           int2* __restrict__ counts, int* __restrict__ max_count) {
     const double4 pi = pos[i];
@@ -58,49 +58,39 @@ __device__ __forceinline__ void build_row(const double4* __restrict__ pos, int b
         if (cnt < g.cap) rows[row_index(i, cnt, g.cap)] = static_cast<uint32_t>(j) | (code << kCodeShift);
         ++cnt;
     };
-    int own;
-    if (g.use_cells) {
-        const int nc = g.ncps;
-        const int cx = c / (nc * nc), cy = (c / nc) % nc, cz = c % nc;
-        for (int dx = -1; dx <= 1; ++dx) {
-            const int x = (cx + dx + nc) % nc;
-            for (int dy = -1; dy <= 1; ++dy) {
-                const int y = (cy + dy + nc) % nc;
-                for (int dz = -1; dz <= 1; ++dz) {
-                    const int cell = (x * nc + y) * nc + (cz + dz + nc) % nc;
-                    const uint32_t code = (dx + 1) * 9 + (dy + 1) * 3 + (dz + 1);
-                    const int e = cell_start[cell + 1];
-                    for (int j = cell_start[cell] > i + 1 ? cell_start[cell] : i + 1; j < e; ++j)
-                        if (within_list(pi, pos[j], g)) push(j, code);
-                }
+    const int nc = g.ncps;
+    const int cx = c / (nc * nc), cy = (c / nc) % nc, cz = c % nc;
+    for (int dx = -1; dx <= 1; ++dx) {
+        const int x = (cx + dx + nc) % nc;
+        for (int dy = -1; dy <= 1; ++dy) {
+            const int y = (cy + dy + nc) % nc;
+            for (int dz = -1; dz <= 1; ++dz) {
+                const int cell = (x * nc + y) * nc + (cz + dz + nc) % nc;
+                const uint32_t code = (dx + 1) * 9 + (dy + 1) * 3 + (dz + 1);
+                const int e = cell_start[cell + 1];
+                for (int j = cell_start[cell] > i + 1 ? cell_start[cell] : i + 1; j < e; ++j)
+                    if (within_list(pi, pos[j], g)) push(j, code);
             }
         }
-        own = cnt;
-        int ox[3], oy[3], oz[3];
-        ascending_offsets(cx, nc, ox);
-        ascending_offsets(cy, nc, oy);
-        ascending_offsets(cz, nc, oz);
-        for (int a = 0; a < 3; ++a) {
-            const int x = (cx + ox[a] + nc) % nc;
-            for (int b = 0; b < 3; ++b) {
-                const int y = (cy + oy[b] + nc) % nc;
-                for (int d = 0; d < 3; ++d) {
-                    const int cell = (x * nc + y) * nc + (cz + oz[d] + nc) % nc;
-                    const uint32_t code = (ox[a] + 1) * 9 + (oy[b] + 1) * 3 + (oz[d] + 1);
-                    const int s = cell_start[cell];
-                    const int e = cell_start[cell + 1] < i ? cell_start[cell + 1] : i;
-                    for (int j = s; j < e; ++j)
-                        if (within_list(pi, pos[j], g)) push(j, code);
-                }
+    }
+    const int own = cnt;
+    int ox[3], oy[3], oz[3];
+    ascending_offsets(cx, nc, ox);
+    ascending_offsets(cy, nc, oy);
+    ascending_offsets(cz, nc, oz);
+    for (int a = 0; a < 3; ++a) {
+        const int x = (cx + ox[a] + nc) % nc;
+        for (int b = 0; b < 3; ++b) {
+            const int y = (cy + oy[b] + nc) % nc;
+            for (int d = 0; d < 3; ++d) {
+                const int cell = (x * nc + y) * nc + (cz + oz[d] + nc) % nc;
+                const uint32_t code = (ox[a] + 1) * 9 + (oy[b] + 1) * 3 + (oz[d] + 1);
+                const int s = cell_start[cell];
+                const int e = cell_start[cell + 1] < i ? cell_start[cell + 1] : i;
+                for (int j = s; j < e; ++j)
+                    if (within_list(pi, pos[j], g)) push(j, code);
             }
         }
-    } else {
-        // Box under 3 cells per side: every particle is a candidate (src/NeighbourList.cpp:45-50)
-        for (int j = i + 1; j < end; ++j)
-            if (within_list(pi, pos[j], g)) push(j, 13u);
-        own = cnt;
-        for (int j = begin; j < i; ++j)
-            if (within_list(pi, pos[j], g)) push(j, 13u);
     }
     const int own_c = own < g.cap ? own : g.cap, all_c = cnt < g.cap ? cnt : g.cap;
     counts[i] = make_int2(own_c, all_c - own_c);
@@ -109,12 +99,53 @@ __device__ __forceinline__ void build_row(const double4* __restrict__ pos, int b
     atomicMax(max_count, padded);
 }
 
+// The row of particle i in a box under 3 cells per side, where every particle of [begin, end) is a candidate
+// (src/NeighbourList.cpp:45-50), by a warp: 32 candidates at once, the accepted placed by the ballot.
+__device__ __forceinline__ void build_row_all(const double4* __restrict__ pos, int begin, int end, const ListGeom& g, int i,
+                                              uint32_t* __restrict__ rows, int2* __restrict__ counts,
+                                              int* __restrict__ max_count) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const double4 pi = load_pos(pos + i);
+    int cnt = 0;
+    auto sweep = [&](int a, int e) {
+#pragma unroll 4
+        for (int j0 = a; j0 < e; j0 += 32) {
+            const int j = j0 + lane;
+            const double4 pj = load_pos(pos + (j < e ? j : i));
+            const bool take = j < e && within_list(pi, pj, g);
+            const unsigned m = __ballot_sync(0xffffffffu, take);
+            const int at = cnt + __popc(m & below);
+            if (take && at < g.cap) rows[row_index(i, at, g.cap)] = static_cast<uint32_t>(j) | (13u << kCodeShift);
+            cnt += __popc(m);
+        }
+    };
+    sweep(i + 1, end);
+    const int own = cnt;
+    sweep(begin, i);
+    const int own_c = own < g.cap ? own : g.cap, all_c = cnt < g.cap ? cnt : g.cap;
+    const int padded = (cnt + 7) & ~7;
+    if (cnt + lane < padded && cnt + lane < g.cap) rows[row_index(i, cnt + lane, g.cap)] = g.sentinel;
+    if (lane == 0) {
+        counts[i] = make_int2(own_c, all_c - own_c);
+        if (padded > *static_cast<volatile int*>(max_count)) atomicMax(max_count, padded);
+    }
+}
+
 // One thread per particle
 __global__ void k_nlist_build(const double4* __restrict__ pos, int n, ListGeom g, const int* __restrict__ cell_of,
                               const int* __restrict__ cell_start, uint32_t* __restrict__ rows,
                               int2* __restrict__ counts, int* __restrict__ max_count) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) build_row(pos, 0, n, g, i, g.use_cells ? cell_of[i] : 0, cell_start, rows, counts, max_count);
+    if (i < n) build_row(pos, g, i, cell_of[i], cell_start, rows, counts, max_count);
+}
+
+// One warp per particle, without cells. (A thread per particle took 155 us at N = 500.)
+__global__ void __launch_bounds__(128) k_nlist_build_all(const double4* __restrict__ pos, int n, ListGeom g,
+                                                         uint32_t* __restrict__ rows, int2* __restrict__ counts,
+                                                         int* __restrict__ max_count) {
+    const int i = static_cast<int>((blockIdx.x * 128 + threadIdx.x) >> 5);
+    if (i < n) build_row_all(pos, 0, n, g, i, rows, counts, max_count);
 }
 
 __global__ void k_own_counts(const int2* __restrict__ counts, int n, int* __restrict__ own) {
