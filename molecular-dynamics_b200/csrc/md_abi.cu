@@ -11,8 +11,8 @@
 #include "md_fp64.cuh"
 #include "md_fx32.cuh"
 #include "md_fx64.cuh"
-#include "md_graph.cuh"
 #include "md_nlist.cuh"
+#include "md_rebuild.cuh"
 #include "md_scan.cuh"
 #include "md_tiles.cuh"
 
@@ -39,6 +39,16 @@ thread_local std::vector<cudaEvent_t>* g_capture_prof = nullptr;
 thread_local size_t g_capture_prof_next = 0;  // next unused event of *g_capture_prof (created before capture)
 thread_local int* g_graph_overflow = nullptr;
 thread_local bool g_capturing = false;  // function attributes are set before a capture, not inside it
+// The step md_run is capturing: where its record goes, and the closing of its float sums when the next step's first
+// kernel is to do it
+struct StepCapture {
+    double* record = nullptr;  // pe, virial, ke
+    bool record_energy = false, record_ke = false;
+    bool defer = false, deferred = false;
+    unsigned long long* acc = nullptr;
+    FinishArgs finish{};
+};
+thread_local StepCapture* g_step = nullptr;
 std::atomic<uint64_t> g_serial{1};  // serial numbers of force fields and lists (md_run's graphs record them)
 
 md_status fail(md_status s, const std::string& msg) {
@@ -127,8 +137,7 @@ struct RunGraph {
     cudaGraphExec_t exec = nullptr;
     std::vector<cudaEvent_t> prof;  // (before, after) each force kernel, when recorded with profiling on
     int rdf_samples = 0;            // g(r) samples per launch
-    uint64_t kernels = 0;           // kernels per launch outside the rebuild bodies
-    uint64_t body_kernels = 0;      // kernels of one rebuild body
+    uint64_t kernels = 0;           // kernels per launch
 };
 
 struct md_system {
@@ -157,13 +166,16 @@ struct md_system {
     // resident grid of k_force_fp32_resident<fixed, energy> (blocks that fit on the SMs at once), 0 until known
     unsigned fp32_resident[2][2] = {{0, 0}, {0, 0}};
     unsigned fx32_resident[2] = {0, 0};  // likewise for k_force_fx32<energy>
-    // md_run's chunk graphs (md_run_graph.inl): the cache, chunk length (0: host loop), test flags, the stream
-    // the rebuild bodies are captured on, device counters ([0] rebuilds, [1] overflow), per-chunk records and
+    // md_run's chunk graphs (md_run_graph.inl): the cache, chunk length (0: host loop), test flags, device counters
+    // ([0] rebuilds, [1] overflow), the step kernel's barrier and block sums, per-chunk records and
     // Bussi draws, the snapshot a chunk restarts from, and the canonical buffer of each double-buffered array
     std::map<std::string, RunGraph> graphs;
     int graph_chunk = 64;
     int graph_flags = 0;
-    cudaStream_t body_stream = nullptr;
+    DevBuf<unsigned> step_barrier;
+    DevBuf<long long> step_sums;
+    unsigned step_resident[2] = {0, 0};  // resident grid of k_step_start<2>, <4> per shared-memory size below
+    size_t step_smem[2] = {0, 0};
     DevBuf<int> graph_state, snap_flag;
     DevBuf<double> chunk_rec, chunk_noise;
     DevBuf<double4> snap_pos, snap_ref, pos_save;
@@ -310,7 +322,7 @@ md_status sync(md_system* s) {
 }
 
 // Kinetic energy into s->scal[0] with the reference's blocked order (no host sync)
-md_status kinetic_async(md_system* s) {
+md_status kinetic_async(md_system* s, double* record = nullptr) {
     const int n = static_cast<int>(s->n);
     const int nb = (n + kChunk - 1) / kChunk;
     if (nb == 0) {
@@ -320,7 +332,7 @@ md_status kinetic_async(md_system* s) {
     MD_CUDA(s->ke_blocks.reserve(nb));
     k_kinetic_blocks<<<nb, kOrderedThreads, 0, s->stream>>>(s->vel.p, s->mass.p, n, s->ke_blocks.p);
     MD_CHECK_LAUNCH();
-    k_sum_blocks<<<1, kChainThreads, 0, s->stream>>>(s->ke_blocks.p, nb, s->scal.p + kScalKE);
+    k_sum_blocks<<<1, kChainThreads, 0, s->stream>>>(s->ke_blocks.p, nb, s->scal.p + kScalKE, record);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
@@ -767,7 +779,8 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
     if (ff->precision != MD_PREC_FP64) MD_TRY(join_energy(ff, s));
     MD_CUDA(ff->out.reserve(4));
     MD_CUDA(ff->inside_count.reserve(1));
-    MD_CUDA(cudaMemsetAsync(ff->inside_count.p, 0, sizeof(unsigned long long), s->stream));
+    // (in a graph the step's first kernel clears the count)
+    if (!g_capturing) MD_CUDA(cudaMemsetAsync(ff->inside_count.p, 0, sizeof(unsigned long long), s->stream));
     if (ff->precision == MD_PREC_FP64) {
         // Inside a CUDA graph's capture (g_capturing) the pair count of a list the graph rebuilt is known only on
         // the device (half_off[n]): the buffers were sized before the capture (graph_prepare_buffers), the record
@@ -806,7 +819,8 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
                     const TileGeom& tg = nl->tiles_geom;
                     const size_t smem = sizeof(double4) * tg.max_staged;
                     MD_CUDA(allow_smem(k_force_fp64_tile, smem));
-                    const KickArgs ka{kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt};
+                    KickArgs ka{kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt};
+                    ka.overflow = g_graph_overflow;
                     k_force_fp64_tile<<<tile_blocks(tg), kTileThreads, smem, s->stream>>>(
                         s->pos.p, n, nl->grid.start.p, nl->cell_sorted.p, tg, ff->lj, nl->rows.p, nl->cap,
                         nl->counts.p, s->force.p, ff->inside_count.p, ka, nl->half_off.p, ew, rec_cap);
@@ -830,7 +844,6 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
                 return MD_OK;
             };
             MD_TRY(choose_variant(s, nl, MD_PREC_FP64, [&](int v) { return launch(v, false, nullptr); }));
-            MD_CUDA(cudaMemsetAsync(ff->inside_count.p, 0, sizeof(unsigned long long), s->stream));
             MD_TRY(profile_mark(s));
             MD_TRY(launch(nl->variant[MD_PREC_FP64], kick_dt > 0.0, sums ? ff->pair_r2[b].p : nullptr));
             MD_TRY(profile_mark(s));
@@ -841,13 +854,11 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
                 const int eb = ff->eb_next;
                 const int grid_blocks = capturing ? static_cast<int>((rec_cap + kChunk - 1) / kChunk) : nb;
                 // the sums' pair count: on the host path the host's (passed as their record capacity); in a graph
-                // the device's, copied to a slot kept with the records (a rebuild for the next step rewrites
-                // half_off). Measured: the copy on every host step made 2000-step runs at 4M a quarter slower.
+                // the device's, copied by the step's first kernel to a slot kept with the records (a rebuild for the
+                // next step rewrites half_off)
                 const long long* count = nullptr;
                 long long sum_cap = pairs;
                 if (capturing) {
-                    k_copy_count<<<1, 1, 0, s->stream>>>(nl->half_off.p + n, ff->epairs.p + b);
-                    MD_CHECK_LAUNCH();
                     count = ff->epairs.p + b;
                     sum_cap = rec_cap;
                 }
@@ -866,7 +877,7 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
                 ff->ew_next = b ^ 1;
                 MD_CUDA(cudaStreamWaitEvent(ff->chain, ff->ev_read[b], 0));
                 MD_TRY(launch_priority(k_sum_pair_blocks, 1, kChainThreads, ff->chain, ff->side_priority, ff->eblocks[eb].p,
-                                       ff->enblocks.p + eb, ff->out.p));
+                                       ff->enblocks.p + eb, ff->out.p, g_step ? g_step->record : nullptr));
                 MD_CUDA(cudaEventRecord(ff->ev_chain[eb], ff->chain));
                 ff->chain_pending[eb] = true;
                 ff->eb_next = eb ^ 1;
@@ -904,7 +915,8 @@ md_status read_energy(md_forcefield* ff, md_system* s, double* pe, double* viria
 md_status kick_drift_async(md_system* s, md_nlist* nl, double dt, bool check_skin, bool write_frames = false) {
     const int n = static_cast<int>(s->n);
     if (n == 0) return MD_OK;
-    if (check_skin) MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
+    // (in a graph the flag is zero but between a drift and the step's first kernel)
+    if (check_skin && !g_capturing) MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
     if (write_frames) {
         const TileGeom& tg = nl->tiles_geom;
         k_kick_drift_frames<<<blocks_for(n + 1, kThreads), kThreads, 0, s->stream>>>(
@@ -1020,7 +1032,6 @@ md_status md_system_destroy(md_system* s) {
     if (s->frame_ready) cudaEventDestroy(s->frame_ready);
     if (s->host_scal) cudaFreeHost(s->host_scal);
     drop_run_graphs(s);
-    if (s->body_stream) cudaStreamDestroy(s->body_stream);
     if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -1880,7 +1891,7 @@ extern "C" md_status md_kinetic_energy_noalloc(const double* vel3, const double*
         MD_CHECK_LAUNCH();
     }
     // (sum of the .x partials, sum of the .y partials) into the result slot; .x is the kinetic energy
-    k_sum_blocks<<<1, kChainThreads, 0, st>>>(scratch, static_cast<int>(nb), result);
+    k_sum_blocks<<<1, kChainThreads, 0, st>>>(scratch, static_cast<int>(nb), result, nullptr);
     MD_CHECK_LAUNCH();
     MD_CUDA(cudaMemcpyAsync(out, result, sizeof(double), cudaMemcpyDeviceToDevice, st));
     return MD_OK;

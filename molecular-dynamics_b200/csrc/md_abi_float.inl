@@ -66,6 +66,31 @@ FixedOffsets fixed_offsets(const md_nlist* nl, const md_system* s) {
     return o;
 }
 
+// Closes a step's fixed-point sums (k_finish_float_energy). While md_run captures a step the sums are left zero for the
+// next one and the run's record is written too; a deferred closing is left to the next step's first kernel.
+md_status finish_float_async(md_forcefield* ff, md_system* s, unsigned long long* acc, bool ke_fused, double energy_unit) {
+    FinishArgs f{};
+    f.out = ff->out.p;
+    f.inside = ff->inside_count.p;
+    f.ke = ke_fused ? s->scal.p + kScalKE : nullptr;
+    f.energy_unit = energy_unit;
+    if (g_step) {
+        f.record = g_step->record;
+        f.record_energy = g_step->record_energy ? 1 : 0;
+        f.record_ke = g_step->record_ke ? 1 : 0;
+        f.clear = 1;
+        if (g_step->defer) {
+            g_step->deferred = true;
+            g_step->acc = acc;
+            g_step->finish = f;
+            return MD_OK;
+        }
+    }
+    k_finish_float_energy<<<1, 1, 0, s->stream>>>(acc, f);
+    MD_CHECK_LAUNCH();
+    return MD_OK;
+}
+
 // MD_PREC_FX64 list forces: fixed-point frames of the current positions, then the global-gather kernel (or the
 // small-box kernel under 3 cells per side); the closing kick and kinetic energy are fused as in the float modes
 // fixed_fresh: the fixed-point frames already match the positions (the previous force kernel drifted them and
@@ -76,7 +101,7 @@ md_status forces_list_fx64_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
     const bool kick = kick_dt > 0.0;
     const Fx64LJ lj = fx64_lj(ff);
     MD_CUDA(ff->fx_acc.reserve(4));
-    if (want_energy || kick) MD_CUDA(cudaMemsetAsync(ff->fx_acc.p, 0, 4 * sizeof(long long), s->stream));
+    if ((want_energy || kick) && !g_capturing) MD_CUDA(cudaMemsetAsync(ff->fx_acc.p, 0, 4 * sizeof(long long), s->stream));
     auto* acc = reinterpret_cast<unsigned long long*>(ff->fx_acc.p);
     nl->variant[MD_PREC_FX64] = 0;
     if (n > 0) {
@@ -94,7 +119,7 @@ md_status forces_list_fx64_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
             if (fuse) {  // the next step's kick and drift, new positions and fixed-point frames to spare buffers
                 MD_CUDA(s->pos2.reserve(n));
                 MD_CUDA(nl->iframes2.reserve(n));
-                MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
+                if (!g_capturing) MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
                 ka.pos_in = s->pos.p;
                 ka.pos_out = s->pos2.p;
                 ka.iframes_out = nl->iframes2.p;
@@ -133,12 +158,7 @@ md_status forces_list_fx64_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
         MD_TRY(profile_mark(s));
     }
     const bool ke_fused = kick && n > 0;
-    if (want_energy || ke_fused) {
-        k_finish_float_energy<<<1, 1, 0, s->stream>>>(acc, ff->out.p, ff->inside_count.p,
-                                                      ke_fused ? s->scal.p + kScalKE : nullptr, 1.0 / kKineticScale,
-                                                      kEnergyUnit64);
-        MD_CHECK_LAUNCH();
-    }
+    if (want_energy || ke_fused) MD_TRY(finish_float_async(ff, s, acc, ke_fused, kEnergyUnit64));
     if (fused_ke) *fused_ke = ke_fused;
     return MD_OK;
 }
@@ -199,7 +219,7 @@ md_status forces_list_fx32_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
     const Fx64LJ dlj = fx64_lj(ff);
     const FloatLJ flj = float_lj(ff);
     MD_CUDA(ff->fx_acc.reserve(4));
-    if (want_energy || kick) MD_CUDA(cudaMemsetAsync(ff->fx_acc.p, 0, 4 * sizeof(long long), s->stream));
+    if ((want_energy || kick) && !g_capturing) MD_CUDA(cudaMemsetAsync(ff->fx_acc.p, 0, 4 * sizeof(long long), s->stream));
     auto* acc = reinterpret_cast<unsigned long long*>(ff->fx_acc.p);
     nl->variant[MD_PREC_FX32] = 0;
     if (n > 0) {
@@ -218,7 +238,7 @@ md_status forces_list_fx32_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
             MD_CUDA(s->pos2.reserve(n));
             MD_CUDA(nl->iframes2.reserve(n));
             MD_CUDA(nl->frames2.reserve(static_cast<size_t>(n) + 1));
-            MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
+            if (!g_capturing) MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
             ka.pos_in = s->pos.p;
             ka.pos_out = s->pos2.p;
             ka.iframes_out = nl->iframes2.p;
@@ -260,12 +280,7 @@ md_status forces_list_fx32_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
         }
     }
     const bool ke_fused = kick && n > 0;
-    if (want_energy || ke_fused) {
-        k_finish_float_energy<<<1, 1, 0, s->stream>>>(acc, ff->out.p, ff->inside_count.p,
-                                                      ke_fused ? s->scal.p + kScalKE : nullptr, 1.0 / kKineticScale,
-                                                      kEnergyUnit64);
-        MD_CHECK_LAUNCH();
-    }
+    if (want_energy || ke_fused) MD_TRY(finish_float_async(ff, s, acc, ke_fused, kEnergyUnit64));
     if (fused_ke) *fused_ke = ke_fused;
     return MD_OK;
 }
@@ -282,7 +297,7 @@ md_status forces_list_float_async(md_forcefield* ff, md_system* s, md_nlist* nl,
     const bool kick = kick_dt > 0.0;
     const FloatLJ lj = float_lj(ff);
     MD_CUDA(ff->fx_acc.reserve(4));
-    if (want_energy || kick) MD_CUDA(cudaMemsetAsync(ff->fx_acc.p, 0, 4 * sizeof(long long), s->stream));
+    if ((want_energy || kick) && !g_capturing) MD_CUDA(cudaMemsetAsync(ff->fx_acc.p, 0, 4 * sizeof(long long), s->stream));
     auto* acc = reinterpret_cast<unsigned long long*>(ff->fx_acc.p);
     if (n > 0) {
         const unsigned g = blocks_for(n, 128);
@@ -350,14 +365,14 @@ md_status forces_list_float_async(md_forcefield* ff, md_system* s, md_nlist* nl,
             // buffer (3n doubles, idle between rebuilds) so the state is untouched
             MD_CUDA(s->vel2.reserve(3 * static_cast<size_t>(n)));
             MD_TRY(choose_variant(s, nl, ff->precision, [&](int v) { return launch(v, true, true, s->vel2.p); }));
-            if (want_energy || kick) MD_CUDA(cudaMemsetAsync(ff->fx_acc.p, 0, 4 * sizeof(long long), s->stream));
+            if ((want_energy || kick) && !g_capturing) MD_CUDA(cudaMemsetAsync(ff->fx_acc.p, 0, 4 * sizeof(long long), s->stream));
             MD_TRY(profile_mark(s));
             if (fuse_drift && kick && nl->use_tiles) {
                 // the next step's kick and drift in the same kernel: new positions and frames go to the spare
                 // buffers (the force loop reads the current ones) and are swapped in after the launch
                 MD_CUDA(s->pos2.reserve(n));
                 MD_CUDA(nl->frames2.reserve(static_cast<size_t>(n) + 1));
-                MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
+                if (!g_capturing) MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
                 drift = KickArgs{s->vel.p, s->mass.p, 0.5 * kick_dt};
                 drift.pos_in = s->pos.p;
                 drift.pos_out = s->pos2.p;
@@ -400,26 +415,22 @@ md_status forces_list_float_async(md_forcefield* ff, md_system* s, md_nlist* nl,
         }
     }
     const bool ke_fused = kick && n > 0;
-    if (want_energy || ke_fused) {
-        k_finish_float_energy<<<1, 1, 0, s->stream>>>(acc, ff->out.p, ff->inside_count.p,
-                                                      ke_fused ? s->scal.p + kScalKE : nullptr, 1.0 / kKineticScale);
-        MD_CHECK_LAUNCH();
-    }
+    if (want_energy || ke_fused) MD_TRY(finish_float_async(ff, s, acc, ke_fused, kEnergyUnit));
     if (fused_ke) *fused_ke = ke_fused;
     return MD_OK;
 }
 
 // Fixed-point kinetic energy of the current velocities into s->scal[kScalKE] (float runs)
-md_status kinetic_fixed_async(md_system* s, md_forcefield* ff) {
+md_status kinetic_fixed_async(md_system* s, md_forcefield* ff, double* record = nullptr) {
     const int n = static_cast<int>(s->n);
     MD_CUDA(ff->fx_acc.reserve(4));
     auto* acc = reinterpret_cast<unsigned long long*>(ff->fx_acc.p) + 3;
-    MD_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long), s->stream));
+    if (!g_capturing) MD_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long), s->stream));
     if (n > 0) {
         k_kinetic_fixed<<<blocks_for(n, kThreads), kThreads, 0, s->stream>>>(s->vel.p, s->mass.p, n, acc);
         MD_CHECK_LAUNCH();
     }
-    k_fixed_to_double<<<1, 1, 0, s->stream>>>(acc, 1.0 / kKineticScale, s->scal.p + kScalKE);
+    k_fixed_to_double<<<1, 1, 0, s->stream>>>(acc, 1.0 / kKineticScale, s->scal.p + kScalKE, record, g_capturing ? 1 : 0);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }

@@ -132,7 +132,7 @@ md_status adj_sum2(md_adjoint* a, const double* x, const double* y, double* out)
     const size_t smem = 4 * kChunk * sizeof(double2);
     k_adj_blocks2<<<blocks_for(nb, 4), 128, smem, a->stream>>>(x, y, a->n, a->blocks.p, nb);
     MD_CHECK_LAUNCH();
-    k_sum_blocks<<<1, kChainThreads, 0, a->stream>>>(a->blocks.p, nb, out);
+    k_sum_blocks<<<1, kChainThreads, 0, a->stream>>>(a->blocks.p, nb, out, nullptr);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
@@ -215,7 +215,7 @@ md_status adj_forward(md_adjoint* a) {
         MD_TRY(adj_sum2(a, a->u.p, a->w.p, a->scal.p + kS_UW));
         k_kinetic_blocks<<<nb, kOrderedThreads, 0, st>>>(a->vel.p, a->mass.p, a->n, a->blocks.p);
         MD_CHECK_LAUNCH();
-        k_sum_blocks<<<1, kChainThreads, 0, st>>>(a->blocks.p, nb, a->scal.p + kS_KE);
+        k_sum_blocks<<<1, kChainThreads, 0, st>>>(a->blocks.p, nb, a->scal.p + kS_KE, nullptr);
         MD_CHECK_LAUNCH();
         k_adj_record<<<1, 1, 0, st>>>(a->scal.p + kS_UW, a->scal.p + kS_KE, a->volume, k, a->U.p, a->W.p, a->KE.p,
                                       a->scal.p + kS_RUN);

@@ -488,16 +488,35 @@ __global__ void k_force_fp32_small(const double4* __restrict__ pos, int n, Box b
     if (kEnergy || kick.vel) flush_sums(e_fx, w_fx, ins, k_fx, acc);
 }
 
-// Converts the fixed-point sums to doubles: (pe, virial) in `energy_unit`s with the double-counted pairs halved
-// into out[0..1], the inside count (halved, an integer) into *inside, and, when ke_out is set, the fused kinetic
-// energy (2^-32 units) into *ke_out.
-__global__ void k_finish_float_energy(const unsigned long long* __restrict__ acc, double* __restrict__ out,
-                                      unsigned long long* __restrict__ inside, double* __restrict__ ke_out,
-                                      double kinetic_unit, double energy_unit = kEnergyUnit) {
-    out[0] = 0.5 * static_cast<double>(static_cast<long long>(acc[0])) * energy_unit;
-    out[1] = 0.5 * static_cast<double>(static_cast<long long>(acc[1])) * energy_unit;
-    *inside = acc[2] / 2;
-    if (ke_out) *ke_out = static_cast<double>(static_cast<long long>(acc[3])) * kinetic_unit;
+// Where a step's fixed-point sums go. Any pointer may be null.
+struct FinishArgs {
+    double* out;                 // (pe, virial)
+    unsigned long long* inside;  // inside-cutoff pairs
+    double* ke;                  // the fused kinetic energy
+    double* record;              // the run's record of the step: pe, virial, ke
+    int record_energy, record_ke;
+    double energy_unit;
+    int clear;                   // leave the sums zero for the next step
+};
+
+// Converts the fixed-point sums to doubles: (pe, virial) in `energy_unit`s with the double-counted pairs halved, the
+// inside count (halved, an integer), the fused kinetic energy (2^-32 units). One thread.
+__device__ __forceinline__ void finish_float_energy(unsigned long long* acc, const FinishArgs& f) {
+    const double pe = 0.5 * static_cast<double>(static_cast<long long>(acc[0])) * f.energy_unit;
+    const double w = 0.5 * static_cast<double>(static_cast<long long>(acc[1])) * f.energy_unit;
+    const double ke = static_cast<double>(static_cast<long long>(acc[3])) * (1.0 / kKineticScale);
+    f.out[0] = pe;
+    f.out[1] = w;
+    *f.inside = acc[2] / 2;
+    if (f.ke) *f.ke = ke;
+    if (f.record && f.record_energy) {
+        f.record[0] = pe;
+        f.record[1] = w;
+    }
+    if (f.record && f.record_ke) f.record[2] = ke;
+    if (f.clear) acc[0] = acc[1] = acc[2] = acc[3] = 0;
 }
+
+__global__ void k_finish_float_energy(unsigned long long* __restrict__ acc, FinishArgs f) { finish_float_energy(acc, f); }
 
 }  // namespace md

@@ -390,25 +390,19 @@ __device__ __forceinline__ void sum_blocks(const double2* __restrict__ block_sum
     if (threadIdx.x < 2) out[threadIdx.x] = sm.ordered.run[threadIdx.x];
 }
 
+// record (a run's records; may be null) gets the kinetic energy too
 __global__ void __launch_bounds__(kChainThreads) k_sum_blocks(const double2* __restrict__ block_sums, int nblocks,
-                                                              double* __restrict__ out) {
+                                                              double* __restrict__ out, double* __restrict__ record) {
     sum_blocks(block_sums, nblocks, out);
+    if (record && threadIdx.x == 0) *record = out[0];
 }
 
-// sum_blocks over the 1024-pair blocks of k_pair_block_sums, as many as it reported
+// sum_blocks over the 1024-pair blocks of k_pair_block_sums, as many as it reported; record (may be null) gets both sums
 __global__ void __launch_bounds__(kChainThreads) k_sum_pair_blocks(const double2* __restrict__ block_sums,
                                                                    const int* __restrict__ nblocks,
-                                                                   double* __restrict__ out) {
+                                                                   double* __restrict__ out, double* __restrict__ record) {
     sum_blocks(block_sums, *nblocks, out);
-}
-
-// The step's pair count into the slot its energy sums read
-__global__ void k_copy_count(const long long* __restrict__ from, long long* __restrict__ to) { *to = *from; }
-
-// In a CUDA graph's list rebuild: the new list's pair count must fit the energy records' buffer, else the graph's
-// run repeats its steps on the host path (state[1], as k_build_done reports a row overflow)
-__global__ void k_pairs_fit(const long long* __restrict__ pair_count, long long rec_cap, int* __restrict__ state) {
-    if (*pair_count > rec_cap) state[1] = 1;
+    if (record && threadIdx.x < 2) record[threadIdx.x] = out[threadIdx.x];
 }
 
 // ---- kinetic energy -----------------------------------------------------------------------------------

@@ -72,22 +72,16 @@ __device__ __forceinline__ float split_r2(const float4& qi, const float4* __rest
 constexpr int kSplitThreads = 128;
 constexpr int kSplitRing = 16;  // far entries staged per lane: at most 11 after a drain (the 8 held back and 3 of an
                                 // open quad) and 4 arriving before the next
-__global__ void __launch_bounds__(kSplitThreads) k_rows_split(const float4* __restrict__ ref_frames, int n,
-                                                              CellOffsets offs, float near2,
-                                                              const uint32_t* __restrict__ rows, int cap,
-                                                              const int2* __restrict__ counts,
-                                                              uint32_t* __restrict__ near_rows,
-                                                              uint32_t* __restrict__ far_rows, int2* __restrict__ counts_nf) {
-    __shared__ float4 s_off[32];
-    __shared__ uint32_t s_near[kSplitThreads / 32][kFx32NearCap][32];
-    __shared__ uint32_t s_far[kSplitThreads / 32][kSplitRing][32];
-    if (threadIdx.x < 32) s_off[threadIdx.x] = offs.off[threadIdx.x];
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+constexpr size_t kSplitSmem = kSplitThreads * (kFx32NearCap + kSplitRing) * sizeof(uint32_t);
+// Particle i's row (one thread); stage is kSplitSmem bytes of shared memory. False if the row was marked.
+__device__ __forceinline__ bool rows_split(uint32_t* stage, const float4* s_off, const float4* __restrict__ ref_frames, int n,
+                                           int i, float near2, const uint32_t* __restrict__ rows, int cap,
+                                           const int2* __restrict__ counts, uint32_t* __restrict__ near_rows,
+                                           uint32_t* __restrict__ far_rows, int2* __restrict__ counts_nf) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    uint32_t(*sn)[32] = s_near[w];
-    uint32_t(*sf)[32] = s_far[w];
+    uint32_t(*sn)[32] = reinterpret_cast<uint32_t(*)[32]>(stage + w * kFx32NearCap * 32);
+    uint32_t(*sf)[32] =
+        reinterpret_cast<uint32_t(*)[32]>(stage + (kSplitThreads / 32) * kFx32NearCap * 32 + w * kSplitRing * 32);
     const float4 qi = ref_frames[i];
     const int2 c = counts[i];
     const int m = c.x + c.y;
@@ -150,25 +144,36 @@ __global__ void __launch_bounds__(kSplitThreads) k_rows_split(const float4* __re
         __stcs(fq + (k >> 2) * 32, make_uint4(v[0], v[1], v[2], v[3]));
     }
     counts_nf[i] = make_int2(over ? -1 : near_len >> 3, far_padded >> 3);
+    return !over;
+}
+
+__global__ void __launch_bounds__(kSplitThreads) k_rows_split(const float4* __restrict__ ref_frames, int n,
+                                                              CellOffsets offs, float near2,
+                                                              const uint32_t* __restrict__ rows, int cap,
+                                                              const int2* __restrict__ counts,
+                                                              uint32_t* __restrict__ near_rows,
+                                                              uint32_t* __restrict__ far_rows, int2* __restrict__ counts_nf) {
+    __shared__ float4 s_off[32];
+    __shared__ uint32_t stage[kSplitSmem / sizeof(uint32_t)];
+    if (threadIdx.x < 32) s_off[threadIdx.x] = offs.off[threadIdx.x];
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) rows_split(stage, s_off, ref_frames, n, i, near2, rows, cap, counts, near_rows, far_rows, counts_nf);
 }
 
 // The rows k_rows_split marked, by the same rule: the near part is the kFx32NearCap closest near entries (of the
 // first kFx32FixNear in row order; the farthest are dropped one at a time, the later of equal ones first).
-// Grid-stride over all particles; only marked rows do work.
-__global__ void __launch_bounds__(128) k_rows_split_fix(const float4* __restrict__ ref_frames, int n, CellOffsets offs,
-                                                        float near2, const uint32_t* __restrict__ rows, int cap,
-                                                        const int2* __restrict__ counts, uint32_t* __restrict__ near_rows,
-                                                        uint32_t* __restrict__ far_rows, int2* __restrict__ counts_nf) {
+// One thread per marked row.
+__device__ __noinline__ void rows_split_fix(const float4* s_off, const float4* __restrict__ ref_frames, int n, int i,
+                                            float near2, const uint32_t* __restrict__ rows, int cap,
+                                            const int2* __restrict__ counts, uint32_t* __restrict__ near_rows,
+                                            uint32_t* __restrict__ far_rows, int2* __restrict__ counts_nf) {
     static_assert(kFx32FixNear < 64, "the kept near entries are a 64-bit mask");
-    __shared__ float4 s_off[32];
-    if (threadIdx.x < 32) s_off[threadIdx.x] = offs.off[threadIdx.x];
-    __syncthreads();
     auto entry = [&](int i, int s) {
         const uint4 q = row_quad(rows, i, s >> 2, cap);
         return (s & 3) == 0 ? q.x : (s & 3) == 1 ? q.y : (s & 3) == 2 ? q.z : q.w;
     };
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (counts_nf[i].x >= 0) continue;
+    {
         const float4 qi = ref_frames[i];
         const int2 c = counts[i];
         const int m = c.x + c.y;
@@ -223,6 +228,19 @@ __global__ void __launch_bounds__(128) k_rows_split_fix(const float4* __restrict
         const int fg = row_close(fb, nf, fq, pad);
         counts_nf[i] = make_int2(ng, fg);
     }
+}
+
+// Grid-stride over all particles; only marked rows do work.
+__global__ void __launch_bounds__(128) k_rows_split_fix(const float4* __restrict__ ref_frames, int n, CellOffsets offs,
+                                                        float near2, const uint32_t* __restrict__ rows, int cap,
+                                                        const int2* __restrict__ counts, uint32_t* __restrict__ near_rows,
+                                                        uint32_t* __restrict__ far_rows, int2* __restrict__ counts_nf) {
+    __shared__ float4 s_off[32];
+    if (threadIdx.x < 32) s_off[threadIdx.x] = offs.off[threadIdx.x];
+    __syncthreads();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        if (counts_nf[i].x < 0)
+            rows_split_fix(s_off, ref_frames, n, i, near2, rows, cap, counts, near_rows, far_rows, counts_nf);
 }
 
 // Thread per particle over its near row and then its far row on a resident grid (each thread takes particles i,

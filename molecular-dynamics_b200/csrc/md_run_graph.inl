@@ -2,10 +2,9 @@
 //
 // A run is cut into chunks of up to s->graph_chunk steps; each chunk is one CUDA graph, cached by everything it
 // records (buffer addresses, sizes, constants and the chunk's step pattern). A step in a graph is the host loop's
-// step (run_steps) with the rebuild decision moved to the device: a one-thread kernel turns the half-skin flag
-// of the last drift into the condition of an IF node whose body is the list rebuild, enqueued by the same
-// kernels as the host path (cell sort, reorder, frames, tiled build; MD_PREC_FX32's near-first rows and the
-// fixed-point frames). So a chunk needs one host synchronisation instead of one per step.
+// step (run_steps) with the rebuild decision moved to the device: the step's first kernel (k_step_start) looks at the
+// half-skin flag of the last drift and rebuilds the list itself when it is set. So a chunk needs one host
+// synchronisation instead of one per step.
 //
 // Addresses: the graph's kernels are recorded with the buffers' addresses, so inside a graph nothing may change
 // which buffer holds what. The rebuild reorders into the spare arrays and copies back (the host path swaps
@@ -13,8 +12,8 @@
 // masses, ids, float and fixed-point frames) in its canonical buffer: the fused drift alternates positions and
 // frames between the two buffers step by step, so a chunk with an odd number of fused steps ends with one copy.
 //
-// Capacity: a rebuild whose rows outgrow the capacity, or whose cells outgrow the shared-memory tile recorded in
-// the graph, sets an error flag (rows are never written out of bounds). The chunk then starts again on the host
+// Capacity: a rebuild whose rows outgrow the capacity, or (a tile force kernel) whose cells outgrow the shared-memory
+// tile recorded in the graph, sets an error flag (rows are never written out of bounds). The chunk then starts again on the host
 // path from a snapshot the graph took at its start (positions, velocities, forces, masses, ids, the list's
 // reference positions, the stale flag and the g(r) histogram): the list of the chunk's start is rebuilt from the
 // reference positions (particles already in cell order, so the reorder is the identity and the rows are the
@@ -60,16 +59,17 @@ md_status record_energy(md_forcefield* ff, md_system* s, double* rec, bool want_
     return MD_OK;
 }
 
-// MD_PREC_FP64 runs as graphs up to this many particles. Measured on the B200 (microseconds per step with energies
-// recorded, graph / host loop): 2,048: 79 / 99; 32,000: 87 / 105; 256,000: 293 / 318; 4,000,000: 3,253 / 2,410.
-// For a large list the ordered energy sums (a 1.1 ms chain at 4M) overlap the next steps on their own streams,
-// which a graph's branches did not match.
-constexpr int64_t kFp64GraphMaxParticles = 1'000'000;
+// Runs go as graphs up to this many particles. A graph saves the host's round trip a step (30 us) and pays with a rebuild
+// on one resident wave of 64-register blocks. Measured on the B200 (microseconds per step with energies recorded,
+// graph / host loop): FX32: 32,000: 39 / 67; 256,000: 122 / 150; 864,000: 363 / 379; 2,048,000: 815 / 796; 4,000,000:
+// 1,587 / 1,507. FP32FX: 864,000: 283 / 301; 2,048,000: 637 / 622. FP64, whose ordered sums overlap the next steps better
+// on their own streams: 32,000: 48 / 79; 256,000: 192 / 218; 500,000: 374 / 356; 864,000: 572 / 560.
+constexpr int64_t kFloatGraphMaxParticles = 1'200'000, kFp64GraphMaxParticles = 400'000;
 
 // Can md_run use graphs for this call? (a tiled list built for this system; the tiled build is the one the device
 // rebuild enqueues)
 bool graph_mode_ok(const md_system* s, const md_forcefield* ff, const md_nlist* nl, int64_t n_steps) {
-    const bool precision = float_precision(ff->precision) ||
+    const bool precision = (float_precision(ff->precision) && s->n <= kFloatGraphMaxParticles) ||
                            (ff->precision == MD_PREC_FP64 && s->n <= kFp64GraphMaxParticles);
     return s->graph_chunk > 0 && n_steps > 0 && s->n > 0 && precision && nlist_current(nl, s) && nl->use_cells &&
            nl->use_tiles && nl->build_pin != 0;
@@ -127,7 +127,7 @@ md_status graph_prepare_buffers(md_system* s, md_forcefield* ff, md_nlist* nl, c
     MD_CUDA(s->snap_mass.reserve(n));
     MD_CUDA(s->snap_ids.reserve(n));
     MD_CUDA(s->snap_flag.reserve(1));
-    if (!s->body_stream) MD_CUDA(cudaStreamCreateWithFlags(&s->body_stream, cudaStreamNonBlocking));
+    MD_CUDA(s->step_barrier.reserve(2));
     if (o.rdf) {
         if (o.rdf->device < 0) {
             o.rdf->device = s->device;
@@ -175,56 +175,106 @@ TileGeom graph_geometry(const md_system* s, const md_nlist* nl) {
     return g;
 }
 
-// NeighbourList::build on the device without host reads (the graph's rebuild body): the same kernels as
-// nlist_build, the reorder copied back into the system's own arrays, the result checked on the device
-md_status device_rebuild_async(md_system* s, md_forcefield* ff, md_nlist* nl, const TileGeom& tg) {
+// Shared memory and particles tested together of the step kernel's list build
+size_t step_smem(const md_nlist* nl, const md_system* s, bool few_cells, CellBuild* bp) {
+    const ListGeom geo{s->box, nl->rl2, nl->grid.ncps, 1, nl->cap, static_cast<uint32_t>(s->n) | (kSentinelCode << kCodeShift)};
+    *bp = cell_build_params(geo, static_cast<double>(s->n) / nl->grid.ncells);
+    size_t smem = cell_build_smem(bp->stage, nl->cap, kRebuildThreads / 32, few_cells ? 2 : 4);
+    if (smem > kBuildSmem) {
+        bp->stage = 0;
+        smem = 0;
+    }
+    return std::max(smem, kSplitSmem);
+}
+
+// The step's first kernel (k_step_start). prepare_only: its shared-memory opt-in and resident grid, before a capture
+md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const StepCapture* last, long long* pair_count,
+                           bool prepare_only = false) {
     const int n = static_cast<int>(s->n);
     CellGrid& g = nl->grid;
-    cudaStream_t st = s->stream;
-    k_zero_ints<<<std::min(blocks_for(g.ncells, kThreads), 148u * 8u), kThreads, 0, st>>>(g.count.p, g.ncells,
-                                                                                       g.cursor.p, g.ncells);
-    MD_CHECK_LAUNCH();
-    k_cell_assign<<<blocks_for(n, kThreads), kThreads, 0, st>>>(s->pos.p, n, g.ncps / s->box.L, g.ncps, g.cell_of.p,
-                                                                g.count.p);
-    MD_CHECK_LAUNCH();
-    exclusive_scan<int, int>(g.count.p, g.ncells, g.start.p, g.tiles.p, st);
-    MD_CHECK_SCAN();
-    k_cell_scatter<<<blocks_for(n, kThreads), kThreads, 0, st>>>(g.cell_of.p, n, g.start.p, g.cursor.p, g.bucket.p);
-    MD_CHECK_LAUNCH();
-    k_cell_rank<<<blocks_for(static_cast<long long>(g.ncells) * 32, kThreads), kThreads, 0, st>>>(
-        g.start.p, g.ncells, g.bucket.p, g.order.p);
-    MD_CHECK_LAUNCH();
-    k_permute<<<blocks_for(n, kThreads), kThreads, 0, st>>>(g.order.p, n, s->pos.p, s->vel.p, s->force.p, s->mass.p,
-                                                            s->ids.p, s->pos2.p, s->vel2.p, s->force2.p, s->mass2.p,
-                                                            s->ids2.p, g.cell_of.p, nl->cell_sorted.p, nl->ref_pos.p);
-    MD_CHECK_LAUNCH();
-    k_copy_back<<<blocks_for(n, kThreads), kThreads, 0, st>>>(n, s->pos2.p, s->vel2.p, s->force2.p, s->mass2.p,
-                                                              s->ids2.p, s->pos.p, s->vel.p, s->force.p, s->mass.p,
-                                                              s->ids.p);
-    MD_CHECK_LAUNCH();
-    const double cell = s->box.L / g.ncps;
-    k_frames<<<blocks_for(n + 1, kThreads), kThreads, 0, st>>>(s->pos.p, n, nl->cell_sorted.p, g.ncps, cell, s->box,
-                                                               nl->frames.p);
-    MD_CHECK_LAUNCH();
-    MD_TRY(cells_build_async(nl, s));
-    k_build_done<<<1, 1, 0, st>>>(nl->flags.p + 1, nl->cap, s->graph_state.p, (s->graph_flags & MD_GRAPH_TEST_RERUN) != 0);
-    MD_CHECK_LAUNCH();
-    if (ff->precision == MD_PREC_FP64) {  // the pair offsets of the energy records, and their count against the buffers
-        k_own_counts<<<blocks_for(n, kThreads), kThreads, 0, st>>>(nl->counts.p, n, nl->tmp_counts.p);
-        MD_CHECK_LAUNCH();
-        exclusive_scan<int, long long>(nl->tmp_counts.p, n, nl->half_off.p, nl->tiles.p, st);
-        MD_CHECK_SCAN();
-        const long long cap = static_cast<long long>(std::min(ff->pair_r2[0].count, ff->pair_r2[1].count));
-        k_pairs_fit<<<1, 1, 0, st>>>(nl->half_off.p + n, cap, s->graph_state.p);
-        MD_CHECK_LAUNCH();
+    const bool few = g.ncells < kWideBuildCells;
+    const int which = few ? 0 : 1;
+    RebuildArgs a{};
+    const size_t smem = step_smem(nl, s, few, &a.build);
+    auto resident = [&](auto kernel) -> md_status {
+        if (s->step_resident[which] != 0 && s->step_smem[which] == smem) return MD_OK;
+        MD_CUDA(allow_smem(kernel, smem));
+        int sms = 0, per_sm = 0;
+        MD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+        MD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kRebuildThreads, smem));
+        if (per_sm < 1) return fail(MD_ERR_CUDA, "the step kernel does not fit an SM");
+        s->step_resident[which] = static_cast<unsigned>(sms * per_sm);
+        s->step_smem[which] = smem;
+        MD_CUDA(s->step_sums.reserve(2 * static_cast<size_t>(s->step_resident[which])));
+        return MD_OK;
+    };
+    if (prepare_only) return few ? resident(k_step_start<2>) : resident(k_step_start<4>);
+    a.n = n;
+    a.ncells = g.ncells;
+    a.ncps = g.ncps;
+    a.inv_cell = g.ncps / s->box.L;
+    a.cell = s->box.L / g.ncps;
+    a.box = s->box;
+    a.pos = s->pos.p;
+    a.pos2 = s->pos2.p;
+    a.vel = s->vel.p;
+    a.vel2 = s->vel2.p;
+    a.force = s->force.p;
+    a.force2 = s->force2.p;
+    a.mass = s->mass.p;
+    a.mass2 = s->mass2.p;
+    a.ids = s->ids.p;
+    a.ids2 = s->ids2.p;
+    a.ref_pos = nl->ref_pos.p;
+    a.cell_of = g.cell_of.p;
+    a.cell_sorted = nl->cell_sorted.p;
+    a.count = g.count.p;
+    a.start = g.start.p;
+    a.slot = reinterpret_cast<int*>(g.order.p);
+    a.bucket = reinterpret_cast<int*>(g.bucket.p);
+    a.block_sums = reinterpret_cast<int*>(s->step_sums.p);
+    a.offset_sums = s->step_sums.p + s->step_resident[which];
+    a.frames = nl->frames.p;
+    a.iframes = ff->precision == MD_PREC_FX64 || ff->precision == MD_PREC_FX32 ? nl->iframes.p : nullptr;
+    a.rows = nl->rows.p;
+    a.counts = nl->counts.p;
+    a.stale = nl->flags.p;
+    a.max_count = nl->flags.p + 1;
+    a.state = s->graph_state.p;
+    a.barrier = s->step_barrier.p;
+    a.report_always = (s->graph_flags & MD_GRAPH_TEST_RERUN) != 0;
+    if (ff->precision == MD_PREC_FP64) {
+        a.half_off = nl->half_off.p;
+        a.rec_cap = static_cast<long long>(std::min(ff->pair_r2[0].count, ff->pair_r2[1].count));
+        a.pair_count = pair_count;
+        a.inside = ff->inside_count.p;
     }
-    if (ff->precision == MD_PREC_FX32)  // the rows just built, split (the float frames are the build's)
-        MD_TRY(split_rows_async(s, nl, nl->frames.p, static_cast<float>(nl->nf_near2), st));
-    if (ff->precision == MD_PREC_FX64 || ff->precision == MD_PREC_FX32) {
-        k_frames_fixed<<<blocks_for(n, kThreads), kThreads, 0, st>>>(s->pos.p, n, nl->cell_sorted.p, g.ncps, cell,
-                                                                     s->box, nl->iframes.p);
-        MD_CHECK_LAUNCH();
+    if (ff->precision == MD_PREC_FX32) {
+        a.near_rows = nl->rows_nf.p;
+        a.far_rows = nl->rows_nf.p + fx32_near_entries(n);
+        a.counts_nf = nl->counts_nf.p;
+        a.near2 = static_cast<float>(nl->nf_near2);
+        a.offs = cell_offsets(nl, s);
     }
+    if (last && last->deferred) {
+        a.acc = last->acc;
+        a.finish = last->finish;
+    }
+    cudaLaunchConfig_t cfg{};
+    // a resident grid, and no more blocks than there is work for
+    cfg.gridDim = dim3(std::min(s->step_resident[which],
+                                std::max(blocks_for(n, kRebuildThreads), static_cast<unsigned>(std::min(g.ncells, 1 << 20)))));
+    cfg.blockDim = dim3(kRebuildThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (few) MD_CUDA(cudaLaunchKernelEx(&cfg, k_step_start<2>, a));
+    else MD_CUDA(cudaLaunchKernelEx(&cfg, k_step_start<4>, a));
+    MD_CHECK_LAUNCH();
     return MD_OK;
 }
 
@@ -268,7 +318,8 @@ std::string graph_key(const md_system* s, const md_forcefield* ff, const md_nlis
                           static_cast<const void*>(ff->eblocks[1].p), static_cast<const void*>(s->ke_blocks.p),
                           static_cast<const void*>(ff->epairs.p), static_cast<const void*>(ff->enblocks.p),
                           static_cast<const void*>(nl->half_off.p), static_cast<const void*>(nl->tmp_counts.p),
-                          static_cast<const void*>(nl->tiles.p),
+                          static_cast<const void*>(nl->tiles.p), static_cast<const void*>(s->step_barrier.p),
+                          static_cast<const void*>(s->step_sums.p),
                           static_cast<const void*>(o.rdf ? o.rdf->hist.p : nullptr)})
         ptr(p);
     for (double v : {static_cast<double>(s->n), s->box.L, static_cast<double>(nl->cap), static_cast<double>(tg.kk),
@@ -290,52 +341,31 @@ std::string graph_key(const md_system* s, const md_forcefield* ff, const md_nlis
     return k;
 }
 
-// One step of a chunk, captured: run_steps' step with the rebuild in a conditional node
+// One step of a chunk, captured: run_steps' step with the rebuild decided on the device. *last carries the closing of the
+// float sums from a step to the next one's first kernel; `close` keeps it in this step (the chunk's last).
 md_status graph_step(md_system* s, md_forcefield* ff, md_nlist* nl, const md_run_options& o, const RunStep& r, int k,
-                     double dt, bool want_energy, bool want_ke, double bussi_c, cudaGraph_t graph, const TileGeom& tg,
-                     uint64_t* body_kernels) {
+                     double dt, bool want_energy, bool want_ke, double bussi_c, StepCapture* last, bool close) {
     const bool float_frames =
         ff->precision == MD_PREC_FP32FX || ff->precision == MD_PREC_FP32 || ff->precision == MD_PREC_FX32;
+    const bool fp64 = ff->precision == MD_PREC_FP64;
     if (!r.drifted_in) MD_TRY(kick_drift_async(s, nl, dt, true, float_frames));
-    cudaGraphConditionalHandle h;
-    MD_CUDA(cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault));
-    k_set_rebuild<<<1, 1, 0, s->stream>>>(h, nl->flags.p);
-    MD_CHECK_LAUNCH();
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t cg = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    MD_CUDA(cudaStreamGetCaptureInfo(s->stream, &cs, nullptr, &cg, &deps, &nd));
-    cudaGraphNodeParams p{};
-    p.type = cudaGraphNodeTypeConditional;
-    p.conditional.handle = h;
-    p.conditional.type = cudaGraphCondTypeIf;
-    p.conditional.size = 1;
-    cudaGraphNode_t node;
-    MD_CUDA(cudaGraphAddNode(&node, cg, deps, nd, &p));
-    MD_CUDA(cudaStreamUpdateCaptureDependencies(s->stream, &node, 1, cudaStreamSetCaptureDependencies));
-    {
-        cudaGraph_t body = p.conditional.phGraph_out[0];
-        const cudaStream_t main = s->stream;
-        uint64_t* saved = g_launches;
-        uint64_t count = 0;
-        g_launches = &count;
-        MD_CUDA(cudaStreamBeginCaptureToGraph(s->body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        s->stream = s->body_stream;
-        const md_status st = device_rebuild_async(s, ff, nl, tg);
-        s->stream = main;
-        g_launches = saved;
-        const cudaError_t e = cudaStreamEndCapture(s->body_stream, &body);
-        MD_TRY(st);
-        MD_CUDA(e);
-        *body_kernels = count;
-    }
-    // the frames are current after a fused drift or a rebuild body; after this step's own drift the fixed-point
+    // FP64: this step's slot of the pair count, once the sums that last read it are done
+    const int b = ff->ew_next;
+    if (fp64 && want_energy && ff->read_pending[b]) MD_CUDA(cudaStreamWaitEvent(s->stream, ff->ev_read[b], 0));
+    MD_TRY(step_start_async(s, ff, nl, last, fp64 && want_energy ? ff->epairs.p + b : nullptr));
+    StepCapture step;
+    step.record = s->chunk_rec.p + 3 * static_cast<size_t>(k);
+    step.record_energy = want_energy;
+    step.record_ke = want_ke && !fp64 && r.thermo == 0;
+    step.defer = r.fuse_out && !close;
+    // the frames are current after a fused drift or a rebuild; after this step's own drift the fixed-point
     // frames are made again (the float frames were written by the drift)
     bool fused_ke = false;
-    MD_TRY(forces_list_async(ff, s, nl, want_energy, dt, true, &fused_ke, r.fuse_out, r.drifted_in));
-    double* rec = s->chunk_rec.p + 3 * static_cast<size_t>(k);
-    MD_TRY(record_energy(ff, s, rec, want_energy));
+    g_step = &step;
+    const md_status st = forces_list_async(ff, s, nl, want_energy, dt, true, &fused_ke, r.fuse_out, r.drifted_in);
+    g_step = nullptr;
+    MD_TRY(st);
+    if (fp64 && want_energy && !ff->side_pending) MD_TRY(record_energy(ff, s, step.record, true));  // no pairs at all
     bool ke_current = fused_ke;
     if (r.thermo) {
         if (!ke_current) MD_TRY(kinetic_async(s));
@@ -351,10 +381,8 @@ md_status graph_step(md_system* s, md_forcefield* ff, md_nlist* nl, const md_run
         ke_current = false;
     }
     if (r.rdf) MD_TRY(rdf_kernel_async(o.rdf, s, nl));
-    if (want_ke) {
-        if (!ke_current) MD_TRY(ff->precision == MD_PREC_FP64 ? kinetic_async(s) : kinetic_fixed_async(s, ff));
-        MD_CUDA(cudaMemcpyAsync(rec + 2, s->scal.p + kScalKE, sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
-    }
+    if (want_ke && !ke_current) MD_TRY(fp64 ? kinetic_async(s, step.record + 2) : kinetic_fixed_async(s, ff, step.record + 2));
+    *last = step;
     return MD_OK;
 }
 
@@ -376,7 +404,7 @@ md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_ru
     // what a capture may not do: opt the tile kernels in to the recorded tile's shared memory, create the
     // profiling events (two per step)
     const size_t tile_smem = sizeof(float4) * (tg.max_staged + 1);
-    MD_TRY(cells_build_async(nl, s, true));
+    MD_TRY(step_start_async(s, ff, nl, nullptr, nullptr, true));
     MD_CUDA(allow_smem(k_force_fp32_tile<true, true>, tile_smem));
     MD_CUDA(allow_smem(k_force_fp32_tile<true, false>, tile_smem));
     MD_CUDA(allow_smem(k_force_fp32_tile<false, true>, tile_smem));
@@ -391,7 +419,7 @@ md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_ru
     cudaGraph_t graph = nullptr;
     MD_CUDA(cudaGraphCreate(&graph, 0));
     uint64_t* saved = g_launches;
-    uint64_t count = 0, body = 0;
+    uint64_t count = 0;
     g_launches = &count;
     const TileGeom host_geom = nl->tiles_geom;
     nl->tiles_geom = tg;  // the tile force kernel, if it is the one in use, records the same bound as the build
@@ -409,9 +437,17 @@ md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_ru
                 if (c != cudaSuccess) st = fail(MD_ERR_CUDA, std::string("graph snapshot: ") + cudaGetErrorString(c));
             }
         };
-        // prologue: clear the device counters and take the snapshot the host restarts from on an overflow
-        if (cudaMemsetAsync(s->graph_state.p, 0, 2 * sizeof(int), s->stream) != cudaSuccess)
-            st = fail(MD_ERR_CUDA, "graph state reset");
+        // prologue: clear what the steps leave cleared (the device counters, the step kernel's barrier, the cell counts,
+        // the float sums and, but after a fused drift, the half-skin flag) and take the snapshot the host restarts from
+        auto zero = [&](void* p, size_t bytes) {
+            if (st == MD_OK && cudaMemsetAsync(p, 0, bytes, s->stream) != cudaSuccess) st = fail(MD_ERR_CUDA, "graph reset");
+        };
+        zero(s->graph_state.p, 2 * sizeof(int));
+        zero(s->step_barrier.p, 2 * sizeof(unsigned));
+        zero(nl->grid.count.p, sizeof(int) * nl->grid.ncells);
+        zero(ff->fx_acc.p, 4 * sizeof(long long));
+        zero(nl->flags.p + 1, sizeof(int));
+        if (!steps.front().drifted_in) zero(nl->flags.p, sizeof(int));
         cp(s->snap_pos.p, s->pos.p, sizeof(double4) * N);
         cp(s->snap_vel.p, s->vel.p, sizeof(double) * 3 * N);
         cp(s->snap_force.p, s->force.p, sizeof(double) * 3 * N);
@@ -422,10 +458,10 @@ md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_ru
         bool rdf = false;
         for (const RunStep& r : steps) rdf |= r.rdf;
         if (rdf) cp(s->snap_hist.p, o.rdf->hist.p, sizeof(unsigned long long) * o.rdf->bins);
+        StepCapture last;
         for (size_t k = 0; k < steps.size() && st == MD_OK; ++k) {
-            uint64_t b = 0;
-            st = graph_step(s, ff, nl, o, steps[k], static_cast<int>(k), dt, want_energy, want_ke, bussi_c, graph, tg, &b);
-            body = b;
+            st = graph_step(s, ff, nl, o, steps[k], static_cast<int>(k), dt, want_energy, want_ke, bussi_c, &last,
+                            k + 1 == steps.size());
             rg.rdf_samples += steps[k].rdf ? 1 : 0;
         }
         // epilogue: positions and frames back into their canonical buffers
@@ -475,7 +511,6 @@ md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_ru
         return fail(MD_ERR_CUDA, std::string("md_run graph instantiate: ") + cudaGetErrorString(ei));
     }
     rg.kernels = count;
-    rg.body_kernels = body;
     auto ins = s->graphs.emplace(key, std::move(rg));
     *out = &ins.first->second;
     return MD_OK;
@@ -655,7 +690,7 @@ md_status run_steps_graph(md_system* s, md_forcefield* ff, md_nlist* nl, double 
             continue;
         }
         drifted = steps.back().fuse_out;
-        s->launches += g->kernels + g->body_kernels * static_cast<uint64_t>(state[0]);
+        s->launches += g->kernels;
         if (state[0] > 0) {  // the rebuilds the graph made, as nlist_build counts them
             rebuilt_on_device = true;
             nl->rebuilds += state[0];

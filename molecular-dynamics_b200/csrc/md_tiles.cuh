@@ -239,7 +239,10 @@ __global__ void __launch_bounds__(kTileThreads) k_force_fp64_tile(
     __shared__ int s_delta[kMaxSegment][32];
     tile_tables(g, cell_start, t);
     const int span = t.kk + 2;
-    if (t.total > g.max_staged) return;
+    if (t.total > g.max_staged) {  // the bound recorded in a graph was outgrown: the host reruns the chunk
+        if (kick.overflow && threadIdx.x == 0) *kick.overflow = 1;
+        return;
+    }
     stage_tile(pos, s_p, t);
     for (int e = threadIdx.x; e < t.kk * 32; e += blockDim.x) {
         const int h = e / 32, code = e % 32;
@@ -321,8 +324,13 @@ __global__ void k_kinetic_fixed(const double* __restrict__ vel, const double* __
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(acc, static_cast<unsigned long long>(v));
 }
 
-__global__ void k_fixed_to_double(const unsigned long long* __restrict__ acc, double unit, double* __restrict__ out) {
-    *out = static_cast<double>(static_cast<long long>(*acc)) * unit;
+// record (a run's records; may be null) gets the value too; clear leaves the sum zero for the next step
+__global__ void k_fixed_to_double(unsigned long long* __restrict__ acc, double unit, double* __restrict__ out,
+                                  double* __restrict__ record, int clear) {
+    const double v = static_cast<double>(static_cast<long long>(*acc)) * unit;
+    *out = v;
+    if (record) *record = v;
+    if (clear) *acc = 0;
 }
 
 // ---- fused drift ------------------------------------------------------------------------------------------
