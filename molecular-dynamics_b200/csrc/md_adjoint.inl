@@ -35,7 +35,8 @@ struct md_adjoint {
     std::vector<std::unique_ptr<DevBuf<double4>>> seg_pos, gen_ref;
     std::vector<std::unique_ptr<DevBuf<double>>> seg_vel;
     std::vector<int> seg_gen;
-    DevBuf<double> ar, av, wv, pe, ps, us, ws, ue, we;
+    DevBuf<double> ar, av, pe, ps, us, ws, ue, we;
+    DevBuf<double4> wv;
     double meanU = 0.0, meanP = 0.0;
     bool forwarded = false;
     int rebuilds = 0;  // list builds of the last forward pass (the first included)
@@ -107,7 +108,7 @@ md_status adj_build(md_adjoint* a, const double4* p) {
     for (int attempt = 0; attempt < 4; ++attempt) {
         MD_CUDA(a->rows.reserve(row_buffer_entries(n, a->cap)));
         MD_CUDA(cudaMemsetAsync(a->flags.p, 0, sizeof(int), st));
-        k_adj_rows<<<blocks_for(n, 128), 128, 0, st>>>(p, n, a->box, a->rl2, g.ncps, g.cell_of.p, g.start.p, g.order.p,
+        k_adj_rows<<<blocks_for(n, 4), 128, 0, st>>>(p, n, a->box, a->rl2, g.ncps, g.cell_of.p, g.start.p, g.order.p,
                                                        a->cap, a->rows.p, a->counts.p, a->flags.p);
         MD_CHECK_LAUNCH();
         MD_CUDA(cudaMemcpyAsync(a->h_flag, a->flags.p, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -120,19 +121,15 @@ md_status adj_build(md_adjoint* a, const double4* p) {
 }
 
 md_status adj_forces(md_adjoint* a) {
-    k_adj_forces<<<blocks_for(a->n, 128), 128, 0, a->stream>>>(a->pos.p, a->n, a->c, a->rows.p, a->cap, a->counts.p,
+    k_adj_forces<<<blocks_for(static_cast<long long>(a->n) * kAdjForceLanes, 128), 128, 0, a->stream>>>(a->pos.p, a->n, a->c, a->rows.p, a->cap, a->counts.p,
                                                                a->force.p, a->u.p, a->w.p);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
 
-// Blocked sums of two per-particle arrays into out[0], out[1]
-md_status adj_sum2(md_adjoint* a, const double* x, const double* y, double* out) {
-    const int nb = (a->n + kChunk - 1) / kChunk;
-    const size_t smem = 4 * kChunk * sizeof(double2);
-    k_adj_blocks2<<<blocks_for(nb, 4), 128, smem, a->stream>>>(x, y, a->n, a->blocks.p, nb);
-    MD_CHECK_LAUNCH();
-    k_sum_blocks<<<1, kChainThreads, 0, a->stream>>>(a->blocks.p, nb, out, nullptr);
+// Block sums of `pairs` pairs of per-particle arrays into a->blocks
+md_status adj_blocks(md_adjoint* a, const AdjArrays& in, int pairs) {
+    k_adj_blocks2<<<dim3((a->n + kChunk - 1) / kChunk, pairs), kChainThreads, 0, a->stream>>>(in, a->n, a->blocks.p);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
@@ -158,23 +155,25 @@ md_status adj_step(md_adjoint* a, bool* rebuilt) {
 // A backward pass at positions p with the weights in a->wv
 md_status adj_pass(md_adjoint* a, const double4* p, double aU, double aW, bool objective) {
     cudaStream_t st = a->stream;
-    k_adj_pass<<<blocks_for(a->n, 128), 128, 0, st>>>(p, a->n, a->c, a->rows.p, a->cap, a->counts.p, a->wv.p, aU, aW,
-                                                      a->ar.p, a->pe.p, a->ps.p, a->us.p, a->ws.p, a->ue.p, a->we.p);
+    auto go = [&](auto kernel, int lanes) {
+        kernel<<<blocks_for(static_cast<long long>(a->n) * lanes, 128), 128, 0, st>>>(
+            p, a->n, a->c, a->rows.p, a->cap, a->counts.p, a->wv.p, aU, aW, a->ar.p, a->pe.p, a->ps.p, a->us.p, a->ws.p,
+            a->ue.p, a->we.p);
+    };
+    if (objective) go(k_adj_pass<true>, 16);
+    else go(k_adj_pass<false>, 8);
     MD_CHECK_LAUNCH();
-    double* sums = a->scal.p + kS_PASS;
-    MD_TRY(adj_sum2(a, a->pe.p, a->ps.p, sums));
-    if (objective) {
-        MD_TRY(adj_sum2(a, a->us.p, a->ws.p, sums + 2));
-        MD_TRY(adj_sum2(a, a->ue.p, a->we.p, sums + 4));
-    }
-    k_adj_theta<<<1, 1, 0, st>>>(sums, a->eps, aU, aW, objective, a->scal.p + kS_THETA);
+    MD_TRY(adj_blocks(a, AdjArrays{{a->pe.p, a->us.p, a->ue.p}, {a->ps.p, a->ws.p, a->we.p}}, objective ? 3 : 1));
+    k_adj_theta<<<1, kChainThreads, 0, st>>>(a->blocks.p, (a->n + kChunk - 1) / kChunk, a->eps, aU, aW, objective,
+                                             a->scal.p + kS_PASS, a->scal.p + kS_THETA);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
 
-md_status adj_weights(md_adjoint* a) {
-    k_adj_weights<<<blocks_for(3ll * a->n, kThreads), kThreads, 0, a->stream>>>(a->av.p, a->mass.p, a->n, a->half_dt,
-                                                                               a->wv.p);
+// The weights of a half kick's pass into a->wv, with the term of av before it (k_adj_weights)
+md_status adj_weights(md_adjoint* a, const double* vel, const double* ar, double aK) {
+    k_adj_weights<<<blocks_for(a->n, kThreads), kThreads, 0, a->stream>>>(a->av.p, vel, ar, a->mass.p, a->n, aK, a->dt,
+                                                                         a->half_dt, a->wv.p);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
@@ -212,13 +211,11 @@ md_status adj_forward(md_adjoint* a) {
         bool rebuilt = false;
         MD_TRY(adj_step(a, &rebuilt));
         a->rebuilds += rebuilt ? 1 : 0;
-        MD_TRY(adj_sum2(a, a->u.p, a->w.p, a->scal.p + kS_UW));
-        k_kinetic_blocks<<<nb, kOrderedThreads, 0, st>>>(a->vel.p, a->mass.p, a->n, a->blocks.p);
+        MD_TRY(adj_blocks(a, AdjArrays{{a->u.p}, {a->w.p}}, 1));
+        k_kinetic_blocks<<<nb, kOrderedThreads, 0, st>>>(a->vel.p, a->mass.p, a->n, a->blocks.p + nb);
         MD_CHECK_LAUNCH();
-        k_sum_blocks<<<1, kChainThreads, 0, st>>>(a->blocks.p, nb, a->scal.p + kS_KE, nullptr);
-        MD_CHECK_LAUNCH();
-        k_adj_record<<<1, 1, 0, st>>>(a->scal.p + kS_UW, a->scal.p + kS_KE, a->volume, k, a->U.p, a->W.p, a->KE.p,
-                                      a->scal.p + kS_RUN);
+        k_adj_record<<<1, kChainThreads, 0, st>>>(a->blocks.p, a->blocks.p + nb, nb, a->scal.p + kS_UW, a->scal.p + kS_KE,
+                                                  a->volume, k, a->U.p, a->W.p, a->KE.p, a->scal.p + kS_RUN);
         MD_CHECK_LAUNCH();
     }
     double run[2];
@@ -241,7 +238,6 @@ md_status adj_backward(md_adjoint* a, double gU, double gP) {
     MD_CUDA(cudaMemsetAsync(a->av.p, 0, sizeof(double) * 3 * n, st));
     MD_CUDA(cudaMemsetAsync(a->scal.p + kS_THETA, 0, 2 * sizeof(double), st));
     const int segments = static_cast<int>((a->steps + a->every - 1) / a->every);
-    const unsigned g3 = blocks_for(3ll * a->n, kThreads);
     for (int sg = segments - 1; sg >= 0; --sg) {
         const int k0 = sg * a->every, k1 = std::min(a->steps, k0 + a->every);
         // recompute the segment from its checkpoint
@@ -281,14 +277,10 @@ md_status adj_backward(md_adjoint* a, double gU, double gP) {
         };
         for (int j = k1; j > k0; --j) {
             const int t = j - k0;
-            k_adj_obj_v<<<g3, kThreads, 0, st>>>(a->av.p, a->seg_vel[t]->p, a->mass.p, a->n, aK);
-            MD_CHECK_LAUNCH();
-            MD_TRY(adj_weights(a));
+            MD_TRY(adj_weights(a, a->seg_vel[t]->p, nullptr, aK));
             MD_TRY(ensure(a->seg_gen[t]));
             MD_TRY(adj_pass(a, a->seg_pos[t]->p, aU, aW, objective));
-            k_adj_drift_back<<<g3, kThreads, 0, st>>>(a->av.p, a->ar.p, a->n, a->dt);
-            MD_CHECK_LAUNCH();
-            MD_TRY(adj_weights(a));
+            MD_TRY(adj_weights(a, nullptr, a->ar.p, 0.0));
             MD_TRY(ensure(a->seg_gen[t - 1]));
             MD_TRY(adj_pass(a, a->seg_pos[t - 1]->p, 0.0, 0.0, false));
         }
@@ -340,12 +332,12 @@ md_status md_adjoint_create(int device, int64_t n, double box_length, const doub
     };
     const size_t N = static_cast<size_t>(n);
     chk(cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking));
-    for (auto* b : {&a->pos, &a->pos0, &a->ref}) chk(b->reserve(N));
-    for (auto* b : {&a->vel, &a->vel0, &a->force, &a->ar, &a->av, &a->wv}) chk(b->reserve(3 * N));
+    for (auto* b : {&a->pos, &a->pos0, &a->ref, &a->wv}) chk(b->reserve(N));
+    for (auto* b : {&a->vel, &a->vel0, &a->force, &a->ar, &a->av}) chk(b->reserve(3 * N));
     for (auto* b : {&a->mass, &a->u, &a->w, &a->pe, &a->ps, &a->us, &a->ws, &a->ue, &a->we}) chk(b->reserve(N));
     chk(a->counts.reserve(N));
     chk(a->flags.reserve(2));
-    chk(a->blocks.reserve((N + kChunk - 1) / kChunk));
+    chk(a->blocks.reserve(3 * ((N + kChunk - 1) / kChunk)));
     chk(a->scal.reserve(16));
     chk(cudaMallocHost(reinterpret_cast<void**>(&a->h_flag), sizeof(int)));
     if (st == MD_OK) {
@@ -354,8 +346,6 @@ md_status md_adjoint_create(int device, int64_t n, double box_length, const doub
         std::vector<double> m(N, 1.0);
         if (mass) m.assign(mass, mass + N);
         chk(cudaMemcpyAsync(a->mass.p, m.data(), sizeof(double) * N, cudaMemcpyHostToDevice, a->stream));
-        chk(cudaFuncSetAttribute(k_adj_blocks2, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(4 * kChunk * sizeof(double2))));
         chk(cudaStreamSynchronize(a->stream));
     }
     if (st != MD_OK) {
