@@ -174,8 +174,8 @@ struct md_system {
     int graph_flags = 0;
     DevBuf<unsigned> step_barrier;
     DevBuf<long long> step_sums;
-    unsigned step_resident[2] = {0, 0};  // resident grid of k_step_start<2>, <4> per shared-memory size below
-    size_t step_smem[2] = {0, 0};
+    unsigned step_resident[3] = {0, 0, 0};  // resident grids of k_step_start's kinds, for the shared memory below
+    size_t step_smem[3] = {0, 0, 0};
     DevBuf<int> graph_state, snap_flag;
     DevBuf<double> chunk_rec, chunk_noise;
     DevBuf<double4> snap_pos, snap_ref, pos_save;
@@ -491,7 +491,9 @@ md_status cells_build_async(md_nlist* nl, md_system* s, bool prepare_only = fals
         MD_CHECK_LAUNCH();
         return MD_OK;
     };
-    return g.ncells >= kWideBuildCells ? go(k_nlist_build_cells<4, 4>, 4, 4) : go(k_nlist_build_cells<8, 2>, 8, 2);
+    if (g.ncells < kWideBuildCells) return go(k_nlist_build_cells<8, 2, 16>, 8, 2);
+    return cell_round(static_cast<double>(s->n) / g.ncells) == 24 ? go(k_nlist_build_cells<4, 4, 24>, 4, 4)
+                                                                  : go(k_nlist_build_cells<4, 4, 16>, 4, 4);
 }
 
 // NeighbourList::build (src/NeighbourList.cpp:55-134) on the device. The reference builds the cell list,

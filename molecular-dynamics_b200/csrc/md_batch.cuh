@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kTile)
 
 // The list build of the stale replicas (build_cell, with slots for indices): blocks take their cells in turn, and groups
 // of particles of replicas under 3 cells per side, a warp per particle. bp.geom's box and cells per side are set per replica.
-template <int kWarps, int kHomes>
+template <int kWarps, int kHomes, int kRound>
 __global__ void __launch_bounds__(32 * kWarps)
     k_b_nlist_build(const BRep* __restrict__ reps, const int* __restrict__ stale_reps, const int* __restrict__ stale_items,
                     const int* __restrict__ work, const double4* __restrict__ pos, const float4* __restrict__ frames,
@@ -382,8 +382,8 @@ __global__ void __launch_bounds__(32 * kWarps)
         bp.geom.use_cells = d.use_cells;
         const int* st = start + d.cell_off + r;
         if (d.use_cells) {
-            build_cell<kWarps, kHomes>(t, sm_cell, frames, pos, st, item - stale_items[lo], static_cast<float>(d.cell), bp,
-                                       rows, counts, max_count);
+            build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, st, item - stale_items[lo],
+                                               static_cast<float>(d.cell), bp, rows, counts, max_count);
         } else {
             const int i0 = (item - stale_items[lo]) * kAllGroup;
             for (int i = i0 + (threadIdx.x >> 5); i < i0 + kAllGroup && i < d.n; i += kWarps)

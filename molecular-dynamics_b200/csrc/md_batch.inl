@@ -145,11 +145,12 @@ md_status b_build_async(md_batch* b, bool prepare_only) {
         bp.stage = 0;
         smem = 0;
     }
-    MD_CUDA(allow_smem(k_b_nlist_build<4, 4>, smem));
+    const auto kernel = cell_round(b->per_cell) == 24 ? k_b_nlist_build<4, 4, 24> : k_b_nlist_build<4, 4, 16>;
+    MD_CUDA(allow_smem(kernel, smem));
     if (prepare_only) return MD_OK;
     const unsigned grid = static_cast<unsigned>(std::min(b->build_items, 148 * 32));
-    k_b_nlist_build<4, 4><<<grid, 128, smem, b->stream>>>(b->reps.p, b->stale_reps.p, b->stale_items.p, b->work.p, b->pos.p,
-                                                          b->frames.p, b->start.p, bp, b->rows.p, b->counts.p, b->flags.p);
+    kernel<<<grid, 128, smem, b->stream>>>(b->reps.p, b->stale_reps.p, b->stale_items.p, b->work.p, b->pos.p, b->frames.p,
+                                           b->start.p, bp, b->rows.p, b->counts.p, b->flags.p);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }

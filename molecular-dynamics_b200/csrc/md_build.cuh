@@ -152,9 +152,18 @@ __device__ __noinline__ void cell_masks_exact(const float4* cand, const uint32_t
     }
 }
 
+// Mask words (32 candidates each) that build_cell's rows are written from at a time, for cells of per_cell particles on
+// average: 16 hold the candidates of a liquid's list of r_l = 2.8; where about that many take a second round nearly
+// empty, 24 (4 homes a warp, kernel alone, 16 / 24: N = 500,000, density 0.85, r_l = 3.2, 20 words: 438 / 406 us;
+// N = 864,000, density 0.8442, r_l = 2.8, 15 words: 545 / 560).
+inline int cell_round(double per_cell) {
+    const double words = 0.8 * kCellItems * per_cell / 32.0;
+    return words > 18.0 && words <= 24.0 ? 24 : 16;
+}
+
 // The rows of one home cell's particles, by the kWarps warps of a block; cell_start is the system's (values are particle
 // indices). `shared` is the block's dynamic shared memory (cell_build_smem).
-template <int kWarps, int kHomes>
+template <int kWarps, int kHomes, int kRound>
 __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const float4* __restrict__ frames,
                                            const double4* __restrict__ pos, const int* __restrict__ cell_start, int cell,
                                            float side, const CellBuild& bp, uint32_t* __restrict__ rows,
@@ -290,12 +299,12 @@ __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const f
         if (__any_sync(kAll, nearest <= bp.margin))
             cell_masks_exact<kHomes>(cand, entries, words, cand + home1 + h0, homes - h0, i0 + h0, pos, bp, masks);
         __syncwarp();
-        // the rows: kLanes lanes per home particle, kWords adjacent mask words a lane, 16 words (512 candidates) at a time
-        constexpr int kLanes = 32 / kHomes, kWords = 16 / kLanes;
+        // the rows: kLanes lanes per home particle, kWords adjacent mask words a lane, kRound words at a time
+        constexpr int kLanes = 32 / kHomes, kWords = kRound / kLanes;
         const int k = lane / kLanes, l = lane % kLanes, h = h0 + k;
         uint32_t* mine = row + k * pitch;
         int len = 0, own = 0;
-        for (int w0 = 0; w0 < words; w0 += 16) {
+        for (int w0 = 0; w0 < words; w0 += kRound) {
             uint32_t bits[kWords];
             int c = 0, c_own = 0;
 #pragma unroll
@@ -362,7 +371,7 @@ __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const f
 }
 
 // One home cell per block
-template <int kWarps, int kHomes>
+template <int kWarps, int kHomes, int kRound>
 __global__ void __launch_bounds__(32 * kWarps) k_nlist_build_cells(const float4* __restrict__ frames,
                                                                    const double4* __restrict__ pos,
                                                                    const int* __restrict__ cell_start, float side,
@@ -370,7 +379,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_nlist_build_cells(const float4*
                                                                    int2* __restrict__ counts, int* __restrict__ max_count) {
     extern __shared__ float4 sm_cell[];
     __shared__ CellItems t;
-    build_cell<kWarps, kHomes>(t, sm_cell, frames, pos, cell_start, blockIdx.x, side, bp, rows, counts, max_count);
+    build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, cell_start, blockIdx.x, side, bp, rows, counts, max_count);
 }
 
 }  // namespace md

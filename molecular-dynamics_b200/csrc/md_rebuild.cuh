@@ -131,7 +131,7 @@ __device__ __forceinline__ void write_prefix(int n, int part, long long before, 
     if (a < n && b == n && threadIdx.x == 0) out[n] = static_cast<Out>(before);
 }
 
-template <int kHomes>
+template <int kHomes, int kRound>
 __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_constant__ RebuildArgs a) {
     extern __shared__ float4 sm_step[];
     __shared__ union Shared {
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
         a.ids[k] = a.ids2[k];
     }
     for (int c = blockIdx.x; c < a.ncells; c += static_cast<int>(gridDim.x)) {
-        build_cell<kRebuildThreads / 32, kHomes>(sh.items, sm_step, a.frames, a.ref_pos, a.start, c,
+        build_cell<kRebuildThreads / 32, kHomes, kRound>(sh.items, sm_step, a.frames, a.ref_pos, a.start, c,
                                                  static_cast<float>(a.cell), a.build, a.rows, a.counts, a.max_count);
         __syncthreads();
     }

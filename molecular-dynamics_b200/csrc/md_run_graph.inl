@@ -193,10 +193,11 @@ md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const 
     const int n = static_cast<int>(s->n);
     CellGrid& g = nl->grid;
     const bool few = g.ncells < kWideBuildCells;
-    const int which = few ? 0 : 1;
+    const int which = few ? 0 : cell_round(static_cast<double>(n) / g.ncells) == 24 ? 2 : 1;
+    const auto kernel = which == 0 ? k_step_start<2, 16> : which == 1 ? k_step_start<4, 16> : k_step_start<4, 24>;
     RebuildArgs a{};
     const size_t smem = step_smem(nl, s, few, &a.build);
-    auto resident = [&](auto kernel) -> md_status {
+    if (prepare_only) {
         if (s->step_resident[which] != 0 && s->step_smem[which] == smem) return MD_OK;
         MD_CUDA(allow_smem(kernel, smem));
         int sms = 0, per_sm = 0;
@@ -207,8 +208,7 @@ md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const 
         s->step_smem[which] = smem;
         MD_CUDA(s->step_sums.reserve(2 * static_cast<size_t>(s->step_resident[which])));
         return MD_OK;
-    };
-    if (prepare_only) return few ? resident(k_step_start<2>) : resident(k_step_start<4>);
+    }
     a.n = n;
     a.ncells = g.ncells;
     a.ncps = g.ncps;
@@ -272,8 +272,7 @@ md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (few) MD_CUDA(cudaLaunchKernelEx(&cfg, k_step_start<2>, a));
-    else MD_CUDA(cudaLaunchKernelEx(&cfg, k_step_start<4>, a));
+    MD_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
