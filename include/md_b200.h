@@ -155,7 +155,8 @@ md_status md_nlist_update(md_nlist* nl, md_system* s, int* rebuilt);
 md_status md_nlist_info(const md_nlist* nl, uint64_t* pair_count, int* rebuild_count, int* cells_per_side,
                         int* reverse_index);
 /* Force kernel choice for one precision: -1 autotunes (the first force call of the list times every
- * available variant and keeps the fastest; MD_PREC_FP64 takes variant 2 untimed), 0 pins global gathers, 1 pins the shared-memory tile kernel (used
+ * available variant and keeps the fastest; MD_PREC_FP64, and the float modes up to 24,576 particles, take
+ * variant 2 untimed), 0 pins global gathers, 1 pins the shared-memory tile kernel (used
  * only while the list has tiles; FP64 and the float modes), 2 pins global gathers with the rows prefetched
  * (FP64: a quad of entries at a time, branch-free; float modes: a group of 8 ahead), 3 the float modes' variant 2
  * with registers capped for occupancy and 4 the same on a resident grid. MD_PREC_FX64 and MD_PREC_FX32 have one

@@ -165,7 +165,7 @@ struct md_system {
     cudaEvent_t frame_ready = nullptr;
     // resident grid of k_force_fp32_resident<fixed, energy> (blocks that fit on the SMs at once), 0 until known
     unsigned fp32_resident[2][2] = {{0, 0}, {0, 0}};
-    unsigned fx32_resident[2] = {0, 0};  // likewise for k_force_fx32<energy>
+    unsigned fx32_resident[6] = {};  // likewise for k_force_fx32<energy, 1, 4 or 8 lanes> (2 lanes index + energy)
     // md_run's chunk graphs (md_run_graph.inl): the cache, chunk length (0: host loop), test flags, device counters
     // ([0] rebuilds, [1] overflow), the step kernel's barrier and block sums, per-chunk records and
     // Bussi draws, the snapshot a chunk restarts from, and the canonical buffer of each double-buffered array
@@ -407,6 +407,7 @@ int initial_capacity(const md_nlist* nl, const md_system* s) {
 }
 
 // Defined in md_abi_float.inl
+int float_lanes(int n);
 md_status frames_async(md_system* s, md_nlist* nl);
 CellOffsets cell_offsets(const md_nlist* nl, const md_system* s);
 
@@ -638,7 +639,8 @@ md_status profile_collect(md_system* s) {
 // Autotuner of the list force kernel: with tiles available, the first force call of a list (per precision)
 // times the global-gather kernel (variant 0) and the shared-memory tile kernel (variant 1) on the current
 // state, two launches each after a warm-up, and keeps the faster. Both variants give the same bits, so the
-// choice never changes a result. md_nlist_set_force_variant pins a variant instead. FP64 always takes variant 2.
+// choice never changes a result. md_nlist_set_force_variant pins a variant instead. FP64, and the float modes
+// with few particles, take variant 2 untimed.
 template <typename Launch>
 md_status choose_variant(md_system* s, md_nlist* nl, int prec, Launch&& launch) {
     // variants available: 0 always, 1 with tiles; for FP64 2 (branch-free quads); for the float modes 2, 3
@@ -648,6 +650,11 @@ md_status choose_variant(md_system* s, md_nlist* nl, int prec, Launch&& launch) 
     if (nl->variant[prec] >= 0 && ((mask >> nl->variant[prec]) & 1u)) return MD_OK;
     if (mask == 1u) {
         nl->variant[prec] = 0;
+        return MD_OK;
+    }
+    if (prec != MD_PREC_FP64 && nl->pinned[prec] < 0 && float_lanes(static_cast<int>(s->n)) > 1) {
+        // small systems: variant 2's several threads per particle beat the other kernels' one (float_lanes)
+        nl->variant[prec] = 2;
         return MD_OK;
     }
     if (prec == MD_PREC_FP64 && nl->pinned[prec] < 0) {

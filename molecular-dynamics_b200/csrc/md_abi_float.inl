@@ -66,6 +66,12 @@ FixedOffsets fixed_offsets(const md_nlist* nl, const md_system* s) {
     return o;
 }
 
+// Threads per particle of the float modes' force kernels by the number of particles. Measured with energies, kicks and
+// drift (B200, us a launch, 1 / 4 / 8 threads): FX32: N = 2,048: 19.1 / 14.9 / 14.2; 10,976: 20.5 / 16.4 / 18.8; 23,328:
+// 21.7 / 19.3 / 24.8; 32,000: 22.3 / 24.7 / 31.2. FX64: 21.1 / 14.5 / 13.1; 22.0 / 15.8 / 16.3; 23.2 / 18.7 / 24.2;
+// 23.5 / 24.9 / 30.2. FP32FX (variant 2): 17.3 / 14.9 / 14.0; 18.1 / 16.6 / 16.9; 19.8 / 18.7 / 24.0; 20.4 / 24.5 / 29.1.
+int float_lanes(int n) { return n <= 4096 ? 8 : n <= 24576 ? 4 : 1; }
+
 // Closes a step's fixed-point sums (k_finish_float_energy). While md_run captures a step the sums are left zero for the
 // next one and the run's record is written too; a deferred closing is left to the next step's first kernel.
 md_status finish_float_async(md_forcefield* ff, md_system* s, unsigned long long* acc, bool ke_fused, double energy_unit) {
@@ -105,7 +111,6 @@ md_status forces_list_fx64_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
     auto* acc = reinterpret_cast<unsigned long long*>(ff->fx_acc.p);
     nl->variant[MD_PREC_FX64] = 0;
     if (n > 0) {
-        const unsigned g = blocks_for(n, 128);
         KickArgs ka{kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt};
         if (nl->use_cells) {
             MD_CUDA(nl->iframes.reserve(n));
@@ -134,12 +139,20 @@ md_status forces_list_fx64_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
             }
             const FixedOffsets offs = fixed_offsets(nl, s);
             MD_TRY(profile_mark(s));
-            if (want_energy)
-                k_force_fx64_rows<true><<<g, 128, 0, s->stream>>>(nl->iframes.p, s->pos.p, n, s->box, lj, offs, nl->rows.p,
-                                                                  nl->cap, nl->counts.p, s->force.p, acc, ka);
-            else
-                k_force_fx64_rows<false><<<g, 128, 0, s->stream>>>(nl->iframes.p, s->pos.p, n, s->box, lj, offs,
-                                                                   nl->rows.p, nl->cap, nl->counts.p, s->force.p, acc, ka);
+            auto go = [&](auto kernel, int lanes) {
+                kernel<<<blocks_for(static_cast<long long>(n) * lanes, 128), 128, 0, s->stream>>>(
+                    nl->iframes.p, s->pos.p, n, s->box, lj, offs, nl->rows.p, nl->cap, nl->counts.p, s->force.p, acc, ka);
+            };
+            const int lanes = float_lanes(n);
+            if (want_energy) {
+                if (lanes == 8) go(k_force_fx64_rows<true, 8>, 8);
+                else if (lanes == 4) go(k_force_fx64_rows<true, 4>, 4);
+                else go(k_force_fx64_rows<true, 1>, 1);
+            } else {
+                if (lanes == 8) go(k_force_fx64_rows<false, 8>, 8);
+                else if (lanes == 4) go(k_force_fx64_rows<false, 4>, 4);
+                else go(k_force_fx64_rows<false, 1>, 1);
+            }
             if (fuse) {
                 MD_CHECK_LAUNCH();
                 swap_buffers(s->pos, s->pos2);
@@ -148,10 +161,10 @@ md_status forces_list_fx64_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
         } else {
             MD_TRY(profile_mark(s));
             if (want_energy)
-                k_force_fx64_small<true><<<g, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p, nl->cap,
+                k_force_fx64_small<true><<<blocks_for(static_cast<long long>(n) * kSmallLanes, 128), 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p, nl->cap,
                                                                    nl->counts.p, s->force.p, acc, ka);
             else
-                k_force_fx64_small<false><<<g, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p, nl->cap,
+                k_force_fx64_small<false><<<blocks_for(static_cast<long long>(n) * kSmallLanes, 128), 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p, nl->cap,
                                                                     nl->counts.p, s->force.p, acc, ka);
         }
         MD_CHECK_LAUNCH();
@@ -254,6 +267,7 @@ md_status forces_list_fx32_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
         }
         const FixedOffsets offs = fixed_offsets(nl, s);
         const CellOffsets foffs = cell_offsets(nl, s);
+        const int lanes = float_lanes(n);
         auto go = [&](auto kernel, unsigned& grid) -> md_status {
             if (grid == 0) {
                 int sms = 0, per_sm = 0;
@@ -262,17 +276,22 @@ md_status forces_list_fx32_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
                 grid = static_cast<unsigned>(std::max(1, sms * per_sm));
             }
             MD_TRY(profile_mark(s));
-            kernel<<<std::min(blocks_for(n, 128), grid), 128, 0, s->stream>>>(
+            kernel<<<std::min(blocks_for(static_cast<long long>(n) * lanes, 128), grid), 128, 0, s->stream>>>(
                 nl->iframes.p, nl->frames.p, s->pos.p, n, s->box, dlj, flj, offs, foffs,
                 reinterpret_cast<const uint4*>(nl->rows_nf.p), static_cast<unsigned>(fx32_near_entries(n) / 4), nl->cap,
                 nl->counts_nf.p, s->force.p, acc, ka);
             MD_CHECK_LAUNCH();
             return profile_mark(s);
         };
-        if (want_energy)
-            MD_TRY(go(k_force_fx32<true>, s->fx32_resident[1]));
-        else
-            MD_TRY(go(k_force_fx32<false>, s->fx32_resident[0]));
+        if (want_energy) {
+            if (lanes == 8) MD_TRY(go(k_force_fx32<true, 8>, s->fx32_resident[5]));
+            else if (lanes == 4) MD_TRY(go(k_force_fx32<true, 4>, s->fx32_resident[3]));
+            else MD_TRY(go(k_force_fx32<true, 1>, s->fx32_resident[1]));
+        } else {
+            if (lanes == 8) MD_TRY(go(k_force_fx32<false, 8>, s->fx32_resident[4]));
+            else if (lanes == 4) MD_TRY(go(k_force_fx32<false, 4>, s->fx32_resident[2]));
+            else MD_TRY(go(k_force_fx32<false, 1>, s->fx32_resident[0]));
+        }
         if (fuse) {
             swap_buffers(s->pos, s->pos2);
             swap_buffers(nl->iframes, nl->iframes2);
@@ -317,7 +336,7 @@ md_status forces_list_float_async(md_forcefield* ff, md_system* s, md_nlist* nl,
                                                : KickArgs{with_kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt};
                 ka.overflow = g_graph_overflow;
                 auto go = [&](auto rows_kernel, auto tile_kernel, auto prefetch_kernel, auto capped_kernel,
-                              auto resident_kernel) -> md_status {
+                              auto resident_kernel, auto lanes4_kernel, auto lanes8_kernel) -> md_status {
                     if (variant == 4) {
                         unsigned& grid = s->fp32_resident[fixed ? 1 : 0][energy ? 1 : 0];
                         if (grid == 0) {
@@ -334,6 +353,12 @@ md_status forces_list_float_async(md_forcefield* ff, md_system* s, md_nlist* nl,
                         tile_kernel<<<tile_blocks(tg), kTileThreads, smem, s->stream>>>(
                             nl->frames.p, s->pos.p, n, nl->grid.start.p, nl->cell_sorted.p, tg, lj, offs, nl->rows.p,
                             nl->cap, nl->counts.p, s->force.p, acc, ka);
+                    } else if (variant == 2 && float_lanes(n) > 1) {
+                        const int lanes = float_lanes(n);
+                        auto lanes_kernel = lanes == 8 ? lanes8_kernel : lanes4_kernel;
+                        lanes_kernel<<<blocks_for(static_cast<long long>(n) * lanes, 128), 128, 0, s->stream>>>(
+                            nl->frames.p, s->pos.p, n, s->box, lj, offs, nl->rows.p, nl->cap, nl->counts.p, s->force.p, acc,
+                            ka);
                     } else if (variant == 2) {
                         prefetch_kernel<<<g, 128, 0, s->stream>>>(nl->frames.p, s->pos.p, n, s->box, lj, offs,
                                                                   nl->rows.p, nl->cap, nl->counts.p, s->force.p, acc, ka);
@@ -350,16 +375,20 @@ md_status forces_list_float_async(md_forcefield* ff, md_system* s, md_nlist* nl,
                 if (fixed)
                     return energy ? go(k_force_fp32_rows<true, true>, k_force_fp32_tile<true, true>,
                                        k_force_fp32_rows<true, true, true>, k_force_fp32_rows<true, true, true, 7>,
-                                       k_force_fp32_resident<true, true>)
+                                       k_force_fp32_resident<true, true>, k_force_fp32_lanes<true, true, 4>,
+                                       k_force_fp32_lanes<true, true, 8>)
                                   : go(k_force_fp32_rows<true, false>, k_force_fp32_tile<true, false>,
                                        k_force_fp32_rows<true, false, true>, k_force_fp32_rows<true, false, true, 7>,
-                                       k_force_fp32_resident<true, false>);
+                                       k_force_fp32_resident<true, false>, k_force_fp32_lanes<true, false, 4>,
+                                       k_force_fp32_lanes<true, false, 8>);
                 return energy ? go(k_force_fp32_rows<false, true>, k_force_fp32_tile<false, true>,
                                    k_force_fp32_rows<false, true, true>, k_force_fp32_rows<false, true, true, 7>,
-                                   k_force_fp32_resident<false, true>)
+                                   k_force_fp32_resident<false, true>, k_force_fp32_lanes<false, true, 4>,
+                                       k_force_fp32_lanes<false, true, 8>)
                               : go(k_force_fp32_rows<false, false>, k_force_fp32_tile<false, false>,
                                    k_force_fp32_rows<false, false, true>, k_force_fp32_rows<false, false, true, 7>,
-                                   k_force_fp32_resident<false, false>);
+                                   k_force_fp32_resident<false, false>, k_force_fp32_lanes<false, false, 4>,
+                                       k_force_fp32_lanes<false, false, 8>);
             };
             // tune on the kernel the steps run (energy and the fused kick), the kick writing into the reorder
             // buffer (3n doubles, idle between rebuilds) so the state is untouched
@@ -394,20 +423,21 @@ md_status forces_list_float_async(md_forcefield* ff, md_system* s, md_nlist* nl,
             MD_TRY(profile_mark(s));
         } else {
             const KickArgs ka{kick ? s->vel.p : nullptr, s->mass.p, 0.5 * kick_dt};
+            const unsigned gs = blocks_for(static_cast<long long>(n) * kSmallLanes, 128);
             MD_TRY(profile_mark(s));
             if (fixed) {
                 if (want_energy)
-                    k_force_fp32_small<true, true><<<g, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p,
+                    k_force_fp32_small<true, true, kSmallLanes><<<gs, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p,
                                                                              nl->cap, nl->counts.p, s->force.p, acc, ka);
                 else
-                    k_force_fp32_small<true, false><<<g, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p,
+                    k_force_fp32_small<true, false, kSmallLanes><<<gs, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p,
                                                                               nl->cap, nl->counts.p, s->force.p, acc, ka);
             } else {
                 if (want_energy)
-                    k_force_fp32_small<false, true><<<g, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p,
+                    k_force_fp32_small<false, true, 1><<<g, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p,
                                                                               nl->cap, nl->counts.p, s->force.p, acc, ka);
                 else
-                    k_force_fp32_small<false, false><<<g, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p,
+                    k_force_fp32_small<false, false, 1><<<g, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p,
                                                                                nl->cap, nl->counts.p, s->force.p, acc, ka);
             }
             MD_CHECK_LAUNCH();

@@ -435,8 +435,7 @@ __global__ void __launch_bounds__(kTile)
         const double f = Fp64Lanes<kLanes>::row(pos, a, d.box, lj, rows, cap, c, s_t[threadIdx.x >> 5], pair_r2, pb, end, ins);
         if (real && u < 3) finish(u, f);
     }
-    ins = __reduce_add_sync(0xffffffffu, ins);
-    if ((threadIdx.x & 31) == 0 && ins) atomicAdd(&acc[4 * r + 2], static_cast<unsigned long long>(ins));
+    count_inside(ins, &acc[4 * r + 2]);
 }
 
 // The float list forces per replica (k_force_fp32_rows and, for replicas under 3 cells per side,

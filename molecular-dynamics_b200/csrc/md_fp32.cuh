@@ -279,9 +279,61 @@ struct FloatAcc {
         }
         return kick.vel ? __double2ll_rn(dmul(dmul(dmul(0.5, kick.mass[i]), ke), kKineticScale)) : 0;
     }
+    // finish for a particle whose kLanes lanes all hold its sums (add_lanes): lane u < 3 does component u, the first lane
+    // what needs all three; the same operations on the same values. The whole warp calls; real: there is a particle.
+    template <int kLanes>
+    __device__ __forceinline__ long long finish_lanes(int i, int n, bool real, int u, double* __restrict__ force,
+                                                      const KickArgs& kick) const {
+        constexpr unsigned kAll = 0xffffffffu;
+        const bool mine = real && u < 3;
+        const size_t o = static_cast<size_t>(u) * n + i;
+        const double F = kFixed ? static_cast<double>(u == 0 ? ax : u == 1 ? ay : az) * kForceUnit
+                                : static_cast<double>(u == 0 ? fx : u == 1 ? fy : fz);
+        if (mine) force[o] = F;
+        if (!kick.vel) return 0;
+        double m = 1.0, v = 0.0, vn = 0.0;
+        if (mine) {
+            m = kick.mass[i];
+            const double dv = ddiv(dmul(kick.half_dt, F), m);
+            v = dadd(kick.vel[o], dv);
+            vn = dadd(v, dv);
+            kick.vel[o] = kick.pos_out ? vn : v;
+        }
+        const double vv = dmul(v, v);
+        const double ke = dadd(dadd(vv, __shfl_down_sync(kAll, vv, 1)), __shfl_down_sync(kAll, vv, 2));
+        if (kick.pos_out) {
+            double x = 0.0, w = 0.0, d2 = 0.0;
+            float q = 0.0f;
+            int qi = 0;
+            if (mine) {
+                const double4 p = kick.pos_in[i], r = kick.ref_pos[i];
+                w = p.w;
+                x = wrap(dadd(u == 0 ? p.x : u == 1 ? p.y : p.z, dmul(kick.dt, vn)), kick.box);
+                const double d = min_image(dsub(x, u == 0 ? r.x : u == 1 ? r.y : r.z), kick.box);
+                d2 = dmul(d, d);
+                const int c = kick.cell_sorted[i], nc = kick.ncps;
+                const int cu = u == 0 ? c / (nc * nc) : u == 1 ? (c / nc) % nc : c % nc;
+                double f = dsub(x, dmul(cu + 0.5, kick.cell));  // frame_of, fixed_frame_of
+                f = dsub(f, dmul(kick.box.L, rint(dmul(f, kick.box.invL))));
+                q = static_cast<float>(f);
+                qi = __double2int_rn(dmul(f, kFrameScale));
+            }
+            const double y = __shfl_down_sync(kAll, x, 1), z = __shfl_down_sync(kAll, x, 2);
+            const double dy2 = __shfl_down_sync(kAll, d2, 1), dz2 = __shfl_down_sync(kAll, d2, 2);
+            const float qy = __shfl_down_sync(kAll, q, 1), qz = __shfl_down_sync(kAll, q, 2);
+            const int iy = __shfl_down_sync(kAll, qi, 1), iz = __shfl_down_sync(kAll, qi, 2);
+            if (real && u == 0) {
+                kick.pos_out[i] = make_double4(x, y, z, w);
+                if (dadd(dadd(d2, dy2), dz2) > kick.max_disp2) *kick.stale = 1;
+                if (kick.frames_out) kick.frames_out[i] = make_float4(q, qy, qz, 0.0f);
+                if (kick.iframes_out) kick.iframes_out[i] = make_int4(qi, iy, iz, 0);
+            }
+        }
+        return real && u == 0 ? __double2ll_rn(dmul(dmul(dmul(0.5, m), ke), kKineticScale)) : 0;
+    }
 };
 
-// Block-level sums of the fixed-point energy, virial, inside count and kinetic energy into acc[0..3]
+// Sums of the fixed-point energy, virial, inside count and kinetic energy into acc[0..3], a warp's at a time
 __device__ __forceinline__ void flush_sums(long long e_fx, long long w_fx, unsigned long long ins, long long k_fx,
                                            unsigned long long* __restrict__ acc) {
     e_fx = warp_sum_i64(e_fx);
@@ -293,6 +345,29 @@ __device__ __forceinline__ void flush_sums(long long e_fx, long long w_fx, unsig
         if (w_fx) atomicAdd(&acc[1], static_cast<unsigned long long>(w_fx));
         if (ins) atomicAdd(&acc[2], ins);
         if (k_fx) atomicAdd(&acc[3], static_cast<unsigned long long>(k_fx));
+    }
+}
+
+// flush_sums a block's at a time, for the kernels with several threads per particle; every thread of the block calls.
+// Atomics on one address are served one after another, and one per warp and sum bounded those kernels (32,000 particles
+// by 4 threads each: 30 us a launch, 24.7 with one per block). The kernels with a thread per particle stay with
+// flush_sums: the block's sums cost FP32's 7 % at N = 500,000 (151 us a launch against 141: the compiler gives the
+// kernel 72 registers instead of 94).
+__device__ __forceinline__ void flush_block_sums(long long e_fx, long long w_fx, unsigned long long ins, long long k_fx,
+                                                 unsigned long long* __restrict__ acc) {
+    __shared__ unsigned long long s_part[32][4];
+    const int warp = threadIdx.x >> 5;
+    const long long v[4] = {warp_sum_i64(e_fx), warp_sum_i64(w_fx), static_cast<long long>(warp_sum_u64(ins)),
+                            warp_sum_i64(k_fx)};
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s_part[warp][q] = static_cast<unsigned long long>(v[q]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        unsigned long long t = 0;
+        for (unsigned w = 0; w < (blockDim.x + 31) / 32; ++w) t += s_part[w][threadIdx.x];
+        if (t) atomicAdd(&acc[threadIdx.x], t);
     }
 }
 
@@ -408,6 +483,96 @@ __device__ __forceinline__ long long fp32_row_split(int i, const float4* __restr
     return a.finish(i, n, force, kick);
 }
 
+// The integer sums of a particle's kLanes lanes added together (every lane gets the total)
+template <int kLanes, bool kFixed, bool kEnergy>
+__device__ __forceinline__ void add_lanes(FloatAcc<kFixed, kEnergy>& a) {
+#pragma unroll
+    for (int o = 1; o < kLanes; o <<= 1) {
+        a.ax += __shfl_xor_sync(0xffffffffu, a.ax, o);
+        a.ay += __shfl_xor_sync(0xffffffffu, a.ay, o);
+        a.az += __shfl_xor_sync(0xffffffffu, a.az, o);
+    }
+}
+
+// fp32_row_split's loop with kLanes threads per particle, lane u taking the groups u, u + kLanes, ...: the fixed-point
+// sums of the lanes are added as integers (FP32: the groups' float sums are handed round and added in row order by every
+// lane), so the bits are the same. For small systems, where a thread per particle leaves most of the GPU without a warp.
+template <bool kFixed, bool kEnergy, int kLanes>
+__global__ void __launch_bounds__(128) k_force_fp32_lanes(const float4* __restrict__ frames,
+                                                          const double4* __restrict__ pos, int n, Box box, FloatLJ lj,
+                                                          CellOffsets offs, const uint32_t* __restrict__ rows, int cap,
+                                                          const int2* __restrict__ counts, double* __restrict__ force,
+                                                          unsigned long long* __restrict__ acc, KickArgs kick) {
+    __shared__ __align__(16) float s_o[4][32];  // s_o[0..1]: the 32 (x, y) pairs; s_o[2]: z
+    if (threadIdx.x < 32) {
+        const float4 o = offs.off[threadIdx.x];
+        reinterpret_cast<float2*>(s_o[0])[threadIdx.x] = make_float2(o.x, o.y);
+        s_o[2][threadIdx.x] = o.z;
+    }
+    __syncthreads();
+    if (kick.frames_out && blockIdx.x == 0 && threadIdx.x == 0)
+        kick.frames_out[n] = make_float4(kSentinelCoord, kSentinelCoord, kSentinelCoord, 0.0f);
+    const float2* s_xy = reinterpret_cast<const float2*>(s_o[0]);
+    const float* s_z = s_o[2];
+    const int u = threadIdx.x % kLanes, i = static_cast<int>((blockIdx.x * 128 + threadIdx.x) / kLanes);
+    const bool real = i < n;
+    const int at = real ? i : 0;
+    const float4 qi = frames[at];
+    const int2 c = real ? counts[at] : make_int2(0, 0);
+    const int groups = (c.x + c.y + 7) >> 3;
+    int rounds = (groups + kLanes - 1) / kLanes;  // of the warp's longest row (FP32 hands its sums round)
+    if (!kFixed) rounds = __reduce_max_sync(0xffffffffu, rounds);
+    FloatAcc<kFixed, kEnergy> a;
+    long long e_fx = 0, w_fx = 0, k_fx = 0;
+    unsigned ins = 0;
+    const uint4* rq = reinterpret_cast<const uint4*>(rows) + static_cast<size_t>(at >> 5) * (cap >> 2) * 32 + (at & 31) + 64 * u;
+    uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0;
+    if (u < groups) {
+        n0 = __ldcs(rq);
+        n1 = __ldcs(rq + 32);
+    }
+    for (int r = 0; r < rounds; ++r) {
+        const int g = r * kLanes + u;
+        const uint4 e0 = n0, e1 = n1;
+        rq += 64 * kLanes;
+        if (g + kLanes < groups) {
+            n0 = __ldcs(rq);
+            n1 = __ldcs(rq + 32);
+        }
+        GroupSums gs;
+        if (g < groups) {
+            gs = float_group<kEnergy>(
+                e0, e1, lj,
+                [=](uint32_t e, float& dx, float& dy, float& dz) {
+                    const uint32_t k = e >> kCodeShift;
+                    const float2 oxy = s_xy[k];
+                    return float_separation(qi, frames[e & kIndexMask], make_float4(oxy.x, oxy.y, s_z[k], 0.0f), dx, dy,
+                                            dz);
+                },
+                [=](uint32_t e) { return exact_inside(pos[at], pos[e & kIndexMask], box, lj.rc2d); }, ins);
+            if (kFixed) a.add_group(gs.x, gs.y, gs.z, gs.e, gs.w, e_fx, w_fx);
+        }
+        if (!kFixed) {
+            long long e = 0, w = 0;
+#pragma unroll
+            for (int t = 0; t < kLanes; ++t) {  // (a group that is not there adds zeros, which change no sum)
+                a.fx = __fadd_rn(a.fx, __shfl_sync(0xffffffffu, gs.x, t, kLanes));
+                a.fy = __fadd_rn(a.fy, __shfl_sync(0xffffffffu, gs.y, t, kLanes));
+                a.fz = __fadd_rn(a.fz, __shfl_sync(0xffffffffu, gs.z, t, kLanes));
+            }
+            if (kEnergy) {
+                e = __float2ll_rn(gs.e * kEnergyScale);
+                w = __float2ll_rn(gs.w * kEnergyScale);
+            }
+            e_fx += e;
+            w_fx += w;
+        }
+    }
+    if (kFixed) add_lanes<kLanes>(a);
+    k_fx = a.template finish_lanes<kLanes>(i, n, real, u, force, kick);
+    if (kEnergy || kick.vel) flush_block_sums(e_fx, w_fx, ins, k_fx, acc);
+}
+
 // Variant 4: fp32_row_split on a resident grid (as many blocks as fit on the SMs at once, each thread taking
 // particles i, i + grid, ...: no block turnover, no partial last wave, one flush of the sums per thread).
 template <bool kFixed, bool kEnergy>
@@ -457,19 +622,23 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_force_fp32_rows(const float
 // Boxes under 3 cells per side (all-pairs candidates): separations come from the double positions with the
 // reference's minimum image, then narrow to float (the reference's mixed path does the same,
 // src/Forcefield.cpp:373-386); the cutoff test uses the double r^2.
-template <bool kFixed, bool kEnergy>
+// kLanes threads per particle (fixed point), lane u taking the groups u, u + kLanes, ...: these boxes hold few particles
+// (N = 500: 42 us a launch by one thread each).
+constexpr int kSmallLanes = 8;
+template <bool kFixed, bool kEnergy, int kLanes>
 __global__ void k_force_fp32_small(const double4* __restrict__ pos, int n, Box box, FloatLJ lj,
                                    const uint32_t* __restrict__ rows, int cap, const int2* __restrict__ counts,
                                    double* __restrict__ force, unsigned long long* __restrict__ acc, KickArgs kick) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    static_assert(kFixed || kLanes == 1, "float accumulation keeps one thread per particle");
+    const int u = threadIdx.x % kLanes, i = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
     long long e_fx = 0, w_fx = 0, k_fx = 0;
     unsigned ins = 0;
+    FloatAcc<kFixed, kEnergy> a;
     if (i < n) {
         const double4 pi = pos[i];
         const int2 c = counts[i];
         const int m = c.x + c.y;
-        FloatAcc<kFixed, kEnergy> a;
-        for (int g0 = 0; g0 < m; g0 += 8) {
+        for (int g0 = 8 * u; g0 < m; g0 += 8 * kLanes) {
             float gx = 0.f, gy = 0.f, gz = 0.f, ge = 0.f, gw = 0.f;
             for (int s = g0; s < g0 + 8 && s < m; ++s) {
                 const double4 pj = pos[rows[row_index(i, s, cap)] & kIndexMask];
@@ -483,9 +652,14 @@ __global__ void k_force_fp32_small(const double4* __restrict__ pos, int n, Box b
             }
             a.add_group(gx, gy, gz, ge, gw, e_fx, w_fx);
         }
+    }
+    if constexpr (kLanes > 1) {
+        add_lanes<kLanes>(a);
+        k_fx = a.template finish_lanes<kLanes>(i, n, i < n, u, force, kick);
+    } else if (i < n) {
         k_fx = a.finish(i, n, force, kick);
     }
-    if (kEnergy || kick.vel) flush_sums(e_fx, w_fx, ins, k_fx, acc);
+    if (kEnergy || kick.vel) flush_block_sums(e_fx, w_fx, ins, k_fx, acc);
 }
 
 // Where a step's fixed-point sums go. Any pointer may be null.

@@ -22,6 +22,19 @@ constexpr int kChainValues = 8;  // values per thread of a one-block ordered sum
 // call (the same operations on the same r^2, so the same bits). Records past rec_cap, the buffer's size in records, are
 // dropped: only a list rebuilt inside a CUDA graph can outgrow the buffer, and the graph's run then reports the overflow
 // and repeats its steps on the host path.
+// A block's inside-cutoff pairs into *inside by one atomic (every thread calls)
+__device__ __forceinline__ void count_inside(unsigned ins, unsigned long long* __restrict__ inside) {
+    __shared__ unsigned s_ins[32];
+    ins = __reduce_add_sync(0xffffffffu, ins);
+    if ((threadIdx.x & 31) == 0) s_ins[threadIdx.x >> 5] = ins;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long t = 0;
+        for (unsigned w = 0; w < (blockDim.x + 31) / 32; ++w) t += s_ins[w];
+        if (t) atomicAdd(inside, t);
+    }
+}
+
 __global__ void k_force_fp64(const double4* __restrict__ pos, int n, Box box, LJ lj, const uint32_t* __restrict__ rows,
                              int cap, const int2* __restrict__ counts, double* __restrict__ force,
                              unsigned long long* __restrict__ inside, double* __restrict__ kick_vel,
@@ -176,8 +189,7 @@ __global__ void __launch_bounds__(128) k_force_fp64_quads(const double4* __restr
             if (kick_vel) kick_vel[o] = dadd(kick_vel[o], ddiv(dmul(half_dt, F[k]), mass[i]));
         }
     }
-    const unsigned total = __reduce_add_sync(0xffffffffu, ins);
-    if ((threadIdx.x & 31) == 0 && total) atomicAdd(inside, static_cast<unsigned long long>(total));
+    count_inside(ins, inside);
 }
 
 // The sums of k_force_fp64_quads with kLanes threads per particle: the lanes evaluate kLanes row entries at once and
@@ -265,8 +277,7 @@ __global__ void __launch_bounds__(128) k_force_fp64_lanes(const double4* __restr
         force[o] = f;
         if (kick_vel) kick_vel[o] = dadd(kick_vel[o], ddiv(dmul(half_dt, f), mass[i]));
     }
-    ins = __reduce_add_sync(0xffffffffu, ins);
-    if ((threadIdx.x & 31) == 0 && ins) atomicAdd(inside, static_cast<unsigned long long>(ins));
+    count_inside(ins, inside);
 }
 
 // Adds x[0], x[stride], ... x[(m - 1) stride] to s one after another. One thread's chain, bound by the latency of an

@@ -247,8 +247,9 @@ __global__ void __launch_bounds__(128) k_rows_split_fix(const float4* __restrict
 // i + grid, ...): the near groups in double on the fixed-point frames (fx64_group, MD_PREC_FX64's sequence), the
 // far groups in float on the float frames (float_group, MD_PREC_FP32FX's sequence); row quads prefetched a group
 // ahead with streaming loads; the fused closing kick, kinetic energy and, with kick.pos_out, the next step's kick
-// and drift writing both kinds of frames, as in the other float modes.
-template <bool kEnergy>
+// and drift writing both kinds of frames, as in the other float modes. With kLanes > 1 threads per particle, lane u takes
+// the groups u, u + kLanes, ... and the lanes' fixed-point sums are added as integers (small systems).
+template <bool kEnergy, int kLanes>
 __global__ void __launch_bounds__(128, 5) k_force_fx32(const int4* __restrict__ iframes, const float4* __restrict__ frames,
                                                     const double4* __restrict__ pos, int n, Box box, Fx64LJ dlj,
                                                     FloatLJ flj, FixedOffsets ioffs, CellOffsets foffs,
@@ -275,24 +276,30 @@ __global__ void __launch_bounds__(128, 5) k_force_fx32(const int4* __restrict__ 
     const float* s_fz = s_fo[2];
     long long e_fx = 0, w_fx = 0, k_fx = 0;
     unsigned ins = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int4 qi = iframes[i];
-        const float4 fi = frames[i];
-        const int2 c = counts[i];
+    const int u = threadIdx.x % kLanes, step = gridDim.x * blockDim.x / kLanes;
+    // (a warp's lanes go on together, those past the end without a row)
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes; i - static_cast<int>(threadIdx.x & 31) / kLanes < n; i += step) {
+        if (kLanes == 1 && i >= n) break;
+        const int at = kLanes == 1 || i < n ? i : 0;
+        const int4 qi = iframes[at];
+        const float4 fi = frames[at];
+        const int2 c = kLanes == 1 || i < n ? counts[at] : make_int2(0, 0);
         const int near_groups = c.x, groups = c.x + c.y;
         FloatAcc<true, kEnergy> a;
         // quad indices into rows_q: the near rows first, the far rows from far_q0 (interleaved layouts)
-        const unsigned far_q = far_q0 + static_cast<unsigned>(i >> 5) * (cap >> 2) * 32 + (i & 31);
-        unsigned rq = near_groups > 0 ? static_cast<unsigned>(i >> 5) * (kFx32NearCap >> 2) * 32 + (i & 31) : far_q;
+        const unsigned far_q = far_q0 + static_cast<unsigned>(at >> 5) * (cap >> 2) * 32 + (at & 31);
+        const unsigned near_q = static_cast<unsigned>(at >> 5) * (kFx32NearCap >> 2) * 32 + (at & 31);
+        unsigned rq = u < near_groups ? near_q + 64 * u : far_q + 64 * (u - near_groups);
         uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0;
-        if (groups > 0) {
+        if (u < groups) {
             n0 = __ldcs(rows_q + rq);
             n1 = __ldcs(rows_q + rq + 32);
         }
-        for (int g = 0; g < groups; ++g) {
+        for (int g = u; g < groups; g += kLanes) {
             const uint4 e0 = n0, e1 = n1;
-            rq = g + 1 == near_groups ? far_q : rq + 64;
-            if (g + 1 < groups) {
+            if (kLanes == 1) rq = g + 1 == near_groups ? far_q : rq + 64;
+            else rq = g + kLanes < near_groups ? rq + 64 * kLanes : far_q + 64 * (g + kLanes - near_groups);
+            if (g + kLanes < groups) {
                 n0 = __ldcs(rows_q + rq);
                 n1 = __ldcs(rows_q + rq + 32);
             }
@@ -300,8 +307,8 @@ __global__ void __launch_bounds__(128, 5) k_force_fx32(const int4* __restrict__ 
                 unsigned gin = 0;
                 bool shell = false;
                 DoubleGroupSums gs =
-                    fx64_group<kEnergy, false>(e0, e1, qi, iframes, s_ixy, s_iz, pos, i, box, dlj, gin, &shell);
-                if (shell) gs = fx64_group_exact<kEnergy>(e0, e1, qi, iframes, s_ixy, s_iz, pos, i, box, dlj, &gin);
+                    fx64_group<kEnergy, false>(e0, e1, qi, iframes, s_ixy, s_iz, pos, at, box, dlj, gin, &shell);
+                if (shell) gs = fx64_group_exact<kEnergy>(e0, e1, qi, iframes, s_ixy, s_iz, pos, at, box, dlj, &gin);
                 ins += gin;
                 a.add_group(gs.x, gs.y, gs.z, gs.e, gs.w, e_fx, w_fx);
             } else {
@@ -313,13 +320,21 @@ __global__ void __launch_bounds__(128, 5) k_force_fx32(const int4* __restrict__ 
                         return float_separation(fi, frames[e & kIndexMask], make_float4(oxy.x, oxy.y, s_fz[k], 0.0f),
                                                 dx, dy, dz);
                     },
-                    [=](uint32_t e) { return exact_inside(pos[i], pos[e & kIndexMask], box, flj.rc2d); }, ins);
+                    [=](uint32_t e) { return exact_inside(pos[at], pos[e & kIndexMask], box, flj.rc2d); }, ins);
                 a.add_group_fine(gs.x, gs.y, gs.z, gs.e, gs.w, e_fx, w_fx);
             }
         }
-        k_fx += a.finish(i, n, force, kick);
+        if constexpr (kLanes > 1) {
+            add_lanes<kLanes>(a);
+            k_fx += a.template finish_lanes<kLanes>(i, n, i < n, u, force, kick);
+        } else {
+            k_fx += a.finish(i, n, force, kick);
+        }
     }
-    if (kEnergy || kick.vel) flush_sums(e_fx, w_fx, ins, k_fx, acc);
+    if (kEnergy || kick.vel) {
+        if constexpr (kLanes > 1) flush_block_sums(e_fx, w_fx, ins, k_fx, acc);
+        else flush_sums(e_fx, w_fx, ins, k_fx, acc);
+    }
 }
 
 }  // namespace md

@@ -139,8 +139,9 @@ __device__ __noinline__ DoubleGroupSums fx64_group_exact(const uint4 e0, const u
 
 // Thread per particle over its row (the layout of k_force_fp32_rows) with the next group's row quads prefetched
 // (streaming loads), frames gathered from global memory; groups run branch-free, a group with a pair in the
-// cutoff shell runs again out of line with the exact test.
-template <bool kEnergy>
+// cutoff shell runs again out of line with the exact test. With kLanes > 1 threads per particle, lane u takes the groups
+// u, u + kLanes, ... and the lanes' fixed-point sums are added as integers (small systems, as k_force_fp32_lanes).
+template <bool kEnergy, int kLanes>
 __global__ void __launch_bounds__(128) k_force_fx64_rows(const int4* __restrict__ frames, const double4* __restrict__ pos,
                                                          int n, Box box, Fx64LJ lj, FixedOffsets offs,
                                                          const uint32_t* __restrict__ rows, int cap,
@@ -158,24 +159,24 @@ __global__ void __launch_bounds__(128) k_force_fx64_rows(const int4* __restrict_
     __syncthreads();
     const int2* s_xy = reinterpret_cast<const int2*>(s_o[0]);
     const int* s_z = s_o[2];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int u = threadIdx.x % kLanes, i = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
     long long e_fx = 0, w_fx = 0, k_fx = 0;
     unsigned ins = 0;
+    FloatAcc<true, kEnergy> a;
     if (i < n) {
         const int4 qi = frames[i];
         const int2 c = counts[i];
         const int groups = (c.x + c.y + 7) >> 3;
-        FloatAcc<true, kEnergy> a;
-        const uint4* rq = reinterpret_cast<const uint4*>(rows) + static_cast<size_t>(i >> 5) * (cap >> 2) * 32 + (i & 31);
+        const uint4* rq = reinterpret_cast<const uint4*>(rows) + static_cast<size_t>(i >> 5) * (cap >> 2) * 32 + (i & 31) + 64 * u;
         uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0;
-        if (groups > 0) {
+        if (u < groups) {
             n0 = __ldcs(rq);
             n1 = __ldcs(rq + 32);
         }
-        for (int g = 0; g < groups; ++g) {
+        for (int g = u; g < groups; g += kLanes) {
             const uint4 e0 = n0, e1 = n1;
-            rq += 64;
-            if (g + 1 < groups) {
+            rq += 64 * kLanes;
+            if (g + kLanes < groups) {
                 n0 = __ldcs(rq);
                 n1 = __ldcs(rq + 32);
             }
@@ -186,26 +187,35 @@ __global__ void __launch_bounds__(128) k_force_fx64_rows(const int4* __restrict_
             ins += gin;
             a.add_group(gs.x, gs.y, gs.z, gs.e, gs.w, e_fx, w_fx);
         }
+    }
+    if constexpr (kLanes > 1) {
+        add_lanes<kLanes>(a);
+        k_fx = a.template finish_lanes<kLanes>(i, n, i < n, u, force, kick);
+    } else if (i < n) {
         k_fx = a.finish(i, n, force, kick);
     }
-    if (kEnergy || kick.vel) flush_sums(e_fx, w_fx, ins, k_fx, acc);
+    if (kEnergy || kick.vel) {
+        if constexpr (kLanes > 1) flush_block_sums(e_fx, w_fx, ins, k_fx, acc);
+        else flush_sums(e_fx, w_fx, ins, k_fx, acc);
+    }
 }
 
 // Boxes under 3 cells per side: separations from the double positions with the reference's minimum image
 // (as k_force_fp32_small), the same double pair terms and fixed-point sums
+// by kSmallLanes threads per particle
 template <bool kEnergy>
 __global__ void k_force_fx64_small(const double4* __restrict__ pos, int n, Box box, Fx64LJ lj,
                                    const uint32_t* __restrict__ rows, int cap, const int2* __restrict__ counts,
                                    double* __restrict__ force, unsigned long long* __restrict__ acc, KickArgs kick) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    long long e_fx = 0, w_fx = 0, k_fx = 0;
+    const int u = threadIdx.x % kSmallLanes, i = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) / kSmallLanes);
+    long long e_fx = 0, w_fx = 0;
     unsigned ins = 0;
+    FloatAcc<true, kEnergy> a;
     if (i < n) {
         const double4 pi = pos[i];
         const int2 c = counts[i];
         const int m = c.x + c.y;
-        FloatAcc<true, kEnergy> a;
-        for (int g0 = 0; g0 < m; g0 += 8) {
+        for (int g0 = 8 * u; g0 < m; g0 += 8 * kSmallLanes) {
             double gx = 0.0, gy = 0.0, gz = 0.0, ge = 0.0, gw = 0.0;
             for (int s = g0; s < g0 + 8 && s < m; ++s) {
                 const double4 pj = pos[rows[row_index(i, s, cap)] & kIndexMask];
@@ -217,9 +227,10 @@ __global__ void k_force_fx64_small(const double4* __restrict__ pos, int n, Box b
             }
             a.add_group(gx, gy, gz, ge, gw, e_fx, w_fx);
         }
-        k_fx = a.finish(i, n, force, kick);
     }
-    if (kEnergy || kick.vel) flush_sums(e_fx, w_fx, ins, k_fx, acc);
+    add_lanes<kSmallLanes>(a);
+    const long long k_fx = a.template finish_lanes<kSmallLanes>(i, n, i < n, u, force, kick);
+    if (kEnergy || kick.vel) flush_block_sums(e_fx, w_fx, ins, k_fx, acc);
 }
 
 }  // namespace md

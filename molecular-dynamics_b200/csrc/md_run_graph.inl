@@ -162,8 +162,12 @@ md_status graph_prepare_buffers(md_system* s, md_forcefield* ff, md_nlist* nl, c
     MD_TRY(grid(k_force_fp32_resident<false, true>, s->fp32_resident[0][1]));
     MD_TRY(grid(k_force_fp32_resident<true, false>, s->fp32_resident[1][0]));
     MD_TRY(grid(k_force_fp32_resident<true, true>, s->fp32_resident[1][1]));
-    MD_TRY(grid(k_force_fx32<false>, s->fx32_resident[0]));
-    MD_TRY(grid(k_force_fx32<true>, s->fx32_resident[1]));
+    MD_TRY(grid(k_force_fx32<false, 1>, s->fx32_resident[0]));
+    MD_TRY(grid(k_force_fx32<true, 1>, s->fx32_resident[1]));
+    MD_TRY(grid(k_force_fx32<false, 4>, s->fx32_resident[2]));
+    MD_TRY(grid(k_force_fx32<true, 4>, s->fx32_resident[3]));
+    MD_TRY(grid(k_force_fx32<false, 8>, s->fx32_resident[4]));
+    MD_TRY(grid(k_force_fx32<true, 8>, s->fx32_resident[5]));
     return MD_OK;
 }
 
