@@ -575,11 +575,13 @@ __global__ void k_b_finish_float(int R, unsigned long long* __restrict__ acc, bo
 }
 
 // Inside-cutoff counts of the FP64 kernel (acc[4 r + 2]) into inside[r]; clears acc
-__global__ void k_b_finish_fp64(int R, unsigned long long* __restrict__ acc, unsigned long long* __restrict__ inside) {
+__global__ void k_b_finish_fp64(int R, unsigned long long* __restrict__ acc, unsigned long long* __restrict__ inside,
+                                double* __restrict__ record) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= R) return;
     unsigned long long* s = acc + 4 * r;
     if (inside) inside[r] = s[2];
+    if (record) record[r] = static_cast<double>(s[2]);
     s[0] = s[1] = s[2] = s[3] = 0;
 }
 
@@ -617,9 +619,28 @@ __global__ void __launch_bounds__(kOrderedThreads)
     if (threadIdx.x == 0) chunk_sums[blockIdx.x] = sm.run[0];
 }
 
+// A step's thermostat: mode 0 none, 1 rescale, 2 Bussi (r1, chi2: the replicas' draws); the factors go to scale
+struct BThermostat {
+    int mode;
+    double c;
+    const double* r1;
+    const double* chi2;
+    double2* scale;
+};
+__device__ __forceinline__ void thermostat_scale(const BThermostat& t, const BRep& d, int r, double kinetic) {
+    double2 out = make_double2(1.0, 0.0);
+    if (t.mode == 1) {
+        const double T = ddiv(dmul(2.0, kinetic), d.dof);
+        if (T > 0.0) out = make_double2(__dsqrt_rn(ddiv(d.temperature, T)), 1.0);
+    } else if (kinetic > 0.0) {
+        out = make_double2(bussi_scale(kinetic, d.dof, d.temperature, t.c, t.r1[r], t.chi2[r]), 1.0);
+    }
+    t.scale[r] = out;
+}
+
 // deterministicSum's outer loop per replica: its block sums added in order; one warp per replica
 __global__ void k_b_sum_chunks(const BRep* __restrict__ reps, int R, const double* __restrict__ chunk_sums,
-                               double* __restrict__ out) {
+                               double* __restrict__ out, BThermostat thermo) {
     const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (r >= R) return;
@@ -634,7 +655,10 @@ __global__ void k_b_sum_chunks(const BRep* __restrict__ reps, int R, const doubl
             if (lane == 0) s = dadd(s, x);
         }
     }
-    if (lane == 0) out[r] = s;
+    if (lane == 0) {
+        out[r] = s;
+        if (thermo.mode) thermostat_scale(thermo, d, r, s);
+    }
 }
 
 // Fixed-point kinetic energy per replica (k_kinetic_fixed) with the pending scale applied, into acc[4 r + 3]
@@ -665,21 +689,9 @@ __global__ void __launch_bounds__(kTile)
 // Thermostat factors per replica into scale[r] = (factor, 1), or (1, 0) to leave the replica alone.
 // mode 1: rescaleVelocities to the replica's temperature (src/Thermostat.cpp:17-30); mode 2: Bussi with the
 // step's draws r1[r], chi2[r] (src/Thermostat.cpp:36-58).
-__global__ void k_b_thermostat(const BRep* __restrict__ reps, int R, int mode, const double* __restrict__ ke, double c,
-                               const double* __restrict__ r1, const double* __restrict__ chi2,
-                               double2* __restrict__ scale) {
+__global__ void k_b_thermostat(const BRep* __restrict__ reps, int R, const double* __restrict__ ke, BThermostat t) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= R) return;
-    const BRep d = reps[r];
-    const double kinetic = ke[r];
-    double2 out = make_double2(1.0, 0.0);
-    if (mode == 1) {
-        const double t = ddiv(dmul(2.0, kinetic), d.dof);
-        if (t > 0.0) out = make_double2(__dsqrt_rn(ddiv(d.temperature, t)), 1.0);
-    } else if (kinetic > 0.0) {
-        out = make_double2(bussi_scale(kinetic, d.dof, d.temperature, c, r1[r], chi2[r]), 1.0);
-    }
-    scale[r] = out;
+    if (r < R) thermostat_scale(t, reps[r], r, ke[r]);
 }
 
 // ---- FP64 energy and virial in the reference's pair order ----------------------------------------------------

@@ -17,6 +17,7 @@ struct md_batch {
     int slots = 0, tiles = 0, cells = 0, chunks = 0;
     int build_items = 0;    // list-build work items of all replicas (cells, or tiles of boxes without cells)
     double per_cell = 0.0;  // particles per cell of the densest replica
+    double mean_cell = 0.0;  // and of all replicas with cells
     std::vector<BRep> reps_h;
     DevBuf<BRep> reps;
     DevBuf<int> tile_rep, chunk_rep;
@@ -68,11 +69,19 @@ struct md_batch {
     // first run, on a state the dynamics has reached, unless md_batch_set_force_variant pinned one
     bool retuned = false;
     uint64_t launches = 0;
+    // FP64 energies of a graph's step: summed on a branch of the graph beside the kinetic energies, the thermostat and the
+    // next step's drift and rebuild (b_enqueue_step), which wait for it before the records are written again
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_records = nullptr, ev_energy = nullptr;
+    bool energy_pending = false;
     ~md_batch() {
         for (auto& g : graphs) cudaGraphExecDestroy(g.second.first);
         if (h_noise) cudaFreeHost(h_noise);
         if (h_rec) cudaFreeHost(h_rec);
         if (h_flags) cudaFreeHost(h_flags);
+        if (ev_records) cudaEventDestroy(ev_records);
+        if (ev_energy) cudaEventDestroy(ev_energy);
+        if (side) cudaStreamDestroy(side);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -145,7 +154,7 @@ md_status b_build_async(md_batch* b, bool prepare_only) {
         bp.stage = 0;
         smem = 0;
     }
-    const auto kernel = cell_round(b->per_cell) == 24 ? k_b_nlist_build<4, 4, 24> : k_b_nlist_build<4, 4, 16>;
+    const auto kernel = cell_round(b->mean_cell) == 24 ? k_b_nlist_build<4, 4, 24> : k_b_nlist_build<4, 4, 16>;
     MD_CUDA(allow_smem(kernel, smem));
     if (prepare_only) return MD_OK;
     const unsigned grid = static_cast<unsigned>(std::min(b->build_items, 148 * 32));
@@ -243,26 +252,27 @@ md_status b_forces(md_batch* b, int variant, bool kick, bool energy) {
     return energy ? b_float_forces<false, true>(b, v, kick) : b_float_forces<false, false>(b, v, kick);
 }
 
-// FP64 kinetic energies in the reference's blocked order into `out` (with the pending scale applied if asked)
-md_status b_kinetic_fp64(md_batch* b, bool scaled, double* out) {
+// FP64 kinetic energies in the reference's blocked order into `out` (with the pending scale applied if asked); with
+// `thermo` also the thermostat's scale from them
+md_status b_kinetic_fp64(md_batch* b, bool scaled, double* out, const BThermostat& thermo = {}) {
     k_b_kinetic_blocks<<<b->chunks, kOrderedThreads, 0, b->stream>>>(b->reps.p, b->chunk_rep.p, b->vel.p, b->mass.p,
                                                                      scaled ? b->scale.p : nullptr, b->chunk_sums.p);
     MD_CHECK_LAUNCH();
     k_b_sum_chunks<<<blocks_for(static_cast<long long>(b->R) * 32, kThreads), kThreads, 0, b->stream>>>(
-        b->reps.p, b->R, b->chunk_sums.p, out);
+        b->reps.p, b->R, b->chunk_sums.p, out, thermo);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
 
 // FP64 energy and virial of every replica in the reference's pair order into pe_out / w_out, from the records of a force
 // launch with `energy`
-md_status b_energy_fp64(md_batch* b, double* pe_out, double* w_out) {
-    k_b_pair_items<<<1, kRepScanThreads, 0, b->stream>>>(b->R, b->pairs.p, b->item_off.p);
+md_status b_energy_fp64(md_batch* b, cudaStream_t st, double* pe_out, double* w_out) {
+    k_b_pair_items<<<1, kRepScanThreads, 0, st>>>(b->R, b->pairs.p, b->item_off.p);
     MD_CHECK_LAUNCH();
-    k_b_energy_blocks<<<148 * 4, kSumWarps * 32, 0, b->stream>>>(b->reps.p, b->R, b->item_off.p, b->pairs.p, b->pair_r2.p,
-                                                                 b->lj, b->cap, b->item_sums.p);
+    k_b_energy_blocks<<<148 * 4, kSumWarps * 32, 0, st>>>(b->reps.p, b->R, b->item_off.p, b->pairs.p, b->pair_r2.p, b->lj,
+                                                          b->cap, b->item_sums.p);
     MD_CHECK_LAUNCH();
-    k_b_sum_items<<<blocks_for(static_cast<long long>(b->R) * 32, kThreads), kThreads, 0, b->stream>>>(
+    k_b_sum_items<<<blocks_for(static_cast<long long>(b->R) * 32, kThreads), kThreads, 0, st>>>(
         b->R, b->item_off.p, b->item_sums.p, pe_out, w_out);
     MD_CHECK_LAUNCH();
     return MD_OK;
@@ -281,13 +291,20 @@ md_status b_observables(md_batch* b, double* pe_out, double* w_out, double* ke_o
         MD_CHECK_LAUNCH();
         return MD_OK;
     }
-    k_b_finish_fp64<<<per_replica(b, kThreads), kThreads, 0, b->stream>>>(b->R, b->acc.p, b->inside.p);
+    k_b_finish_fp64<<<per_replica(b, kThreads), kThreads, 0, b->stream>>>(b->R, b->acc.p, b->inside.p, nullptr);
     MD_CHECK_LAUNCH();
-    MD_TRY(b_energy_fp64(b, pe_out, w_out));
+    MD_TRY(b_energy_fp64(b, b->stream, pe_out, w_out));
     return b_kinetic_fp64(b, true, ke_out);
 }
 
-// One step of every replica (src/Integrator.cpp:18-30, then the thermostat); `k` is the step's index in its
+// The stream waits for the energy branch of an earlier step
+md_status b_join_energy(md_batch* b) {
+    if (b->energy_pending) MD_CUDA(cudaStreamWaitEvent(b->stream, b->ev_energy, 0));
+    b->energy_pending = false;
+    return MD_OK;
+}
+
+// One step of every replica (src/Integrator.cpp:18-30, then the thermostat), into a graph; `k` is the step's index in its
 // chunk, `step` its number in the run (1-based), `rec` the sample's records or null.
 md_status b_enqueue_step(md_batch* b, int k, int64_t step, double* rec) {
     cudaStream_t st = b->stream;
@@ -312,29 +329,43 @@ md_status b_enqueue_step(md_batch* b, int k, int64_t step, double* rec) {
     }
     MD_TRY(b_rebuild_async(b));
     const bool sample = rec != nullptr;
+    // the last sums read the records and the inside counts that the force kernel writes
+    MD_TRY(b_join_energy(b));
     MD_TRY(b_forces(b, b->variant, true, sample));
     const int R = b->R;
+    BThermostat th{};
+    if (thermo)
+        th = {b->opt.thermostat, b->bussi_c, b->noise.p + static_cast<size_t>(k) * R,
+              b->noise.p + static_cast<size_t>(b->chunk + k) * R, b->scale.p};
     if (fl) {
         k_b_finish_float<<<per_replica(b, kThreads), kThreads, 0, st>>>(R, b->acc.p, true, b->ke.p,
                                                                         sample ? rec : nullptr,
                                                                         sample ? rec + R : nullptr, b->inside.p);
         MD_CHECK_LAUNCH();
+        if (sample) {
+            k_b_record_inside<<<per_replica(b, kThreads), kThreads, 0, st>>>(R, b->inside.p, rec + 3 * R);
+            MD_CHECK_LAUNCH();
+        }
+        if (thermo) {
+            k_b_thermostat<<<per_replica(b, kThreads), kThreads, 0, st>>>(b->reps.p, R, b->ke.p, th);
+            MD_CHECK_LAUNCH();
+        }
     } else {
-        k_b_finish_fp64<<<per_replica(b, kThreads), kThreads, 0, st>>>(R, b->acc.p, b->inside.p);
+        cudaStream_t branch = st;
+        if (sample) {
+            MD_CUDA(cudaEventRecord(b->ev_records, st));
+            MD_CUDA(cudaStreamWaitEvent(b->side, b->ev_records, 0));
+            branch = b->side;
+        }
+        k_b_finish_fp64<<<per_replica(b, kThreads), kThreads, 0, branch>>>(R, b->acc.p, b->inside.p,
+                                                                           sample ? rec + 3 * R : nullptr);
         MD_CHECK_LAUNCH();
-        if (thermo) MD_TRY(b_kinetic_fp64(b, false, b->ke.p));
-        if (sample) MD_TRY(b_energy_fp64(b, rec, rec + R));
-    }
-    if (sample) {
-        k_b_record_inside<<<per_replica(b, kThreads), kThreads, 0, st>>>(R, b->inside.p, rec + 3 * R);
-        MD_CHECK_LAUNCH();
-    }
-    if (thermo) {
-        const double* r1 = b->noise.p + static_cast<size_t>(k) * R;
-        const double* chi2 = b->noise.p + static_cast<size_t>(b->chunk + k) * R;
-        k_b_thermostat<<<per_replica(b, kThreads), kThreads, 0, st>>>(b->reps.p, R, b->opt.thermostat, b->ke.p,
-                                                                      b->bussi_c, r1, chi2, b->scale.p);
-        MD_CHECK_LAUNCH();
+        if (sample) {
+            MD_TRY(b_energy_fp64(b, branch, rec, rec + R));
+            MD_CUDA(cudaEventRecord(b->ev_energy, branch));
+            b->energy_pending = true;
+        }
+        if (thermo) MD_TRY(b_kinetic_fp64(b, false, b->ke.p, th));
     }
     if (sample) {
         if (fl) {
@@ -375,6 +406,8 @@ md_status b_graph(md_batch* b, int len, cudaGraphExec_t* out, uint64_t* kernels)
                                                      : nullptr;
         st = b_enqueue_step(b, k, step, rec);
     }
+    if (st == MD_OK) st = b_join_energy(b);
+    b->energy_pending = false;
     const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
     g_capturing = false;
     g_launches = saved;
@@ -605,6 +638,7 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
     b->reps_h.resize(replicas);
     std::vector<int> tile_rep(b->tiles), chunk_rep;
     int off = 0, cell_off = 0, chunk_off = 0;
+    double celled = 0.0, cells_used = 0.0;
     for (int r = 0; r < replicas; ++r) {
         BRep& d = b->reps_h[r];
         const int n = static_cast<int>(n_atoms[r]);
@@ -624,7 +658,11 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
         d.tile_off = off / kTile;
         d.chunk_off = chunk_off;
         b->build_items += md::build_items(d);
-        if (d.use_cells) b->per_cell = std::max(b->per_cell, static_cast<double>(d.n) / d.ncells);
+        if (d.use_cells) {
+            b->per_cell = std::max(b->per_cell, static_cast<double>(d.n) / d.ncells);
+            celled += d.n;
+            cells_used += d.ncells;
+        }
         for (int t = 0; t < d.np / kTile; ++t) tile_rep[d.tile_off + t] = r;
         const int nch = (n + kChunk - 1) / kChunk;
         for (int c = 0; c < nch; ++c) chunk_rep.push_back(r);
@@ -632,6 +670,7 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
         cell_off += d.ncells;
         chunk_off += nch;
     }
+    if (cells_used > 0.0) b->mean_cell = celled / cells_used;
     b->cells = cell_off;
     b->chunks = chunk_off;
     // initial row capacity: the full r_l sphere at the densest replica with a margin (or the caller's)
@@ -649,6 +688,8 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
     };
     const size_t S = slots, R = replicas;
     chk(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
+    chk(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
+    for (cudaEvent_t* ev : {&b->ev_records, &b->ev_energy}) chk(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
     chk(b->reps.reserve(R));
     chk(b->tile_rep.reserve(b->tiles));
     chk(b->chunk_rep.reserve(b->chunks));
