@@ -18,6 +18,7 @@ struct md_batch {
     int build_items = 0;    // list-build work items of all replicas (cells, or tiles of boxes without cells)
     double per_cell = 0.0;  // particles per cell of the densest replica
     double mean_cell = 0.0;  // and of all replicas with cells
+    int most_n = 0, most_cells = 0;  // the largest replica's particles, the most cells of one
     std::vector<BRep> reps_h;
     DevBuf<BRep> reps;
     DevBuf<int> tile_rep, chunk_rep;
@@ -164,12 +165,23 @@ md_status b_build_async(md_batch* b, bool prepare_only) {
     return MD_OK;
 }
 
+// Replicas small enough to be resorted by a block each (k_b_resort)
+bool one_block_resort(const md_batch* b) { return b->most_n <= kResortMost && b->most_cells <= kResortCells; }
+
 // The list rebuild of every replica flagged stale (all of them when the flags were set by the host)
 md_status b_rebuild_async(md_batch* b) {
     cudaStream_t st = b->stream;
     k_b_stale_lists<<<1, kListThreads, 0, st>>>(b->reps.p, b->R, b->stale.p, b->stale_reps.p, b->stale_tiles.p,
                                                 b->stale_items.p, b->work.p, b->rebuilds.p);
     MD_CHECK_LAUNCH();
+    if (one_block_resort(b)) {
+        k_b_resort<<<std::min(b->R, 148 * 2), kResortThreads, resort_smem(b->most_n, b->most_cells), st>>>(
+            b->reps.p, b->stale_reps.p, b->work.p, b->most_n, b->most_cells, b->pos.p, b->vel.p, b->force.p, b->mass.p,
+            b->ids.p, b->pos2.p, b->vel2.p, b->force2.p, b->mass2.p, b->ids2.p, b->start.p, b->cell_sorted.p, b->ref_pos.p,
+            b->frames.p);
+        MD_CHECK_LAUNCH();
+        return b_build_async(b, false);
+    }
     const unsigned gt = rebuild_grid(b), gr = replica_grid(b);
     k_b_cell_assign<<<gt, kTile, 0, st>>>(b->reps.p, b->tile_rep.p, b->stale_tiles.p, b->work.p, b->pos.p, b->cell_of.p,
                                           b->count.p);
@@ -663,6 +675,8 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
             celled += d.n;
             cells_used += d.ncells;
         }
+        b->most_n = std::max(b->most_n, d.n);
+        b->most_cells = std::max(b->most_cells, d.ncells);
         for (int t = 0; t < d.np / kTile; ++t) tile_rep[d.tile_off + t] = r;
         const int nch = (n + kChunk - 1) / kChunk;
         for (int c = 0; c < nch; ++c) chunk_rep.push_back(r);
