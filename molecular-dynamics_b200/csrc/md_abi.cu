@@ -149,6 +149,7 @@ struct md_system {
     DevBuf<double> vel, vel2, force, force2, mass, mass2;
     DevBuf<uint64_t> ids, ids2;
     DevBuf<double2> ke_blocks;
+    DevBuf<unsigned> ke_done;    // k_kinetic_sum's count of finished blocks, zero between launches
     DevBuf<double> scal;         // device scalars, indexed by the kScal* constants
     double* host_scal = nullptr; // pinned mirror of scal
     uint64_t layout = 0;         // bumps whenever the particle order changes
@@ -321,22 +322,6 @@ md_status sync(md_system* s) {
     return MD_OK;
 }
 
-// Kinetic energy into s->scal[0] with the reference's blocked order (no host sync)
-md_status kinetic_async(md_system* s, double* record = nullptr) {
-    const int n = static_cast<int>(s->n);
-    const int nb = (n + kChunk - 1) / kChunk;
-    if (nb == 0) {
-        MD_CUDA(cudaMemsetAsync(s->scal.p + kScalKE, 0, sizeof(double), s->stream));
-        return MD_OK;
-    }
-    MD_CUDA(s->ke_blocks.reserve(nb));
-    k_kinetic_blocks<<<nb, kOrderedThreads, 0, s->stream>>>(s->vel.p, s->mass.p, n, s->ke_blocks.p);
-    MD_CHECK_LAUNCH();
-    k_sum_blocks<<<1, kChainThreads, 0, s->stream>>>(s->ke_blocks.p, nb, s->scal.p + kScalKE, record);
-    MD_CHECK_LAUNCH();
-    return MD_OK;
-}
-
 md_status scale_async(md_system* s) {
     const long long count = 3 * s->n;
     if (count == 0) return MD_OK;
@@ -347,6 +332,50 @@ md_status scale_async(md_system* s) {
 }
 
 double dof_of(int64_t n) { return 3.0 * static_cast<double>(n) - 3.0; }
+
+// A thermostat's factor (s->scal[kScalFactor]) from s->scal[kScalKE]
+md_status thermostat_factor_async(md_system* s, const Thermostat& t) {
+    k_thermostat_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, t);
+    MD_CHECK_LAUNCH();
+    return MD_OK;
+}
+
+// Kinetic energy into s->scal[kScalKE] (and *record) with the reference's blocked order (no host sync); with `scale` the
+// velocities are scaled by the pending factor first, with a thermostat its factor follows
+md_status kinetic_async(md_system* s, double* record = nullptr, bool scale = false, const Thermostat& t = {}) {
+    const int n = static_cast<int>(s->n);
+    const int nb = (n + kChunk - 1) / kChunk;
+    MD_CUDA(s->ke_blocks.reserve(std::max(nb, 1)));
+    if (nb > 0 && nb <= kChainSerial) {
+        k_kinetic_sum<<<nb, kOrderedThreads, 0, s->stream>>>(
+            s->vel.p, s->mass.p, n, scale ? s->scal.p + kScalFactor : nullptr, reinterpret_cast<double*>(s->ke_blocks.p),
+            s->ke_done.p, s->scal.p + kScalKE, record, t);
+        MD_CHECK_LAUNCH();
+        return MD_OK;
+    }
+    if (scale) MD_TRY(scale_async(s));
+    if (nb == 0) {
+        MD_CUDA(cudaMemsetAsync(s->scal.p + kScalKE, 0, sizeof(double), s->stream));
+    } else {
+        k_kinetic_blocks<<<nb, kOrderedThreads, 0, s->stream>>>(s->vel.p, s->mass.p, n, s->ke_blocks.p);
+        MD_CHECK_LAUNCH();
+        k_sum_blocks<<<1, kChainThreads, 0, s->stream>>>(s->ke_blocks.p, nb, s->scal.p + kScalKE, record);
+        MD_CHECK_LAUNCH();
+    }
+    return t.mode ? thermostat_factor_async(s, t) : MD_OK;
+}
+
+// A thermostat's factor for the current velocities (ke_current: s->scal[kScalKE] holds their kinetic energy); the
+// velocities are scaled by whoever comes next (scale_async, or kinetic_async with `scale`)
+md_status thermostat_async(md_system* s, const Thermostat& t, bool ke_current) {
+    return ke_current ? thermostat_factor_async(s, t) : kinetic_async(s, nullptr, false, t);
+}
+Thermostat rescale_thermostat(md_system* s, double target) {
+    return {1, dof_of(s->n), target, 0.0, nullptr, nullptr, s->scal.p + kScalFactor};
+}
+Thermostat bussi_thermostat(md_system* s, double temperature, double c, const double* r1, const double* chi2) {
+    return {2, dof_of(s->n), temperature, c, r1, chi2, s->scal.p + kScalFactor};
+}
 
 // src/Forcefield.cpp:8-15 and the constant factors of pairTerms (:25-36)
 LJ lj_constants(double epsilon, double sigma, double cutoff) {
@@ -1011,6 +1040,8 @@ md_status md_system_create(int64_t n, double box_length, int device, md_system**
     chk(s->mass.reserve(n));
     chk(s->ids.reserve(n));
     chk(s->scal.reserve(8));
+    chk(s->ke_done.reserve(1));
+    if (st == MD_OK) chk(cudaMemsetAsync(s->ke_done.p, 0, sizeof(unsigned), s->stream));
     chk(cudaMallocHost(reinterpret_cast<void**>(&s->host_scal), 8 * sizeof(double)));
     if (st == MD_OK && n > 0) {
         chk(cudaMemsetAsync(s->pos.p, 0, sizeof(double4) * n, s->stream));
@@ -1278,9 +1309,7 @@ md_status md_scale_velocities(md_system* s, double scale) {
 md_status md_rescale_velocities(md_system* s, double target) {
     if (!s) return fail(MD_ERR_INVALID, "null system");
     MD_TRY(use_system(s));
-    MD_TRY(kinetic_async(s));
-    k_rescale_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, dof_of(s->n), target, s->scal.p + kScalFactor);
-    MD_CHECK_LAUNCH();
+    MD_TRY(thermostat_async(s, rescale_thermostat(s, target), false));
     MD_TRY(scale_async(s));
     return sync(s);
 }
@@ -1293,10 +1322,7 @@ md_status md_bussi_apply(md_system* s, double temperature, double tau, double dt
     s->host_scal[kScalR1 + 1] = chi2;
     MD_CUDA(cudaMemcpyAsync(s->scal.p + kScalR1, s->host_scal + kScalR1, 2 * sizeof(double), cudaMemcpyHostToDevice,
                             s->stream));
-    MD_TRY(kinetic_async(s));
-    k_bussi_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, dof_of(s->n), temperature, c, s->scal.p + kScalR1,
-                                           s->scal.p + kScalR1 + 1, s->scal.p + kScalFactor);
-    MD_CHECK_LAUNCH();
+    MD_TRY(thermostat_async(s, bussi_thermostat(s, temperature, c, s->scal.p + kScalR1, s->scal.p + kScalR1 + 1), false));
     MD_TRY(scale_async(s));
     return sync(s);
 }

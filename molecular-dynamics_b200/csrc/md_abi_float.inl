@@ -558,25 +558,22 @@ md_status run_steps(md_system* s, md_forcefield* ff, md_nlist* nl, double dt, in
             MD_CUDA(cudaMemcpyAsync(rec.p + 3 * k, ff->out.p, 2 * sizeof(double), cudaMemcpyDeviceToDevice, es));
             if (es != s->stream) MD_CUDA(cudaEventRecord(ff->ev_done, es));  // the join covers the copy too
         }
+        bool scale_next = false;
         bool ke_current = fused_ke && !exact_ke;  // scal[kScalKE] holds this step's kinetic energy
         const bool rescale = o.thermostat == 1 && o.rescale_every > 0 && step % o.rescale_every == 0;
         if (rescale || o.thermostat == 2) {
-            if (!ke_current) MD_TRY(kinetic_async(s));
-            if (rescale) {
-                const double target = step <= o.melt_until ? o.melt_temperature : o.rescale_temperature;
-                k_rescale_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, dof_of(s->n), target,
-                                                         s->scal.p + kScalFactor);
-            } else {
-                k_bussi_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, dof_of(s->n), o.bussi_temperature, bussi_c,
-                                                       noise.p + k, noise.p + n_steps + k, s->scal.p + kScalFactor);
-            }
-            MD_CHECK_LAUNCH();
-            MD_TRY(scale_async(s));
+            const double target = step <= o.melt_until ? o.melt_temperature : o.rescale_temperature;
+            MD_TRY(thermostat_async(s, rescale ? rescale_thermostat(s, target)
+                                               : bussi_thermostat(s, o.bussi_temperature, bussi_c, noise.p + k,
+                                                                  noise.p + n_steps + k),
+                                    ke_current));
+            scale_next = exact_ke && ke;  // with the kinetic energy below
+            if (!scale_next) MD_TRY(scale_async(s));
             ke_current = false;
         }
         if (o.rdf && o.rdf_every > 0 && step % o.rdf_every == 0) MD_TRY(rdf_sample_async(o.rdf, s, nl));
         if (ke) {
-            if (!ke_current) MD_TRY(exact_ke ? kinetic_async(s) : kinetic_fixed_async(s, ff));
+            if (!ke_current) MD_TRY(exact_ke ? kinetic_async(s, nullptr, scale_next) : kinetic_fixed_async(s, ff));
             MD_CUDA(cudaMemcpyAsync(rec.p + 3 * k + 2, s->scal.p + kScalKE, sizeof(double), cudaMemcpyDeviceToDevice,
                                     s->stream));
         }

@@ -493,18 +493,18 @@ __global__ void k_kick(double* __restrict__ vel, const double* __restrict__ forc
 
 // ---- thermostats ----------------------------------------------------------------------------------------
 
-// Scale factors computed on the device from the device kinetic energy, so no host round trip is needed.
-// scale[0] = factor, scale[1] = 1 to apply or 0 to leave the velocities alone.
-// rescaleVelocities (src/Thermostat.cpp:17-30)
-__global__ void k_rescale_factor(const double* __restrict__ ke, double dof, double target, double* __restrict__ scale) {
-    const double t = ddiv(dmul(2.0, ke[0]), dof);  // System::temperature (src/System.cpp:79-82)
-    if (t <= 0.0) {
-        scale[1] = 0.0;
-        return;
-    }
-    scale[0] = __dsqrt_rn(ddiv(target, t));
-    scale[1] = 1.0;
-}
+// A thermostat's scale factor from the kinetic energy on the device, so no host round trip is needed: mode 1
+// rescaleVelocities (src/Thermostat.cpp:17-30), 2 BussiThermostat::apply with the step's draws (src/Thermostat.cpp:36-58),
+// 0 none. scale[0] = factor, scale[1] = 1 to apply or 0 to leave the velocities alone.
+struct Thermostat {
+    int mode;
+    double dof;
+    double temperature;
+    double c;
+    const double* r1;
+    const double* chi2;
+    double* scale;
+};
 
 // BussiThermostat::apply's velocity scale, equation A7 (src/Thermostat.cpp:40-57), for kinetic > 0
 __device__ __forceinline__ double bussi_scale(double kinetic, double dof, double temperature, double c, double r1,
@@ -517,17 +517,71 @@ __device__ __forceinline__ double bussi_scale(double kinetic, double dof, double
     return __dsqrt_rn(ddiv(nk, kinetic));
 }
 
-// BussiThermostat::apply (src/Thermostat.cpp:36-58), with r1 and chi2 given
-__global__ void k_bussi_factor(const double* __restrict__ ke, double dof, double temperature, double c,
-                               const double* __restrict__ r1p, const double* __restrict__ chi2p,
-                               double* __restrict__ scale) {
-    const double kinetic = ke[0];
-    if (kinetic <= 0.0) {
-        scale[1] = 0.0;
-        return;
+__device__ __forceinline__ void thermostat_factor(const Thermostat& t, double kinetic) {
+    double factor = 0.0;
+    bool apply;
+    if (t.mode == 1) {
+        const double now = ddiv(dmul(2.0, kinetic), t.dof);  // System::temperature (src/System.cpp:79-82)
+        apply = !(now <= 0.0);
+        if (apply) factor = __dsqrt_rn(ddiv(t.temperature, now));
+    } else {
+        apply = !(kinetic <= 0.0);
+        if (apply) factor = bussi_scale(kinetic, t.dof, t.temperature, t.c, *t.r1, *t.chi2);
     }
-    scale[0] = bussi_scale(kinetic, dof, temperature, c, r1p[0], chi2p[0]);
-    scale[1] = 1.0;
+    if (apply) t.scale[0] = factor;
+    t.scale[1] = apply ? 1.0 : 0.0;
+}
+
+__global__ void k_thermostat_factor(const double* __restrict__ ke, Thermostat t) { thermostat_factor(t, ke[0]); }
+
+// k_kinetic_blocks, k_sum_blocks and what stands before and after them in one launch, for at most kChainSerial blocks:
+// with `scale` the velocities are scaled first (k_scale_velocities), the last block to finish (counted in *done, which it
+// leaves zero) adds the blocks' sums in order, and with a thermostat it makes its factor. A thermostat's step waits for
+// all of it, and small systems spend that time in launches: N = 2,048 (B200) 3.2 + 3.4 us for the sum and the factor and
+// 3.5 for the scaling, each after a launch of its own, around the 6.1 of k_kinetic_blocks.
+__global__ void __launch_bounds__(kOrderedThreads)
+    k_kinetic_sum(double* vel, const double* __restrict__ mass, int n, const double* __restrict__ scale,
+                  double* __restrict__ block_sums, unsigned* __restrict__ done, double* __restrict__ out,
+                  double* __restrict__ record, Thermostat thermostat) {
+    __shared__ OrderedSmem<1, kChunk / kOrderedThreads> sm;
+    __shared__ double s_sums[kChainSerial];
+    __shared__ bool s_last;
+    const int i0 = blockIdx.x * kChunk;
+    const int m = n - i0 < kChunk ? n - i0 : kChunk;
+    const bool scaled = scale && scale[1] != 0.0;
+    const double factor = scaled ? scale[0] : 1.0;
+    if (threadIdx.x == 0) sm.run[0] = 0.0;
+    ordered_sum(sm, m, [&](long long k, double* v) {
+        const int i = i0 + static_cast<int>(k);
+        double c[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) c[q] = vel[q * static_cast<size_t>(n) + i];
+        if (scaled) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                c[q] = dmul(c[q], factor);
+                vel[q * static_cast<size_t>(n) + i] = c[q];
+            }
+        }
+        v[0] = dmul(dmul(0.5, mass[i]), norm2(c[0], c[1], c[2]));
+    });
+    if (threadIdx.x == 0) {
+        block_sums[blockIdx.x] = sm.run[0];
+        __threadfence();
+        s_last = gridDim.x == 1 || atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += kOrderedThreads) s_sums[k] = __ldcg(block_sums + k);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double kinetic = add_in_order(s_sums, 1, static_cast<int>(gridDim.x), 0.0);
+        *out = kinetic;
+        if (record) *record = kinetic;
+        if (thermostat.mode) thermostat_factor(thermostat, kinetic);
+        if (gridDim.x > 1) *done = 0u;
+    }
 }
 
 __global__ void k_scale_velocities(double* __restrict__ vel, long long count, const double* __restrict__ scale) {

@@ -369,22 +369,20 @@ md_status graph_step(md_system* s, md_forcefield* ff, md_nlist* nl, const md_run
     g_step = nullptr;
     MD_TRY(st);
     if (fp64 && want_energy && !ff->side_pending) MD_TRY(record_energy(ff, s, step.record, true));  // no pairs at all
+    bool scale_next = false;
     bool ke_current = fused_ke;
     if (r.thermo) {
-        if (!ke_current) MD_TRY(kinetic_async(s));
-        if (r.thermo == 1) {
-            k_rescale_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, dof_of(s->n), r.target, s->scal.p + kScalFactor);
-        } else {
-            const double* noise = s->chunk_noise.p;
-            k_bussi_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, dof_of(s->n), o.bussi_temperature, bussi_c,
-                                                   noise + k, noise + s->graph_chunk + k, s->scal.p + kScalFactor);
-        }
-        MD_CHECK_LAUNCH();
-        MD_TRY(scale_async(s));
+        const double* noise = s->chunk_noise.p;
+        MD_TRY(thermostat_async(s, r.thermo == 1 ? rescale_thermostat(s, r.target)
+                                                 : bussi_thermostat(s, o.bussi_temperature, bussi_c, noise + k,
+                                                                    noise + s->graph_chunk + k),
+                                ke_current));
+        scale_next = fp64 && want_ke;  // with the kinetic energy below
+        if (!scale_next) MD_TRY(scale_async(s));
         ke_current = false;
     }
     if (r.rdf) MD_TRY(rdf_kernel_async(o.rdf, s, nl));
-    if (want_ke && !ke_current) MD_TRY(fp64 ? kinetic_async(s, step.record + 2) : kinetic_fixed_async(s, ff, step.record + 2));
+    if (want_ke && !ke_current) MD_TRY(fp64 ? kinetic_async(s, step.record + 2, scale_next) : kinetic_fixed_async(s, ff, step.record + 2));
     *last = step;
     return MD_OK;
 }
@@ -571,21 +569,20 @@ md_status host_step(md_system* s, md_forcefield* ff, md_nlist* nl, double dt, in
     MD_TRY(forces_list_async(ff, s, nl, want_energy, dt, true, &fused_ke, fuse, drifted_in && !rebuilt));
     *fused_out = fuse;
     MD_TRY(record_energy(ff, s, rec + 3 * k, want_energy));
+    bool scale_next = false;
     bool ke_current = fused_ke;
     if (r.thermo) {
-        if (!ke_current) MD_TRY(kinetic_async(s));
-        if (r.thermo == 1)
-            k_rescale_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, dof_of(s->n), r.target, s->scal.p + kScalFactor);
-        else
-            k_bussi_factor<<<1, 1, 0, s->stream>>>(s->scal.p + kScalKE, dof_of(s->n), o.bussi_temperature, bussi_c,
-                                                   noise + k, noise + n_steps + k, s->scal.p + kScalFactor);
-        MD_CHECK_LAUNCH();
-        MD_TRY(scale_async(s));
+        MD_TRY(thermostat_async(s, r.thermo == 1 ? rescale_thermostat(s, r.target)
+                                                 : bussi_thermostat(s, o.bussi_temperature, bussi_c, noise + k,
+                                                                    noise + n_steps + k),
+                                ke_current));
+        scale_next = ff->precision == MD_PREC_FP64 && want_ke;
+        if (!scale_next) MD_TRY(scale_async(s));
         ke_current = false;
     }
     if (r.rdf) MD_TRY(rdf_sample_async(o.rdf, s, nl));
     if (want_ke) {
-        if (!ke_current) MD_TRY(ff->precision == MD_PREC_FP64 ? kinetic_async(s) : kinetic_fixed_async(s, ff));
+        if (!ke_current) MD_TRY(ff->precision == MD_PREC_FP64 ? kinetic_async(s, nullptr, scale_next) : kinetic_fixed_async(s, ff));
         MD_CUDA(cudaMemcpyAsync(rec + 3 * k + 2, s->scal.p + kScalKE, sizeof(double), cudaMemcpyDeviceToDevice,
                                 s->stream));
     }
