@@ -472,7 +472,7 @@ md_status rdf_kernel_async(md_rdf* r, md_system* s, md_nlist* nl) {
     if (n > 0) {
         const size_t smem = sizeof(unsigned int) * r->bins;
         MD_CUDA(allow_smem(k_rdf_sample, smem));
-        k_rdf_sample<<<blocks_for(n, kThreads), kThreads, smem, s->stream>>>(
+        k_rdf_sample<<<blocks_for(static_cast<long long>(n) * kRdfLanes, kThreads), kThreads, smem, s->stream>>>(
             s->pos.p, n, s->box, nl->rows.p, nl->cap, nl->counts.p, r->rmax * r->rmax, r->bin_width, r->bins, r->hist.p);
         MD_CHECK_LAUNCH();
     }
