@@ -159,8 +159,8 @@ md_status md_nlist_info(const md_nlist* nl, uint64_t* pair_count, int* rebuild_c
  * variant 2 untimed), 0 pins global gathers, 1 pins the shared-memory tile kernel (used
  * only while the list has tiles; FP64 and the float modes), 2 pins global gathers with the rows prefetched
  * (FP64: a quad of entries at a time, branch-free; float modes: a group of 8 ahead), 3 the float modes' variant 2
- * with registers capped for occupancy and 4 the same on a resident grid. MD_PREC_FX64 and MD_PREC_FX32 have one
- * kernel each (variant 0). Every variant gives the same bits. md_nlist_force_variant reports the variant in use
+ * with registers capped for occupancy and 4 the same on a resident grid; a list that loses the tiles of a pinned
+ * variant 1 goes on as with -1. MD_PREC_FX64 and MD_PREC_FX32 have one kernel each (variant 0). Every variant gives the same bits. md_nlist_force_variant reports the variant in use
  * (-1 until the first force call). */
 md_status md_nlist_set_force_variant(md_nlist* nl, int precision, int variant);
 md_status md_nlist_force_variant(const md_nlist* nl, int precision, int* variant);

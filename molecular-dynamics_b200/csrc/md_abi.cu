@@ -665,35 +665,38 @@ md_status profile_collect(md_system* s) {
     return MD_OK;
 }
 
-// Autotuner of the list force kernel: with tiles available, the first force call of a list (per precision)
-// times the global-gather kernel (variant 0) and the shared-memory tile kernel (variant 1) on the current
-// state, two launches each after a warm-up, and keeps the faster. Both variants give the same bits, so the
-// choice never changes a result. md_nlist_set_force_variant pins a variant instead. FP64, and the float modes
-// with few particles, take variant 2 untimed.
+// The list force kernel's variant, chosen at the first force call of a list (per precision) unless
+// md_nlist_set_force_variant pinned one that is available. Every variant of a precision gives the same bits, so the choice
+// never changes a result. Variants: 0 always; 1 (shared-memory tile) with tiles; FP64: 2 (branch-free quads or lanes);
+// float modes: 2, 3 and 4 (prefetching global gathers; 3 with capped registers, 4 on a resident grid).
+bool keep_or_pin(md_nlist* nl, int prec, unsigned mask) {
+    auto available = [&](int v) { return v >= 0 && ((mask >> v) & 1u); };
+    if (available(nl->variant[prec])) return true;
+    if (!available(nl->pinned[prec])) return false;
+    nl->variant[prec] = nl->pinned[prec];
+    return true;
+}
+
+// FP64: variant 2 untimed, also for a pin that is not available (the tile kernel on a list without tiles; timing launches
+// would add to the inside-cutoff count). Nothing to time: with records, variants 0 / 1 / 2 take 63 / 47 / 12 us at
+// N = 2,048, 72 / 56 / 24 at 32,000, 243 / 295 / 118 at 256,000 and 574 / 763 / 313 at 864,000.
+void choose_fp64_variant(md_nlist* nl) {
+    if (!keep_or_pin(nl, MD_PREC_FP64, 5u | (nl->use_tiles ? 2u : 0u))) nl->variant[MD_PREC_FP64] = 2;
+}
+
+// Float modes: variant 2 untimed with few particles, else the fastest on the current state, two launches of each timed
+// after a warm-up.
 template <typename Launch>
 md_status choose_variant(md_system* s, md_nlist* nl, int prec, Launch&& launch) {
-    // variants available: 0 always, 1 with tiles; for FP64 2 (branch-free quads); for the float modes 2, 3
-    // and 4 (prefetching global gathers; the second with capped registers, the third on a resident grid)
-    unsigned mask = 1u | (nl->use_tiles ? 2u : 0u) | (prec == MD_PREC_FP32FX || prec == MD_PREC_FP32 ? 28u : 0u) |
-                    (prec == MD_PREC_FP64 ? 4u : 0u);
-    if (nl->variant[prec] >= 0 && ((mask >> nl->variant[prec]) & 1u)) return MD_OK;
+    const unsigned mask = 1u | (nl->use_tiles ? 2u : 0u) | (prec == MD_PREC_FP32FX || prec == MD_PREC_FP32 ? 28u : 0u);
+    if (keep_or_pin(nl, prec, mask)) return MD_OK;
     if (mask == 1u) {
         nl->variant[prec] = 0;
         return MD_OK;
     }
-    if (prec != MD_PREC_FP64 && nl->pinned[prec] < 0 && float_lanes(static_cast<int>(s->n)) > 1) {
+    if (nl->pinned[prec] < 0 && float_lanes(static_cast<int>(s->n)) > 1) {
         // small systems: variant 2's several threads per particle beat the other kernels' one (float_lanes)
         nl->variant[prec] = 2;
-        return MD_OK;
-    }
-    if (prec == MD_PREC_FP64 && nl->pinned[prec] < 0) {
-        // nothing to time: with records, variants 0 / 1 / 2 take 63 / 47 / 12 us at N = 2,048, 72 / 56 / 24 at 32,000,
-        // 243 / 295 / 118 at 256,000 and 574 / 763 / 313 at 864,000
-        nl->variant[prec] = 2;
-        return MD_OK;
-    }
-    if (nl->pinned[prec] >= 0 && ((mask >> nl->pinned[prec]) & 1u)) {
-        nl->variant[prec] = nl->pinned[prec];
         return MD_OK;
     }
     cudaEvent_t e0, e1;
@@ -881,7 +884,7 @@ md_status forces_list_async(md_forcefield* ff, md_system* s, md_nlist* nl, bool 
                 MD_CHECK_LAUNCH();
                 return MD_OK;
             };
-            MD_TRY(choose_variant(s, nl, MD_PREC_FP64, [&](int v) { return launch(v, false, nullptr); }));
+            choose_fp64_variant(nl);
             MD_TRY(profile_mark(s));
             MD_TRY(launch(nl->variant[MD_PREC_FP64], kick_dt > 0.0, sums ? ff->pair_r2[b].p : nullptr));
             MD_TRY(profile_mark(s));
