@@ -589,12 +589,12 @@ md_status host_step(md_system* s, md_forcefield* ff, md_nlist* nl, double dt, in
     return MD_OK;
 }
 
-// A chunk whose graph hit an overflow: back to the snapshot, the chunk start's list rebuilt from its reference
-// positions (an identity reorder, the same rows; the host grows the capacity or the tile), then the chunk's
-// steps on the host path
+// A chunk whose graph hit an overflow: back to the snapshot (which holds the g(r) histogram if the chunk samples it:
+// `sampled`; a chunk that does not has not changed it), the chunk start's list rebuilt from its reference positions (an
+// identity reorder, the same rows; the host grows the capacity or the tile), then the chunk's steps on the host path
 md_status recover_chunk(md_system* s, md_forcefield* ff, md_nlist* nl, double dt, int64_t n_steps,
                         const md_run_options& o, int64_t b, int64_t e, bool want_energy, bool want_ke,
-                        const double* noise, double* rec, double bussi_c, bool* drifted_io) {
+                        const double* noise, double* rec, double bussi_c, bool sampled, bool* drifted_io) {
     const size_t N = static_cast<size_t>(s->n);
     cudaStream_t st = s->stream;
     MD_CUDA(s->pos_save.reserve(N));
@@ -604,7 +604,7 @@ md_status recover_chunk(md_system* s, md_forcefield* ff, md_nlist* nl, double dt
     MD_CUDA(cudaMemcpyAsync(s->force.p, s->snap_force.p, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, st));
     MD_CUDA(cudaMemcpyAsync(s->mass.p, s->snap_mass.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
     MD_CUDA(cudaMemcpyAsync(s->ids.p, s->snap_ids.p, sizeof(uint64_t) * N, cudaMemcpyDeviceToDevice, st));
-    if (o.rdf && o.rdf->device >= 0)
+    if (sampled)
         MD_CUDA(cudaMemcpyAsync(o.rdf->hist.p, s->snap_hist.p, sizeof(unsigned long long) * o.rdf->bins,
                                 cudaMemcpyDeviceToDevice, st));
     const int rebuilds = nl->rebuilds;
@@ -685,7 +685,7 @@ md_status run_steps_graph(md_system* s, md_forcefield* ff, md_nlist* nl, double 
         if (state[1] != 0) {
             s->graph_recoveries++;
             MD_TRY(recover_chunk(s, ff, nl, dt, n_steps, o, b, e, want_energy, want_ke, noise.p, rec.p, bussi_c,
-                                 &drifted));
+                                 g->rdf_samples > 0, &drifted));
             if (graph_mode_ok(s, ff, nl, n_steps)) MD_TRY(normalize_buffers(s, nl));
             continue;
         }
