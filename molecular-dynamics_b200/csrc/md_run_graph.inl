@@ -391,6 +391,8 @@ md_status graph_step(md_system* s, md_forcefield* ff, md_nlist* nl, const md_run
 md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_run_options& o,
                       const std::vector<RunStep>& steps, double dt, bool want_energy, bool want_ke, double bussi_c,
                       RunGraph** out) {
+    // what the key names and a capture may not make: the step kernel's block sums, with its resident grid and opt-in
+    MD_TRY(step_start_async(s, ff, nl, nullptr, nullptr, true));
     const TileGeom tg = graph_geometry(s, nl);
     const std::string key = graph_key(s, ff, nl, o, steps, dt, want_energy, want_ke, bussi_c, tg);
     auto it = s->graphs.find(key);
@@ -405,7 +407,6 @@ md_status chunk_graph(md_system* s, md_forcefield* ff, md_nlist* nl, const md_ru
     // what a capture may not do: opt the tile kernels in to the recorded tile's shared memory, create the
     // profiling events (two per step)
     const size_t tile_smem = sizeof(float4) * (tg.max_staged + 1);
-    MD_TRY(step_start_async(s, ff, nl, nullptr, nullptr, true));
     MD_CUDA(allow_smem(k_force_fp32_tile<true, true>, tile_smem));
     MD_CUDA(allow_smem(k_force_fp32_tile<true, false>, tile_smem));
     MD_CUDA(allow_smem(k_force_fp32_tile<false, true>, tile_smem));
