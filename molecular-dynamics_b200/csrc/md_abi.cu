@@ -115,12 +115,21 @@ constexpr int kThreads = 256;
 // Dynamic shared memory above this gets the opt-in attribute: static shared memory (at most 16 KB in these
 // kernels) counts against the same 48 KB default, so the threshold leaves room for it.
 constexpr size_t kSmemNoOptIn = 32 * 1024;
+constexpr size_t kSmemOptIn = 64 * 1024;  // least limit asked for: above the default, whatever the static part
 
-// Opt a kernel in to `bytes` of dynamic shared memory (not while md_run captures a graph: it sets them first)
+// Opt a kernel in to `bytes` of dynamic shared memory (not while md_run captures a graph: it sets them first). The limit
+// belongs to the kernel, for every system of the process, so it is only ever raised: another system's launches, now or in a
+// graph it captures later, may need more than this one's.
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
     if (g_capturing || bytes <= kSmemNoOptIn) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    const int limit = static_cast<int>(std::max(bytes, kSmemOptIn));
+    static std::mutex raising;  // (one for each type of kernel)
+    std::lock_guard<std::mutex> lock(raising);
+    cudaFuncAttributes now{};
+    const cudaError_t e = cudaFuncGetAttributes(&now, kernel);
+    if (e != cudaSuccess || now.maxDynamicSharedSizeBytes >= limit) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
 }
 
 // Slots of md_system::scal (device scalars)

@@ -202,8 +202,8 @@ md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const 
     RebuildArgs a{};
     const size_t smem = step_smem(nl, s, few, &a.build);
     if (prepare_only) {
-        if (s->step_resident[which] != 0 && s->step_smem[which] == smem) return MD_OK;
         MD_CUDA(allow_smem(kernel, smem));
+        if (s->step_resident[which] != 0 && s->step_smem[which] == smem) return MD_OK;
         int sms = 0, per_sm = 0;
         MD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
         MD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kRebuildThreads, smem));
