@@ -53,7 +53,16 @@ std::atomic<uint64_t> g_serial{1};  // serial numbers of force fields and lists 
 
 md_status fail(md_status s, const std::string& msg) {
     g_error = msg;
+    // a reported error is taken off the runtime's record, where the launches of the next call would find it
+    if (s == MD_ERR_CUDA) cudaGetLastError();
     return s;
+}
+
+// Keeps the first error of a list of calls that are all made
+void note(md_status& st, cudaError_t e) {
+    if (e == cudaSuccess) return;
+    if (st == MD_OK) st = fail(MD_ERR_CUDA, cudaGetErrorString(e));
+    cudaGetLastError();
 }
 
 #define MD_CUDA(call)                                                                                  \
@@ -1042,9 +1051,7 @@ md_status md_system_create(int64_t n, double box_length, int device, md_system**
     s->n = n;
     s->box = Box{box_length, 1.0 / box_length, 0.25 * box_length};
     md_status st = MD_OK;
-    auto chk = [&](cudaError_t e) {
-        if (e != cudaSuccess && st == MD_OK) st = fail(MD_ERR_CUDA, cudaGetErrorString(e));
-    };
+    auto chk = [&](cudaError_t e) { note(st, e); };
     chk(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     chk(s->pos.reserve(n));
     chk(s->vel.reserve(3 * n));

@@ -327,9 +327,7 @@ md_status md_adjoint_create(int device, int64_t n, double box_length, const doub
         a->cap = ((static_cast<int>(1.35 * est) + 24) + 7) & ~7;
     }
     md_status st = MD_OK;
-    auto chk = [&](cudaError_t e) {
-        if (e != cudaSuccess && st == MD_OK) st = fail(MD_ERR_CUDA, cudaGetErrorString(e));
-    };
+    auto chk = [&](cudaError_t e) { note(st, e); };
     const size_t N = static_cast<size_t>(n);
     chk(cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking));
     for (auto* b : {&a->pos, &a->pos0, &a->ref, &a->wv}) chk(b->reserve(N));

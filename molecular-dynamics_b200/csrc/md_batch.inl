@@ -697,9 +697,7 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
         b->cap = ((static_cast<int>(1.35 * est) + 24) + 7) & ~7;
     }
     md_status st = MD_OK;
-    auto chk = [&](cudaError_t e) {
-        if (e != cudaSuccess && st == MD_OK) st = fail(MD_ERR_CUDA, cudaGetErrorString(e));
-    };
+    auto chk = [&](cudaError_t e) { note(st, e); };
     const size_t S = slots, R = replicas;
     chk(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     chk(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
