@@ -402,13 +402,14 @@ md_status b_graph(md_batch* b, int len, cudaGraphExec_t* out, uint64_t* kernels)
         *kernels = it->second.second;
         return MD_OK;
     }
+    MD_TRY(b_build_async(b, true));
+    if (!float_mode(b) && b->opt.energy_every > 0) MD_TRY(b_alloc_records(b));
+    cudaGraph_t graph = nullptr;
+    MD_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    // (nothing returns between here and the end of the capture: the launch counter points into this frame)
     uint64_t count = 0;
     uint64_t* saved = g_launches;
     g_launches = &count;
-    cudaGraph_t graph = nullptr;
-    MD_TRY(b_build_async(b, true));
-    if (!float_mode(b) && b->opt.energy_every > 0) MD_TRY(b_alloc_records(b));
-    MD_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     g_capturing = true;
     md_status st = MD_OK;
     const int every = b->opt.energy_every;
