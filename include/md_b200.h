@@ -248,9 +248,11 @@ md_status md_run_prepare(md_system* s, md_forcefield* ff, md_nlist* nl, double d
                          const md_run_options* opts, int record);
 /* md_run's graph chunk length (1..1024 steps; 0 runs every step from the host) and test flags:
  * MD_GRAPH_TEST_RERUN makes every list rebuild on the device report an overflow, so that each chunk with a rebuild
- * reruns on the host path from its starting state (for tests of that path; the results are the same bits).
- * Drops the system's cached graphs. */
+ * reruns on the host path from its starting state (for tests of that path; the results are the same bits);
+ * MD_GRAPH_TEST_GIVE_UP makes the barriers inside such a rebuild wait for a block that does not exist, so that they
+ * give up (after about a quarter of a second) and the chunk reruns likewise. Drops the system's cached graphs. */
 #define MD_GRAPH_TEST_RERUN 1
+#define MD_GRAPH_TEST_GIVE_UP 2
 md_status md_system_set_graph(md_system* s, int chunk_steps, int flags);
 /* Graph chunk length, graphs cached, chunk graphs launched and chunks rerun on the host path. Any may be NULL. */
 md_status md_system_graph_info(const md_system* s, int* chunk_steps, uint64_t* graphs, uint64_t* launches,

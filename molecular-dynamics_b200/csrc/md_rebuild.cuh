@@ -22,7 +22,7 @@
 namespace md {
 
 constexpr int kRebuildThreads = 128;
-constexpr unsigned kBarrierPolls = 1u << 22;  // some seconds
+constexpr unsigned kBarrierPolls = 1u << 20;  // 0.23 s (N = 4,000, B200), for a wait whose partners are resident and at most some ms behind
 constexpr int kDirectScan = 16384;            // cells up to which a block adds up the counts before its own
 
 struct RebuildArgs {
@@ -44,6 +44,7 @@ struct RebuildArgs {
     int *stale, *max_count, *state;
     unsigned* barrier;  // [0] arrivals, [1] blocks done
     int report_always;
+    unsigned missing;   // for tests: blocks that the barriers wait for in vain
     // FP64: pair offsets, the records' capacity, and this step's copy of the pair count
     long long* half_off;  // nullptr: none kept
     long long* offset_sums;
@@ -61,18 +62,19 @@ struct RebuildArgs {
 };
 
 // All blocks have arrived when the count passes the next multiple of the grid. False (in every thread) if it gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned* count, int* state) {
+__device__ __forceinline__ bool grid_barrier(const RebuildArgs& a) {
     __shared__ bool ok;
+    unsigned* count = a.barrier;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        const unsigned at = atomicAdd(count, 1u), target = (at / gridDim.x + 1u) * gridDim.x;
+        const unsigned at = atomicAdd(count, 1u), target = (at / gridDim.x + 1u) * gridDim.x + a.missing;
         unsigned polls = 0, v;
         do {
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
         } while (v < target && ++polls < kBarrierPolls);
         ok = v >= target;
-        if (!ok) atomicExch(state + 1, 1);
+        if (!ok) atomicExch(a.state + 1, 1);
         __threadfence();
     }
     __syncthreads();
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
         a.cell_of[i] = c;
         a.slot[i] = atomicAdd(&a.count[c], 1);
     }
-    if (!grid_barrier(a.barrier, a.state)) return;
+    if (!grid_barrier(a)) return;
     if (first) *a.stale = 0;  // every block has read it
     // the cells' first particles (src/CellList.cpp:42-46)
     {
@@ -174,16 +176,16 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
             for (int k = p0 + static_cast<int>(threadIdx.x); k < p1; k += kRebuildThreads) mine += a.count[k];
             mine = block_sum(mine);
             if (threadIdx.x == 0) a.block_sums[blockIdx.x] = static_cast<int>(mine);
-            if (!grid_barrier(a.barrier, a.state)) return;
+            if (!grid_barrier(a)) return;
             for (int k = threadIdx.x; k < static_cast<int>(blockIdx.x); k += kRebuildThreads) before += a.block_sums[k];
             before = block_sum(before);
         }
         write_prefix(a.ncells, part, before, a.start, [&](int k) { return a.count[k]; });
     }
-    if (!grid_barrier(a.barrier, a.state)) return;
+    if (!grid_barrier(a)) return;
     for (int i = t0; i < n; i += stride) a.bucket[a.start[a.cell_of[i]] + a.slot[i]] = i;
     for (int c = t0; c < a.ncells; c += stride) a.count[c] = 0;
-    if (!grid_barrier(a.barrier, a.state)) return;
+    if (!grid_barrier(a)) return;
     // the stable order: a particle's place in its cell is the number of smaller indices there (src/CellList.cpp:48-51);
     // the reorder (src/System.cpp:42-64) into the spare arrays, and the list's own copies
     if (first) a.frames[n] = make_float4(kSentinelCoord, kSentinelCoord, kSentinelCoord, 0.0f);
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
         a.frames[k] = frame_of(p, c, a.ncps, a.cell, a.box);
         if (a.iframes) a.iframes[k] = fixed_frame_of(p, c, a.ncps, a.cell, a.box);
     }
-    if (!grid_barrier(a.barrier, a.state)) return;
+    if (!grid_barrier(a)) return;
     // the reordered arrays back into their places (the graph's kernels were recorded with those addresses)
     for (int k = t0; k < n; k += stride) {
         a.pos[k] = a.pos2[k];
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
         __syncthreads();
     }
     if (a.near_rows) {
-        if (!grid_barrier(a.barrier, a.state)) return;
+        if (!grid_barrier(a)) return;
         if (threadIdx.x < 32) sh.s_off[threadIdx.x] = a.offs.off[threadIdx.x];
         __syncthreads();
         for (int i = t0; i < n; i += stride) {
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
         }
     }
     if (a.half_off) {  // the half-list offsets (src/NeighbourList.cpp:116-127)
-        if (!grid_barrier(a.barrier, a.state)) return;
+        if (!grid_barrier(a)) return;
         const int part = (n + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
         const int p0 = min(n, static_cast<int>(blockIdx.x) * part), p1 = min(n, p0 + part);
         long long before = 0;
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
         for (int k = p0 + static_cast<int>(threadIdx.x); k < p1; k += kRebuildThreads) mine += a.counts[k].x;
         mine = block_sum(mine);
         if (threadIdx.x == 0) a.offset_sums[blockIdx.x] = mine;
-        if (!grid_barrier(a.barrier, a.state)) return;
+        if (!grid_barrier(a)) return;
         for (int k = threadIdx.x; k < static_cast<int>(blockIdx.x); k += kRebuildThreads) before += a.offset_sums[k];
         before = block_sum(before);
         write_prefix(n, part, before, a.half_off, [&](int k) { return a.counts[k].x; });

@@ -247,6 +247,7 @@ md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const 
     a.state = s->graph_state.p;
     a.barrier = s->step_barrier.p;
     a.report_always = (s->graph_flags & MD_GRAPH_TEST_RERUN) != 0;
+    a.missing = (s->graph_flags & MD_GRAPH_TEST_GIVE_UP) != 0 ? 1 : 0;
     if (ff->precision == MD_PREC_FP64) {
         a.half_off = nl->half_off.p;
         a.rec_cap = static_cast<long long>(std::min(ff->pair_r2[0].count, ff->pair_r2[1].count));
