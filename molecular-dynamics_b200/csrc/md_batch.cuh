@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kTile)
         mass[a] = mass2[a];
         ids[a] = ids2[a];
         ref_pos[a] = p;
-        frames[a] = frame_of(p, cell_sorted[a], d.ncps, d.cell, d.box);
+        frames[a] = list_frame_of(p, cell_sorted[a], d.ncps, d.cell, d.box);
     }
 }
 
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(kResortThreads)
             ids[a] = ids2[a];
             ref_pos[a] = p;
             cell_sorted[a] = c;
-            frames[a] = frame_of(p, c, d.ncps, d.cell, d.box);
+            frames[a] = list_frame_of(p, c, d.ncps, d.cell, d.box);
         }
         __syncthreads();  // the next replica's cells go where this one's are read
     }

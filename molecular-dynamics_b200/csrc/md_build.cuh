@@ -13,11 +13,12 @@
 //
 // The test: r^2 - r_l^2 = (|h|^2 - r_l^2) + |c|^2 - 2 h.c, three FMAs from sums kept per home h and candidate c, for two
 // homes at a time in packed instructions. Exactness: a candidate is accepted when that is below -margin. With
-// coordinates of at most 1.6 cell sides (c) and 0.501 (h) and sides under 4/3 r_l, all roundings together stay below
+// coordinates of at most 1.5 cell sides (c) and 0.5 (h) and sides under 4/3 r_l, all roundings together stay below
 // 7e-6 r_l^2, and the margin is 1e-5 r_l^2 + 1e-4. Every lane keeps the smallest |r^2 - r_l^2| it has met; when it falls
 // inside the margin (about one group of homes in fifty) the group is tested again with the reference's double test
-// deciding those candidates. So the rows are the reference's, bit for bit. A cell with particles outside those bounds
-// (positions outside the box) or more candidates than the shared memory holds goes through build_row.
+// deciding those candidates. So the rows are the reference's, bit for bit. A cell that has a position outside the box among
+// its candidates (list_frame_of marks them: such a particle lies outside its cell, and with 3 cells a side the frames may
+// then name another image than the nearest), or more candidates than the shared memory holds, goes through build_row.
 //
 // What bounds it: instruction issue (65 % of the slots; about 480 warp instructions a particle: a third in laying out the
 // candidates, a seventh in the tests, the rest in the rows). A thread per particle walking its candidates one by one took
@@ -62,7 +63,7 @@ struct CellItems {
     int off[kCellItems + 1];
     int own_items;  // the items before this one are j > i
     int home;       // item of the home cell's first copy (the second is the last item)
-    int odd;        // a particle outside the test's bounds
+    int odd;        // a position outside the box
 };
 
 // Fills t for home cell `cell` (one warp)
@@ -192,10 +193,7 @@ __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const f
         float4 c[kItems];
         unsigned kept[kItems];
         bool odd = false;
-        auto keep = [&](const float4& q, int code) {
-            odd |= code == 13 ? !(fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))) <= half) : !(q.w <= 7.68f * side * side);
-            return code == 13 || cell_reachable(q, half, bp.prune);
-        };
+        auto keep = [&](const float4& q, int code) { return code == 13 || cell_reachable(q, half, bp.prune); };
 #pragma unroll
         for (int q = 0; q < kItems; ++q) {
             const int r = warp * kItems + q;
@@ -208,12 +206,15 @@ __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const f
             if (r < kCellItems) {
                 const int4 item = t.cell[r];
                 const float4 shift = t.shift[r];
+                odd |= c[q].w != 0.0f;
                 c[q] = cell_candidate(c[q], shift);
                 kept[q] = __ballot_sync(kAll, lane < item.y && keep(c[q], item.z));
                 int more = 0;
-                for (int u = 32; u < item.y; u += 32)
-                    more += __popc(__ballot_sync(
-                        kAll, u + lane < item.y && keep(cell_candidate(frames[item.x + u + lane], shift), item.z)));
+                for (int u = 32; u < item.y; u += 32) {
+                    const float4 f = frames[min(item.x + u + lane, item.x + item.y - 1)];
+                    odd |= f.w != 0.0f;
+                    more += __popc(__ballot_sync(kAll, u + lane < item.y && keep(cell_candidate(f, shift), item.z)));
+                }
                 if (lane == 0) t.off[r + 1] = __popc(kept[q]) + more;
             }
         }

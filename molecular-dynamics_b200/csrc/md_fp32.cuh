@@ -51,6 +51,15 @@ __device__ __forceinline__ float4 frame_of(const double4& p, int c, int ncps, do
     return make_float4(static_cast<float>(d[0]), static_cast<float>(d[1]), static_cast<float>(d[2]), 0.0f);
 }
 
+// frame_of where a list is built: w tells the build that the position lies outside the box (0 inside). Only there do the
+// frames of a cell and its neighbours give every pair's minimum image.
+__device__ __forceinline__ float4 list_frame_of(const double4& p, int c, int ncps, double cell, const Box& box) {
+    float4 f = frame_of(p, c, ncps, cell, box);
+    const bool in = p.x >= 0.0 && p.x <= box.L && p.y >= 0.0 && p.y <= box.L && p.z >= 0.0 && p.z <= box.L;
+    f.w = in ? 0.0f : 1.0f;
+    return f;
+}
+
 constexpr double kFrameScale = 268435456.0;  // 2^28 fixed-point frame units per unit length
 constexpr double kFrameUnit = 1.0 / 268435456.0;
 
@@ -388,7 +397,7 @@ __global__ void k_frames(const double4* __restrict__ pos, int n, const int* __re
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) frames[n] = make_float4(kSentinelCoord, kSentinelCoord, kSentinelCoord, 0.0f);
     if (i >= n) return;
-    frames[i] = frame_of(pos[i], cell_sorted[i], ncps, cell, box);
+    frames[i] = list_frame_of(pos[i], cell_sorted[i], ncps, cell, box);
 }
 
 // Thread per particle over its row with neighbour frames gathered from global memory (L1/L2); rows are read

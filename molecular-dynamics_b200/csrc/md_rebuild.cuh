@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
         a.ids2[k] = a.ids[i];
         a.ref_pos[k] = p;
         a.cell_sorted[k] = c;
-        a.frames[k] = frame_of(p, c, a.ncps, a.cell, a.box);
+        a.frames[k] = list_frame_of(p, c, a.ncps, a.cell, a.box);
         if (a.iframes) a.iframes[k] = fixed_frame_of(p, c, a.ncps, a.cell, a.box);
     }
     if (!grid_barrier(a)) return;
