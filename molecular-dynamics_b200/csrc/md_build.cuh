@@ -113,14 +113,18 @@ __device__ __forceinline__ void cell_items(const int* __restrict__ cell_start, i
 
 // A candidate: its position c in the home cell's frame, and |c|^2
 __device__ __forceinline__ float4 cell_candidate(const float4& f, const float4& shift) {
-    const float x = f.x + shift.x, y = f.y + shift.y, z = f.z + shift.z;
-    return make_float4(x, y, z, fmaf(x, x, fmaf(y, y, __fmul_rn(z, z))));
+    const float x = __fadd_rn(f.x, shift.x), y = __fadd_rn(f.y, shift.y), z = __fadd_rn(f.z, shift.z);
+    return make_float4(x, y, z, __fmaf_rn(x, x, __fmaf_rn(y, y, __fmul_rn(z, z))));
 }
 
-// Is a candidate within reach of the home cube [-half, half]^3?
+// Is a candidate within reach of the home cube [-half, half]^3? Candidates are counted and then laid out by the same test, so
+// its roundings are spelled out: a product that the compiler fused with the difference in one of the two places only would
+// leave a slot that nothing writes.
+__device__ __forceinline__ float cell_half(float side) { return __fmul_rn(0.501f, side); }
 __device__ __forceinline__ bool cell_reachable(const float4& c, float half, float prune) {
-    const float x = fmaxf(fabsf(c.x) - half, 0.0f), y = fmaxf(fabsf(c.y) - half, 0.0f), z = fmaxf(fabsf(c.z) - half, 0.0f);
-    return fmaf(x, x, fmaf(y, y, z * z)) <= prune;
+    const float x = fmaxf(__fsub_rn(fabsf(c.x), half), 0.0f), y = fmaxf(__fsub_rn(fabsf(c.y), half), 0.0f),
+                z = fmaxf(__fsub_rn(fabsf(c.z), half), 0.0f);
+    return __fmaf_rn(x, x, __fmaf_rn(y, y, __fmul_rn(z, z))) <= prune;
 }
 
 // r^2 - r_l^2 of a candidate and two home particles: (-2 h, |h|^2 - r_l^2) in (hx, hy, hz, hk)
@@ -185,7 +189,7 @@ __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const f
     const int i0 = t.cell[kCellItems - 1].x, homes = t.cell[kCellItems - 1].y;
     if (homes == 0) return;
     const unsigned below = (1u << lane) - 1u;
-    const float half = 0.501f * side;
+    const float half = cell_half(side);
     {
         // Each warp takes kItems of the items, a particle per lane, all their loads in flight at once; the kept ones are
         // counted, then laid out. (A cell of more than 32 particles goes through the rest in a loop.)
