@@ -193,8 +193,8 @@ struct md_system {
     int graph_flags = 0;
     DevBuf<unsigned> step_barrier;
     DevBuf<long long> step_sums;
-    unsigned step_resident[3] = {0, 0, 0};  // resident grids of k_step_start's kinds, for the shared memory below
-    size_t step_smem[3] = {0, 0, 0};
+    unsigned step_resident[4] = {};  // resident grids of k_step_start's kinds, for the shared memory below
+    size_t step_smem[4] = {};
     DevBuf<int> graph_state, snap_flag;
     DevBuf<double> chunk_rec, chunk_noise;
     DevBuf<double4> snap_pos, snap_ref, pos_save;
@@ -251,13 +251,16 @@ struct md_nlist {
     bool use_cells = false;
     DevBuf<uint32_t> rows;
     DevBuf<int2> counts;
-    DevBuf<int> tmp_counts, cell_sorted, flags;  // flags: [0] stale, [1] max row, [2] device rebuild count
+    DevBuf<int> tmp_counts, cell_sorted, flags;  // flags: [0] stale, [1] max row, [2, 3] tile_geometry's, [4] full_cells' length,
+                                              // [5] build_stamp of the last build with a position outside the box
     DevBuf<long long> half_off, rev_off, tiles;
     DevBuf<double4> ref_pos;
     DevBuf<float4> frames;  // per-particle float coordinates for the float kernels (n + 1, sentinel last)
     DevBuf<float4> frames2; // the frames a force kernel with the fused next drift writes (then swapped in)
     DevBuf<int4> iframes;   // fixed-point frames of MD_PREC_FX64 (n)
     DevBuf<int4> iframes2;  // the fixed-point frames a FX64 force kernel with the fused next drift writes
+    DevBuf<int> full_cells; // sparse systems: cells that a build leaves to whole blocks
+    int cell_most = 0;      // most candidates of a cell (27 cells and itself), an eighth more or up to twice as many
     bool use_tiles = false; // shared-memory tile kernels (3+ cells per side and tiles that fit)
     TileGeom tiles_geom{};
     int build_kernel = -1;  // list build of the last rebuild: 0 thread per particle, 1 tiles
@@ -455,18 +458,17 @@ int initial_capacity(const md_nlist* nl, const md_system* s) {
 
 // Defined in md_abi_float.inl
 int float_lanes(int n);
-md_status frames_async(md_system* s, md_nlist* nl);
+md_status frames_async(md_system* s, md_nlist* nl, int stamp = 0);
 CellOffsets cell_offsets(const md_nlist* nl, const md_system* s);
 
 #ifndef MD_TILE_HOME_TARGET
 #define MD_TILE_HOME_TARGET 96.0
 #endif
-constexpr int kMaxStage = 4096;  // candidates of a cell held in shared memory (64 KB)
 constexpr double kTileHomeTarget = MD_TILE_HOME_TARGET;  // home particles per tile block aimed at
 
-// Segment length and shared-memory size of the tile kernels for this build. Segments aim at ~96 home
-// particles per block. The largest staged tile of the geometry is measured on the device (the cells only
-// change at rebuilds, so it holds until the next one); it must fit 3072 slots (96 KB of double4 for the
+// Segment length and shared-memory size of the tile kernels for this build, and the most candidates that a cell has (for
+// the list build). Segments aim at ~96 home particles per block. The largest staged tile of the geometry is measured on the
+// device (the cells only change at rebuilds, so it holds until the next one); it must fit 3072 slots (96 KB of double4 for the
 // FP64 kernel), shrinking kk down to one cell. Beyond 6000 slots the global-gather kernels are used instead.
 md_status tile_geometry(md_nlist* nl, md_system* s, bool* use) {
     *use = false;
@@ -476,19 +478,23 @@ md_status tile_geometry(md_nlist* nl, md_system* s, bool* use) {
     int kk = static_cast<int>(std::lround(kTileHomeTarget / std::max(avg, 1.0)));
     kk = std::clamp(kk, 1, std::min(kMaxSegment, nc - 2));
     TileGeom& g = nl->tiles_geom;
-    for (;;) {
+    for (bool first = true;; first = false) {
         g.ncps = nc;
         g.kk = kk;
         g.nseg = (nc + kk - 1) / kk;
         g.cell = s->box.L / nc;
         g.box = s->box;
-        MD_CUDA(cudaMemsetAsync(nl->flags.p + 2, 0, sizeof(int), s->stream));
+        MD_CUDA(cudaMemsetAsync(nl->flags.p + 2, 0, 2 * sizeof(int), s->stream));
         const long long segs = static_cast<long long>(nc) * nc * g.nseg;
-        k_tile_max_staged<<<blocks_for(segs, 128), 128, 0, s->stream>>>(nl->grid.start.p, g, nl->flags.p + 2);
+        k_tile_max_staged<<<blocks_for(segs + (first ? nl->grid.ncells : 0), 128), 128, 0, s->stream>>>(
+            nl->grid.start.p, g, first ? nl->grid.ncells : 0, nl->flags.p + 2);
         MD_CHECK_LAUNCH();
-        int staged = 0;
-        MD_CUDA(cudaMemcpyAsync(&staged, nl->flags.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+        int most[2] = {0, 0};
+        MD_CUDA(cudaMemcpyAsync(most, nl->flags.p + 2, sizeof most, cudaMemcpyDeviceToHost, s->stream));
         MD_TRY(sync(s));
+        const int staged = most[0];
+        // (with room to drift: graphs are kept by the build's sizes)
+        if (first && (most[1] > nl->cell_most || 2 * most[1] < nl->cell_most)) nl->cell_most = most[1] + most[1] / 8;
         g.max_staged = std::max(staged, 1);
         if (staged <= 3072 || kk == 1) {
             *use = staged <= 6000;
@@ -500,48 +506,120 @@ md_status tile_geometry(md_nlist* nl, md_system* s, bool* use) {
 
 unsigned tile_blocks(const TileGeom& g) { return static_cast<unsigned>(g.ncps) * g.ncps * g.nseg; }
 
-// Parameters of the cell build (md_build.cuh) for a list of radius^2 g.rl2 and cells of per_cell particles on average
-CellBuild cell_build_params(const ListGeom& g, double per_cell) {
+constexpr size_t kBuildSmem = 200 * 1024;
+// Names the build in progress in flags[5]
+int build_stamp(const md_nlist* nl) { return static_cast<int>(nl->builds % 1'000'000'000) + 1; }
+// Is the list of a system of ncells cells with per_cell particles each built a cell per warp (build_cells_sparse)? With few
+// cells a block finishes one sooner (N = 2,000, 9.3 a cell: 100 us a whole build against 122). In md_run's graphs, whose
+// rebuilds have no other kernel (FP32FX, us a step, cell per block / per warp): N = 500,000, 6.8 a cell: 162 / 136; 800,000,
+// 9.4 a cell: 230 / 214. cells_build_async's host-path builds go on to a cell per block at 9 (N = 100,000, 9.4 a cell: 184 us
+// a whole build, by warps 190; 7.2 a cell: 188 / 152).
+constexpr int kWideBuildCells = 148 * 14;
+bool sparse_cells(double ncells, double per_cell) { return per_cell < (ncells < kWideBuildCells ? 6.0 : 10.5); }
+
+// Parameters of the cell build (md_build.cuh) for a list of radius^2 g.rl2 and cells of per_cell particles on average, for
+// blocks of `warps` warps with `homes` particles each and room for at least `room` candidates. Returns the dynamic shared
+// memory.
+size_t cell_build_params(CellBuild& bp, const ListGeom& g, double per_cell, int room, int warps, int homes) {
     const double margin = 1e-5 * g.rl2 + 1e-4;
-    CellBuild bp{};
+    bp = CellBuild{};
     bp.geom = g;
     bp.rl2 = static_cast<float>(g.rl2);
     bp.margin = static_cast<float>(margin);
     bp.prune = static_cast<float>(g.rl2 * 1.0001 + 2.0 * margin);  // well past what the test could accept
-    // room for the candidates of nearly every cell of a uniform system (four fifths of 28 cells and six deviations)
-    const double mean = 0.8 * kCellItems * per_cell;
-    bp.stage = (std::min(static_cast<int>(mean + 6.0 * std::sqrt(mean)), kMaxStage) + 31) & ~31;
-    return bp;
+    // room for the candidates of nearly every cell of a uniform system: four fifths of 28 cells and six deviations
+    const double near = 0.8 * kCellItems * per_cell, stage = std::max(near + 6.0 * std::sqrt(near), static_cast<double>(room));
+    const size_t row_smem = cell_build_smem(0, g.cap, warps, homes), word = cell_build_smem(32, g.cap, warps, homes) - row_smem;
+    if (row_smem + word > kBuildSmem) return 0;  // rows too long for the shared memory: stage 0
+    const int words = std::min(static_cast<int>(stage) / 32 + 1, static_cast<int>((kBuildSmem - row_smem) / word));
+    bp.stage = 32 * words;
+    return cell_build_smem(bp.stage, g.cap, warps, homes);
 }
 
-// The list build kernel (md_build.cuh) on the system's stream, from the cells, frames and positions of this build; with
-// prepare_only its shared-memory opt-in alone, which a capture may not make. Blocks of 4 warps, 4 particles a warp at a
-// time, spend the fewest instructions (N = 864,000: 514 us; 2 particles: 551; blocks of 2 warps: 720); with few cells, 8
-// warps and 2 particles finish a cell soonest (N = 2,048: 90 us a whole rebuild against 102). Rows too long for the
-// shared memory go through the kernel's thread-per-particle path (stage 0).
-constexpr int kWideBuildCells = 148 * 14;
-constexpr size_t kBuildSmem = 200 * 1024;
-md_status cells_build_async(md_nlist* nl, md_system* s, bool prepare_only = false) {
+// Room for the fullest cell of a system that is not uniform: `most` candidates (all of its 27 cells and itself again), of
+// which four fifths are within reach; 0 for a uniform one
+int build_room(int most, double per_cell) { return most > 1.6 * kCellItems * per_cell ? static_cast<int>(0.85 * most) : 0; }
+
+// Cells that a warp looks at together: enough warps first
+int sparse_group(double ncells) { return std::clamp(static_cast<int>(ncells / (148 * 32)), 1, 32); }
+
+// The share of a warp in a sparse system (build_cells_sparse): the fullest cell's candidates (most; 0: not known), none left
+// out, up to kMostWarpStage; fuller cells go to a block. Returns the dynamic shared memory, 0 if rows are too long for it.
+size_t sparse_build_params(CellBuild& bp, double ncells, double per_cell, int most) {
+    const int want = most > 0 ? most : static_cast<int>(1.5 * kCellItems * per_cell) + 32;
+    bp.warp_stage = std::min((want + 31) & ~31, kMostWarpStage);
+    bp.group = sparse_group(ncells);
+    const size_t smem = kSparseWarps * sparse_smem_warp(bp.warp_stage, bp.geom.cap);
+    if (smem <= kBuildSmem) return smem;
+    bp.warp_stage = 0;
+    return 0;
+}
+
+// The list build kernel for the cells, frames and positions of this build, on the system's stream. They write the same rows.
+// Times are whole builds (B200, us; uniform systems of r_l = 2.8 unless said otherwise).
+//   - thin gases (under 3 particles a cell, no full cell): a thread per particle; a block or warp per cell spends itself on
+//     near-empty cells: N = 100,000, density 0.03: tile 306, cells 652, threads 145; 0.1: 217, 329, 170; N = 864,000,
+//     density 0.1: 830, 2,158, 513. Below 50,000 particles a warp per cell is as good: N = 8,000, density 0.1: 118 against 141.
+//   - tiles: large systems that are neither gas nor liquid, where cells hold too few particles to fill a warp (N = 864,000,
+//     density 0.3 / 0.5 / 0.6: tile 600 / 688 / 711, cells 905 / 782 / 748) or few of them hold all (a slab in a third of
+//     the box: 895 against 938 by warps and blocks); at density 0.8442: 727 against 680. And cells of 100 and more, whose
+//     candidates leave room for a block or two on an SM (N = 100,000, r_l = 5.5: 930 against 1,003).
+//   - a warp per cell (sparse_cells), and blocks for the cells that are too full for it: N = 100,000, density 0.3: cells 188,
+//     tile 174, warps 152; a slab of 32,000: tile 144, warps 148; a droplet of 8,000: 146, 142.
+//   - a block per cell: blocks of 4 warps, 4 particles a warp at a time, spend the fewest instructions (N = 864,000: 514 us;
+//     2 particles: 551; blocks of 2 warps: 720). With few cells, 8 warps and 2 particles finish a cell soonest (N = 2,048: 90
+//     us against 102), and with cells of 50 and more they bring twice the warps onto an SM (N = 864,000, r_l = 4: 1,397
+//     against 1,855).
+md_status cells_build_async(md_nlist* nl, md_system* s) {
     const CellGrid& g = nl->grid;
     const ListGeom geo{s->box, nl->rl2, g.ncps, 1, nl->cap, static_cast<uint32_t>(s->n) | (kSentinelCode << kCodeShift)};
-    CellBuild bp = cell_build_params(geo, static_cast<double>(s->n) / g.ncells);
-    auto go = [&](auto kernel, int warps, int homes) -> md_status {
-        size_t smem = cell_build_smem(bp.stage, nl->cap, warps, homes);
-        if (smem > kBuildSmem) {
-            bp.stage = 0;
-            smem = 0;
-        }
+    const double per_cell = static_cast<double>(s->n) / g.ncells;
+    const float side = static_cast<float>(s->box.L / g.ncps);
+    CellBuild bp;
+    auto go = [&](auto kernel, int warps, int homes, unsigned blocks) -> md_status {
+        const size_t smem = cell_build_params(bp, geo, per_cell, build_room(nl->cell_most, per_cell), warps, homes);
         MD_CUDA(allow_smem(kernel, smem));
-        if (prepare_only) return MD_OK;
-        kernel<<<g.ncells, 32 * warps, smem, s->stream>>>(nl->frames.p, s->pos.p, g.start.p,
-                                                          static_cast<float>(s->box.L / g.ncps), bp, nl->rows.p,
-                                                          nl->counts.p, nl->flags.p + 1);
+        kernel<<<blocks, 32 * warps, smem, s->stream>>>(nl->frames.p, s->pos.p, g.start.p, side, bp, nl->rows.p, nl->counts.p,
+                                                        nl->flags.p + 1, nl->full_cells.p, nl->flags.p + 4);
         MD_CHECK_LAUNCH();
         return MD_OK;
     };
-    if (g.ncells < kWideBuildCells) return go(k_nlist_build_cells<8, 2, 16>, 8, 2);
-    return cell_round(static_cast<double>(s->n) / g.ncells) == 24 ? go(k_nlist_build_cells<4, 4, 24>, 4, 4)
-                                                                  : go(k_nlist_build_cells<4, 4, 16>, 4, 4);
+    const int n = static_cast<int>(s->n);
+    const bool gas = nl->cell_most <= kMostWarpStage;  // no cell that a warp could not build
+    if (gas && per_cell < 3.0 && n >= 50'000) {
+        k_nlist_build<<<blocks_for(n, 128), 128, 0, s->stream>>>(s->pos.p, n, geo, nl->cell_sorted.p, g.start.p, nl->rows.p,
+                                                                  nl->counts.p, nl->flags.p + 1);
+        MD_CHECK_LAUNCH();
+        return MD_OK;
+    }
+    if (nl->use_tiles && (per_cell >= 100.0 || (n >= 200'000 && per_cell < 15.0 && !(gas && per_cell < 4.0)))) {
+        cell_build_params(bp, geo, per_cell, 0, 4, 4);
+        const TileBuild tb{geo, bp.rl2 - bp.margin, bp.rl2 + bp.margin, build_stamp(nl)};
+        const size_t smem = sizeof(float4) * nl->tiles_geom.max_staged;
+        MD_CUDA(allow_smem(k_nlist_build_tile, smem));
+        k_nlist_build_tile<<<tile_blocks(nl->tiles_geom), kTileThreads, smem, s->stream>>>(
+            nl->frames.p, s->pos.p, g.start.p, nl->cell_sorted.p, nl->tiles_geom, tb, cell_offsets(nl, s), nl->flags.p + 5,
+            nl->rows.p, nl->counts.p, nl->flags.p + 1);
+        MD_CHECK_LAUNCH();
+        return MD_OK;
+    }
+    if (per_cell < 9.0 && sparse_cells(g.ncells, per_cell)) {
+        cell_build_params(bp, geo, per_cell, 0, kSparseWarps, kSparseHomes);
+        const size_t smem = sparse_build_params(bp, g.ncells, per_cell, nl->cell_most);
+        if (bp.warp_stage) {
+            MD_CUDA(nl->full_cells.reserve(g.ncells));
+            MD_CUDA(allow_smem(k_nlist_build_sparse, smem));
+            k_nlist_build_sparse<<<blocks_for(g.ncells, kSparseWarps * bp.group), 32 * kSparseWarps, smem, s->stream>>>(
+                nl->frames.p, s->pos.p, g.start.p, g.ncells, side, bp, nl->rows.p, nl->counts.p, nl->flags.p + 1,
+                nl->full_cells.p, nl->flags.p + 4);
+            MD_CHECK_LAUNCH();
+            if (nl->cell_most <= bp.warp_stage) return MD_OK;  // no cell is too full for a warp
+            return go(k_nlist_build_cells<4, 4, 16, true>, 4, 4, std::min(g.ncells, 148 * 8));
+        }
+    }
+    if (g.ncells < kWideBuildCells || per_cell >= 50.0) return go(k_nlist_build_cells<8, 2, 16, false>, 8, 2, g.ncells);
+    return cell_round(per_cell) == 24 ? go(k_nlist_build_cells<4, 4, 24, false>, 4, 4, g.ncells)
+                                      : go(k_nlist_build_cells<4, 4, 16, false>, 4, 4, g.ncells);
 }
 
 // NeighbourList::build (src/NeighbourList.cpp:55-134) on the device. The reference builds the cell list,
@@ -573,19 +651,19 @@ md_status nlist_build(md_nlist* nl, md_system* s) {
         for (int& v : nl->variant) v = -1;  // a new system: tune the force kernels again
     }
     MD_CUDA(nl->counts.reserve(n));
-    MD_CUDA(nl->flags.reserve(4));
+    MD_CUDA(nl->flags.reserve(6));
     MD_CUDA(nl->half_off.reserve(n + 1));
     MD_CUDA(nl->tmp_counts.reserve(n));
     MD_CUDA(nl->tiles.reserve(scan_tiles_needed(n)));
     nl->use_tiles = false;
     if (nl->use_cells && n > 0) {
-        MD_TRY(frames_async(s, nl));  // float frames of the new cells (the tile build's prefilter reads them)
+        MD_TRY(frames_async(s, nl, build_stamp(nl)));  // float frames of the new cells (the list builds read them)
         MD_TRY(tile_geometry(nl, s, &nl->use_tiles));
     }
     const uint32_t sentinel = static_cast<uint32_t>(n) | (kSentinelCode << kCodeShift);
     for (int attempt = 0; attempt < 4; ++attempt) {
         MD_CUDA(nl->rows.reserve(row_buffer_entries(n, nl->cap)));
-        MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, 4 * sizeof(int), s->stream));
+        MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, 5 * sizeof(int), s->stream));
         if (n > 0 && nl->use_tiles && nl->build_pin != 0) {
             MD_TRY(cells_build_async(nl, s));
             nl->build_kernel = 1;

@@ -38,11 +38,13 @@ CellOffsets cell_offsets(const md_nlist* nl, const md_system* s) {
     return o;
 }
 
-md_status frames_async(md_system* s, md_nlist* nl) {
+// stamp (not 0): flags[5] gets it if a position lies outside the box
+md_status frames_async(md_system* s, md_nlist* nl, int stamp) {
     const int n = static_cast<int>(s->n);
     MD_CUDA(nl->frames.reserve(static_cast<size_t>(n) + 1));
     k_frames<<<blocks_for(n + 1, kThreads), kThreads, 0, s->stream>>>(s->pos.p, n, nl->cell_sorted.p, nl->grid.ncps,
-                                                                      cell_side(nl, s), s->box, nl->frames.p);
+                                                                      cell_side(nl, s), s->box, nl->frames.p,
+                                                                      nl->flags.p + 5, stamp);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }
@@ -212,7 +214,7 @@ md_status ensure_near_first(md_forcefield* ff, md_system* s, md_nlist* nl) {
     MD_CUDA(nl->frames2.reserve(static_cast<size_t>(n) + 1));
     k_frames<<<blocks_for(n + 1, kThreads), kThreads, 0, s->stream>>>(nl->ref_pos.p, n, nl->cell_sorted.p,
                                                                       nl->grid.ncps, cell_side(nl, s), s->box,
-                                                                      nl->frames2.p);
+                                                                      nl->frames2.p, nullptr, 0);
     MD_CHECK_LAUNCH();
     MD_TRY(split_rows_async(s, nl, nl->frames2.p, static_cast<float>(near2), s->stream));
     nl->nf_build = nl->builds;

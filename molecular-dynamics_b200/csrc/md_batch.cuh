@@ -42,7 +42,7 @@ struct BRep {
     int ncps;            // cells per side
     int ncells;          // ncps^3
     int cell_off;        // first cell of the count/cursor arrays
-    int use_cells;       // ncps >= 3 (src/NeighbourList.cpp:69)
+    int use_cells;       // ncps >= 3 (src/NeighbourList.cpp:69); 2: so few particles a cell that threads build rows
     int tile_off;        // first tile
     int chunk_off;       // first 1024-particle block of the kinetic-energy sums
 };
@@ -144,9 +144,12 @@ __global__ void k_b_clear_scale(int R, double2* __restrict__ scale) {
 
 // ---- rebuild ------------------------------------------------------------------------------------------------
 
-// Work items of a replica's list build: its cells, or groups of kAllGroup slots in a box under 3 cells per side
+// Work items of a replica's list build: its cells, its tiles where threads build rows, or groups of kAllGroup slots in a box
+// under 3 cells per side
 constexpr int kAllGroup = 16;
-__host__ __device__ __forceinline__ int build_items(const BRep& d) { return d.use_cells ? d.ncells : d.np / kAllGroup; }
+__host__ __device__ __forceinline__ int build_items(const BRep& d) {
+    return d.use_cells == 1 ? d.ncells : d.use_cells == 2 ? d.np / kTile : d.np / kAllGroup;
+}
 
 // One block. Reads and clears the stale flags, lists the stale replicas and their tiles in replica order
 // (work[0] replicas, work[1] tiles, work[2] list-build items, those before stale replica w in stale_items[w]) and counts
@@ -465,13 +468,15 @@ __global__ void __launch_bounds__(kResortThreads)
 }
 
 // The list build of the stale replicas (build_cell, with slots for indices): blocks take their cells in turn, and groups
-// of particles of replicas under 3 cells per side, a warp per particle. bp.geom's box and cells per side are set per replica.
+// of particles of replicas under 3 cells per side, a warp per particle. In thin gases (kThinReplica) a block takes a tile, a
+// thread per particle. bp.geom's box and cells per side are set per replica. max_count as in build_cell.
 template <int kWarps, int kHomes, int kRound>
 __global__ void __launch_bounds__(32 * kWarps)
     k_b_nlist_build(const BRep* __restrict__ reps, const int* __restrict__ stale_reps, const int* __restrict__ stale_items,
                     const int* __restrict__ work, const double4* __restrict__ pos, const float4* __restrict__ frames,
-                    const int* __restrict__ start, CellBuild bp, uint32_t* __restrict__ rows, int2* __restrict__ counts,
-                    int* __restrict__ max_count) {
+                    const int* __restrict__ start, const int* __restrict__ cell_sorted, CellBuild bp,
+                    uint32_t* __restrict__ rows, int2* __restrict__ counts, int* __restrict__ max_count) {
+    static_assert(kTile == 32 * kWarps, "a thread per particle of a tile");
     extern __shared__ float4 sm_cell[];
     __shared__ CellItems t;
     const int nr = work[0], total = work[2];
@@ -487,11 +492,15 @@ __global__ void __launch_bounds__(32 * kWarps)
         bp.geom.ncps = d.ncps;
         bp.geom.use_cells = d.use_cells;
         const int* st = start + d.cell_off + r;
-        if (d.use_cells) {
-            build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, st, item - stale_items[lo],
-                                               static_cast<float>(d.cell), bp, rows, counts, max_count);
+        const int part = item - stale_items[lo];
+        if (d.use_cells == 1) {
+            build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, st, part, static_cast<float>(d.cell), bp, rows, counts,
+                                               max_count);
+        } else if (d.use_cells == 2) {
+            const int i = part * kTile + static_cast<int>(threadIdx.x);
+            if (i < d.n) build_row(pos, bp.geom, d.off + i, cell_sorted[d.off + i], st, rows, counts, max_count);
         } else {
-            const int i0 = (item - stale_items[lo]) * kAllGroup;
+            const int i0 = part * kAllGroup;
             for (int i = i0 + (threadIdx.x >> 5); i < i0 + kAllGroup && i < d.n; i += kWarps)
                 build_row_all(pos, d.off, d.off + d.n, bp.geom, d.off + i, rows, counts, max_count);
         }

@@ -18,6 +18,7 @@ struct md_batch {
     int build_items = 0;    // list-build work items of all replicas (cells, or tiles of boxes without cells)
     double per_cell = 0.0;  // particles per cell of the densest replica
     double mean_cell = 0.0;  // and of all replicas with cells
+    int room = 0, stage = 0;  // candidates of a cell that the list build is asked to hold, and holds
     int most_n = 0, most_cells = 0;  // the largest replica's particles, the most cells of one
     std::vector<BRep> reps_h;
     DevBuf<BRep> reps;
@@ -145,24 +146,39 @@ unsigned per_replica(const md_batch* b, int threads) { return blocks_for(b->R, t
 
 bool float_mode(const md_batch* b) { return b->opt.precision != MD_PREC_FP64; }
 
+void b_drop_graphs(md_batch* b) {
+    for (auto& g : b->graphs) cudaGraphExecDestroy(g.second.first);
+    b->graphs.clear();
+}
+
+// Replicas with fewer particles a cell than this have their rows built by a thread per particle: a block a
+// cell spends itself on empty cells (64 gases of 2,048 at density 0.005, 0.12 a cell, us a step: 265 by cells, 87; 128 of 500
+// at 0.05, 1.5 a cell: 51 by cells)
+constexpr double kThinReplica = 0.5;
+
 // The list build kernel over the stale replicas' cells (prepare_only: its shared-memory opt-in alone, which a capture
 // may not make). Rows too long for the kernel's shared memory go through its thread-per-particle path (stage 0).
 md_status b_build_async(md_batch* b, bool prepare_only) {
     const ListGeom geo{Box{}, b->rl2, 0, 1, b->cap, static_cast<uint32_t>(b->slots) | (kSentinelCode << kCodeShift)};
-    CellBuild bp = cell_build_params(geo, b->per_cell);
-    size_t smem = cell_build_smem(bp.stage, b->cap, 4, 4);
-    if (smem > kBuildSmem) {
-        bp.stage = 0;
-        smem = 0;
-    }
+    CellBuild bp;
+    const size_t smem = cell_build_params(bp, geo, b->per_cell, b->room, 4, 4);
+    b->stage = bp.stage;
     const auto kernel = cell_round(b->mean_cell) == 24 ? k_b_nlist_build<4, 4, 24> : k_b_nlist_build<4, 4, 16>;
     MD_CUDA(allow_smem(kernel, smem));
     if (prepare_only) return MD_OK;
     const unsigned grid = static_cast<unsigned>(std::min(b->build_items, 148 * 32));
     kernel<<<grid, 128, smem, b->stream>>>(b->reps.p, b->stale_reps.p, b->stale_items.p, b->work.p, b->pos.p, b->frames.p,
-                                           b->start.p, bp, b->rows.p, b->counts.p, b->flags.p);
+                                           b->start.p, b->cell_sorted.p, bp, b->rows.p, b->counts.p, b->flags.p);
     MD_CHECK_LAUNCH();
     return MD_OK;
+}
+
+// A build that met a cell with many more candidates than it has room for (such cells go through build_row): room for it from
+// the next captured graph on
+void b_adapt_room(md_batch* b) {
+    if (b->h_flags[1] <= b->stage + b->stage / 4) return;
+    b->room = b->h_flags[1] + b->h_flags[1] / 8;
+    b_drop_graphs(b);
 }
 
 // Replicas small enough to be resorted by a block each (k_b_resort)
@@ -439,11 +455,6 @@ md_status b_graph(md_batch* b, int len, cudaGraphExec_t* out, uint64_t* kernels)
     return MD_OK;
 }
 
-void b_drop_graphs(md_batch* b) {
-    for (auto& g : b->graphs) cudaGraphExecDestroy(g.second.first);
-    b->graphs.clear();
-}
-
 md_status b_copy(void* dst, const void* src, size_t bytes, md_batch* b) {
     MD_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, b->stream));
     return MD_OK;
@@ -579,10 +590,11 @@ md_status b_initial_build(md_batch* b) {
         MD_TRY(b_alloc_rows(b));
         std::vector<int> ones(b->R, 1);
         MD_CUDA(cudaMemcpyAsync(b->stale.p, ones.data(), sizeof(int) * b->R, cudaMemcpyHostToDevice, b->stream));
-        MD_CUDA(cudaMemsetAsync(b->flags.p, 0, sizeof(int), b->stream));
+        MD_CUDA(cudaMemsetAsync(b->flags.p, 0, 2 * sizeof(int), b->stream));
         MD_TRY(b_rebuild_async(b));
-        MD_CUDA(cudaMemcpyAsync(b->h_flags, b->flags.p, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+        MD_CUDA(cudaMemcpyAsync(b->h_flags, b->flags.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
         MD_TRY(bsync(b));
+        b_adapt_room(b);
         if (b->h_flags[0] <= b->cap) {
             // a repeated build sorted an already sorted state (identity order); it counts once
             std::vector<unsigned long long> one(b->R, 1);
@@ -670,12 +682,14 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
         d.use_cells = d.ncps >= 3 ? 1 : 0;  // src/NeighbourList.cpp:69
         d.tile_off = off / kTile;
         d.chunk_off = chunk_off;
-        b->build_items += md::build_items(d);
         if (d.use_cells) {
-            b->per_cell = std::max(b->per_cell, static_cast<double>(d.n) / d.ncells);
+            const double per_cell = static_cast<double>(d.n) / d.ncells;
+            b->per_cell = std::max(b->per_cell, per_cell);
             celled += d.n;
             cells_used += d.ncells;
+            if (per_cell < kThinReplica) d.use_cells = 2;
         }
+        b->build_items += md::build_items(d);
         b->most_n = std::max(b->most_n, d.n);
         b->most_cells = std::max(b->most_cells, d.ncells);
         for (int t = 0; t < d.np / kTile; ++t) tile_rep[d.tile_off + t] = r;
@@ -723,7 +737,7 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
     chk(b->stale_tiles.reserve(b->tiles));
     chk(b->work.reserve(3));
     chk(b->item_off.reserve(R + 1));
-    chk(b->flags.reserve(1));
+    chk(b->flags.reserve(2));
     chk(b->acc.reserve(4 * R));
     for (auto* buf : {&b->rebuilds, &b->inside, &b->s_rebuilds}) chk(buf->reserve(R));
     for (auto* buf : {&b->ke, &b->tmp_pe, &b->tmp_w}) chk(buf->reserve(R));
@@ -898,7 +912,7 @@ md_status md_batch_run_records(md_batch* b, int64_t n_steps, double* pe, double*
             if (b->opt.thermostat == 2)
                 MD_CUDA(cudaMemcpyAsync(b->noise.p, draws, sizeof(double) * half, cudaMemcpyHostToDevice, b->stream));
             MD_TRY(b_snapshot(b, false));
-            MD_CUDA(cudaMemsetAsync(b->flags.p, 0, sizeof(int), b->stream));
+            MD_CUDA(cudaMemsetAsync(b->flags.p, 0, 2 * sizeof(int), b->stream));
             MD_TRY(b_graph(b, len, &g, &kernels));
             MD_CUDA(cudaGraphLaunch(g, b->stream));
             b->launches += kernels;
@@ -906,7 +920,7 @@ md_status md_batch_run_records(md_batch* b, int64_t n_steps, double* pe, double*
             if (samples > 0)
                 MD_CUDA(cudaMemcpyAsync(b->h_rec, b->rec.p, sizeof(double) * kRecRows * samples * R, cudaMemcpyDeviceToHost,
                                         b->stream));
-            MD_CUDA(cudaMemcpyAsync(b->h_flags, b->flags.p, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+            MD_CUDA(cudaMemcpyAsync(b->h_flags, b->flags.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
             // the next chunk's draws are made while this one runs
             const int64_t next = done + len;
             if (attempt == 0 && next < n_steps)
@@ -917,6 +931,7 @@ md_status md_batch_run_records(md_batch* b, int64_t n_steps, double* pe, double*
                 continue;
             }
             ok = true;
+            b_adapt_room(b);
             for (int s = 0; s < samples; ++s) {
                 const int64_t row = done / (every > 0 ? every : 1) + s;
                 for (int r = 0; r < R; ++r) {

@@ -37,10 +37,13 @@ struct CellBuild {
     float rl2;      // r_l^2
     float margin;   // |float r^2 - r_l^2| up to this: decided in double
     float prune;    // candidates farther than this from the home cube (squared) are left out
-    int stage;      // candidates the shared memory holds (multiple of 32)
+    int stage;      // candidates the shared memory holds (multiple of 32; 0: rows too long, every cell through build_row)
+    int warp_stage; // sparse systems: candidates that a warp lays out by itself (multiple of 32); 0: blocks build every cell
+    int group;      // cells that a warp looks at together then (at most 32)
 };
 
 constexpr int kCellItems = 28;  // 27 cells, the home cell twice
+constexpr float kCellFar = 1.0e30f;  // |c|^2 of an empty candidate
 
 __host__ __device__ inline int cell_row_pitch(int cap) { return cap + 4; }
 inline size_t cell_build_smem(int stage, int cap, int warps, int homes) {
@@ -139,18 +142,18 @@ __device__ __forceinline__ float2 cell_gap(const float4& q, const float2& hx, co
 // reference's double test on the candidates inside the margin. Out of line: one group in fifty comes here.
 template <int kHomes>
 __device__ __noinline__ void cell_masks_exact(const float4* cand, const uint32_t* entries, int words, const float4* home,
-                                              int left, int i, const double4* __restrict__ pos, const CellBuild& bp,
-                                              uint32_t* masks) {
+                                              int left, int i, const double4* __restrict__ pos, const ListGeom geom,
+                                              float rl2, float margin, uint32_t* masks) {
     const int lane = threadIdx.x & 31;
     for (int k = 0; k < kHomes && k < left; ++k) {
         const float4 f = home[k];
         const float2 hx = make_float2(-2.0f * f.x, 0.0f), hy = make_float2(-2.0f * f.y, 0.0f),
-                     hz = make_float2(-2.0f * f.z, 0.0f), hk = make_float2(f.w - bp.rl2, 0.0f);
+                     hz = make_float2(-2.0f * f.z, 0.0f), hk = make_float2(f.w - rl2, 0.0f);
         for (int w = 0; w < words; ++w) {
             const float gap = cell_gap(cand[32 * w + lane], hx, hy, hz, hk).x;
-            bool take = gap < -bp.margin;
-            if (fabsf(gap) <= bp.margin)
-                take = within_list(pos[i + k], pos[entries[32 * w + lane] & kIndexMask], bp.geom);
+            bool take = gap < -margin;
+            if (fabsf(gap) <= margin)
+                take = within_list(pos[i + k], pos[entries[32 * w + lane] & kIndexMask], geom);
             const unsigned m = __ballot_sync(0xffffffffu, take);
             if (lane == 0) masks[w * kHomes + k] = m;
         }
@@ -166,23 +169,167 @@ inline int cell_round(double per_cell) {
     return words > 18.0 && words <= 24.0 ? 24 : 16;
 }
 
+// kHomes home particles for the test: (-2 h, |h|^2 - r_l^2) in pairs
+template <int kHomes>
+struct CellHomes {
+    float2 x[kHomes / 2], y[kHomes / 2], z[kHomes / 2], k[kHomes / 2];
+};
+// home[k]: the candidate of the group's particle k < left
+template <int kHomes>
+__device__ __forceinline__ CellHomes<kHomes> cell_homes(const float4* home, int left, float rl2) {
+    CellHomes<kHomes> hm;
+#pragma unroll
+    for (int k = 0; k < kHomes; ++k) {
+        float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float sq = kCellFar;
+        if (k < left) {
+            f = home[k];
+            sq = f.w - rl2;
+        }
+        (k & 1 ? hm.x[k / 2].y : hm.x[k / 2].x) = -2.0f * f.x;
+        (k & 1 ? hm.y[k / 2].y : hm.y[k / 2].x) = -2.0f * f.y;
+        (k & 1 ? hm.z[k / 2].y : hm.z[k / 2].x) = -2.0f * f.z;
+        (k & 1 ? hm.k[k / 2].y : hm.k[k / 2].x) = sq;
+    }
+    return hm;
+}
+
+// The masks of a group of homes over `words` words of candidates (one warp): masks[w * kHomes + k]. home: the group's
+// candidates, i: its first particle, left: its real ones.
+template <int kHomes>
+__device__ __forceinline__ void cell_masks(const float4* cand, const uint32_t* entries, int words, const float4* home, int left,
+                                           int i, const double4* __restrict__ pos, const CellBuild& bp, uint32_t* masks) {
+    static_assert(kHomes == 2 || kHomes == 4, "masks are stored as 8 or 16 bytes");
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const CellHomes<kHomes> hm = cell_homes<kHomes>(home, left, bp.rl2);
+    float nearest = kCellFar;
+    for (int w = 0; w < words; ++w) {
+        const float4 q = cand[32 * w + lane];
+        unsigned m[kHomes];
+#pragma unroll
+        for (int p = 0; p < kHomes / 2; ++p) {
+            const float2 gap = cell_gap(q, hm.x[p], hm.y[p], hm.z[p], hm.k[p]);
+            nearest = fminf(nearest, fminf(fabsf(gap.x), fabsf(gap.y)));
+            m[2 * p] = __ballot_sync(kAll, gap.x < -bp.margin);
+            m[2 * p + 1] = __ballot_sync(kAll, gap.y < -bp.margin);
+        }
+        if (lane == 0) {
+            if constexpr (kHomes == 4) reinterpret_cast<uint4*>(masks)[w] = make_uint4(m[0], m[1], m[2], m[3]);
+            else reinterpret_cast<uint2*>(masks)[w] = make_uint2(m[0], m[1]);
+        }
+    }
+    if (__any_sync(kAll, nearest <= bp.margin))
+        cell_masks_exact<kHomes>(cand, entries, words, home, left, i, pos, bp.geom, bp.rl2, bp.margin, masks);
+    __syncwarp();
+}
+
+// Where the home cell's two copies and the items before a row's j < i lie among a cell's candidates
+struct CellOrder {
+    int home0, home1, own_end;
+};
+
+// Adds the accepted candidates of `words` words to the rows of a group of homes (one warp): kLanes lanes per home particle, kWords adjacent mask words a lane, kRound words at a time. h: this lane's home
+// particle in the cell (real: there is one), mine: its row in shared memory, len and own: its entries so far.
+template <int kHomes, int kRound>
+__device__ __forceinline__ void cell_append(const uint32_t* entries, const uint32_t* masks, int words, const CellOrder& order, int h, bool real, int cap, uint32_t* mine, int& len,
+                                            int& own) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int kLanes = 32 / kHomes, kWords = kRound / kLanes;
+    const int lane = threadIdx.x & 31, k = lane / kLanes, l = lane % kLanes;
+    for (int w0 = 0; w0 < words; w0 += kRound) {
+        uint32_t bits[kWords];
+        int c = 0, c_own = 0;
+#pragma unroll
+        for (int u = 0; u < kWords; ++u) {
+            const int w = w0 + l * kWords + u, v = 32 * w;
+            bits[u] = real && w < words ? masks[w * kHomes + k] : 0u;
+            // in the home cell's first copy j > i, in the second j < i
+            bits[u] &= (~bits_from(order.home0 - v) | bits_from(order.home0 + h + 1 - v)) & ~bits_from(order.home1 + h - v);
+            c += __popc(bits[u]);
+            c_own += __popc(bits[u] & ~bits_from(order.own_end - v));
+        }
+        int inc = c | (c_own << 16);  // both counts in one scan (kRound words hold far fewer than 65,536)
+#pragma unroll
+        for (int o = 1; o < kLanes; o <<= 1) {
+            const int y = __shfl_up_sync(kAll, inc, o, kLanes);
+            inc += l >= o ? y : 0;
+        }
+        int at = len + (inc & 0xffff) - c;
+        const int sums = __shfl_sync(kAll, inc, kLanes - 1, kLanes);
+        len += sums & 0xffff;
+        own += sums >> 16;
+        const bool fits = __all_sync(kAll, len <= cap);
+#pragma unroll
+        for (int u = 0; u < kWords; ++u) {
+            uint32_t left = __brev(bits[u]);  // the first candidate in the highest bit
+            const uint32_t* in = entries + 32 * (w0 + l * kWords + u);
+            if (fits) {
+                uint32_t* out = mine + at;
+                at += __popc(left);
+                while (left) {
+                    const int b = __clz(left);
+                    left ^= 0x80000000u >> b;
+                    *out++ = in[b];
+                }
+            } else {
+                for (; left; ++at) {
+                    const int b = __clz(left);
+                    left ^= 0x80000000u >> b;
+                    if (at < cap) mine[at] = in[b];
+                }
+            }
+        }
+    }
+}
+
+// Pads the rows of a group of homes and writes them and their counts out (one warp). row: the group's rows in shared memory;
+// i: its first particle, the others as in cell_append. Returns this lane's padded length, within the capacity or not.
+template <int kHomes>
+__device__ __forceinline__ int cell_write(uint32_t* row, int i, bool real, int len, int own, const CellBuild& bp,
+                                          uint32_t* __restrict__ rows, int2* __restrict__ counts) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int kLanes = 32 / kHomes;
+    const int lane = threadIdx.x & 31, k = lane / kLanes, l = lane % kLanes, cap = bp.geom.cap, pitch = cell_row_pitch(cap);
+    const int padded = real ? (len + 7) & ~7 : 0;
+    if (real) {
+        if (l < 8 && len + l < padded && len + l < cap) row[k * pitch + len + l] = bp.geom.sentinel;
+        // a row past the capacity keeps counts within it, so every reader stays in bounds until the host has seen
+        // max_count, which reports the full length
+        const int own_c = min(own, cap);
+        if (l == 0) counts[i + k] = make_int2(own_c, min(len, cap) - own_c);
+    }
+    const int my_quads = __shfl_sync(kAll, min(padded, cap) >> 2, (lane % kHomes) * kLanes);
+    __syncwarp();
+    // quad q of home particle o by lane (q, o): neighbouring lanes write neighbouring particles' quads
+    const int o = lane % kHomes, io = i + o;
+    uint4* out = reinterpret_cast<uint4*>(rows) + static_cast<size_t>(io >> 5) * (cap >> 2) * 32 + (io & 31);
+    for (int q = lane / kHomes; q < my_quads; q += kLanes)
+        out[32 * q] = *reinterpret_cast<const uint4*>(row + o * pitch + 4 * q);
+    __syncwarp();
+    return padded;
+}
+
+__device__ __forceinline__ void report_longest(int longest, int* max_count) {
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) == 0 && longest > *static_cast<volatile int*>(max_count)) atomicMax(max_count, longest);
+}
+
 // The rows of one home cell's particles, by the kWarps warps of a block; cell_start is the system's (values are particle
-// indices). `shared` is the block's dynamic shared memory (cell_build_smem).
+// indices). `shared` is the block's dynamic shared memory (cell_build_smem). max_count[0] gets the longest padded row,
+// max_count[1] the candidates of a cell that goes through build_row for having too many.
 template <int kWarps, int kHomes, int kRound>
 __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const float4* __restrict__ frames,
                                            const double4* __restrict__ pos, const int* __restrict__ cell_start, int cell,
                                            float side, const CellBuild& bp, uint32_t* __restrict__ rows,
                                            int2* __restrict__ counts, int* __restrict__ max_count) {
-    static_assert(kHomes == 2 || kHomes == 4, "masks are stored as 8 or 16 bytes");
-    constexpr float kFar = 1.0e30f;
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int cap = bp.geom.cap, max_words = bp.stage >> 5;
     float4* cand = shared;
     uint32_t* entries = reinterpret_cast<uint32_t*>(cand + bp.stage);
     uint32_t* masks = entries + bp.stage + warp * kHomes * max_words;  // masks[w * kHomes + k]
-    const int pitch = cell_row_pitch(cap);
-    uint32_t* row = entries + bp.stage + kWarps * kHomes * max_words + warp * kHomes * pitch;
+    uint32_t* row = entries + bp.stage + kWarps * kHomes * max_words + warp * kHomes * cell_row_pitch(cap);
 
     if (warp == 0) cell_items(cell_start, bp.geom.ncps, cell, side, t);
     __syncthreads();
@@ -235,6 +382,7 @@ __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const f
         }
         __syncthreads();
         if (t.odd || t.off[kCellItems] > bp.stage) {
+            if (threadIdx.x == 0) atomicMax(max_count + 1, t.off[kCellItems]);
             for (int h = threadIdx.x; h < homes; h += 32 * kWarps)
                 build_row(pos, bp.geom, i0 + h, cell, cell_start, rows, counts, max_count);
             return;
@@ -264,127 +412,144 @@ __device__ __forceinline__ void build_cell(CellItems& t, float4* shared, const f
             }
         }
         const int total = t.off[kCellItems];
-        if (warp == 0 && total + lane < ((total + 31) & ~31)) cand[total + lane] = make_float4(0.0f, 0.0f, 0.0f, kFar);
+        if (warp == 0 && total + lane < ((total + 31) & ~31)) cand[total + lane] = make_float4(0.0f, 0.0f, 0.0f, kCellFar);
     }
     __syncthreads();
     const int words = (t.off[kCellItems] + 31) >> 5;
-    const int home0 = t.off[t.home], home1 = t.off[kCellItems - 1], own_end = t.off[t.own_items];
+    const CellOrder order{t.off[t.home], t.off[kCellItems - 1], t.off[t.own_items]};
+    const int k = lane / (32 / kHomes);
     int longest = 0;
     for (int h0 = warp * kHomes; h0 < homes; h0 += kWarps * kHomes) {
-        float2 hx[kHomes / 2], hy[kHomes / 2], hz[kHomes / 2], hk[kHomes / 2];  // (-2 h, |h|^2 - r_l^2) in pairs
-#pragma unroll
-        for (int k = 0; k < kHomes; ++k) {
-            float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            float sq = kFar;
-            if (h0 + k < homes) {
-                f = cand[home1 + h0 + k];
-                sq = f.w - bp.rl2;
-            }
-            (k & 1 ? hx[k / 2].y : hx[k / 2].x) = -2.0f * f.x;
-            (k & 1 ? hy[k / 2].y : hy[k / 2].x) = -2.0f * f.y;
-            (k & 1 ? hz[k / 2].y : hz[k / 2].x) = -2.0f * f.z;
-            (k & 1 ? hk[k / 2].y : hk[k / 2].x) = sq;
-        }
-        float nearest = kFar;
-        for (int w = 0; w < words; ++w) {
-            const float4 q = cand[32 * w + lane];
-            unsigned m[kHomes];
-#pragma unroll
-            for (int p = 0; p < kHomes / 2; ++p) {
-                const float2 gap = cell_gap(q, hx[p], hy[p], hz[p], hk[p]);
-                nearest = fminf(nearest, fminf(fabsf(gap.x), fabsf(gap.y)));
-                m[2 * p] = __ballot_sync(kAll, gap.x < -bp.margin);
-                m[2 * p + 1] = __ballot_sync(kAll, gap.y < -bp.margin);
-            }
-            if (lane == 0) {
-                if constexpr (kHomes == 4) reinterpret_cast<uint4*>(masks)[w] = make_uint4(m[0], m[1], m[2], m[3]);
-                else reinterpret_cast<uint2*>(masks)[w] = make_uint2(m[0], m[1]);
-            }
-        }
-        if (__any_sync(kAll, nearest <= bp.margin))
-            cell_masks_exact<kHomes>(cand, entries, words, cand + home1 + h0, homes - h0, i0 + h0, pos, bp, masks);
-        __syncwarp();
-        // the rows: kLanes lanes per home particle, kWords adjacent mask words a lane, kRound words at a time
-        constexpr int kLanes = 32 / kHomes, kWords = kRound / kLanes;
-        const int k = lane / kLanes, l = lane % kLanes, h = h0 + k;
-        uint32_t* mine = row + k * pitch;
+        const bool real = h0 + k < homes;
+        cell_masks<kHomes>(cand, entries, words, cand + order.home1 + h0, homes - h0, i0 + h0, pos, bp, masks);
         int len = 0, own = 0;
-        for (int w0 = 0; w0 < words; w0 += kRound) {
-            uint32_t bits[kWords];
-            int c = 0, c_own = 0;
-#pragma unroll
-            for (int u = 0; u < kWords; ++u) {
-                const int w = w0 + l * kWords + u, v0 = 32 * w;
-                bits[u] = h < homes && w < words ? masks[w * kHomes + k] : 0u;
-                // in the home cell's first copy j > i, in the second j < i
-                bits[u] &= (~bits_from(home0 - v0) | bits_from(home0 + h + 1 - v0)) & ~bits_from(home1 + h - v0);
-                c += __popc(bits[u]);
-                c_own += __popc(bits[u] & ~bits_from(own_end - v0));
-            }
-            int inc = c | (c_own << 16);  // both counts in one scan (a row has far fewer than 65,536 entries)
-#pragma unroll
-            for (int o = 1; o < kLanes; o <<= 1) {
-                const int y = __shfl_up_sync(kAll, inc, o, kLanes);
-                inc += l >= o ? y : 0;
-            }
-            int at = len + (inc & 0xffff) - c;
-            const int sums = __shfl_sync(kAll, inc, kLanes - 1, kLanes);
-            len += sums & 0xffff;
-            own += sums >> 16;
-            const bool fits = __all_sync(kAll, len <= cap);
-#pragma unroll
-            for (int u = 0; u < kWords; ++u) {
-                uint32_t left = __brev(bits[u]);  // the first candidate in the highest bit
-                const uint32_t* in = entries + 32 * (w0 + l * kWords + u);
-                if (fits) {
-                    uint32_t* out = mine + at;
-                    at += __popc(left);
-                    while (left) {
-                        const int b = __clz(left);
-                        left ^= 0x80000000u >> b;
-                        *out++ = in[b];
-                    }
-                } else {
-                    for (; left; ++at) {
-                        const int b = __clz(left);
-                        left ^= 0x80000000u >> b;
-                        if (at < cap) mine[at] = in[b];
-                    }
-                }
-            }
-        }
-        const int padded = h < homes ? (len + 7) & ~7 : 0;
-        if (h < homes) {
-            if (l < 8 && len + l < padded && len + l < cap) mine[len + l] = bp.geom.sentinel;
-            // a row past the capacity keeps counts within it, so every reader stays in bounds until the host has seen
-            // max_count, which reports the full length
-            const int own_c = min(own, cap);
-            if (l == 0) counts[i0 + h] = make_int2(own_c, min(len, cap) - own_c);
-            longest = max(longest, padded);
-        }
-        const int my_quads = __shfl_sync(kAll, min(padded, cap) >> 2, (lane % kHomes) * kLanes);
-        __syncwarp();
-        // quad q of home particle o by lane (q, o): neighbouring lanes write neighbouring particles' quads
-        const int o = lane % kHomes, i = i0 + h0 + o;
-        uint4* out = reinterpret_cast<uint4*>(rows) + static_cast<size_t>(i >> 5) * (cap >> 2) * 32 + (i & 31);
-        for (int q = lane / kHomes; q < my_quads; q += kLanes)
-            out[32 * q] = *reinterpret_cast<const uint4*>(row + o * pitch + 4 * q);
-        __syncwarp();
+        cell_append<kHomes, kRound>(entries, masks, words, order, h0 + k, real, cap, row + k * cell_row_pitch(cap),
+                                    len, own);
+        longest = max(longest, cell_write<kHomes>(row, i0 + h0, real, len, own, bp, rows, counts));
     }
-    longest = __reduce_max_sync(kAll, longest);
-    if (lane == 0 && longest > *static_cast<volatile int*>(max_count)) atomicMax(max_count, longest);
+    report_longest(longest, max_count);
 }
 
-// One home cell per block
-template <int kWarps, int kHomes, int kRound>
-__global__ void __launch_bounds__(32 * kWarps) k_nlist_build_cells(const float4* __restrict__ frames,
-                                                                   const double4* __restrict__ pos,
-                                                                   const int* __restrict__ cell_start, float side,
-                                                                   CellBuild bp, uint32_t* __restrict__ rows,
-                                                                   int2* __restrict__ counts, int* __restrict__ max_count) {
+// Sparse systems: a cell's rows by one warp, all its candidates laid out one after another without regard to reach (a lane
+// per item writes the item's entries, then a lane per candidate fetches it). `mem` is the warp's shared memory
+// (sparse_smem). False, and nothing written, if there are more candidates than it holds.
+template <int kHomes, int kRound>
+__device__ __forceinline__ bool build_cell_warp(float4* mem, const float4* __restrict__ frames,
+                                                const double4* __restrict__ pos, const int* __restrict__ cell_start,
+                                                int cell, float side, const CellBuild& bp, uint32_t* __restrict__ rows,
+                                                int2* __restrict__ counts, int* __restrict__ max_count) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, cap = bp.geom.cap;
+    CellItems& t = *reinterpret_cast<CellItems*>(mem);
+    float4* cand = mem + sizeof(CellItems) / sizeof(float4);
+    uint32_t* entries = reinterpret_cast<uint32_t*>(cand + bp.warp_stage);
+    uint32_t* masks = entries + bp.warp_stage;
+    uint32_t* row = masks + kHomes * (bp.warp_stage >> 5);
+    cell_items(cell_start, bp.geom.ncps, cell, side, t);
+    __syncwarp();
+    const int4 item = lane < kCellItems ? t.cell[lane] : make_int4(0, 0, 0, 0);
+    int inc = item.y;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kAll, inc, o);
+        if (lane >= o) inc += y;
+    }
+    const int total = __shfl_sync(kAll, inc, 31), words = (total + 31) >> 5;
+    if (total > bp.warp_stage) return false;
+    if (lane <= kCellItems) t.off[lane] = inc - item.y;
+    for (int q = 0; q < item.y; ++q)
+        entries[inc - item.y + q] = static_cast<uint32_t>(item.x + q) | (static_cast<uint32_t>(item.z) << kCodeShift);
+    __syncwarp();
+    bool odd = false;
+    for (int v = lane; v < 32 * words; v += 32) {
+        float4 q = make_float4(0.0f, 0.0f, 0.0f, kCellFar);
+        if (v < total) {
+            const uint32_t e = entries[v];
+            const int code = static_cast<int>(e >> kCodeShift);
+            const float4 f = frames[e & kIndexMask];
+            odd |= f.w != 0.0f;
+            q = cell_candidate(f, make_float4((code / 9 - 1) * side, (code / 3 % 3 - 1) * side, (code % 3 - 1) * side, 0.0f));
+        }
+        cand[v] = q;
+    }
+    const int i0 = t.cell[kCellItems - 1].x, homes = t.cell[kCellItems - 1].y;
+    if (__any_sync(kAll, odd)) {
+        for (int h = lane; h < homes; h += 32) build_row(pos, bp.geom, i0 + h, cell, cell_start, rows, counts, max_count);
+        return true;
+    }
+    __syncwarp();
+    const CellOrder order{t.off[t.home], t.off[kCellItems - 1], t.off[t.own_items]};
+    const int k = lane / (32 / kHomes);
+    int longest = 0;
+    for (int h0 = 0; h0 < homes; h0 += kHomes) {
+        const bool real = h0 + k < homes;
+        cell_masks<kHomes>(cand, entries, words, cand + order.home1 + h0, homes - h0, i0 + h0, pos, bp, masks);
+        int len = 0, own = 0;
+        cell_append<kHomes, kRound>(entries, masks, words, order, h0 + k, real, cap, row + k * cell_row_pitch(cap), len,
+                                    own);
+        longest = max(longest, cell_write<kHomes>(row, i0 + h0, real, len, own, bp, rows, counts));
+    }
+    report_longest(longest, max_count);
+    return true;
+}
+
+// Sparse systems: the warps of a block go through the cells [c0, c0 + bp.group) each, past the empty ones. The cells that are
+// too full for a warp (a droplet's, in a box that is otherwise empty) go to a list, for blocks to build: full(cell) adds one.
+constexpr int kSparseWarps = 4, kSparseHomes = 4;
+constexpr int kMostWarpStage = 320;
+__host__ __device__ inline size_t sparse_smem_warp(int warp_stage, int cap) {
+    return sizeof(CellItems) + (sizeof(float4) + sizeof(uint32_t)) * warp_stage +
+           sizeof(uint32_t) * kSparseHomes * (static_cast<size_t>(cell_row_pitch(cap)) + warp_stage / 32);
+}
+template <typename Full>
+__device__ __forceinline__ void build_cells_sparse(float4* shared, const float4* __restrict__ frames,
+                                                   const double4* __restrict__ pos, const int* __restrict__ cell_start,
+                                                   int ncells, int c0, float side, const CellBuild& bp,
+                                                   uint32_t* __restrict__ rows, int2* __restrict__ counts,
+                                                   int* __restrict__ max_count, Full full) {
+    static_assert(sizeof(CellItems) % 16 == 0, "the candidates behind it are 16-byte vectors");
+    const int lane = threadIdx.x & 31, c = c0 + lane;
+    float4* mem = shared + (threadIdx.x >> 5) * (sparse_smem_warp(bp.warp_stage, bp.geom.cap) / sizeof(float4));
+    unsigned todo = __ballot_sync(0xffffffffu, lane < bp.group && c < ncells && cell_start[c] < cell_start[c + 1]);
+    while (todo) {
+        const int cell = c0 + __ffs(todo) - 1;
+        todo &= todo - 1;
+        const bool done = bp.warp_stage != 0 && build_cell_warp<kSparseHomes, 16>(mem, frames, pos, cell_start, cell, side, bp,
+                                                                                  rows, counts, max_count);
+        if (!done && lane == 0) full(cell);
+        __syncwarp();
+    }
+}
+
+// One home cell per block, or, with `list`, the `*listed` cells of the list in turn
+template <int kWarps, int kHomes, int kRound, bool kList>
+__global__ void __launch_bounds__(32 * kWarps)
+    k_nlist_build_cells(const float4* __restrict__ frames, const double4* __restrict__ pos,
+                        const int* __restrict__ cell_start, float side, CellBuild bp, uint32_t* __restrict__ rows,
+                        int2* __restrict__ counts, int* __restrict__ max_count, const int* __restrict__ list,
+                        const int* __restrict__ listed) {
     extern __shared__ float4 sm_cell[];
     __shared__ CellItems t;
-    build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, cell_start, blockIdx.x, side, bp, rows, counts, max_count);
+    if constexpr (kList) {
+        for (int k = blockIdx.x, n = *listed; k < n; k += gridDim.x) {
+            build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, cell_start, list[k], side, bp, rows, counts, max_count);
+            __syncthreads();  // the shared memory goes to the next cell
+        }
+    } else {
+        build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, cell_start, blockIdx.x, side, bp, rows, counts, max_count);
+    }
+}
+
+// Sparse systems: a cell per warp; list and *listed (zero before) get the cells left for k_nlist_build_cells
+__global__ void __launch_bounds__(32 * kSparseWarps, 7)
+    k_nlist_build_sparse(const float4* __restrict__ frames, const double4* __restrict__ pos,
+                         const int* __restrict__ cell_start, int ncells, float side, CellBuild bp,
+                         uint32_t* __restrict__ rows, int2* __restrict__ counts, int* __restrict__ max_count,
+                         int* __restrict__ list, int* __restrict__ listed) {
+    extern __shared__ float4 sm_cell[];
+    build_cells_sparse(sm_cell, frames, pos, cell_start, ncells,
+                       static_cast<int>(blockIdx.x * kSparseWarps + (threadIdx.x >> 5)) * bp.group, side, bp, rows, counts,
+                       max_count, [&](int cell) { list[atomicAdd(listed, 1)] = cell; });
 }
 
 }  // namespace md

@@ -391,13 +391,16 @@ __device__ __forceinline__ float4 code_offset(int code, float cell) {
     return make_float4(o[0], o[1], o[2], 0.0f);
 }
 
-// Frames: q = minimum-image (r - centre of the particle's build cell), in float. frames[n] is the sentinel.
+// Frames: q = minimum-image (r - centre of the particle's build cell), in float. frames[n] is the sentinel. *outside gets
+// `stamp` if a position lies outside the box (stamp 0: not asked for).
 __global__ void k_frames(const double4* __restrict__ pos, int n, const int* __restrict__ cell_sorted, int ncps,
-                         double cell, Box box, float4* __restrict__ frames) {
+                         double cell, Box box, float4* __restrict__ frames, int* __restrict__ outside, int stamp) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) frames[n] = make_float4(kSentinelCoord, kSentinelCoord, kSentinelCoord, 0.0f);
     if (i >= n) return;
-    frames[i] = list_frame_of(pos[i], cell_sorted[i], ncps, cell, box);
+    const float4 f = list_frame_of(pos[i], cell_sorted[i], ncps, cell, box);
+    frames[i] = f;
+    if (stamp != 0 && f.w != 0.0f) *outside = stamp;
 }
 
 // Thread per particle over its row with neighbour frames gathered from global memory (L1/L2); rows are read

@@ -39,6 +39,7 @@ struct RebuildArgs {
     float4* frames;
     int4* iframes;  // nullptr: none kept
     CellBuild build;
+    int *list, *listed;  // sparse systems: the cells left to blocks
     uint32_t* rows;
     int2* counts;
     int *stale, *max_count, *state;
@@ -133,7 +134,7 @@ __device__ __forceinline__ void write_prefix(int n, int part, long long before, 
     if (a < n && b == n && threadIdx.x == 0) out[n] = static_cast<Out>(before);
 }
 
-template <int kHomes, int kRound>
+template <int kHomes, int kRound, bool kSparse>
 __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_constant__ RebuildArgs a) {
     extern __shared__ float4 sm_step[];
     __shared__ union Shared {
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
     if (!grid_barrier(a)) return;
     for (int i = t0; i < n; i += stride) a.bucket[a.start[a.cell_of[i]] + a.slot[i]] = i;
     for (int c = t0; c < a.ncells; c += stride) a.count[c] = 0;
+    if (kSparse && first) *a.listed = 0;
     if (!grid_barrier(a)) return;
     // the stable order: a particle's place in its cell is the number of smaller indices there (src/CellList.cpp:48-51);
     // the reorder (src/System.cpp:42-64) into the spare arrays, and the list's own copies
@@ -219,9 +221,20 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
         a.mass[k] = a.mass2[k];
         a.ids[k] = a.ids2[k];
     }
-    for (int c = blockIdx.x; c < a.ncells; c += static_cast<int>(gridDim.x)) {
-        build_cell<kRebuildThreads / 32, kHomes, kRound>(sh.items, sm_step, a.frames, a.ref_pos, a.start, c,
-                                                 static_cast<float>(a.cell), a.build, a.rows, a.counts, a.max_count);
+    int cells = a.ncells;
+    if constexpr (kSparse) {  // a cell per warp, and then the cells too full for one by blocks (build_cells_sparse)
+        const int per = kSparseWarps * a.build.group;
+        const int mine = static_cast<int>(blockIdx.x) * per + static_cast<int>(threadIdx.x >> 5) * a.build.group;
+        for (int c = mine; c < a.ncells; c += static_cast<int>(gridDim.x) * per)
+            build_cells_sparse(sm_step, a.frames, a.ref_pos, a.start, a.ncells, c, static_cast<float>(a.cell), a.build, a.rows,
+                               a.counts, a.max_count, [&](int cell) { a.list[atomicAdd(a.listed, 1)] = cell; });
+        if (!grid_barrier(a)) return;
+        cells = *static_cast<volatile int*>(a.listed);
+    }
+    for (int k = blockIdx.x; k < cells; k += static_cast<int>(gridDim.x)) {
+        build_cell<kRebuildThreads / 32, kHomes, kRound>(sh.items, sm_step, a.frames, a.ref_pos, a.start,
+                                                         kSparse ? a.list[k] : k, static_cast<float>(a.cell), a.build, a.rows,
+                                                         a.counts, a.max_count);
         __syncthreads();
     }
     if (a.near_rows) {

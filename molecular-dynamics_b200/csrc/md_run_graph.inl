@@ -66,13 +66,34 @@ md_status record_energy(md_forcefield* ff, md_system* s, double* rec, bool want_
 // on their own streams: 32,000: 48 / 79; 256,000: 192 / 218; 500,000: 374 / 356; 864,000: 572 / 560.
 constexpr int64_t kFloatGraphMaxParticles = 1'200'000, kFp64GraphMaxParticles = 400'000;
 
+bool sparse_build(const md_nlist* nl, const md_system* s) {
+    return sparse_cells(nl->grid.ncells, static_cast<double>(s->n) / nl->grid.ncells);
+}
+
+// Parameters and shared memory of the step kernel's list build
+size_t step_smem(const md_nlist* nl, const md_system* s, CellBuild* bp) {
+    const bool few_cells = !sparse_build(nl, s) && nl->grid.ncells < kWideBuildCells;
+    const ListGeom geo{s->box, nl->rl2, nl->grid.ncps, 1, nl->cap, static_cast<uint32_t>(s->n) | (kSentinelCode << kCodeShift)};
+    const double per_cell = static_cast<double>(s->n) / nl->grid.ncells;
+    size_t smem = cell_build_params(*bp, geo, per_cell, build_room(nl->cell_most, per_cell), kRebuildThreads / 32,
+                                    few_cells ? 2 : 4);
+    if (sparse_build(nl, s)) smem = std::max(smem, sparse_build_params(*bp, nl->grid.ncells, per_cell, nl->cell_most));
+    return std::max(smem, kSplitSmem);
+}
+
+// Shared memory up to which two blocks of the step kernel fit an SM. Past it (lists of about 170 particles a cell and more)
+// a rebuild on the resident grid costs more than the host's round trips: N = 100,000, r_l = 6, FP32FX: 541 us a step in
+// graphs, 390 in the host loop; r_l = 5 (two blocks): 248 in graphs.
+constexpr size_t kStepSmem = 110 * 1024;
+
 // Can md_run use graphs for this call? (a tiled list built for this system; the tiled build is the one the device
 // rebuild enqueues)
 bool graph_mode_ok(const md_system* s, const md_forcefield* ff, const md_nlist* nl, int64_t n_steps) {
     const bool precision = (float_precision(ff->precision) && s->n <= kFloatGraphMaxParticles) ||
                            (ff->precision == MD_PREC_FP64 && s->n <= kFp64GraphMaxParticles);
+    CellBuild build;
     return s->graph_chunk > 0 && n_steps > 0 && s->n > 0 && precision && nlist_current(nl, s) && nl->use_cells &&
-           nl->use_tiles && nl->build_pin != 0;
+           nl->use_tiles && nl->build_pin != 0 && step_smem(nl, s, &build) <= kStepSmem;
 }
 
 // Live data of a double-buffered array into its canonical buffer (recorded by the graphs); count elements
@@ -128,6 +149,7 @@ md_status graph_prepare_buffers(md_system* s, md_forcefield* ff, md_nlist* nl, c
     MD_CUDA(s->snap_ids.reserve(n));
     MD_CUDA(s->snap_flag.reserve(1));
     MD_CUDA(s->step_barrier.reserve(2));
+    if (sparse_build(nl, s)) MD_CUDA(nl->full_cells.reserve(nl->grid.ncells));
     if (o.rdf) {
         if (o.rdf->device < 0) {
             o.rdf->device = s->device;
@@ -179,28 +201,19 @@ TileGeom graph_geometry(const md_system* s, const md_nlist* nl) {
     return g;
 }
 
-// Shared memory and particles tested together of the step kernel's list build
-size_t step_smem(const md_nlist* nl, const md_system* s, bool few_cells, CellBuild* bp) {
-    const ListGeom geo{s->box, nl->rl2, nl->grid.ncps, 1, nl->cap, static_cast<uint32_t>(s->n) | (kSentinelCode << kCodeShift)};
-    *bp = cell_build_params(geo, static_cast<double>(s->n) / nl->grid.ncells);
-    size_t smem = cell_build_smem(bp->stage, nl->cap, kRebuildThreads / 32, few_cells ? 2 : 4);
-    if (smem > kBuildSmem) {
-        bp->stage = 0;
-        smem = 0;
-    }
-    return std::max(smem, kSplitSmem);
-}
-
 // The step's first kernel (k_step_start). prepare_only: its shared-memory opt-in and resident grid, before a capture
 md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const StepCapture* last, long long* pair_count,
                            bool prepare_only = false) {
     const int n = static_cast<int>(s->n);
     CellGrid& g = nl->grid;
-    const bool few = g.ncells < kWideBuildCells;
-    const int which = few ? 0 : cell_round(static_cast<double>(n) / g.ncells) == 24 ? 2 : 1;
-    const auto kernel = which == 0 ? k_step_start<2, 16> : which == 1 ? k_step_start<4, 16> : k_step_start<4, 24>;
+    const bool sparse = sparse_build(nl, s), few = !sparse && g.ncells < kWideBuildCells;
+    const int which = sparse ? 3 : few ? 0 : cell_round(static_cast<double>(n) / g.ncells) == 24 ? 2 : 1;
+    const auto kernel = which == 0   ? k_step_start<2, 16, false>
+                        : which == 1 ? k_step_start<4, 16, false>
+                        : which == 2 ? k_step_start<4, 24, false>
+                                     : k_step_start<4, 16, true>;
     RebuildArgs a{};
-    const size_t smem = step_smem(nl, s, few, &a.build);
+    const size_t smem = step_smem(nl, s, &a.build);
     if (prepare_only) {
         MD_CUDA(allow_smem(kernel, smem));
         if (s->step_resident[which] != 0 && s->step_smem[which] == smem) return MD_OK;
@@ -240,6 +253,8 @@ md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const 
     a.offset_sums = s->step_sums.p + s->step_resident[which];
     a.frames = nl->frames.p;
     a.iframes = ff->precision == MD_PREC_FX64 || ff->precision == MD_PREC_FX32 ? nl->iframes.p : nullptr;
+    a.list = nl->full_cells.p;
+    a.listed = nl->flags.p + 4;
     a.rows = nl->rows.p;
     a.counts = nl->counts.p;
     a.stale = nl->flags.p;
@@ -323,13 +338,16 @@ std::string graph_key(const md_system* s, const md_forcefield* ff, const md_nlis
                           static_cast<const void*>(ff->epairs.p), static_cast<const void*>(ff->enblocks.p),
                           static_cast<const void*>(nl->half_off.p), static_cast<const void*>(nl->tmp_counts.p),
                           static_cast<const void*>(nl->tiles.p), static_cast<const void*>(s->step_barrier.p),
-                          static_cast<const void*>(s->step_sums.p),
+                          static_cast<const void*>(s->step_sums.p), static_cast<const void*>(nl->full_cells.p),
                           static_cast<const void*>(o.rdf ? o.rdf->hist.p : nullptr)})
         ptr(p);
+    CellBuild build;
+    step_smem(nl, s, &build);
     for (double v : {static_cast<double>(s->n), s->box.L, static_cast<double>(nl->cap), static_cast<double>(tg.kk),
                      static_cast<double>(tg.nseg), static_cast<double>(tg.max_staged), static_cast<double>(tg.ncps),
                      static_cast<double>(nl->variant[ff->precision]), static_cast<double>(ff->precision), ff->eps,
-                     ff->sigma, ff->rc, nl->rl2, nl->max_disp2, nl->nf_near2, dt, want_energy ? 1.0 : 0.0,
+                     ff->sigma, ff->rc, nl->rl2, nl->max_disp2, nl->nf_near2, static_cast<double>(build.stage),
+                     static_cast<double>(build.warp_stage), dt, want_energy ? 1.0 : 0.0,
                      want_ke ? 1.0 : 0.0, bussi_c, o.bussi_temperature, s->profile ? 1.0 : 0.0,
                      static_cast<double>(s->graph_chunk), o.rdf ? o.rdf->rmax : 0.0,
                      static_cast<double>(o.rdf ? o.rdf->bins : 0), static_cast<double>(ff->serial),

@@ -1,4 +1,4 @@
-// Shared-memory cell tiles for the list force kernels (boxes of at least 3 cells per side).
+// Shared-memory cell tiles for the list force kernels and one of the list builds (boxes of at least 3 cells per side).
 //
 // Work decomposition: one thread block per "segment" = kk consecutive cells along z of one (x, y) cell
 // column. The block stages into shared memory every particle its home atoms can pair with: the 9 columns
@@ -18,6 +18,7 @@
 #include "md_common.cuh"
 #include "md_fp32.cuh"
 #include "md_fp64.cuh"
+#include "md_nlist.cuh"
 
 namespace md {
 
@@ -125,24 +126,43 @@ __device__ __forceinline__ void stage_tile(const T* __restrict__ src, T* dst, co
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// Largest staged particle count over all segments of this geometry (one thread per segment); sizes the
-// shared tile until the next rebuild, since the cell contents only change at rebuilds.
-__global__ void k_tile_max_staged(const int* __restrict__ cell_start, TileGeom g, int* __restrict__ out) {
+// Largest staged particle count over all segments of this geometry (one thread per segment) into out[0]; sizes the
+// shared tile until the next rebuild, since the cell contents only change at rebuilds. With ncells, also the most
+// candidates of a cell for the list build (its 27 cells, itself twice; one thread per cell) into out[1].
+__global__ void k_tile_max_staged(const int* __restrict__ cell_start, TileGeom g, int ncells, int* __restrict__ out) {
+    const int n = g.ncps, segs = n * n * g.nseg;
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = g.ncps;
-    if (b >= n * n * g.nseg) return;
-    const int seg = b % g.nseg, col = b / g.nseg;
-    const int cx = col / n, cy = col % n, z0 = seg * g.kk;
-    const int span = min(g.kk, n - z0) + 2;
     int total = 0;
-    for (int c = 0; c < 9; ++c) {
-        const int x = (cx + c / 3 - 1 + n) % n, y = (cy + c % 3 - 1 + n) % n;
-        for (int u = 0; u < span; ++u) {
-            const int cell = (x * n + y) * n + (z0 - 1 + u + n) % n;
-            total += cell_start[cell + 1] - cell_start[cell];
+    if (b < segs) {
+        const int seg = b % g.nseg, col = b / g.nseg;
+        const int cx = col / n, cy = col % n, z0 = seg * g.kk;
+        const int span = min(g.kk, n - z0) + 2;
+        for (int c = 0; c < 9; ++c) {
+            const int x = (cx + c / 3 - 1 + n) % n, y = (cy + c % 3 - 1 + n) % n;
+            for (int u = 0; u < span; ++u) {
+                const int cell = (x * n + y) * n + (z0 - 1 + u + n) % n;
+                total += cell_start[cell + 1] - cell_start[cell];
+            }
+        }
+        atomicMax(out, total);
+        total = 0;
+    } else if (b - segs < ncells) {
+        const int home = b - segs, own = cell_start[home + 1] - cell_start[home];
+        if (own > 0) {
+            const int cx = home / (n * n), cy = (home / n) % n, cz = home % n;
+            total = own;
+            for (int c = 0; c < 9; ++c) {
+                const int x = (cx + c / 3 - 1 + n) % n, y = (cy + c % 3 - 1 + n) % n, row = (x * n + y) * n;
+                // the z cells are neighbours in memory but at the box's faces
+                const int lo = max(cz - 1, 0), hi = min(cz + 1, n - 1);
+                total += cell_start[row + hi + 1] - cell_start[row + lo];
+                if (cz == 0) total += cell_start[row + n] - cell_start[row + n - 1];
+                if (cz == n - 1) total += cell_start[row + 1] - cell_start[row];
+            }
         }
     }
-    atomicMax(out, total);
+    total = __reduce_max_sync(0xffffffffu, total);
+    if ((threadIdx.x & 31) == 0 && total > *static_cast<volatile int*>(out + 1)) atomicMax(out + 1, total);
 }
 
 // Staged cell of code (dx, dy, dz) seen from home z offset h (0-based in the segment)
@@ -150,6 +170,140 @@ __device__ __forceinline__ int staged_cell(int code, int h, int span) {
     const int dxy = code / 3;        // (dx + 1) * 3 + (dy + 1)
     const int dz = code % 3 - 1;
     return dxy * span + h + 1 + dz;
+}
+
+// ---- list build -------------------------------------------------------------------------------------------
+
+// NeighbourList::build pass 1 (src/NeighbourList.cpp:75-111) on a tile, a thread per home particle walking its candidates:
+// the build for large systems that are neither a uniform liquid nor a gas (cells_build_async says where the line lies).
+// Candidates come from staged float frames; one is accepted when float r^2 < r_l^2 - margin, rejected when float
+// r^2 > r_l^2 + margin, and otherwise decided by the reference's double test on the global positions (a thin shell of
+// candidates). The margin bounds the float error of r^2 for positions inside the box (each coordinate carries under 4e-7
+// absolute error); a tile with a position outside it (list_frame_of; *outside_stamp
+// tells whether this build has one at all) goes through build_row. Row order: own pairs (j > i) in
+// the reference's candidate order, then the j < i that list i, ascending. Bound by instruction issue (about 25 a candidate).
+struct TileBuild {
+    ListGeom geom;
+    float lo, hi;  // r_l^2 -+ margin
+    int stamp;     // this build's (build_stamp)
+};
+
+// Candidates [u0, u1) of one cell decided as the float scan does, except those in the thin shell, which the reference's
+// double test decides; appended from the row length cnt on
+__device__ __noinline__ void rescan_cell_exact(const float4* q, int jbase, int u0, int u1, const float4 qo, uint32_t code,
+                                               const TileBuild& b, const double4 pi, const double4* __restrict__ pos,
+                                               uint32_t* row, int& cnt) {
+    for (int u = u0; u < u1; ++u) {
+        const float4 qj = q[u];
+        const float dx = qo.x - qj.x, dy = qo.y - qj.y, dz = qo.z - qj.z;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        bool take = r2 < b.lo;
+        if (!take && r2 <= b.hi) take = within_list(pi, pos[jbase + u], b.geom);
+        if (take) {
+            if (cnt < b.geom.cap) row[(cnt >> 2) * 128 + (cnt & 3)] = static_cast<uint32_t>(jbase + u) | (code << kCodeShift);
+            ++cnt;
+        }
+    }
+}
+
+// Appends to a row the candidates u in [u0, u1) of one cell that are within r_l of particle i: candidate u has the float
+// frame q[u] and the index jbase + u, qo = q_i + the cell's image offset, row is particle i's interleaved row (entry s at
+// row[(s >> 2) * 128 + (s & 3)]) and cnt its length. The loop runs branch-free, with a predicated store; if any candidate
+// falls in the thin shell, the cell is scanned again from its first slot. Entries past the capacity are counted only.
+__device__ __forceinline__ void scan_cell(const float4* q, int jbase, int u0, int u1, const float4& qo, uint32_t code,
+                                          const TileBuild& b, const double4& pi, const double4* __restrict__ pos,
+                                          uint32_t* row, int& cnt) {
+    const int cnt0 = cnt;
+    bool shell = false;
+    const uint32_t vbase = static_cast<uint32_t>(jbase) | (code << kCodeShift);  // entry of candidate u: vbase + u
+    const float2 nxy = make_float2(-qo.x, -qo.y);
+    const float nz = -qo.z;
+    auto scan = [&](auto put) {
+        for (int u = u0; u < u1; ++u) {
+            const float4 qj = q[u];
+            const float2 d = __fadd2_rn(make_float2(qj.x, qj.y), nxy);
+            const float dz = __fadd_rn(qj.z, nz);
+            const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, dz * dz));
+            const bool take = r2 < b.lo;
+            shell |= !take && r2 <= b.hi;
+            put(take, vbase + static_cast<uint32_t>(u));
+            cnt += take ? 1 : 0;
+        }
+    };
+    if (cnt + (u1 - u0) <= b.geom.cap) {  // every candidate fits: no capacity test per candidate
+        scan([&](bool take, uint32_t entry) {
+            asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.u32 t, %2, 0;\n\t@t st.global.u32 [%0], %1;\n\t}" ::"l"(
+                             row + (cnt + 31 * (cnt & ~3))),  // (cnt >> 2) * 128 + (cnt & 3)
+                         "r"(entry), "r"(static_cast<unsigned>(take))
+                         : "memory");
+        });
+    } else {
+        scan([&](bool take, uint32_t entry) {
+            if (take && cnt < b.geom.cap) row[(cnt >> 2) * 128 + (cnt & 3)] = entry;
+        });
+    }
+    if (shell) {
+        cnt = cnt0;
+        rescan_cell_exact(q, jbase, u0, u1, qo, code, b, pi, pos, row, cnt);
+    }
+}
+
+__global__ void __launch_bounds__(kTileThreads) k_nlist_build_tile(
+    const float4* __restrict__ frames, const double4* __restrict__ pos, const int* __restrict__ cell_start,
+    const int* __restrict__ cell_sorted, TileGeom g, const __grid_constant__ TileBuild b, CellOffsets offs,
+    const int* __restrict__ outside_stamp, uint32_t* __restrict__ rows, int2* __restrict__ counts,
+    int* __restrict__ max_count) {
+    extern __shared__ float4 s_q[];
+    __shared__ TileTables t;
+    tile_tables(g, cell_start, t);
+    if (t.total > g.max_staged) {  // (not after tile_geometry has measured this build's cells)
+        if (threadIdx.x == 0) atomicMax(max_count, 1 << 30);
+        return;
+    }
+    stage_tile(frames, s_q, t);
+    cp_async_wait();
+    __syncthreads();
+    bool outside = false;
+    if (*outside_stamp == b.stamp)
+        for (int k = threadIdx.x; k < t.total; k += blockDim.x) outside |= s_q[k].w != 0.0f;
+    if (__syncthreads_or(outside)) {
+        for (int i = t.home_begin + threadIdx.x; i < t.home_end; i += blockDim.x)
+            build_row(pos, b.geom, i, cell_sorted[i], cell_start, rows, counts, max_count);
+        return;
+    }
+    const int n = g.ncps, span = t.kk + 2, cap = b.geom.cap;
+    for (int i = t.home_begin + threadIdx.x; i < t.home_end; i += blockDim.x) {
+        const float4 qi = frames[i];
+        const double4 pi = pos[i];
+        const int z = cell_sorted[i] % n, h = (z - t.z0 + n) % n;
+        int cnt = 0;
+        uint32_t* row = rows + static_cast<size_t>(i >> 5) * (cap >> 2) * 128 + (i & 31) * 4;
+        // the staged cell of `code`: its particles after i, or those before it
+        auto scan = [&](uint32_t code, bool after) {
+            const int sc = staged_cell(static_cast<int>(code), h, span), gs = t.gstart[sc], all = t.count[sc];
+            const float4 o = offs.off[code];
+            scan_cell(s_q + t.off[sc], gs, after ? max(0, i + 1 - gs) : 0, after ? all : min(all, i - gs),
+                      make_float4(qi.x + o.x, qi.y + o.y, qi.z + o.z, 0.0f), code, b, pi, pos, row, cnt);
+        };
+        // own pairs: 27 cells in (dx, dy, dz) order, increasing j inside each (src/CellList.cpp:55-83)
+        for (uint32_t code = 0; code < 27; ++code) scan(code, true);
+        const int own = cnt;
+        // the j < i that list i, increasing j: cells in increasing cell id
+        int ox[3], oy[3], oz[3];
+        ascending_offsets(t.cx, n, ox);
+        ascending_offsets(t.cy, n, oy);
+        ascending_offsets(z, n, oz);
+        for (int u = 0; u < 3; ++u)
+            for (int v = 0; v < 3; ++v)
+                for (int w = 0; w < 3; ++w) scan((ox[u] + 1) * 9 + (oy[v] + 1) * 3 + (oz[w] + 1), false);
+        // a row past the capacity keeps counts within it, so every reader stays in bounds until the host has seen
+        // max_count, which reports the full length
+        const int own_c = min(own, cap);
+        counts[i] = make_int2(own_c, min(cnt, cap) - own_c);
+        const int padded = (cnt + 7) & ~7;
+        for (int s = cnt; s < padded && s < cap; ++s) row[(s >> 2) * 128 + (s & 3)] = b.geom.sentinel;
+        atomicMax(max_count, padded);
+    }
 }
 
 // ---- float forces -----------------------------------------------------------------------------------------
