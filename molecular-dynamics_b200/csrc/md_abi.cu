@@ -459,6 +459,7 @@ int initial_capacity(const md_nlist* nl, const md_system* s) {
 // Defined in md_abi_float.inl
 int float_lanes(int n);
 md_status frames_async(md_system* s, md_nlist* nl, int stamp = 0);
+double cell_side(const md_nlist* nl, const md_system* s);
 CellOffsets cell_offsets(const md_nlist* nl, const md_system* s);
 
 #ifndef MD_TILE_HOME_TARGET
@@ -1048,17 +1049,17 @@ md_status read_energy(md_forcefield* ff, md_system* s, double* pe, double* viria
 }
 
 // Half kick + drift + wrap; with check_skin also the list's half-skin test into nl->flags[0]; with
-// write_frames also the float frames of the new positions (the list must be current and use tiles).
+// write_frames also the float frames of the new positions (the list must be current and have cells).
 md_status kick_drift_async(md_system* s, md_nlist* nl, double dt, bool check_skin, bool write_frames = false) {
     const int n = static_cast<int>(s->n);
     if (n == 0) return MD_OK;
     // (in a graph the flag is zero but between a drift and the step's first kernel)
     if (check_skin && !g_capturing) MD_CUDA(cudaMemsetAsync(nl->flags.p, 0, sizeof(int), s->stream));
     if (write_frames) {
-        const TileGeom& tg = nl->tiles_geom;
         k_kick_drift_frames<<<blocks_for(n + 1, kThreads), kThreads, 0, s->stream>>>(
             s->pos.p, s->vel.p, s->force.p, s->mass.p, n, 0.5 * dt, dt, s->box, check_skin ? nl->ref_pos.p : nullptr,
-            nl->max_disp2, check_skin ? nl->flags.p : nullptr, nl->cell_sorted.p, tg.ncps, tg.cell, nl->frames.p);
+            nl->max_disp2, check_skin ? nl->flags.p : nullptr, nl->cell_sorted.p, nl->grid.ncps, cell_side(nl, s),
+            nl->frames.p);
     } else {
         k_kick_drift<<<blocks_for(n, kThreads), kThreads, 0, s->stream>>>(
             s->pos.p, s->vel.p, s->force.p, s->mass.p, n, 0.5 * dt, dt, s->box, check_skin ? nl->ref_pos.p : nullptr,
@@ -1070,10 +1071,11 @@ md_status kick_drift_async(md_system* s, md_nlist* nl, double dt, bool check_ski
 
 // The first half of VelocityVerletIntegrator::step (src/Integrator.cpp:18-30): kick, drift and wrap, then
 // NeighbourList::update. The staleness flag is read back (one 4-byte copy); a stale or never-built list is
-// rebuilt. Afterwards the float frames match the positions whenever the list uses tiles.
+// rebuilt. Afterwards the float frames match the positions wherever the float kernels read them (a list with cells, whether
+// or not its tiles fit the shared memory).
 md_status drift_and_update(md_system* s, md_forcefield* ff, md_nlist* nl, double dt, bool* rebuilt) {
     const bool current = nlist_current(nl, s);
-    const bool frames = current && nl->use_tiles &&
+    const bool frames = current && nl->use_cells &&
                         (ff->precision == MD_PREC_FP32FX || ff->precision == MD_PREC_FP32 || ff->precision == MD_PREC_FX32);
     MD_TRY(kick_drift_async(s, nl, dt, current, frames));
     bool stale = true;
