@@ -160,8 +160,8 @@ md_status md_nlist_info(const md_nlist* nl, uint64_t* pair_count, int* rebuild_c
  * only while the list has tiles; FP64 and the float modes), 2 pins global gathers with the rows prefetched
  * (FP64: a quad of entries at a time, branch-free; float modes: a group of 8 ahead), 3 the float modes' variant 2
  * with registers capped for occupancy and 4 the same on a resident grid; a list that loses the tiles of a pinned
- * variant 1 goes on as with -1. MD_PREC_FX64 and MD_PREC_FX32 have one kernel each (variant 0). Every variant gives the same bits. md_nlist_force_variant reports the variant in use
- * (-1 until the first force call). */
+ * variant 1 goes on as with -1. MD_PREC_FX64 and MD_PREC_FX32 have one kernel each (variant 0). Every variant gives
+ * the same bits. md_nlist_force_variant reports the variant in use (-1 until the first force call). */
 md_status md_nlist_set_force_variant(md_nlist* nl, int precision, int variant);
 md_status md_nlist_force_variant(const md_nlist* nl, int precision, int* variant);
 /* List build kernel: -1 and 1 choose by the system's size and density among the builds by cells, tiles and particles
@@ -303,6 +303,8 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
 md_status md_batch_destroy(md_batch* b);
 /* Replicas, particles (sum of n), neighbour row capacity, kernels launched so far. Any may be NULL. */
 md_status md_batch_info(const md_batch* b, int* replicas, int64_t* atoms, int* capacity, uint64_t* launches);
+/* Graphs that the batch keeps and graphs that it has captured so far. Either may be NULL. */
+md_status md_batch_graph_info(const md_batch* b, uint64_t* graphs, uint64_t* captured);
 md_status md_batch_stream(md_batch* b, void** stream);
 /* n_steps steps of every replica. With energy_every = k, row s of the records (replica r at [s * replicas + r])
  * is step (s + 1) k of this run; arrays hold n_steps / k rows each and may be NULL. */

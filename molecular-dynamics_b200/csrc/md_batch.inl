@@ -61,6 +61,7 @@ struct md_batch {
     double* h_rec = nullptr;    // pinned: one chunk of records
     int* h_flags = nullptr;     // pinned
     std::map<int, std::pair<cudaGraphExec_t, uint64_t>> graphs;  // chunk length -> (graph, kernels in it)
+    uint64_t captured = 0;  // graphs captured since the batch was made
     struct Variant {
         int apb, tpa;
         bool prefetch;
@@ -156,12 +157,17 @@ void b_drop_graphs(md_batch* b) {
 // at 0.05, 1.5 a cell: 51 by cells)
 constexpr double kThinReplica = 0.5;
 
+// The list build's parameters with room for `room` candidates, as far as the shared memory goes; returns its size
+size_t b_build_params(const md_batch* b, int room, CellBuild& bp) {
+    const ListGeom geo{Box{}, b->rl2, 0, 1, b->cap, static_cast<uint32_t>(b->slots) | (kSentinelCode << kCodeShift)};
+    return cell_build_params(bp, geo, b->per_cell, room, 4, 4);
+}
+
 // The list build kernel over the stale replicas' cells (prepare_only: its shared-memory opt-in alone, which a capture
 // may not make). Rows too long for the kernel's shared memory go through its thread-per-particle path (stage 0).
 md_status b_build_async(md_batch* b, bool prepare_only) {
-    const ListGeom geo{Box{}, b->rl2, 0, 1, b->cap, static_cast<uint32_t>(b->slots) | (kSentinelCode << kCodeShift)};
     CellBuild bp;
-    const size_t smem = cell_build_params(bp, geo, b->per_cell, b->room, 4, 4);
+    const size_t smem = b_build_params(b, b->room, bp);
     b->stage = bp.stage;
     const auto kernel = cell_round(b->mean_cell) == 24 ? k_b_nlist_build<4, 4, 24> : k_b_nlist_build<4, 4, 16>;
     MD_CUDA(allow_smem(kernel, smem));
@@ -174,10 +180,14 @@ md_status b_build_async(md_batch* b, bool prepare_only) {
 }
 
 // A build that met a cell with many more candidates than it has room for (such cells go through build_row): room for it from
-// the next captured graph on
+// the next captured graph on, unless the shared memory has no more
 void b_adapt_room(md_batch* b) {
     if (b->h_flags[1] <= b->stage + b->stage / 4) return;
-    b->room = b->h_flags[1] + b->h_flags[1] / 8;
+    const int room = b->h_flags[1] + b->h_flags[1] / 8;
+    CellBuild bp;
+    b_build_params(b, room, bp);
+    if (bp.stage <= b->stage) return;
+    b->room = room;
     b_drop_graphs(b);
 }
 
@@ -450,6 +460,7 @@ md_status b_graph(md_batch* b, int len, cudaGraphExec_t* out, uint64_t* kernels)
     cudaGraphDestroy(graph);
     if (ei != cudaSuccess) return fail(MD_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ei));
     b->graphs[len] = {exec, count};
+    b->captured += 1;
     *out = exec;
     *kernels = count;
     return MD_OK;
@@ -827,6 +838,13 @@ md_status md_batch_info(const md_batch* b, int* replicas, int64_t* atoms, int* c
     if (atoms) *atoms = b->atoms;
     if (capacity) *capacity = b->cap;
     if (launches) *launches = b->launches;
+    return MD_OK;
+}
+
+md_status md_batch_graph_info(const md_batch* b, uint64_t* graphs, uint64_t* captured) {
+    if (!b) return fail(MD_ERR_INVALID, "null batch");
+    if (graphs) *graphs = b->graphs.size();
+    if (captured) *captured = b->captured;
     return MD_OK;
 }
 

@@ -91,6 +91,7 @@ def _load():
         "md_batch_create": (_I, [_I, _I, C.POINTER(C.c_int64), _PD, _PD, _PU64, _PD, _PD, _PD,
                                  C.POINTER(md_batch_options), _PP]),
         "md_batch_destroy": (_I, [_P]), "md_batch_info": (_I, [_P, _PI, C.POINTER(C.c_int64), _PI, _PU64]),
+        "md_batch_graph_info": (_I, [_P, _PU64, _PU64]),
         "md_batch_stream": (_I, [_P, _PP]), "md_batch_run": (_I, [_P, _I64, _PD, _PD, _PD]),
         "md_batch_run_records": (_I, [_P, _I64, _PD, _PD, _PD, _PD]),
         "md_batch_set_thermostat": (_I, [_P, _I, _I, _D, _PD, _PU64]),
@@ -631,6 +632,11 @@ class Batch:
         atoms, launches = C.c_int64(), C.c_uint64()
         _check(LIB.md_batch_info(self.h, C.byref(r), C.byref(atoms), C.byref(cap), C.byref(launches)))
         return dict(replicas=r.value, atoms=atoms.value, capacity=cap.value, launches=launches.value)
+
+    def graph_info(self) -> dict:
+        kept, captured = C.c_uint64(), C.c_uint64()
+        _check(LIB.md_batch_graph_info(self.h, C.byref(kept), C.byref(captured)))
+        return dict(graphs=kept.value, captured=captured.value)
 
     def run(self, n_steps: int, record: bool = True, inside: bool = False):
         """n_steps steps of every replica; returns (pe, virial, ke) arrays of shape (n_steps // energy_every,
