@@ -467,6 +467,26 @@ __global__ void __launch_bounds__(kResortThreads)
     }
 }
 
+// The stale replica of a list-build item: the last w with stale_items[w] <= item
+__device__ __forceinline__ int build_item_replica(const int* __restrict__ stale_items, int nr, int item) {
+    int lo = 0, hi = nr;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (stale_items[mid] <= item) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// kAllGroup particles of a replica under 3 cells per side by the block's warps
+template <int kWarps>
+__device__ __forceinline__ void build_group_all(const BRep& d, int group, const double4* __restrict__ pos, const ListGeom& g,
+                                                uint32_t* __restrict__ rows, int2* __restrict__ counts,
+                                                int* __restrict__ max_count) {
+    const int i0 = group * kAllGroup;
+    for (int i = i0 + static_cast<int>(threadIdx.x >> 5); i < i0 + kAllGroup && i < d.n; i += kWarps)
+        build_row_all(pos, d.off, d.off + d.n, g, d.off + i, rows, counts, max_count);
+}
+
 // The list build of the stale replicas (build_cell, with slots for indices): blocks take their cells in turn, and groups
 // of particles of replicas under 3 cells per side, a warp per particle. In thin gases (kThinReplica) a block takes a tile, a
 // thread per particle. bp.geom's box and cells per side are set per replica. max_count as in build_cell.
@@ -481,18 +501,13 @@ __global__ void __launch_bounds__(32 * kWarps)
     __shared__ CellItems t;
     const int nr = work[0], total = work[2];
     for (int item = blockIdx.x; item < total; item += gridDim.x) {
-        int lo = 0, hi = nr;  // the replica: last w with stale_items[w] <= item
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (stale_items[mid] <= item) lo = mid; else hi = mid;
-        }
-        const int r = stale_reps[lo];
+        const int w = build_item_replica(stale_items, nr, item), r = stale_reps[w];
         const BRep d = reps[r];
         bp.geom.box = d.box;
         bp.geom.ncps = d.ncps;
         bp.geom.use_cells = d.use_cells;
         const int* st = start + d.cell_off + r;
-        const int part = item - stale_items[lo];
+        const int part = item - stale_items[w];
         if (d.use_cells == 1) {
             build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, st, part, static_cast<float>(d.cell), bp, rows, counts,
                                                max_count);
@@ -500,11 +515,23 @@ __global__ void __launch_bounds__(32 * kWarps)
             const int i = part * kTile + static_cast<int>(threadIdx.x);
             if (i < d.n) build_row(pos, bp.geom, d.off + i, cell_sorted[d.off + i], st, rows, counts, max_count);
         } else {
-            const int i0 = part * kAllGroup;
-            for (int i = i0 + (threadIdx.x >> 5); i < i0 + kAllGroup && i < d.n; i += kWarps)
-                build_row_all(pos, d.off, d.off + d.n, bp.geom, d.off + i, rows, counts, max_count);
+            build_group_all<kWarps>(d, part, pos, bp.geom, rows, counts, max_count);
         }
         __syncthreads();  // the shared memory goes to the next item
+    }
+}
+
+// The same for a batch whose replicas are all under 3 cells per side, without build_cell's registers, stack and shared memory
+__global__ void __launch_bounds__(kTile)
+    k_b_nlist_build_all(const BRep* __restrict__ reps, const int* __restrict__ stale_reps, const int* __restrict__ stale_items,
+                        const int* __restrict__ work, const double4* __restrict__ pos, ListGeom g, uint32_t* __restrict__ rows,
+                        int2* __restrict__ counts, int* __restrict__ max_count) {
+    const int nr = work[0], total = work[2];
+    for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        const int w = build_item_replica(stale_items, nr, item);
+        const BRep d = reps[stale_reps[w]];
+        g.box = d.box;
+        build_group_all<kTile / 32>(d, item - stale_items[w], pos, g, rows, counts, max_count);
     }
 }
 

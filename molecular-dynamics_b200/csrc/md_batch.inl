@@ -169,10 +169,17 @@ md_status b_build_async(md_batch* b, bool prepare_only) {
     CellBuild bp;
     const size_t smem = b_build_params(b, b->room, bp);
     b->stage = bp.stage;
+    const unsigned grid = static_cast<unsigned>(std::min(b->build_items, 148 * 32));
+    if (b->per_cell == 0.0) {  // no replica has cells
+        if (prepare_only) return MD_OK;
+        k_b_nlist_build_all<<<grid, kTile, 0, b->stream>>>(b->reps.p, b->stale_reps.p, b->stale_items.p, b->work.p, b->pos.p,
+                                                           bp.geom, b->rows.p, b->counts.p, b->flags.p);
+        MD_CHECK_LAUNCH();
+        return MD_OK;
+    }
     const auto kernel = cell_round(b->mean_cell) == 24 ? k_b_nlist_build<4, 4, 24> : k_b_nlist_build<4, 4, 16>;
     MD_CUDA(allow_smem(kernel, smem));
     if (prepare_only) return MD_OK;
-    const unsigned grid = static_cast<unsigned>(std::min(b->build_items, 148 * 32));
     kernel<<<grid, 128, smem, b->stream>>>(b->reps.p, b->stale_reps.p, b->stale_items.p, b->work.p, b->pos.p, b->frames.p,
                                            b->start.p, b->cell_sorted.p, bp, b->rows.p, b->counts.p, b->flags.p);
     MD_CHECK_LAUNCH();
