@@ -1743,8 +1743,12 @@ md_status md_forces_all_pairs(md_forcefield* ff, md_system* s, double* pe, doubl
     const int n = static_cast<int>(s->n);
     MD_TRY(join_energy(ff, s));
     MD_CUDA(ff->out.reserve(4));
-    MD_CUDA(cudaMemsetAsync(ff->out.p, 0, 3 * sizeof(double), s->stream));
-    if (n > 0) {
+    if (n == 0) MD_CUDA(cudaMemsetAsync(ff->out.p, 0, 3 * sizeof(double), s->stream));
+    if (n > 0 && n <= kFewParticles) {
+        k_all_pairs_few<<<1, 32 * kFewParticles, 0, s->stream>>>(s->pos.p, n, s->box, ff->lj, s->force.p, ff->out.p);
+        MD_CHECK_LAUNCH();
+    } else if (n > 0) {
+        MD_CUDA(cudaMemsetAsync(ff->out.p, 0, 3 * sizeof(double), s->stream));
         MD_CUDA(ff->own_pairs.reserve(n));
         MD_CUDA(ff->own_off.reserve(static_cast<size_t>(n) + 1));
         MD_CUDA(ff->own_tiles.reserve(scan_tiles_needed(n)));

@@ -700,6 +700,60 @@ __global__ void __launch_bounds__(128) k_all_pairs(const double4* __restrict__ p
     }
 }
 
+// The same for n <= 32 in one launch: warp p takes particle p, one thread adds the pairs' (E, W) in order; out = potential,
+// virial, inside pairs. (Through k_all_pairs, the offsets' scan and k_sum_pairs, with the pair count read back in between, a
+// call on 2 particles takes 62 us, with this kernel 22.)
+constexpr int kFewParticles = 32;
+__global__ void __launch_bounds__(32 * kFewParticles) k_all_pairs_few(const double4* __restrict__ pos, int n, Box box, LJ lj,
+                                                                      double* __restrict__ force, double* __restrict__ out) {
+    __shared__ double2 s_rec[kFewParticles][kFewParticles];
+    __shared__ int s_own[kFewParticles];
+    const int p = threadIdx.x >> 5, i = threadIdx.x & 31;
+    if (p < n) {
+        bool in = i < n && i != p;
+        double dx = 0.0, dy = 0.0, dz = 0.0, r2 = 0.0, fr = 0.0, e = 0.0;
+        if (in) {
+            const double4 pp = pos[p], q = pos[i];
+            dx = min_image(dsub(pp.x, q.x), box);
+            dy = min_image(dsub(pp.y, q.y), box);
+            dz = min_image(dsub(pp.z, q.z), box);
+            r2 = norm2(dx, dy, dz);
+            in = !(r2 >= lj.rc2);
+        }
+        if (in) pair_terms(r2, lj, fr, e);
+        const bool mine = in && i > p && r2 < lj.rc2;
+        const unsigned own = __ballot_sync(0xffffffffu, mine);
+        if (mine) s_rec[p][__popc(own & ((1u << i) - 1u))] = make_double2(e, dmul(fr, r2));
+        if (i == 0) s_own[p] = __popc(own);
+        dx = dmul(fr, dx);
+        dy = dmul(fr, dy);
+        dz = dmul(fr, dz);
+        double fx = 0.0, fy = 0.0, fz = 0.0;
+        for (unsigned mask = __ballot_sync(0xffffffffu, in); mask; mask &= mask - 1) {
+            const int t = __ffs(mask) - 1;
+            fx = dadd(fx, __shfl_sync(0xffffffffu, dx, t));
+            fy = dadd(fy, __shfl_sync(0xffffffffu, dy, t));
+            fz = dadd(fz, __shfl_sync(0xffffffffu, dz, t));
+        }
+        if (i < 3) force[static_cast<size_t>(i) * n + p] = i == 0 ? fx : i == 1 ? fy : fz;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double pe = 0.0, w = 0.0;
+        int inside = 0;
+        for (int k = 0; k < n; ++k) {
+            for (int t = 0; t < s_own[k]; ++t) {
+                pe = dadd(pe, s_rec[k][t].x);
+                w = dadd(w, s_rec[k][t].y);
+            }
+            inside += s_own[k];
+        }
+        out[0] = pe;
+        out[1] = w;
+        out[2] = static_cast<double>(inside);
+    }
+}
+
 // The all-pairs records added to the running (potential, virial) in out[0..1]; out[2] = inside pairs so far. One block.
 __global__ void __launch_bounds__(2 * kOrderedThreads) k_sum_pairs(const double2* __restrict__ rec, long long m,
                                                                    double* __restrict__ out, double inside) {
