@@ -513,10 +513,14 @@ int build_stamp(const md_nlist* nl) { return static_cast<int>(nl->builds % 1'000
 // Is the list of a system of ncells cells with per_cell particles each built a cell per warp (build_cells_sparse)? With few
 // cells a block finishes one sooner (N = 2,000, 9.3 a cell: 100 us a whole build against 122). In md_run's graphs, whose
 // rebuilds have no other kernel (FP32FX, us a step, cell per block / per warp): N = 500,000, 6.8 a cell: 162 / 136; 800,000,
-// 9.4 a cell: 230 / 214. cells_build_async's host-path builds go on to a cell per block at 9 (N = 100,000, 9.4 a cell: 184 us
-// a whole build, by warps 190; 7.2 a cell: 188 / 152).
+// 9.4 a cell: 230 / 214. The host path's builds go on to a cell per block at 9 (N = 100,000, 9.4 a cell: 184 us a whole build,
+// by warps 190; 7.2 a cell: 188 / 152).
 constexpr int kWideBuildCells = 148 * 14;
 bool sparse_cells(double ncells, double per_cell) { return per_cell < (ncells < kWideBuildCells ? 6.0 : 10.5); }
+
+// Particles in the fullest cells and those around them, about; from kFullCell on a cell fills the lanes of a block's warps
+double full_cells(const md_nlist* nl) { return static_cast<double>(nl->cell_most) / kCellItems; }
+constexpr double kFullCell = 18.0;
 
 // Parameters of the cell build (md_build.cuh) for a list of radius^2 g.rl2 and cells of per_cell particles on average, for
 // blocks of `warps` warps with `homes` particles each and room for at least `room` candidates. Returns the dynamic shared
@@ -556,21 +560,39 @@ size_t sparse_build_params(CellBuild& bp, double ncells, double per_cell, int mo
     return 0;
 }
 
-// The list build kernel for the cells, frames and positions of this build, on the system's stream. They write the same rows.
-// Times are whole builds (B200, us; uniform systems of r_l = 2.8 unless said otherwise).
-//   - thin gases (under 3 particles a cell, no full cell): a thread per particle; a block or warp per cell spends itself on
-//     near-empty cells: N = 100,000, density 0.03: tile 306, cells 652, threads 145; 0.1: 217, 329, 170; N = 864,000,
-//     density 0.1: 830, 2,158, 513. Below 50,000 particles a warp per cell is as good: N = 8,000, density 0.1: 118 against 141.
-//   - tiles: large systems that are neither gas nor liquid, where cells hold too few particles to fill a warp (N = 864,000,
-//     density 0.3 / 0.5 / 0.6: tile 600 / 688 / 711, cells 905 / 782 / 748) or few of them hold all (a slab in a third of
-//     the box: 895 against 938 by warps and blocks); at density 0.8442: 727 against 680. And cells of 100 and more, whose
-//     candidates leave room for a block or two on an SM (N = 100,000, r_l = 5.5: 930 against 1,003).
-//   - a warp per cell (sparse_cells), and blocks for the cells that are too full for it: N = 100,000, density 0.3: cells 188,
-//     tile 174, warps 152; a slab of 32,000: tile 144, warps 148; a droplet of 8,000: 146, 142.
-//   - a block per cell: blocks of 4 warps, 4 particles a warp at a time, spend the fewest instructions (N = 864,000: 514 us;
-//     2 particles: 551; blocks of 2 warps: 720). With few cells, 8 warps and 2 particles finish a cell soonest (N = 2,048: 90
-//     us against 102), and with cells of 50 and more they bring twice the warps onto an SM (N = 864,000, r_l = 4: 1,397
-//     against 1,855).
+// Which list build kernel suits the cells of a system (all write the same rows). `full` is about how many particles the fullest
+// cells hold. Times are whole builds (B200, us; uniform systems of r_l = 2.8 unless said otherwise).
+//   - threads: thin gases (under 3 particles a cell, no full cell); a block or warp per cell spends itself on near-empty cells:
+//     N = 100,000, density 0.03: tile 306, cells 652, threads 145; 0.1: 217, 329, 170; N = 864,000, density 0.1: 830, 2,158,
+//     513. Below 50,000 particles a warp per cell is as good: N = 8,000, density 0.1: 118 against 141.
+//   - tiles: cells of 100 and more, whose candidates leave room for a block or two on an SM, but in small systems (r_l = 5.8:
+//     liquid of 100,000 993 against 1,201 by 8-warp blocks, of 20,000 403 / 343; droplet of 300,000 in a tenth of the box 2,100
+//     / 2,664, of 20,000 627 / 499). And large systems that are neither gas nor liquid, where cells hold too few particles to
+//     fill a warp (N = 864,000, density 0.3 / 0.5: 600 / 688 against 905 / 782 by cells; 0.65: 721 / 699).
+//   - blocks of 8 warps: 2 particles a warp at a time; with cells of 35 and more they bring twice the warps onto an SM
+//     (864,000, r_l = 3.3 / 3.5 / 4: 1,065 / 1,105 / 1,397 against 1,116 / 1,299 / 1,855 with 4 warps; slab of 300,000 in a third
+//     of the box, r_l = 4.3: 719 / 954, tile 783), and with few cells they finish one soonest (N = 2,048: 90 against 102).
+//   - blocks of 4 warps: 4 particles a warp at a time spend the fewest instructions (N = 864,000: 514 us alone; 2 particles: 551;
+//     blocks of 2 warps: 720). Where full cells are few, blocks pass the empty ones sooner than warps do and leave none to a
+//     second kernel (slab of 100,000: 189, warps 219, tile 212; droplet of 100,000: 195 / 324 / 236; of 300,000: 416 / 743 / 430).
+//   - warps: sparse systems (sparse_cells) without full cells, and with few of them in a box that is nearly empty (droplet of
+//     100,000 in a hundredth of the box, r_l = 4.3: 668, 4-warp blocks 872, tile 774); 100,000 at density 0.3: 149, tile 182.
+enum class BuildKind { threads, tiles, warps, blocks4, blocks8 };
+BuildKind build_kind(const md_nlist* nl, int n) {
+    const int ncells = nl->grid.ncells;
+    const double per_cell = static_cast<double>(n) / ncells, full = full_cells(nl);
+    const bool gas = nl->cell_most <= kMostWarpStage;  // no cell that a warp could not build
+    const BuildKind blocks = ncells < kWideBuildCells ? BuildKind::blocks8 : BuildKind::blocks4;
+    if (gas && per_cell < 3.0 && n >= 50'000) return BuildKind::threads;
+    if (full >= 100.0 && n >= 30'000) return BuildKind::tiles;
+    if (per_cell >= 1.0 && full >= kFullCell) return full >= 40.0 ? BuildKind::blocks8 : blocks;
+    if (n >= 200'000 && per_cell < 15.0 && !(gas && per_cell < 4.0)) return BuildKind::tiles;
+    if (per_cell < 9.0 && sparse_cells(ncells, per_cell))
+        return gas || per_cell < 1.0 ? BuildKind::warps : BuildKind::tiles;
+    return blocks;
+}
+
+// The list build kernel for the cells, frames and positions of this build, on the system's stream
 md_status cells_build_async(md_nlist* nl, md_system* s) {
     const CellGrid& g = nl->grid;
     const ListGeom geo{s->box, nl->rl2, g.ncps, 1, nl->cap, static_cast<uint32_t>(s->n) | (kSentinelCode << kCodeShift)};
@@ -586,14 +608,14 @@ md_status cells_build_async(md_nlist* nl, md_system* s) {
         return MD_OK;
     };
     const int n = static_cast<int>(s->n);
-    const bool gas = nl->cell_most <= kMostWarpStage;  // no cell that a warp could not build
-    if (gas && per_cell < 3.0 && n >= 50'000) {
+    const BuildKind kind = build_kind(nl, n);
+    if (kind == BuildKind::threads) {
         k_nlist_build<<<blocks_for(n, 128), 128, 0, s->stream>>>(s->pos.p, n, geo, nl->cell_sorted.p, g.start.p, nl->rows.p,
                                                                   nl->counts.p, nl->flags.p + 1);
         MD_CHECK_LAUNCH();
         return MD_OK;
     }
-    if (nl->use_tiles && (per_cell >= 100.0 || (n >= 200'000 && per_cell < 15.0 && !(gas && per_cell < 4.0)))) {
+    if (kind == BuildKind::tiles) {
         cell_build_params(bp, geo, per_cell, 0, 4, 4);
         const TileBuild tb{geo, bp.rl2 - bp.margin, bp.rl2 + bp.margin, build_stamp(nl)};
         const size_t smem = sizeof(float4) * nl->tiles_geom.max_staged;
@@ -604,7 +626,7 @@ md_status cells_build_async(md_nlist* nl, md_system* s) {
         MD_CHECK_LAUNCH();
         return MD_OK;
     }
-    if (per_cell < 9.0 && sparse_cells(g.ncells, per_cell)) {
+    if (kind == BuildKind::warps) {
         cell_build_params(bp, geo, per_cell, 0, kSparseWarps, kSparseHomes);
         const size_t smem = sparse_build_params(bp, g.ncells, per_cell, nl->cell_most);
         if (bp.warp_stage) {
@@ -618,7 +640,7 @@ md_status cells_build_async(md_nlist* nl, md_system* s) {
             return go(k_nlist_build_cells<4, 4, 16, true>, 4, 4, std::min(g.ncells, 148 * 8));
         }
     }
-    if (g.ncells < kWideBuildCells || per_cell >= 50.0) return go(k_nlist_build_cells<8, 2, 16, false>, 8, 2, g.ncells);
+    if (kind == BuildKind::blocks8) return go(k_nlist_build_cells<8, 2, 16, false>, 8, 2, g.ncells);
     return cell_round(per_cell) == 24 ? go(k_nlist_build_cells<4, 4, 24, false>, 4, 4, g.ncells)
                                       : go(k_nlist_build_cells<4, 4, 16, false>, 4, 4, g.ncells);
 }

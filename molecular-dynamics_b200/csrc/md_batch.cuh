@@ -508,6 +508,8 @@ __global__ void __launch_bounds__(32 * kWarps)
         bp.geom.use_cells = d.use_cells;
         const int* st = start + d.cell_off + r;
         const int part = item - stale_items[w];
+        // an empty cell (the same for the whole block); replicas whose cells are hardly ever empty don't wait for the look
+        if (d.use_cells == 1 && d.n < 8 * d.ncells && st[part] == st[part + 1]) continue;
         if (d.use_cells == 1) {
             build_cell<kWarps, kHomes, kRound>(t, sm_cell, frames, pos, st, part, static_cast<float>(d.cell), bp, rows, counts,
                                                max_count);

@@ -152,10 +152,27 @@ void b_drop_graphs(md_batch* b) {
     b->graphs.clear();
 }
 
-// Replicas with fewer particles a cell than this have their rows built by a thread per particle: a block a
-// cell spends itself on empty cells (64 gases of 2,048 at density 0.005, 0.12 a cell, us a step: 265 by cells, 87; 128 of 500
-// at 0.05, 1.5 a cell: 51 by cells)
-constexpr double kThinReplica = 0.5;
+// Replicas with fewer particles a cell than this, and not many more around a particle (a droplet's cells are full), have their
+// rows built by a thread per particle: a block per cell spends itself on near-empty cells (us a step, FP32FX, by cells /
+// threads: 128 gases of 2,000 at 0.25, 0.7, 1.5, 2.7 and 5.8 a cell 247 / 46, 173 / 49, 122 / 50, 93 / 53, 77 / 66; 4 of them 31
+// / 24, 28 / 24, 26 / 25, 24 / 25, 24 / 28)
+constexpr double kThinReplica = 3.0, kThinCell = 5.0;
+
+// Particles in a particle's cell on average
+double cell_around(const BRep& d, const double* pos4) {
+    std::vector<int> cells(d.n);
+    auto coord = [&](double x) { return std::clamp(static_cast<int>(x * d.inv_cell), 0, d.ncps - 1); };
+    for (int i = 0; i < d.n; ++i)
+        cells[i] = (coord(pos4[4 * static_cast<size_t>(i)]) * d.ncps + coord(pos4[4 * static_cast<size_t>(i) + 1])) * d.ncps +
+                   coord(pos4[4 * static_cast<size_t>(i) + 2]);
+    std::sort(cells.begin(), cells.end());
+    double sum = 0.0;
+    for (size_t a = 0, b; a < cells.size(); a = b) {
+        for (b = a; b < cells.size() && cells[b] == cells[a];) ++b;
+        sum += static_cast<double>(b - a) * static_cast<double>(b - a);
+    }
+    return sum / d.n;
+}
 
 // The list build's parameters with room for `room` candidates, as far as the shared memory goes; returns its size
 size_t b_build_params(const md_batch* b, int room, CellBuild& bp) {
@@ -682,6 +699,7 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
     std::vector<int> tile_rep(b->tiles), chunk_rep;
     int off = 0, cell_off = 0, chunk_off = 0;
     double celled = 0.0, cells_used = 0.0;
+    int64_t atoms_before = 0;
     for (int r = 0; r < replicas; ++r) {
         BRep& d = b->reps_h[r];
         const int n = static_cast<int>(n_atoms[r]);
@@ -705,7 +723,7 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
             b->per_cell = std::max(b->per_cell, per_cell);
             celled += d.n;
             cells_used += d.ncells;
-            if (per_cell < kThinReplica) d.use_cells = 2;
+            if (per_cell < kThinReplica && cell_around(d, pos4 + 4 * atoms_before) < kThinCell) d.use_cells = 2;
         }
         b->build_items += md::build_items(d);
         b->most_n = std::max(b->most_n, d.n);
@@ -714,6 +732,7 @@ md_status md_batch_create(int device, int replicas, const int64_t* n_atoms, cons
         const int nch = (n + kChunk - 1) / kChunk;
         for (int c = 0; c < nch; ++c) chunk_rep.push_back(r);
         off += d.np;
+        atoms_before += n;
         cell_off += d.ncells;
         chunk_off += nch;
     }

@@ -22,7 +22,8 @@
 namespace md {
 
 constexpr int kRebuildThreads = 128;
-constexpr unsigned kBarrierPolls = 1u << 20;  // 0.23 s (N = 4,000, B200), for a wait whose partners are resident and at most some ms behind
+// 0.23 s (N = 4,000, B200), for a wait whose partners are resident and at most some ms behind
+constexpr unsigned kBarrierPolls = 1u << 20;
 constexpr int kDirectScan = 16384;            // cells up to which a block adds up the counts before its own
 
 struct RebuildArgs {
@@ -224,19 +225,21 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_step_start(const __grid_
     int cells = a.ncells;
     if constexpr (kSparse) {  // a cell per warp, and then the cells too full for one by blocks (build_cells_sparse)
         const int per = kSparseWarps * a.build.group;
-        const int mine = static_cast<int>(blockIdx.x) * per + static_cast<int>(threadIdx.x >> 5) * a.build.group;
-        for (int c = mine; c < a.ncells; c += static_cast<int>(gridDim.x) * per)
-            build_cells_sparse(sm_step, a.frames, a.ref_pos, a.start, a.ncells, c, static_cast<float>(a.cell), a.build, a.rows,
-                               a.counts, a.max_count, [&](int cell) { a.list[atomicAdd(a.listed, 1)] = cell; });
+        const int first_cell = static_cast<int>(threadIdx.x >> 5) * a.build.group;
+        block_turns((a.ncells + per - 1) / per, [&](int k) {
+            build_cells_sparse(sm_step, a.frames, a.ref_pos, a.start, a.ncells, k * per + first_cell, static_cast<float>(a.cell),
+                               a.build, a.rows, a.counts, a.max_count,
+                               [&](int cell) { a.list[atomicAdd(a.listed, 1)] = cell; });
+        });
         if (!grid_barrier(a)) return;
         cells = *static_cast<volatile int*>(a.listed);
     }
-    for (int k = blockIdx.x; k < cells; k += static_cast<int>(gridDim.x)) {
+    block_turns(cells, [&](int k) {
         build_cell<kRebuildThreads / 32, kHomes, kRound>(sh.items, sm_step, a.frames, a.ref_pos, a.start,
                                                          kSparse ? a.list[k] : k, static_cast<float>(a.cell), a.build, a.rows,
                                                          a.counts, a.max_count);
         __syncthreads();
-    }
+    });
     if (a.near_rows) {
         if (!grid_barrier(a)) return;
         if (threadIdx.x < 32) sh.s_off[threadIdx.x] = a.offs.off[threadIdx.x];

@@ -65,9 +65,22 @@ md_status record_energy(md_forcefield* ff, md_system* s, double* rec, bool want_
 // 1,587 / 1,507. FP32FX: 864,000: 283 / 301; 2,048,000: 637 / 622. FP64, whose ordered sums overlap the next steps better
 // on their own streams: 32,000: 48 / 79; 256,000: 192 / 218; 500,000: 374 / 356; 864,000: 572 / 560.
 constexpr int64_t kFloatGraphMaxParticles = 1'200'000, kFp64GraphMaxParticles = 400'000;
+// Fuller cells than that liquid's (28 and more: longer cutoffs, denser systems) cost such a rebuild more than their share (us a
+// step, graph / host loop): liquid, r_l = 3.2: FX32 of 380,000 308 / 327, of 800,000 611 / 573; FP64 of 380,000 474 / 441;
+// r_l = 4.3: FP32FX of 100,000 121 / 139, FX32 of 200,000 278 / 270, FP32FX slab of 300,000 in a third of the box 348 / 279;
+// FP64 of 50,000 196 / 180. But not in a nearly empty box, whose cells the host path is slow at too: droplet of 300,000 in a
+// hundredth of the box, r_l = 4.3: FP32FX 309 / 369, FP64 660 / 646.
+int64_t graph_max_particles(const md_nlist* nl, const md_system* s, bool fp64) {
+    const double full = full_cells(nl), per_cell = static_cast<double>(s->n) / nl->grid.ncells;
+    double most = static_cast<double>(fp64 ? kFp64GraphMaxParticles : kFloatGraphMaxParticles);
+    if (full > 28.0 && per_cell >= 1.0) most *= std::pow(28.0 / full, fp64 ? 1.5 : 2.0);
+    return static_cast<int64_t>(most);
+}
 
+// Does the step kernel build the list a cell per warp? (not where full cells are many: the host path's builds go by blocks there)
 bool sparse_build(const md_nlist* nl, const md_system* s) {
-    return sparse_cells(nl->grid.ncells, static_cast<double>(s->n) / nl->grid.ncells);
+    const double per_cell = static_cast<double>(s->n) / nl->grid.ncells;
+    return sparse_cells(nl->grid.ncells, per_cell) && !(per_cell >= 3.0 && full_cells(nl) >= kFullCell);
 }
 
 // Parameters and shared memory of the step kernel's list build
@@ -89,11 +102,11 @@ constexpr size_t kStepSmem = 110 * 1024;
 // Can md_run use graphs for this call? (a tiled list built for this system; the tiled build is the one the device
 // rebuild enqueues)
 bool graph_mode_ok(const md_system* s, const md_forcefield* ff, const md_nlist* nl, int64_t n_steps) {
-    const bool precision = (float_precision(ff->precision) && s->n <= kFloatGraphMaxParticles) ||
-                           (ff->precision == MD_PREC_FP64 && s->n <= kFp64GraphMaxParticles);
+    const bool fp64 = ff->precision == MD_PREC_FP64;
     CellBuild build;
-    return s->graph_chunk > 0 && n_steps > 0 && s->n > 0 && precision && nlist_current(nl, s) && nl->use_cells &&
-           nl->use_tiles && nl->build_pin != 0 && step_smem(nl, s, &build) <= kStepSmem;
+    return s->graph_chunk > 0 && n_steps > 0 && s->n > 0 && (fp64 || float_precision(ff->precision)) &&
+           nlist_current(nl, s) && nl->use_cells && nl->use_tiles && nl->build_pin != 0 &&
+           s->n <= graph_max_particles(nl, s, fp64) && step_smem(nl, s, &build) <= kStepSmem;
 }
 
 // Live data of a double-buffered array into its canonical buffer (recorded by the graphs); count elements
