@@ -263,8 +263,8 @@ struct md_nlist {
     int cell_most = 0;      // most candidates of a cell (27 cells and itself), an eighth more or up to twice as many
     bool use_tiles = false; // shared-memory tile kernels (3+ cells per side and tiles that fit)
     TileGeom tiles_geom{};
-    int build_kernel = -1;  // list build of the last rebuild: 0 thread per particle, 1 tiles
-    int build_pin = -1;     // set by md_nlist_set_build_variant (-1: tiles where available)
+    int build_kernel = -1;  // list build of the last rebuild: 0 pinned or no tiles (a thread per particle), 1 chosen (build_kind)
+    int build_pin = -1;     // set by md_nlist_set_build_variant (0: a thread per particle)
     int variant[5] = {-1, -1, -1, -1, -1};  // force kernel per precision (0 global gathers, 1 tile; -1 untuned)
     int pinned[5] = {-1, -1, -1, -1, -1};   // set by md_nlist_set_force_variant
     uint64_t builds = 0;                    // list builds so far (names the rows of the last one)
@@ -572,8 +572,8 @@ size_t sparse_build_params(CellBuild& bp, double ncells, double per_cell, int mo
 //   - blocks of 8 warps: 2 particles a warp at a time; with cells of 35 and more they bring twice the warps onto an SM
 //     (864,000, r_l = 3.3 / 3.5 / 4: 1,065 / 1,105 / 1,397 against 1,116 / 1,299 / 1,855 with 4 warps; slab of 300,000 in a third
 //     of the box, r_l = 4.3: 719 / 954, tile 783), and with few cells they finish one soonest (N = 2,048: 90 against 102).
-//   - blocks of 4 warps: 4 particles a warp at a time spend the fewest instructions (N = 864,000: 514 us alone; 2 particles: 551;
-//     blocks of 2 warps: 720). Where full cells are few, blocks pass the empty ones sooner than warps do and leave none to a
+//   - blocks of 4 warps: 4 particles a warp at a time spend the fewest instructions (N = 864,000, 2 particles 7 % more time,
+//     blocks of 2 warps 40 %). Where full cells are few, blocks pass the empty ones sooner than warps do and leave none to a
 //     second kernel (slab of 100,000: 189, warps 219, tile 212; droplet of 100,000: 195 / 324 / 236; of 300,000: 416 / 743 / 430).
 //   - warps: sparse systems (sparse_cells) without full cells, and with few of them in a box that is nearly empty (droplet of
 //     100,000 in a hundredth of the box, r_l = 4.3: 668, 4-warp blocks 872, tile 774); 100,000 at density 0.3: 149, tile 182.

@@ -162,12 +162,13 @@ md_status forces_list_fx64_async(md_forcefield* ff, md_system* s, md_nlist* nl, 
             }
         } else {
             MD_TRY(profile_mark(s));
+            const unsigned gs = blocks_for(static_cast<long long>(n) * kSmallLanes, 128);
             if (want_energy)
-                k_force_fx64_small<true><<<blocks_for(static_cast<long long>(n) * kSmallLanes, 128), 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p, nl->cap,
-                                                                   nl->counts.p, s->force.p, acc, ka);
-            else
-                k_force_fx64_small<false><<<blocks_for(static_cast<long long>(n) * kSmallLanes, 128), 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p, nl->cap,
+                k_force_fx64_small<true><<<gs, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p, nl->cap,
                                                                     nl->counts.p, s->force.p, acc, ka);
+            else
+                k_force_fx64_small<false><<<gs, 128, 0, s->stream>>>(s->pos.p, n, s->box, lj, nl->rows.p, nl->cap,
+                                                                     nl->counts.p, s->force.p, acc, ka);
         }
         MD_CHECK_LAUNCH();
         MD_TRY(profile_mark(s));

@@ -121,8 +121,8 @@ md_status adj_build(md_adjoint* a, const double4* p) {
 }
 
 md_status adj_forces(md_adjoint* a) {
-    k_adj_forces<<<blocks_for(static_cast<long long>(a->n) * kAdjForceLanes, 128), 128, 0, a->stream>>>(a->pos.p, a->n, a->c, a->rows.p, a->cap, a->counts.p,
-                                                               a->force.p, a->u.p, a->w.p);
+    k_adj_forces<<<blocks_for(static_cast<long long>(a->n) * kAdjForceLanes, 128), 128, 0, a->stream>>>(
+        a->pos.p, a->n, a->c, a->rows.p, a->cap, a->counts.p, a->force.p, a->u.p, a->w.p);
     MD_CHECK_LAUNCH();
     return MD_OK;
 }

@@ -20,10 +20,10 @@
 // its candidates (list_frame_of marks them: such a particle lies outside its cell, and with 3 cells a side the frames may
 // then name another image than the nearest), or more candidates than the shared memory holds, goes through build_row.
 //
-// What bounds it: instruction issue (65 % of the slots; about 480 warp instructions a particle: a third in laying out the
-// candidates, a seventh in the tests, the rest in the rows). A thread per particle walking its candidates one by one took
-// 630 and scattered 4-byte stores, and left small systems to a few long chains. Measured (B200, kernel alone): N = 864,000:
-// 0.60 ms, now 0.51; 2,048: 36 us, now 15.
+// What bounds it: instruction issue (71 % of the slots; 482 warp instructions a particle: a third in laying out the candidates,
+// a seventh in the tests, the rest in the rows). A thread per particle walking its candidates one by one (k_nlist_build_tile)
+// takes 630 and scattered 4-byte stores, and leaves small systems to a few long chains. Measured (B200, kernel alone, liquid,
+// tiles / cells): N = 4,000,000: 2.59 / 2.28 ms; 864,000: 0.60 / 0.53; 2,048: 36 / 15 us.
 #pragma once
 
 #include "md_common.cuh"
@@ -162,8 +162,8 @@ __device__ __noinline__ void cell_masks_exact(const float4* cand, const uint32_t
 
 // Mask words (32 candidates each) that build_cell's rows are written from at a time, for cells of per_cell particles on
 // average: 16 hold the candidates of a liquid's list of r_l = 2.8; where about that many take a second round nearly
-// empty, 24 (4 homes a warp, kernel alone, 16 / 24: N = 500,000, density 0.85, r_l = 3.2, 20 words: 438 / 406 us;
-// N = 864,000, density 0.8442, r_l = 2.8, 15 words: 545 / 560).
+// empty, 24 (4 homes a warp, kernel alone with the same code otherwise, 16 / 24: N = 500,000, density 0.85, r_l = 3.2, 20
+// words: 438 / 406 us; N = 864,000, density 0.8442, r_l = 2.8, 15 words: 545 / 560).
 inline int cell_round(double per_cell) {
     const double words = 0.8 * kCellItems * per_cell / 32.0;
     return words > 18.0 && words <= 24.0 ? 24 : 16;
@@ -229,11 +229,12 @@ struct CellOrder {
     int home0, home1, own_end;
 };
 
-// Adds the accepted candidates of `words` words to the rows of a group of homes (one warp): kLanes lanes per home particle, kWords adjacent mask words a lane, kRound words at a time. h: this lane's home
-// particle in the cell (real: there is one), mine: its row in shared memory, len and own: its entries so far.
+// Adds the accepted candidates of `words` words to the rows of a group of homes (one warp): kLanes lanes per home particle,
+// kWords adjacent mask words a lane, kRound words at a time. h: this lane's home particle in the cell (real: there is one),
+// mine: its row in shared memory, len and own: its entries so far.
 template <int kHomes, int kRound>
-__device__ __forceinline__ void cell_append(const uint32_t* entries, const uint32_t* masks, int words, const CellOrder& order, int h, bool real, int cap, uint32_t* mine, int& len,
-                                            int& own) {
+__device__ __forceinline__ void cell_append(const uint32_t* entries, const uint32_t* masks, int words, const CellOrder& order,
+                                            int h, bool real, int cap, uint32_t* mine, int& len, int& own) {
     constexpr unsigned kAll = 0xffffffffu;
     constexpr int kLanes = 32 / kHomes, kWords = kRound / kLanes;
     const int lane = threadIdx.x & 31, k = lane / kLanes, l = lane % kLanes;

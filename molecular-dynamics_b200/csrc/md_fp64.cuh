@@ -12,16 +12,6 @@ constexpr int kChainValues = 8;  // values per thread of a one-block ordered sum
 
 // ---- forces -----------------------------------------------------------------------------------------
 
-// computeForcesDeterministic's per-particle sum (src/Forcefield.cpp:264-320): particle i adds F(i, j) over
-// its own pairs in list order, then subtracts F(j, i) over the pairs where it is second, in increasing pair
-// index. Pairs outside the cutoff contribute an exact zero in the reference and are skipped here. The
-// inside-cutoff count is the number of own pairs with r^2 < r_c^2 (a sum of whole numbers, exact).
-// With kick_vel set it also applies the closing half kick, v += (half_dt F) / m, with k_kick's sequence.
-// With pair_r2 set, own pair s of particle i also stores its r^2, inside the cutoff or not, for the ordered energy sums
-// at index half_off[i] + s; k_pair_block_sums recomputes the pair's E and (F/r) r^2 from it with the same pair_terms
-// call (the same operations on the same r^2, so the same bits). Records past rec_cap, the buffer's size in records, are
-// dropped: only a list rebuilt inside a CUDA graph can outgrow the buffer, and the graph's run then reports the overflow
-// and repeats its steps on the host path.
 // A block's inside-cutoff pairs into *inside by one atomic (every thread calls)
 __device__ __forceinline__ void count_inside(unsigned ins, unsigned long long* __restrict__ inside) {
     __shared__ unsigned s_ins[32];
@@ -35,6 +25,16 @@ __device__ __forceinline__ void count_inside(unsigned ins, unsigned long long* _
     }
 }
 
+// computeForcesDeterministic's per-particle sum (src/Forcefield.cpp:264-320): particle i adds F(i, j) over
+// its own pairs in list order, then subtracts F(j, i) over the pairs where it is second, in increasing pair
+// index. Pairs outside the cutoff contribute an exact zero in the reference and are skipped here. The
+// inside-cutoff count is the number of own pairs with r^2 < r_c^2 (a sum of whole numbers, exact).
+// With kick_vel set it also applies the closing half kick, v += (half_dt F) / m, with k_kick's sequence.
+// With pair_r2 set, own pair s of particle i also stores its r^2, inside the cutoff or not, for the ordered energy sums
+// at index half_off[i] + s; k_pair_block_sums recomputes the pair's E and (F/r) r^2 from it with the same pair_terms
+// call (the same operations on the same r^2, so the same bits). Records past rec_cap, the buffer's size in records, are
+// dropped: only a list rebuilt inside a CUDA graph can outgrow the buffer, and the graph's run then reports the overflow
+// and repeats its steps on the host path.
 __global__ void k_force_fp64(const double4* __restrict__ pos, int n, Box box, LJ lj, const uint32_t* __restrict__ rows,
                              int cap, const int2* __restrict__ counts, double* __restrict__ force,
                              unsigned long long* __restrict__ inside, double* __restrict__ kick_vel,

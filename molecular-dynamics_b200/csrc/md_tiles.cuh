@@ -179,9 +179,9 @@ __device__ __forceinline__ int staged_cell(int code, int h, int span) {
 // Candidates come from staged float frames; one is accepted when float r^2 < r_l^2 - margin, rejected when float
 // r^2 > r_l^2 + margin, and otherwise decided by the reference's double test on the global positions (a thin shell of
 // candidates). The margin bounds the float error of r^2 for positions inside the box (each coordinate carries under 4e-7
-// absolute error); a tile with a position outside it (list_frame_of; *outside_stamp
-// tells whether this build has one at all) goes through build_row. Row order: own pairs (j > i) in
-// the reference's candidate order, then the j < i that list i, ascending. Bound by instruction issue (about 25 a candidate).
+// absolute error); a tile with a position outside it (list_frame_of; *outside_stamp tells whether this build has one at all)
+// goes through build_row. Row order: own pairs (j > i) in the reference's candidate order, then the j < i that list i,
+// ascending. Bound by instruction issue (about 25 a candidate).
 struct TileBuild {
     ListGeom geom;
     float lo, hi;  // r_l^2 -+ margin
