@@ -85,8 +85,7 @@ def args_parse():
     p.add_argument("--force-variant", type=int, default=-1,
                    help="list force kernel of the headline run: -1 autotunes, 0-4 pin one (md_nlist_set_force_variant)")
     p.add_argument("--graph-chunk", type=int, default=64,
-                   help="md_run's CUDA-graph chunk length (md_system_set_graph); 0 runs every step from the host, as "
-                        "profilers need (ncu cannot profile kernels in graphs with conditional nodes)")
+                   help="md_run's CUDA-graph chunk length (md_system_set_graph); 0 runs every step from the host")
     p.add_argument("--profile-region", action="store_true",
                    help="bracket the timed steps with cudaProfilerStart/Stop (for ncu --profile-from-start off)")
     return p.parse_args()
