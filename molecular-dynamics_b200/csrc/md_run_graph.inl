@@ -162,7 +162,6 @@ md_status graph_prepare_buffers(md_system* s, md_forcefield* ff, md_nlist* nl, c
     MD_CUDA(s->snap_ids.reserve(n));
     MD_CUDA(s->snap_flag.reserve(1));
     MD_CUDA(s->step_barrier.reserve(2));
-    if (sparse_build(nl, s)) MD_CUDA(nl->full_cells.reserve(nl->grid.ncells));
     if (o.rdf) {
         if (o.rdf->device < 0) {
             o.rdf->device = s->device;
@@ -214,7 +213,8 @@ TileGeom graph_geometry(const md_system* s, const md_nlist* nl) {
     return g;
 }
 
-// The step's first kernel (k_step_start). prepare_only: its shared-memory opt-in and resident grid, before a capture
+// The step's first kernel (k_step_start). prepare_only: its shared-memory opt-in, resident grid and list of full cells, before
+// a capture
 md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const StepCapture* last, long long* pair_count,
                            bool prepare_only = false) {
     const int n = static_cast<int>(s->n);
@@ -228,6 +228,8 @@ md_status step_start_async(md_system* s, md_forcefield* ff, md_nlist* nl, const 
     RebuildArgs a{};
     const size_t smem = step_smem(nl, s, &a.build);
     if (prepare_only) {
+        // (here and not once a run: a chunk that ran again on the host path may have changed the kind)
+        if (sparse) MD_CUDA(nl->full_cells.reserve(g.ncells));
         MD_CUDA(allow_smem(kernel, smem));
         if (s->step_resident[which] != 0 && s->step_smem[which] == smem) return MD_OK;
         int sms = 0, per_sm = 0;
