@@ -90,7 +90,12 @@ size_t step_smem(const md_nlist* nl, const md_system* s, CellBuild* bp) {
     const double per_cell = static_cast<double>(s->n) / nl->grid.ncells;
     size_t smem = cell_build_params(*bp, geo, per_cell, build_room(nl->cell_most, per_cell), kRebuildThreads / 32,
                                     few_cells ? 2 : 4);
-    if (sparse_build(nl, s)) smem = std::max(smem, sparse_build_params(*bp, nl->grid.ncells, per_cell, nl->cell_most));
+    if (sparse_build(nl, s)) {
+        smem = std::max(smem, sparse_build_params(*bp, nl->grid.ncells, per_cell, nl->cell_most));
+        // full cells lie together: short runs spread them over the warps (droplet of 300,000, FP32FX, us a step with up to 32 /
+        // 8 / 4 cells a warp: 152 / 133 / 123; in a hundredth of the box 159 / 131 / 129; thin slab of 100,000: 53 / 56 / 57)
+        if (nl->cell_most > kMostWarpStage) bp->group = std::min(bp->group, 4);
+    }
     return std::max(smem, kSplitSmem);
 }
 
